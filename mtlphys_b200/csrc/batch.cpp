@@ -472,7 +472,7 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         const uint32_t cap = round_up(std::max<uint32_t>(b->N, 1u), 256u);
         const size_t v4 = size_t(cap) * 16, u = size_t(cap) * 4;
         const size_t longs = (size_t(cap) / kSegMax + 2) * 4;
-        const size_t ptotal = 5 * v4 + 19 * u + longs + 32 * 256;
+        const size_t ptotal = 5 * v4 + 20 * u + longs + 32 * 256;
         MP_ALLOC(b->particle_block, ptotal, b->device);
         MP_CUDA(cudaMemset(b->particle_block, 0, ptotal));
         char* pb = static_cast<char*>(b->particle_block);
@@ -491,6 +491,7 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         a.off = reinterpret_cast<uint32_t*>(take(u));
         a.tmp = reinterpret_cast<uint32_t*>(take(u));
         a.sidx = reinterpret_cast<uint32_t*>(take(u));
+        a.qpos = reinterpret_cast<uint32_t*>(take(u));
         a.scell = reinterpret_cast<uint32_t*>(take(u));
         a.ncount = reinterpret_cast<uint32_t*>(take(u));
         a.lambdas = reinterpret_cast<float*>(take(u));

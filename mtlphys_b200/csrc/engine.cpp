@@ -11,6 +11,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -325,6 +326,44 @@ size_t elem_bytes(uint32_t which) {
     }
 }
 
+// The lambda passes' prefilter (quantize() in pbf_device.cuh) for parameters
+// p: positions in steps u = cell_size / units, differences modulo 256 steps.
+//   - A pair within h differs by at most h / u steps on an axis.  Flooring
+//     both positions (the query's y and z rounded instead) and the borrow of
+//     the byte below shift a byte's difference by less than 1 step on x and 1.5
+//     on y and z, together sqrt(1 + 1.5^2 + 1.5^2) < 2.3453 steps, plus
+//     `fuzz` per axis for FP32 rounding of coordinates and offsets.  q_thr is
+//     the square of h / u plus that (plus 1: byte 3 can hold a borrow).
+//   - Bytes hold differences up to 127 steps: units <= (127 - slack) / (h / cs).
+//     Candidates up to 2 cells away must not wrap to within range:
+//     256 - 2 units >= h / u + slack.  (A wrapped candidate only costs an exact
+//     test, so particles that drifted further are no concern.)
+// At cell_size = h: 84 steps a cell, and 9% more candidates pass than are in
+// range.  Coordinates too large for FP32 to resolve a step, or a cell much
+// smaller than h, switch the prefilter off (every candidate passes).
+void set_prefilter(const mp_pbf_params& p, StepConsts& c) {
+    c.q_units = 0;
+    c.q_inv = 0.0f;
+    c.q_thr = 1 << 30;
+    c.q_lim = 0.0f;
+    const double cs = p.cell_size, h = p.h;
+    const double slack = 4.0;
+    const int units = int(std::floor(std::min((127.0 - slack) * cs / h, (256.0 - slack) / (2.0 + h / cs))));
+    if (units < 1) return;
+    const double u = cs / units;
+    const double lim = 32768.0 * u;  // beyond it from its cell, a particle skips the prefilter
+    double most = 2.0 * lim;
+    for (int a = 0; a < 3; ++a)
+        most = std::max(most, std::max(std::fabs(double(p.bounds_min[a])), std::fabs(double(p.bounds_max[a]))) + 2.0 * lim);
+    const double fuzz = 0.02 + 4.0 * most * 0x1p-23 / u;
+    const double r = h / u * (1.0 + 1e-5) + 2.3453 + 1.7321 * fuzz;
+    if (h / u + 1.5 + fuzz > 127.0 || fuzz > 1.0) return;
+    c.q_units = units;
+    c.q_inv = float(double(units) / cs);
+    c.q_thr = int(std::floor(r * r)) + 2;
+    c.q_lim = float(lim);
+}
+
 // writePBFParams (Engine.cpp:551-572) and the shader literals, in FP32 like
 // the reference, for a scene of n particles on grid g stepped by dt.
 StepConsts make_consts(const mp_pbf_params& p, const GridDev& g, uint32_t n, float dt, bool sphere) {
@@ -373,6 +412,7 @@ StepConsts make_consts(const mp_pbf_params& p, const GridDev& g, uint32_t n, flo
     c.sph_gravity = p.sphere_gravity;
     c.sph_drag = p.sphere_drag;
     c.sph_rest = p.sphere_restitution;
+    set_prefilter(p, c);
     return c;
 }
 
@@ -514,7 +554,7 @@ struct mp_engine {
         particle_block = nullptr;
         list_block = nullptr;
         d.pos = d.vel = d.prev = d.sorted_a = d.sorted_b = nullptr;
-        d.hash = d.off = d.tmp = d.sidx = d.scell = d.ncount = d.long_list = nullptr;
+        d.hash = d.off = d.tmp = d.sidx = d.qpos = d.scell = d.ncount = d.long_list = nullptr;
         d.lambdas = d.foam = nullptr;
         d.row_masks = nullptr;
         d.mask_overflow = nullptr;
@@ -545,7 +585,7 @@ struct mp_engine {
         free_particles();
         const size_t v4 = size_t(cap) * 16, u = size_t(cap) * 4;
         const size_t longs = (size_t(cap) / mpb::kSegMax + 2) * 4;
-        const size_t total = 5 * v4 + 8 * u + longs + 16 * 256;
+        const size_t total = 5 * v4 + 9 * u + longs + 16 * 256;
         MP_ALLOC(particle_block, total, device);
         char* b = static_cast<char*>(particle_block);
         auto take = [&](size_t bytes) {
@@ -562,6 +602,7 @@ struct mp_engine {
         d.off = reinterpret_cast<uint32_t*>(take(u));
         d.tmp = reinterpret_cast<uint32_t*>(take(u));
         d.sidx = reinterpret_cast<uint32_t*>(take(u));
+        d.qpos = reinterpret_cast<uint32_t*>(take(u));
         d.scell = reinterpret_cast<uint32_t*>(take(u));
         d.ncount = reinterpret_cast<uint32_t*>(take(u));
         d.lambdas = reinterpret_cast<float*>(take(u));

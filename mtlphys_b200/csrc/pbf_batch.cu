@@ -288,16 +288,16 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     if (!grid_barrier(a, &s_ok)) return;
     if (cells_ok)
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
-            sort_gather_item(s, a.tmp, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a, a.long_list,
-                             a.long_count);
+            sort_gather_item(sc[a.scene_of[s]].c, s, a.tmp, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
+                             a.qpos, a.long_list, a.long_count);
     if (!grid_barrier(a, &s_ok)) return;
     {
         const uint32_t nl = cells_ok ? *a.long_count : 0u;
         for (uint32_t li = blockIdx.x; li < nl; li += gridDim.x) {
             const uint32_t cell = a.long_list[li];
             const SceneDev& sd = sc[a.scene_of[a.tmp[a.cstart[cell]]]];
-            long_segment(cell, sd.p0, sd.p0 + sd.c.n, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
-                         s_warp);
+            long_segment(sd.c, cell, sd.p0, sd.p0 + sd.c.n, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
+                         a.qpos, s_warp);
         }
     }
     if (!grid_barrier(a, &s_ok)) return;
@@ -329,25 +329,25 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             const StepConsts& c = sc[a.scene_of[s]].c;
             if (it == 0) {
                 if (last)
-                    lambda_first_item<true>(c, s, a.sorted_a, lam_out, a.scell, a.cstart, a.sidx,
+                    lambda_first_item<true>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
                                             a.lambdas, a.ncount, rmi);
                 else
-                    lambda_first_item<false>(c, s, a.sorted_a, lam_out, a.scell, a.cstart, a.sidx,
+                    lambda_first_item<false>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
                                              a.lambdas, a.ncount, rmi);
             } else if (last) {
-                lambda_item<true>(c, s, a.sorted_a, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi);
+                lambda_item<true>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi);
             } else {
-                lambda_item<false>(c, s, a.sorted_a, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi);
+                lambda_item<false>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi);
             }
         }
         if (!grid_barrier(a, &s_ok)) return;
         for (uint32_t s = pb + gtid; s < pe; s += gsize) {
             const SceneDev& sd = sc[a.scene_of[s]];
             if (last)
-                delta_item<true, SN>(sd.c, s, lam_out, a.sorted_a, a.scell, a.cstart, a.sidx, &sd.sphere,
+                delta_item<true, SN>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.scell, a.cstart, a.sidx, &sd.sphere,
                                  a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec);
             else
-                delta_item<false, SN>(sd.c, s, lam_out, a.sorted_a, a.scell, a.cstart, a.sidx, &sd.sphere,
+                delta_item<false, SN>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.scell, a.cstart, a.sidx, &sd.sphere,
                                   a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec);
         }
         if (!last && !grid_barrier(a, &s_ok)) return;

@@ -39,7 +39,7 @@ struct BatchArgs {
     uint32_t p_begin, p_end;          // particles (= slots) of this launch
     uint32_t iterations;
     float4 *pos, *vel, *prev, *sorted_a, *sorted_b;
-    uint32_t *hash, *off, *tmp, *sidx, *scell, *ncount;
+    uint32_t *hash, *off, *tmp, *sidx, *scell, *ncount, *qpos;
     float *lambdas, *foam;
     uint32_t *counts, *cstart, *tile_sums;
     uint32_t max_cells;               // capacity of counts / cstart minus one

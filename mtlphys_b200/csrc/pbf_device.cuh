@@ -53,6 +53,11 @@ struct StepConsts {
     float foam_maxn, foam_lo, foam_hi;
     int sphere;  // 1: sphere-drop scene (sphere state lives in device memory)
     float sph_gravity, sph_drag, sph_rest;
+    // byte-quantized distance prefilter of the lambda passes (set_prefilter):
+    int q_units;   // quantization steps per cell
+    float q_inv;   // q_units / cellSize
+    int q_thr;     // largest quantized squared distance an in-range pair can have
+    float q_lim;   // particles further than this from their cell's corner skip the prefilter
 };
 
 // Device-resident sphere state: center xyz, velocity xyz, radius.
@@ -122,6 +127,26 @@ __device__ __forceinline__ float anchor_z(const GridDev& g, int c) {
 // count and the solver so that integer outputs are reproducible.
 __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+}
+
+// ---- quantized positions ------------------------------------------------------
+//
+// A slot's position in steps of cellSize / q_units, each axis modulo 256, x, y
+// and z in bytes 0, 1 and 2 (byte 3 zero).  The byte-wise difference of two of
+// these words, as signed bytes, is the offset between the positions to within
+// a step or so whenever they are within h of each other, so one subtraction
+// and one __dp4a test a candidate; what passes is tested again exactly.
+// (cx, cy, cz): dense coordinates of the slot's hash cell, l the offset from
+// that cell's lower corner.  BIAS: the query's word, rounded instead of
+// floored on y and z, which centres the borrows of a 32-bit subtraction.
+template <bool BIAS>
+__device__ __forceinline__ uint32_t quantize(const StepConsts& c, int cx, int cy, int cz, float lx,
+                                             float ly, float lz) {
+    const float b = BIAS ? 0.5f : 0.0f;
+    const uint32_t x = uint32_t(cx * c.q_units) + uint32_t(__float2int_rd(__fmul_rn(lx, c.q_inv)));
+    const uint32_t y = uint32_t(cy * c.q_units) + uint32_t(__float2int_rd(__fmaf_rn(ly, c.q_inv, b)));
+    const uint32_t z = uint32_t(cz * c.q_units) + uint32_t(__float2int_rd(__fmaf_rn(lz, c.q_inv, b)));
+    return (x & 0xffu) | ((y & 0xffu) << 8) | ((z & 0xffu) << 16);
 }
 
 // ---- SPH helpers ------------------------------------------------------------

@@ -235,24 +235,24 @@ k_scatter(uint32_t n, const uint32_t* __restrict__ hash, const uint32_t* __restr
 }
 
 __global__ void __launch_bounds__(256)
-k_sort_gather(uint32_t n, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ hash,
+k_sort_gather(StepConsts c, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ hash,
               const uint32_t* __restrict__ cstart, const float4* __restrict__ pos,
-              uint32_t* __restrict__ sidx, float4* __restrict__ sorted,
+              uint32_t* __restrict__ sidx, float4* __restrict__ sorted, uint32_t* __restrict__ qpos,
               uint32_t* __restrict__ long_list, uint32_t* __restrict__ long_count) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) sort_gather_item(s, tmp, hash, cstart, pos, sidx, sorted, long_list, long_count);
+    if (s < c.n) sort_gather_item(c, s, tmp, hash, cstart, pos, sidx, sorted, qpos, long_list, long_count);
 }
 
 // One block per queued long segment.
 __global__ void __launch_bounds__(256)
-k_long_segments(uint32_t n, const uint32_t* __restrict__ hash, const uint32_t* __restrict__ cstart,
+k_long_segments(StepConsts c, const uint32_t* __restrict__ hash, const uint32_t* __restrict__ cstart,
                 const float4* __restrict__ pos, uint32_t* __restrict__ sidx,
-                float4* __restrict__ sorted, const uint32_t* __restrict__ long_list,
+                float4* __restrict__ sorted, uint32_t* __restrict__ qpos, const uint32_t* __restrict__ long_list,
                 const uint32_t* __restrict__ long_count) {
     __shared__ uint32_t s_warp[8];
     const uint32_t total = *long_count;
     for (uint32_t li = blockIdx.x; li < total; li += gridDim.x)
-        long_segment(long_list[li], 0u, n, hash, cstart, pos, sidx, sorted, s_warp);
+        long_segment(c, long_list[li], 0u, c.n, hash, cstart, pos, sidx, sorted, qpos, s_warp);
 }
 
 __global__ void __launch_bounds__(256)
@@ -299,12 +299,12 @@ cudaError_t launch_hash_pass(const StepConsts& c, const DevState& d, bool predic
     k_scatter<<<cdiv(n, 256), 256, 0, s>>>(n, d.hash, d.off, d.cstart, d.tmp);
     tend(t, "scatter", s);
     tbegin(t, s);
-    k_sort_gather<<<cdiv(n, 256), 256, 0, s>>>(n, d.tmp, d.hash, d.cstart, d.pos, d.sidx,
-                                                d.sorted_a, d.long_list, d.long_count);
+    k_sort_gather<<<cdiv(n, 256), 256, 0, s>>>(c, d.tmp, d.hash, d.cstart, d.pos, d.sidx,
+                                                d.sorted_a, d.qpos, d.long_list, d.long_count);
     tend(t, "sort_gather", s);
     tbegin(t, s);
-    k_long_segments<<<148, 256, 0, s>>>(n, d.hash, d.cstart, d.pos, d.sidx, d.sorted_a,
-                                        d.long_list, d.long_count);
+    k_long_segments<<<148, 256, 0, s>>>(c, d.hash, d.cstart, d.pos, d.sidx, d.sorted_a,
+                                        d.qpos, d.long_list, d.long_count);
     tend(t, "long_segments", s);
     return cudaGetLastError();
 }

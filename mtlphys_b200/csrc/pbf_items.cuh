@@ -34,6 +34,7 @@
 namespace mpb {
 
 constexpr unsigned kFull = 0xffffffffu;
+constexpr int kPassAll = 1 << 30;  // a prefilter threshold every candidate passes
 
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
@@ -120,15 +121,30 @@ __device__ __forceinline__ void scatter_item(uint32_t i, const uint32_t* __restr
     tmp[cstart[hash[i]] + off[i]] = i;
 }
 
+// A particle's place in sorted order: its index, predicted position and
+// quantized position.
+__device__ __forceinline__ void place(const StepConsts& c, uint32_t d, uint32_t j, const float4& p,
+                                      uint32_t* __restrict__ sidx, float4* __restrict__ sorted,
+                                      uint32_t* __restrict__ qpos) {
+    int cx, cy, cz;
+    cell_of(c.g, p.x, p.y, p.z, cx, cy, cz);
+    sidx[d] = j;
+    sorted[d] = p;
+    qpos[d] = quantize<false>(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, __fsub_rn(p.x, anchor_x(c.g, cx)),
+                              __fsub_rn(p.y, anchor_y(c.g, cy)), __fsub_rn(p.z, anchor_z(c.g, cz)));
+}
+
 // Stable re-rank inside the cell segment + gatherPositions: the slot's
 // particle j moves to cellStart + (number of particles of its cell with a
 // smaller index).  Segments longer than kSegMax are queued instead.
-__device__ __forceinline__ void sort_gather_item(uint32_t s, const uint32_t* __restrict__ tmp,
+__device__ __forceinline__ void sort_gather_item(const StepConsts& sc, uint32_t s,
+                                                 const uint32_t* __restrict__ tmp,
                                                  const uint32_t* __restrict__ hash,
                                                  const uint32_t* __restrict__ cstart,
                                                  const float4* __restrict__ pos,
                                                  uint32_t* __restrict__ sidx,
                                                  float4* __restrict__ sorted,
+                                                 uint32_t* __restrict__ qpos,
                                                  uint32_t* __restrict__ long_list,
                                                  uint32_t* __restrict__ long_count) {
     const uint32_t j = tmp[s];
@@ -140,19 +156,18 @@ __device__ __forceinline__ void sort_gather_item(uint32_t s, const uint32_t* __r
     }
     uint32_t rank = 0;
     for (uint32_t k = a; k < b; ++k) rank += (tmp[k] < j) ? 1u : 0u;
-    const uint32_t d = a + rank;
-    sidx[d] = j;
-    sorted[d] = pos[j];
+    place(sc, a + rank, j, pos[j], sidx, sorted, qpos);
 }
 
 // A long segment, by the whole block: rank(j) = number of particles j' < j of
 // cell c, from a block-wide scan over the particle indices [p0, p1) that can
 // hold the cell's particles.  s_warp: blockDim.x / 32 words of shared memory.
-__device__ inline void long_segment(uint32_t c, uint32_t p0, uint32_t p1,
+__device__ inline void long_segment(const StepConsts& sc, uint32_t c, uint32_t p0, uint32_t p1,
                                     const uint32_t* __restrict__ hash,
                                     const uint32_t* __restrict__ cstart,
                                     const float4* __restrict__ pos, uint32_t* __restrict__ sidx,
-                                    float4* __restrict__ sorted, uint32_t* s_warp) {
+                                    float4* __restrict__ sorted, uint32_t* __restrict__ qpos,
+                                    uint32_t* s_warp) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t a = cstart[c], len = cstart[c + 1] - a;
     uint32_t running = 0;
@@ -167,11 +182,7 @@ __device__ inline void long_segment(uint32_t c, uint32_t p0, uint32_t p1,
             if (w < warp) before += s_warp[w];
             blk += s_warp[w];
         }
-        if (f) {
-            const uint32_t d = a + running + before + __popc(m & lanemask_lt());
-            sidx[d] = j;
-            sorted[d] = pos[j];
-        }
+        if (f) place(sc, a + running + before + __popc(m & lanemask_lt()), j, pos[j], sidx, sorted, qpos);
         running += blk;
         __syncthreads();
     }
@@ -209,14 +220,15 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
 // ---- solver ------------------------------------------------------------------
 
 // In-range masks of one lambda pass.  For each particle and each of the 9
-// stencil rows, bit i is set when candidate slot b0 + i of that row lies
-// within h.  The delta pass of the same iteration sees the same positions and
-// the same stencil, hence exactly the same in-range pairs, so it walks these
-// bits instead of sweeping the 27 cells again.  Row-major layout (row r of
-// slot s at r * stride + s): the warp's stores and loads of one row coalesce.
-// A row longer than 32 candidates keeps the bits of its first 32 and sets bit
-// r of overflow[s]; the delta pass distance-tests that row's remaining
-// candidates again.  rows == nullptr disables the masks.
+// stencil rows [b0, b3), bit i is set when candidate slot (b0 & ~3) + i lies
+// within h (the row's first slot rounded down to a 16-byte boundary of the
+// quantized positions).  The delta pass of the same iteration sees the same
+// positions and the same stencil, hence exactly the same in-range pairs, so it
+// walks these bits instead of sweeping the 27 cells again.  Row-major layout
+// (row r of slot s at r * stride + s): the warp's stores and loads of one row
+// coalesce.  A row that does not end within 32 slots of its rounded start keeps
+// those bits and sets bit r of overflow[s]; the delta pass distance-tests that
+// row's remaining candidates again.
 struct RowMasks {
     uint32_t* rows;
     uint32_t* overflow;
@@ -298,114 +310,120 @@ __device__ __forceinline__ void delta_add(const StepConsts& c, float li, float l
     }
 }
 
+// First slot of a row mask: the row's first slot, rounded down to a 16-byte
+// boundary of the quantized positions.
+__device__ __forceinline__ uint32_t row_base(uint32_t b0) { return b0 & ~3u; }
+
 // Two-phase sweep of the 27-cell stencil around cell (cx, cy, cz).  Each row
 // (3 consecutive cells, one contiguous slot range) is taken in chunks of 32
-// candidates: phase 1 loads every candidate once, does only the distance test
-// and sets a bit for each one within h; phase 2 visits just the set bits and
-// calls body(k, q, rx, ry, rz, r2) with k the candidate's slot.  The in-range
-// body, about an eighth of the candidates, then runs on most lanes of the warp
-// instead of on the few lanes whose candidate happened to be in range.
+// candidates.
+//
+// Phase 1 tests the byte-quantized positions qsrc (quantize() above): per
+// candidate one 32-bit subtraction, one __dp4a whose sum starts at -threshold
+// and one funnel shift that collects its sign bit; one 16-byte load brings four
+// candidates.  The threshold admits every pair the exact test could accept
+// (set_prefilter), about 9% more than are in range.  Phase 2 visits just the
+// set bits, loads the candidate's position, applies the exact FP32 test and
+// calls body(k, q, rx, ry, rz, r2), k the candidate's slot; a candidate that
+// fails loses its bit.  So masks, counts and sums are those of the exact test
+// alone.
+// Both passes are bound by instruction issue: testing the FP32 positions took
+// about 12 instructions and a 16-byte load per candidate, this takes 3 and a
+// quarter of one.  On the 1,003,520-particle dam break, k_lambda 286 M -> 214 M
+// warp instructions, 309-327 -> 281 us; the step 2.35 -> 2.16 ms.
 //
 // ANCHORED = false: (px, py, pz) is the absolute FP32 position and r = p - q.
-// ANCHORED = true:  (px, py, pz) is the offset l from the anchor of hash cell
-// (pcx, pcy, pcz); r = ((A_i - A_cell(k)) + l_i) - l_k, A_i - A_cell(k) exact.
-// XW = true: each candidate carries the x anchor of its own hash cell in w
-// (the delta pass's output), so its x term is (A_i - q.w) + l_i, the same
-// value as the per-cell term the row would otherwise select by slot.
+// ANCHORED = true:  (px, py, pz) is the offset l from the anchor (aix, aiy,
+// aiz) of the particle's hash cell and each candidate carries the x anchor of
+// its own hash cell in w (the delta pass's output):
+// r = ((A_i - A_cell(k)) + l_i) - l_k, A_i - A_cell(k) exact.
 //
-// With masks, every row of the stencil stores the bits of its first chunk (the
-// particle's own bit cleared) for the delta pass, and a row longer than one
-// chunk sets its bit in the overflow word.  Returns the number of in-range
-// candidates, the particle itself included.
-template <bool ANCHORED, bool XW = false, class Body>
+// Every row of the stencil stores the bits of its first chunk (the particle's
+// own bit cleared) for the delta pass, and a row longer than one chunk sets
+// its bit in the overflow word.  Returns the number of in-range candidates
+// other than the particle itself.
+template <bool ANCHORED, class Body>
 __device__ __forceinline__ uint32_t sweep(const StepConsts& c, const float4* __restrict__ src,
+                                          const uint32_t* __restrict__ qsrc,
                                           const uint32_t* __restrict__ cstart, int cx, int cy, int cz,
-                                          float px, float py, float pz, int pcx, int pcy, int pcz,
-                                          uint32_t s, const RowMasks* masks, Body&& body) {
+                                          float px, float py, float pz, float aix, float aiy, float aiz,
+                                          uint32_t qi, int nthr, uint32_t s, const RowMasks& masks,
+                                          Body&& body) {
     const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
     const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
     const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
     const int nx = x1 - x0 + 1;
     uint32_t hits = 0, over = 0;
     if (nx <= 0) {  // drifted more than a cell outside a scene's sub-grid: no candidates
-        if (masks) {
-            for (int z = z0; z <= z1; ++z)
-                for (int y = y0; y <= y1; ++y)
-                    masks->rows[uint32_t((z - z0) * 3 + (y - y0)) * masks->stride + s] = 0u;
-            masks->overflow[s] = 0u;
-        }
+        for (int z = z0; z <= z1; ++z)
+            for (int y = y0; y <= y1; ++y)
+                masks.rows[uint32_t((z - z0) * 3 + (y - y0)) * masks.stride + s] = 0u;
+        masks.overflow[s] = 0u;
         return 0;
-    }
-#ifndef MPB_NO_XW
-    constexpr bool kXW = ANCHORED && XW;
-#else
-    constexpr bool kXW = false;
-#endif
-    float ox0 = px, ox1 = px, ox2 = px;
-    float aix = 0.0f, aiy = 0.0f, aiz = 0.0f;
-    if (ANCHORED) {
-        aix = anchor_x(c.g, pcx);
-        aiy = anchor_y(c.g, pcy);
-        aiz = anchor_z(c.g, pcz);
-        ox0 = __fadd_rn(__fsub_rn(aix, anchor_x(c.g, x0)), px);
-        ox1 = __fadd_rn(__fsub_rn(aix, anchor_x(c.g, x0 + 1)), px);
-        ox2 = __fadd_rn(__fsub_rn(aix, anchor_x(c.g, x0 + 2)), px);
     }
     for (int z = z0; z <= z1; ++z) {
         const float oz = ANCHORED ? __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z)), pz) : pz;
         for (int y = y0; y <= y1; ++y) {
             const float oy = ANCHORED ? __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y)), py) : py;
             const uint32_t base = cell_hash(c.g, x0, y, z);
-            const uint32_t b0 = cstart[base], b1 = cstart[base + 1];
-            const uint32_t b2 = nx > 1 ? cstart[base + 2] : b1;
-            const uint32_t b3 = nx > 2 ? cstart[base + 3] : b2;
-            uint32_t first = 0;  // bits of the first chunk (the whole row if b3 - b0 <= 32)
-            for (uint32_t c0 = b0; c0 < b3; c0 += 32) {
-                const uint32_t c1 = min(c0 + 32u, b3);
-                uint32_t mask = 0;
-                if (!ANCHORED) {
-                    // the first pass: a running bit (measured faster here, not in
-                    // the anchored passes)
-                    uint32_t bit = 1u;
-                    for (uint32_t k = c0; k < c1; ++k, bit <<= 1) {
-                        const float4 q = __ldg(&src[k]);
-                        const float r2 = dist2(__fsub_rn(px, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
-                        if (r2 < c.h2) mask |= bit;
+            const uint32_t b0 = cstart[base], b3 = cstart[base + uint32_t(nx)];
+            const uint32_t a0 = row_base(b0);
+            const uint32_t row = uint32_t((z - z0) * 3 + (y - y0));
+            uint32_t first = 0;  // bits of the first chunk (the whole row if b3 - a0 <= 32)
+            if (b0 < b3) {
+                uint32_t lo = b0 - a0;  // candidates of the chunk before the row
+                for (uint32_t c0 = a0; c0 < b3; c0 += 32) {
+                    const uint32_t c1 = min(c0 + 32u, b3);
+                    uint32_t mask = 0, k = c0;
+                    for (; k < c1; k += 4) {
+                        const uint4 q = __ldg(reinterpret_cast<const uint4*>(qsrc + k));
+                        const int d0 = int(qi - q.x), d1 = int(qi - q.y);
+                        const int d2 = int(qi - q.z), d3 = int(qi - q.w);
+                        mask = __funnelshift_l(uint32_t(__dp4a(d0, d0, nthr)), mask, 1);
+                        mask = __funnelshift_l(uint32_t(__dp4a(d1, d1, nthr)), mask, 1);
+                        mask = __funnelshift_l(uint32_t(__dp4a(d2, d2, nthr)), mask, 1);
+                        mask = __funnelshift_l(uint32_t(__dp4a(d3, d3, nthr)), mask, 1);
                     }
-                } else {
-                    for (uint32_t k = c0; k < c1; ++k) {
-                        const float4 q = __ldg(&src[k]);
-                        const float ox =
-                            kXW ? __fadd_rn(__fsub_rn(aix, q.w), px) : (k < b1 ? ox0 : (k < b2 ? ox1 : ox2));
-                        const float r2 = dist2(__fsub_rn(ox, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
-                        mask |= uint32_t(r2 < c.h2) << (k - c0);
+                    // first candidate in the top of the k - c0 bits: to bit 0;
+                    // then drop what lies outside the row, and the particle itself
+                    mask = __brev(mask) >> (32u - (k - c0));
+                    mask &= (0xffffffffu << lo) & (0xffffffffu >> (32u - (c1 - c0)));
+                    lo = 0;
+                    if (s - c0 < 32u) mask &= ~(1u << (s - c0));
+                    uint32_t todo = mask;
+                    while (todo) {
+                        const uint32_t bit = todo & (0u - todo);
+                        const uint32_t j = c0 + uint32_t(__ffs(todo) - 1);
+                        todo ^= bit;
+                        const float4 q = __ldg(&src[j]);
+                        const float ox = ANCHORED ? __fadd_rn(__fsub_rn(aix, q.w), px) : px;
+                        const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
+                        const float r2 = dist2(rx, ry, rz);
+                        if (r2 < c.h2)
+                            body(j, q, rx, ry, rz, r2);
+                        else
+                            mask ^= bit;
                     }
+                    hits += __popc(mask);
+                    if (c0 == a0) first = mask;
                 }
-                if (c0 == b0) first = mask;
-                hits += __popc(mask);
-                // the particle's own slot gets no body (its r is 0)
-                if (s - c0 < 32u) mask &= ~(1u << (s - c0));
-                while (mask) {
-                    const uint32_t k = c0 + uint32_t(__ffs(mask) - 1);
-                    mask &= mask - 1;
-                    const float4 q = __ldg(&src[k]);
-                    const float ox = kXW ? __fadd_rn(__fsub_rn(aix, q.w), px) : (k < b1 ? ox0 : (k < b2 ? ox1 : ox2));
-                    const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
-                    body(k, q, rx, ry, rz, dist2(rx, ry, rz));
-                }
+                if (b3 - a0 > 32u) over |= 1u << row;
             }
-            if (masks) {
-                // every row of the stencil is stored, empty ones as 0; a long
-                // row stores its first 32 candidates and flags the rest
-                const uint32_t row = uint32_t((z - z0) * 3 + (y - y0));
-                const uint32_t self = s - b0;
-                masks->rows[row * masks->stride + s] = self < 32u ? (first & ~(1u << self)) : first;
-                if (b3 - b0 > 32u) over |= 1u << row;
-            }
+            masks.rows[row * masks.stride + s] = first;
         }
     }
-    if (masks) masks->overflow[s] = over;
+    masks.overflow[s] = over;
     return hits;
+}
+
+// The prefilter's arguments of a particle at offset l from the corner of its
+// hash cell (dense coordinates): its quantized word, and minus the threshold.  A
+// particle far outside the grid (or not finite) tests every candidate exactly.
+__device__ __forceinline__ int prefilter(const StepConsts& c, int hx, int hy, int hz, float lx, float ly,
+                                         float lz, uint32_t& qi) {
+    qi = quantize<true>(c, hx, hy, hz, lx, ly, lz);
+    const bool near = fabsf(lx) < c.q_lim && fabsf(ly) < c.q_lim && fabsf(lz) < c.q_lim;
+    return near ? -c.q_thr : -kPassAll;
 }
 
 // First lambda pass: absolute FP32 predicted positions (reference arithmetic,
@@ -414,6 +432,7 @@ __device__ __forceinline__ uint32_t sweep(const StepConsts& c, const float4* __r
 template <bool LAST>
 __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t s,
                                                   const float4* __restrict__ cur,
+                                                  const uint32_t* __restrict__ qpos,
                                                   float4* __restrict__ nxt,
                                                   uint32_t* __restrict__ scell,
                                                   const uint32_t* __restrict__ cstart,
@@ -423,27 +442,26 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t 
     const float4 p = cur[s];
     int cx, cy, cz;
     cell_of(c.g, p.x, p.y, p.z, cx, cy, cz);
-    LambdaAcc acc;
-    acc.self(c);
-    const uint32_t cnt = sweep<false>(c, cur, cstart, cx, cy, cz, p.x, p.y, p.z, cx, cy, cz, s,
-                                      rm.rows ? &rm : nullptr,
-                                      [&](uint32_t k, const float4&, float rx, float ry, float rz,
-                                          float r2) {
-                                          acc.add(c, rx, ry, rz, r2);
-                                      });
-    const float lambda = acc.lambda(c);
     // l = p - A(c): exact for the particle's own cell (Sterbenz) unless the
     // cell reaches a zero coordinate from below, where it rounds once, by at
     // most half an ulp of the cell size; so the anchored state starts equal to
     // the FP32 predicted position.
-    nxt[s] = make_float4(__fsub_rn(p.x, anchor_x(c.g, cx)), __fsub_rn(p.y, anchor_y(c.g, cy)),
-                         __fsub_rn(p.z, anchor_z(c.g, cz)), lambda);
+    const float lx = __fsub_rn(p.x, anchor_x(c.g, cx)), ly = __fsub_rn(p.y, anchor_y(c.g, cy));
+    const float lz = __fsub_rn(p.z, anchor_z(c.g, cz));
+    uint32_t qi;
+    const int nthr = prefilter(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, lx, ly, lz, qi);
+    LambdaAcc acc;
+    acc.self(c);
+    const uint32_t cnt = sweep<false>(c, cur, qpos, cstart, cx, cy, cz, p.x, p.y, p.z, 0.0f, 0.0f, 0.0f, qi,
+                                      nthr, s, rm,
+                                      [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
+                                          acc.add(c, rx, ry, rz, r2);
+                                      });
+    const float lambda = acc.lambda(c);
+    nxt[s] = make_float4(lx, ly, lz, lambda);
     scell[s] = cell_local(c.g, cx, cy, cz);
     const uint32_t j = sidx[s];
-    // the particle itself was counted iff its own distance test passed
-    // (false for a non-finite position)
-    const uint32_t self = dist2(p.x - p.x, p.y - p.y, p.z - p.z) < c.h2 ? 1u : 0u;
-    ncount[j] = cnt - self;
+    ncount[j] = cnt;
     if (LAST) lambdas[j] = lambda;
 }
 
@@ -451,7 +469,8 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t 
 // output, (l, x anchor of the hash cell) per slot.
 template <bool LAST>
 __device__ __forceinline__ void lambda_item(const StepConsts& c, uint32_t s,
-                                            const float4* __restrict__ cur, float4* __restrict__ nxt,
+                                            const float4* __restrict__ cur,
+                                            const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
                                             const uint32_t* __restrict__ scell,
                                             const uint32_t* __restrict__ cstart,
                                             const uint32_t* __restrict__ sidx,
@@ -459,14 +478,16 @@ __device__ __forceinline__ void lambda_item(const StepConsts& c, uint32_t s,
     const float4 l = cur[s];
     int pcx, pcy, pcz, cx, cy, cz;
     decode_cell(c.g, scell[s], pcx, pcy, pcz);
-    cell_of(c.g, __fadd_rn(anchor_x(c.g, pcx), l.x), __fadd_rn(anchor_y(c.g, pcy), l.y),
-            __fadd_rn(anchor_z(c.g, pcz), l.z), cx, cy, cz);
+    const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
+    cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
+    uint32_t qi;
+    const int nthr = prefilter(c, pcx + c.g.lx, pcy + c.g.ly, pcz + c.g.lz, l.x, l.y, l.z, qi);
     LambdaAcc acc;
     acc.self(c);
-    sweep<true, true>(c, cur, cstart, cx, cy, cz, l.x, l.y, l.z, pcx, pcy, pcz, s, rm.rows ? &rm : nullptr,
-                      [&](uint32_t k, const float4&, float rx, float ry, float rz, float r2) {
-                          acc.add(c, rx, ry, rz, r2);
-                      });
+    sweep<true>(c, cur, qpos, cstart, cx, cy, cz, l.x, l.y, l.z, ax, ay, az, qi, nthr, s, rm,
+                [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
+                    acc.add(c, rx, ry, rz, r2);
+                });
     const float lambda = acc.lambda(c);
     nxt[s] = make_float4(l.x, l.y, l.z, lambda);
     if (LAST) lambdas[sidx[s]] = lambda;
@@ -528,7 +549,7 @@ __device__ __forceinline__ void finalize_particle(const StepConsts& c, uint32_t 
 // own bit cleared), walked with the anchored neighbour vector of sweep<true>:
 // body(k, q, rx, ry, rz, r2) for each, in sweep<true>'s order (rows in
 // stencil order, slots ascending).  The candidates of a long row past its
-// first 32 are distance-tested again.  (cx, cy, cz): the stencil cell of the
+// first chunk are distance-tested again.  (cx, cy, cz): the stencil cell of the
 // particle at offset l from anchor (ax, ay, az).
 template <class Body>
 __device__ __forceinline__ void masked_pairs(const StepConsts& c, const float4* __restrict__ src,
@@ -555,8 +576,9 @@ __device__ __forceinline__ void masked_pairs(const StepConsts& c, const float4* 
             const uint32_t base = cell_hash(c.g, x0, y, z);
             const uint32_t b0 = cstart[base], b1 = cstart[base + 1];
             const uint32_t b2 = nx > 1 ? cstart[base + 2] : b1;
+            const uint32_t a0 = row_base(b0);
             while (mask) {
-                const uint32_t k = b0 + uint32_t(__ffs(mask) - 1);
+                const uint32_t k = a0 + uint32_t(__ffs(mask) - 1);
                 mask &= mask - 1;
                 const float ox = k < b1 ? ox0 : (k < b2 ? ox1 : ox2);
                 const float4 q = __ldg(&src[k]);
@@ -566,7 +588,7 @@ __device__ __forceinline__ void masked_pairs(const StepConsts& c, const float4* 
             }
             if (long_row) {
                 const uint32_t b3 = nx > 2 ? cstart[base + 3] : b2;
-                for (uint32_t k = b0 + 32u; k < b3; ++k) {
+                for (uint32_t k = a0 + 32u; k < b3; ++k) {
                     const float ox = k < b1 ? ox0 : (k < b2 ? ox1 : ox2);
                     const float4 q = __ldg(&src[k]);
                     const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y);
@@ -586,6 +608,7 @@ __device__ __forceinline__ void masked_pairs(const StepConsts& c, const float4* 
 template <bool LAST, uint32_t SN = 0>
 __device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
                                            const float4* __restrict__ src, float4* __restrict__ dst,
+                                           uint32_t* __restrict__ qpos,
                                            const uint32_t* __restrict__ scell,
                                            const uint32_t* __restrict__ cstart,
                                            const uint32_t* __restrict__ sidx,
@@ -605,15 +628,7 @@ __device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
     auto body = [&](uint32_t, const float4& q, float rx, float ry, float rz, float r2) {
         delta_add<SN>(c, l.w, q.w, rx, ry, rz, r2, dx, dy, dz);
     };
-#ifdef MPB_PARTICLE_OVERFLOW
-    if (rm.rows != nullptr && rm.overflow[s] == 0u)
-#else
-    if (rm.rows != nullptr)
-#endif
-        masked_pairs(c, src, cstart, rm, s, l, ax, ay, az, cx, cy, cz, body);
-    else
-        sweep<true>(c, src, cstart, cx, cy, cz, l.x, l.y, l.z, pcx, pcy, pcz, s,
-                    static_cast<const RowMasks*>(nullptr), body);
+    masked_pairs(c, src, cstart, rm, s, l, ax, ay, az, cx, cy, cz, body);
     dx = __fmul_rn(dx, c.delta_scale);
     dy = __fmul_rn(dy, c.delta_scale);
     dz = __fmul_rn(dz, c.delta_scale);
@@ -646,8 +661,10 @@ __device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
     if (!LAST) {
         // w: the x anchor of the particle's hash cell, for the next lambda
         // pass's neighbour vectors
-        dst[s] = make_float4(float(__dsub_rn(X, double(ax))), float(__dsub_rn(Y, double(ay))),
-                             float(__dsub_rn(Z, double(az))), ax);
+        const float lx = float(__dsub_rn(X, double(ax))), ly = float(__dsub_rn(Y, double(ay)));
+        const float lz = float(__dsub_rn(Z, double(az)));
+        dst[s] = make_float4(lx, ly, lz, ax);
+        qpos[s] = quantize<false>(c, pcx + c.g.lx, pcy + c.g.ly, pcz + c.g.lz, lx, ly, lz);
         return;
     }
     finalize_particle(c, sidx[s], X, Y, Z, pos, vel, prev, ncount, foam, err);

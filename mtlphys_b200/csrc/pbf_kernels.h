@@ -20,9 +20,10 @@ struct DevState {
     uint32_t* off;          // rank of the particle's atomic increment in its cell
     uint32_t* tmp;          // unstable cell-grouped order (before the stable fix-up)
     uint32_t* sidx;         // sortedIndex: slot -> particle, stable within a cell
+    uint32_t* qpos;         // quantized position per sorted slot (the lambda passes' prefilter)
     uint32_t* scell;        // hash cell per sorted slot (anchor of the solver state)
     uint32_t* row_masks;            // 9 x mask_stride in-range bits per stencil row
-    uint32_t* mask_overflow;        // bit r: row r exceeded 32 candidates (delta re-tests the rest)
+    uint32_t* mask_overflow;        // bit r: row r does not fit its 32 bits (delta re-tests the rest)
     uint32_t mask_stride;
     uint32_t* ncount;       // neighbour count per particle
     float* lambdas;         // last lambda per particle

@@ -41,35 +41,35 @@ constexpr uint32_t kSB = MPB_SOLVER_BLOCK;
 
 template <bool LAST>
 __global__ void __launch_bounds__(kSB, MPB_LAMBDA_MIN_BLOCKS * 256 / kSB)
-k_lambda_first(StepConsts c, const float4* __restrict__ cur, float4* __restrict__ nxt,
+k_lambda_first(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
                uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
                const uint32_t* __restrict__ sidx, float* __restrict__ lambdas,
                uint32_t* __restrict__ ncount, RowMasks rm) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < c.n) lambda_first_item<LAST>(c, s, cur, nxt, scell, cstart, sidx, lambdas, ncount, rm);
+    if (s < c.n) lambda_first_item<LAST>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm);
 }
 
 template <bool LAST>
 __global__ void __launch_bounds__(kSB, MPB_LAMBDA_MIN_BLOCKS * 256 / kSB)
-k_lambda(StepConsts c, const float4* __restrict__ cur, float4* __restrict__ nxt,
+k_lambda(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
          const uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
          const uint32_t* __restrict__ sidx, float* __restrict__ lambdas, RowMasks rm) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < c.n) lambda_item<LAST>(c, s, cur, nxt, scell, cstart, sidx, lambdas, rm);
+    if (s < c.n) lambda_item<LAST>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm);
 }
 
 // SN = 4: the reference's s_corr exponent, fixed at compile time (the host
 // launches this instance when scorr_n == 4); SN = 0 reads it from c.
 template <bool LAST, uint32_t SN>
 __global__ void __launch_bounds__(kSB, (LAST ? MPB_DELTA_MIN_BLOCKS : MPB_DELTA_MID_MIN_BLOCKS) * 256 / kSB)
-k_delta(StepConsts c, const float4* __restrict__ src, float4* __restrict__ dst,
+k_delta(StepConsts c, const float4* __restrict__ src, float4* __restrict__ dst, uint32_t* __restrict__ qpos,
         const uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
         const uint32_t* __restrict__ sidx, const SphereState* __restrict__ sphere,
         float4* __restrict__ pos, float4* __restrict__ vel, const float4* __restrict__ prev,
         const uint32_t* __restrict__ ncount, float* __restrict__ foam, uint32_t* err, RowMasks rm) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < c.n)
-        delta_item<LAST, SN>(c, s, src, dst, scell, cstart, sidx, sphere, pos, vel, prev, ncount, foam,
+        delta_item<LAST, SN>(c, s, src, dst, qpos, scell, cstart, sidx, sphere, pos, vel, prev, ncount, foam,
                              err, rm, nullptr);
 }
 
@@ -77,10 +77,10 @@ template <bool LAST>
 void launch_delta(const StepConsts& c, const DevState& d, const RowMasks& rm, cudaStream_t s) {
     const dim3 grid(cdiv(c.n, kSB));
     if (c.scorr_n == 4)
-        k_delta<LAST, 4><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.scell, d.cstart, d.sidx, d.sphere,
+        k_delta<LAST, 4><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.scell, d.cstart, d.sidx, d.sphere,
                                               d.pos, d.vel, d.prev, d.ncount, d.foam, d.err, rm);
     else
-        k_delta<LAST, 0><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.scell, d.cstart, d.sidx, d.sphere,
+        k_delta<LAST, 0><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.scell, d.cstart, d.sidx, d.sphere,
                                               d.pos, d.vel, d.prev, d.ncount, d.foam, d.err, rm);
 }
 
@@ -114,16 +114,16 @@ cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t itera
         const bool first = it == 0, last = it + 1 == iterations;
         tbegin(t, s);
         if (first && last)
-            k_lambda_first<true><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.sorted_b, d.scell, d.cstart,
+            k_lambda_first<true><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart,
                                                       d.sidx, d.lambdas, d.ncount, rm);
         else if (first)
-            k_lambda_first<false><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.sorted_b, d.scell, d.cstart,
+            k_lambda_first<false><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart,
                                                        d.sidx, d.lambdas, d.ncount, rm);
         else if (last)
-            k_lambda<true><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.sorted_b, d.scell, d.cstart, d.sidx,
+            k_lambda<true><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart, d.sidx,
                                                 d.lambdas, rm);
         else
-            k_lambda<false><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.sorted_b, d.scell, d.cstart, d.sidx,
+            k_lambda<false><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart, d.sidx,
                                                  d.lambdas, rm);
         tend(t, first ? "lambda_count" : "lambda", s);
         tbegin(t, s);
