@@ -420,7 +420,8 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         total += counts[s];
         worst_cells += grids[s].cells;
     }
-    if (total >= (1ull << 31)) return fail(MP_ERR_INVALID_ARGUMENT, "too many particles");
+    // slots are 30-bit numbers in the pair queues (a batch this size needs 176 GB)
+    if (total > (1ull << 30)) return fail(MP_ERR_INVALID_ARGUMENT, "too many particles");
     if (worst_cells >= (1ull << 31) - 1) return fail(MP_ERR_INVALID_ARGUMENT, "scene grids too large");
     // seed every scene on the host
     std::vector<float> pos(4 * size_t(total), 0.0f), tmp;
@@ -472,7 +473,7 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         const uint32_t cap = round_up(std::max<uint32_t>(b->N, 1u), 256u);
         const size_t v4 = size_t(cap) * 16, u = size_t(cap) * 4;
         const size_t longs = (size_t(cap) / kSegMax + 2) * 4;
-        const size_t ptotal = 5 * v4 + 20 * u + longs + 32 * 256;
+        const size_t ptotal = 5 * v4 + 21 * u + longs + 32 * 256;
         MP_ALLOC(b->particle_block, ptotal, b->device);
         MP_CUDA(cudaMemset(b->particle_block, 0, ptotal));
         char* pb = static_cast<char*>(b->particle_block);
@@ -496,6 +497,7 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         a.ncount = reinterpret_cast<uint32_t*>(take(u));
         a.lambdas = reinterpret_cast<float*>(take(u));
         a.foam = reinterpret_cast<float*>(take(u));
+        a.xa = reinterpret_cast<float*>(take(u));
         uint32_t* so = reinterpret_cast<uint32_t*>(take(u));
         a.scene_of = so;
         a.row_masks = reinterpret_cast<uint32_t*>(take(9 * u));

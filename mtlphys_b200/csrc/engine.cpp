@@ -555,7 +555,7 @@ struct mp_engine {
         list_block = nullptr;
         d.pos = d.vel = d.prev = d.sorted_a = d.sorted_b = nullptr;
         d.hash = d.off = d.tmp = d.sidx = d.qpos = d.scell = d.ncount = d.long_list = nullptr;
-        d.lambdas = d.foam = nullptr;
+        d.lambdas = d.foam = d.xa = nullptr;
         d.row_masks = nullptr;
         d.mask_overflow = nullptr;
         d.mask_stride = 0;
@@ -585,7 +585,7 @@ struct mp_engine {
         free_particles();
         const size_t v4 = size_t(cap) * 16, u = size_t(cap) * 4;
         const size_t longs = (size_t(cap) / mpb::kSegMax + 2) * 4;
-        const size_t total = 5 * v4 + 9 * u + longs + 16 * 256;
+        const size_t total = 5 * v4 + 10 * u + longs + 18 * 256;
         MP_ALLOC(particle_block, total, device);
         char* b = static_cast<char*>(particle_block);
         auto take = [&](size_t bytes) {
@@ -607,6 +607,7 @@ struct mp_engine {
         d.ncount = reinterpret_cast<uint32_t*>(take(u));
         d.lambdas = reinterpret_cast<float*>(take(u));
         d.foam = reinterpret_cast<float*>(take(u));
+        d.xa = reinterpret_cast<float*>(take(u));
         d.long_list = reinterpret_cast<uint32_t*>(take(longs));
         MP_CUDA(cudaMemset(particle_block, 0, total));
         // 9 row masks (4 bytes each) + an overflow flag per particle

@@ -123,6 +123,7 @@ template <uint32_t BS, uint32_t SN>
 __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(BatchArgs a) {
     __shared__ uint32_t s_warp[BS / 32 + 1];
     __shared__ int s_ok;
+    extern __shared__ uint2 queue[];  // kQueue entries per thread
     const uint32_t gtid = blockIdx.x * BS + threadIdx.x;
     // an earlier launch gave up on a barrier and left the barrier counter
     // mid-count: do nothing until the host has re-armed the batch
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     if (cells_ok)
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             sort_gather_item(sc[a.scene_of[s]].c, s, a.tmp, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
-                             a.qpos, a.long_list, a.long_count);
+                             a.qpos, a.xa, a.long_list, a.long_count);
     if (!grid_barrier(a, &s_ok)) return;
     {
         const uint32_t nl = cells_ok ? *a.long_count : 0u;
@@ -297,7 +298,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             const uint32_t cell = a.long_list[li];
             const SceneDev& sd = sc[a.scene_of[a.tmp[a.cstart[cell]]]];
             long_segment(sd.c, cell, sd.p0, sd.p0 + sd.c.n, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
-                         a.qpos, s_warp);
+                         a.qpos, a.xa, s_warp);
         }
     }
     if (!grid_barrier(a, &s_ok)) return;
@@ -329,29 +330,42 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             const StepConsts& c = sc[a.scene_of[s]].c;
             if (it == 0) {
                 if (last)
-                    lambda_first_item<true>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
-                                            a.lambdas, a.ncount, rmi);
+                    lambda_first_item<true, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                                            a.lambdas, a.ncount, rmi, queue);
                 else
-                    lambda_first_item<false>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
-                                             a.lambdas, a.ncount, rmi);
+                    lambda_first_item<false, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                                             a.lambdas, a.ncount, rmi, queue);
             } else if (last) {
-                lambda_item<true>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi);
+                lambda_item<true, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi, queue);
             } else {
-                lambda_item<false>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi);
+                lambda_item<false, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi, queue);
             }
         }
         if (!grid_barrier(a, &s_ok)) return;
         for (uint32_t s = pb + gtid; s < pe; s += gsize) {
             const SceneDev& sd = sc[a.scene_of[s]];
             if (last)
-                delta_item<true, SN>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.scell, a.cstart, a.sidx, &sd.sphere,
-                                 a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec);
+                delta_item<true, SN, BS>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx, &sd.sphere,
+                                 a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec, queue);
             else
-                delta_item<false, SN>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.scell, a.cstart, a.sidx, &sd.sphere,
-                                  a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec);
+                delta_item<false, SN, BS>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx, &sd.sphere,
+                                  a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec, queue);
         }
         if (!last && !grid_barrier(a, &s_ok)) return;
     }
+}
+
+// Dynamic shared memory of a launch: the blocks' pair queues (beyond the 48 KB
+// a kernel may use unasked at BS = 512).
+template <uint32_t BS>
+constexpr size_t queue_bytes() {
+    return size_t(kQueue) * BS * sizeof(uint2);
+}
+
+template <uint32_t BS>
+cudaError_t allow_shared(const void* fn) {
+    if (queue_bytes<BS>() <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(queue_bytes<BS>()));
 }
 
 template <uint32_t BS>
@@ -359,17 +373,22 @@ cudaError_t launch_bs(const BatchArgs& args, uint32_t blocks, cudaStream_t s) {
     void* kargs[] = {const_cast<BatchArgs*>(&args)};
     const void* fn = args.scorr4 ? reinterpret_cast<const void*>(&k_batch_step<BS, 4>)
                                  : reinterpret_cast<const void*>(&k_batch_step<BS, 0>);
-    return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(BS), kargs, 0, s);
+    const cudaError_t e = allow_shared<BS>(fn);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(BS), kargs, queue_bytes<BS>(), s);
 }
 
 // Blocks of both instances that fit on one SM at once (the smaller count).
 template <uint32_t BS>
 int occupancy_bs() {
-    int n0 = 0, n4 = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n0, k_batch_step<BS, 0>, BS, 0) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n4, k_batch_step<BS, 4>, BS, 0) != cudaSuccess)
-        return 0;
-    return n0 < n4 ? n0 : n4;
+    int n[2] = {0, 0};
+    const void* fns[2] = {reinterpret_cast<const void*>(&k_batch_step<BS, 0>),
+                          reinterpret_cast<const void*>(&k_batch_step<BS, 4>)};
+    for (int i = 0; i < 2; ++i)
+        if (allow_shared<BS>(fns[i]) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[i], fns[i], BS, queue_bytes<BS>()) != cudaSuccess)
+            return 0;
+    return n[0] < n[1] ? n[0] : n[1];
 }
 
 }  // namespace

@@ -40,7 +40,7 @@ struct BatchArgs {
     uint32_t iterations;
     float4 *pos, *vel, *prev, *sorted_a, *sorted_b;
     uint32_t *hash, *off, *tmp, *sidx, *scell, *ncount, *qpos;
-    float *lambdas, *foam;
+    float *lambdas, *foam, *xa;
     uint32_t *counts, *cstart, *tile_sums;
     uint32_t max_cells;               // capacity of counts / cstart minus one
     uint32_t *long_list, *long_count;

@@ -238,21 +238,22 @@ __global__ void __launch_bounds__(256)
 k_sort_gather(StepConsts c, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ hash,
               const uint32_t* __restrict__ cstart, const float4* __restrict__ pos,
               uint32_t* __restrict__ sidx, float4* __restrict__ sorted, uint32_t* __restrict__ qpos,
-              uint32_t* __restrict__ long_list, uint32_t* __restrict__ long_count) {
+              float* __restrict__ xa, uint32_t* __restrict__ long_list, uint32_t* __restrict__ long_count) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < c.n) sort_gather_item(c, s, tmp, hash, cstart, pos, sidx, sorted, qpos, long_list, long_count);
+    if (s < c.n) sort_gather_item(c, s, tmp, hash, cstart, pos, sidx, sorted, qpos, xa, long_list, long_count);
 }
 
 // One block per queued long segment.
 __global__ void __launch_bounds__(256)
 k_long_segments(StepConsts c, const uint32_t* __restrict__ hash, const uint32_t* __restrict__ cstart,
                 const float4* __restrict__ pos, uint32_t* __restrict__ sidx,
-                float4* __restrict__ sorted, uint32_t* __restrict__ qpos, const uint32_t* __restrict__ long_list,
+                float4* __restrict__ sorted, uint32_t* __restrict__ qpos, float* __restrict__ xa,
+                const uint32_t* __restrict__ long_list,
                 const uint32_t* __restrict__ long_count) {
     __shared__ uint32_t s_warp[8];
     const uint32_t total = *long_count;
     for (uint32_t li = blockIdx.x; li < total; li += gridDim.x)
-        long_segment(c, long_list[li], 0u, c.n, hash, cstart, pos, sidx, sorted, qpos, s_warp);
+        long_segment(c, long_list[li], 0u, c.n, hash, cstart, pos, sidx, sorted, qpos, xa, s_warp);
 }
 
 __global__ void __launch_bounds__(256)
@@ -300,11 +301,11 @@ cudaError_t launch_hash_pass(const StepConsts& c, const DevState& d, bool predic
     tend(t, "scatter", s);
     tbegin(t, s);
     k_sort_gather<<<cdiv(n, 256), 256, 0, s>>>(c, d.tmp, d.hash, d.cstart, d.pos, d.sidx,
-                                                d.sorted_a, d.qpos, d.long_list, d.long_count);
+                                                d.sorted_a, d.qpos, d.xa, d.long_list, d.long_count);
     tend(t, "sort_gather", s);
     tbegin(t, s);
     k_long_segments<<<148, 256, 0, s>>>(c, d.hash, d.cstart, d.pos, d.sidx, d.sorted_a,
-                                        d.qpos, d.long_list, d.long_count);
+                                        d.qpos, d.xa, d.long_list, d.long_count);
     tend(t, "long_segments", s);
     return cudaGetLastError();
 }

@@ -121,16 +121,18 @@ __device__ __forceinline__ void scatter_item(uint32_t i, const uint32_t* __restr
     tmp[cstart[hash[i]] + off[i]] = i;
 }
 
-// A particle's place in sorted order: its index, predicted position and
-// quantized position.
+// A particle's place in sorted order: its index, predicted position, quantized
+// position and the x anchor of its cell.
 __device__ __forceinline__ void place(const StepConsts& c, uint32_t d, uint32_t j, const float4& p,
                                       uint32_t* __restrict__ sidx, float4* __restrict__ sorted,
-                                      uint32_t* __restrict__ qpos) {
+                                      uint32_t* __restrict__ qpos, float* __restrict__ xa) {
     int cx, cy, cz;
     cell_of(c.g, p.x, p.y, p.z, cx, cy, cz);
     sidx[d] = j;
     sorted[d] = p;
-    qpos[d] = quantize<false>(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, __fsub_rn(p.x, anchor_x(c.g, cx)),
+    const float ax = anchor_x(c.g, cx);
+    xa[d] = ax;
+    qpos[d] = quantize<false>(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, __fsub_rn(p.x, ax),
                               __fsub_rn(p.y, anchor_y(c.g, cy)), __fsub_rn(p.z, anchor_z(c.g, cz)));
 }
 
@@ -144,7 +146,7 @@ __device__ __forceinline__ void sort_gather_item(const StepConsts& sc, uint32_t 
                                                  const float4* __restrict__ pos,
                                                  uint32_t* __restrict__ sidx,
                                                  float4* __restrict__ sorted,
-                                                 uint32_t* __restrict__ qpos,
+                                                 uint32_t* __restrict__ qpos, float* __restrict__ xa,
                                                  uint32_t* __restrict__ long_list,
                                                  uint32_t* __restrict__ long_count) {
     const uint32_t j = tmp[s];
@@ -156,7 +158,7 @@ __device__ __forceinline__ void sort_gather_item(const StepConsts& sc, uint32_t 
     }
     uint32_t rank = 0;
     for (uint32_t k = a; k < b; ++k) rank += (tmp[k] < j) ? 1u : 0u;
-    place(sc, a + rank, j, pos[j], sidx, sorted, qpos);
+    place(sc, a + rank, j, pos[j], sidx, sorted, qpos, xa);
 }
 
 // A long segment, by the whole block: rank(j) = number of particles j' < j of
@@ -167,7 +169,7 @@ __device__ inline void long_segment(const StepConsts& sc, uint32_t c, uint32_t p
                                     const uint32_t* __restrict__ cstart,
                                     const float4* __restrict__ pos, uint32_t* __restrict__ sidx,
                                     float4* __restrict__ sorted, uint32_t* __restrict__ qpos,
-                                    uint32_t* s_warp) {
+                                    float* __restrict__ xa, uint32_t* s_warp) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t a = cstart[c], len = cstart[c + 1] - a;
     uint32_t running = 0;
@@ -182,7 +184,8 @@ __device__ inline void long_segment(const StepConsts& sc, uint32_t c, uint32_t p
             if (w < warp) before += s_warp[w];
             blk += s_warp[w];
         }
-        if (f) place(sc, a + running + before + __popc(m & lanemask_lt()), j, pos[j], sidx, sorted, qpos);
+        if (f)
+            place(sc, a + running + before + __popc(m & lanemask_lt()), j, pos[j], sidx, sorted, qpos, xa);
         running += blk;
         __syncthreads();
     }
@@ -241,6 +244,14 @@ struct RowMasks {
 // functions (the single-scene kernels, the persistent batch kernel) rounds
 // identically and gives bit-identical results.
 
+// 1 / sqrt(x) of a normal x (the value of rsqrtf without its handling of
+// subnormal arguments).
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // densityLambdaSorted's sums for one particle (Constraints.metal:99-121): the
 // density starts at the particle's own W(0) whether or not its slot lies in
 // the stencil of its current cell (a particle can drift two cells from its
@@ -253,17 +264,20 @@ struct LambdaAcc {
     __device__ __forceinline__ void self(const StepConsts& c) {
         dens = __fmul_rn(__fmul_rn(__fmul_rn(c.poly6, c.h2), c.h2), c.h2);
     }
+    // no effect unless r2 < h^2
     __device__ __forceinline__ void add(const StepConsts& c, float rx, float ry, float rz, float r2) {
         const float d = __fsub_rn(c.h2, r2);
-        dens = __fmaf_rn(__fmul_rn(__fmul_rn(c.poly6, d), d), d, dens);
-        if (r2 > 1e-12f) {
-            const float rinv = rsqrtf(r2);
-            const float hd = fmaxf(__fsub_rn(c.h, __fmul_rn(r2, rinv)), 0.0f);
-            const float sc = __fmul_rn(__fmul_rn(__fmul_rn(-c.spiky, hd), hd), rinv);
+        const float w = __fmul_rn(__fmul_rn(c.poly6, d), d);
+        const float rinv = rsqrt_normal(r2);
+        const float hd = fmaxf(__fsub_rn(c.h, __fmul_rn(r2, rinv)), 0.0f);
+        const float sc = __fmul_rn(__fmul_rn(__fmul_rn(-c.spiky, hd), hd), rinv);
+        const float sc2 = __fmul_rn(sc, sc);
+        if (r2 < c.h2) dens = __fmaf_rn(w, d, dens);
+        if (r2 < c.h2 && r2 > 1e-12f) {
             gx = __fmaf_rn(sc, rx, gx);
             gy = __fmaf_rn(sc, ry, gy);
             gz = __fmaf_rn(sc, rz, gz);
-            gsq = __fmaf_rn(__fmul_rn(sc, sc), r2, gsq);
+            gsq = __fmaf_rn(sc2, r2, gsq);
         }
     }
     __device__ __forceinline__ float lambda(const StepConsts& c) const {
@@ -293,17 +307,17 @@ __device__ __forceinline__ float scorr_pow(float x, uint32_t n) {
 // applies c.delta_scale once to the sum):
 //   (lambda_i + lambda_j - k (W / W(dq))^n) (h - r)^2 / r  r
 // W / W(dq) = d^3 poly6 / W(dq) (c.scorr_pq); the sum of lambdas and s_corr is
-// one fused multiply-add.
+// one fused multiply-add.  No effect unless r2 < h^2.
 template <uint32_t N = 0>
 __device__ __forceinline__ void delta_add(const StepConsts& c, float li, float lj, float rx, float ry,
                                           float rz, float r2, float& dx, float& dy, float& dz) {
-    if (r2 > 1e-12f) {
-        const float d = __fsub_rn(c.h2, r2);
-        const float ratio = __fmul_rn(__fmul_rn(__fmul_rn(d, d), d), c.scorr_pq);
-        const float rinv = rsqrtf(r2);
-        const float hd = fmaxf(__fsub_rn(c.h, __fmul_rn(r2, rinv)), 0.0f);
-        const float coef = __fmul_rn(__fmaf_rn(-c.scorr_k, scorr_pow<N>(ratio, c.scorr_n), __fadd_rn(li, lj)),
-                                     __fmul_rn(__fmul_rn(hd, hd), rinv));
+    const float d = __fsub_rn(c.h2, r2);
+    const float ratio = __fmul_rn(__fmul_rn(__fmul_rn(d, d), d), c.scorr_pq);
+    const float rinv = rsqrt_normal(r2);
+    const float hd = fmaxf(__fsub_rn(c.h, __fmul_rn(r2, rinv)), 0.0f);
+    const float coef = __fmul_rn(__fmaf_rn(-c.scorr_k, scorr_pow<N>(ratio, c.scorr_n), __fadd_rn(li, lj)),
+                                 __fmul_rn(__fmul_rn(hd, hd), rinv));
+    if (r2 < c.h2 && r2 > 1e-12f) {
         dx = __fmaf_rn(coef, rx, dx);
         dy = __fmaf_rn(coef, ry, dy);
         dz = __fmaf_rn(coef, rz, dz);
@@ -314,6 +328,62 @@ __device__ __forceinline__ void delta_add(const StepConsts& c, float li, float l
 // boundary of the quantized positions.
 __device__ __forceinline__ uint32_t row_base(uint32_t b0) { return b0 & ~3u; }
 
+// Offsets of a particle to the three stencil rows along y and along z.
+struct RowOffsets {
+    float y0, y1, y2, z0, z1, z2;
+};
+
+// Per-thread queue of row chunks with candidates to visit, in shared memory:
+// entry e of thread t at (e * BS + t), 8 bytes: the chunk's bits (first
+// candidate in bit 31), and its first slot (a multiple of 4, below 2^30) with the
+// row's y index in bits 0-1 and z index in bits 30-31.  The lanes of a warp have
+// very different numbers of candidates per row but similar totals: walking all
+// rows' bits in one loop, each lane moving to its next chunk by itself with a
+// predicated load, takes 38 iterations where row by row takes 87 (lattice or
+// disordered fluid at rest density, 31 pairs per particle).  k_lambda on the
+// 1,003,520-particle dam break: 214 M -> 150 M warp instructions, 17 -> 25 of 32
+// threads active, 281 -> 184 us; k_delta 161 M -> 95 M, 14 -> 27, 150-171 -> 130 us.
+// 16-byte entries that hold the two offsets instead of the row's indices leave
+// too little of the SM's memory for L1 (k_delta 258 us, 13% hits).
+constexpr uint32_t kQueue = 10;  // 9 rows and a second chunk of one of them
+
+template <uint32_t BS>
+struct PairQueue {
+    uint32_t base;       // shared-memory address of this thread's entry 0
+    uint32_t tail;       // where the next entry goes
+    uint32_t pairs = 0;  // bits in the queue
+
+    __device__ __forceinline__ explicit PairQueue(uint2* shared)
+        : base(uint32_t(__cvta_generic_to_shared(shared + threadIdx.x))), tail(base) {}
+    __device__ __forceinline__ bool full() const { return tail == base + kQueue * BS * 8u; }
+    __device__ __forceinline__ void push(uint32_t mask, uint32_t first, uint32_t y, uint32_t z) {
+        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(tail), "r"(mask), "r"(first | y | (z << 30)));
+        tail += BS * 8u;
+        pairs += __popc(mask);
+    }
+    // visit(slot, oy, oz) for every bit, in the order queued; empties the queue
+    template <class Visit>
+    __device__ __forceinline__ void drain(const RowOffsets& o, Visit&& visit) {
+        uint32_t at = base, mask = 0, first = 0;
+        for (; pairs > 0; --pairs) {
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.eq.u32 p, %0, 0;\n\t"
+                "@p ld.shared.v2.b32 {%0, %1}, [%2];\n\t"
+                "@p add.u32 %2, %2, %3;\n\t}"
+                : "+r"(mask), "+r"(first), "+r"(at)
+                : "n"(BS * 8u));
+            uint32_t t;
+            asm("bfind.shiftamt.u32 %0, %1;" : "=r"(t) : "r"(mask));
+            mask &= 0x7fffffffu >> t;
+            const float oy = (first & 2u) ? o.y2 : ((first & 1u) ? o.y1 : o.y0);
+            const float oz = int(first) < 0 ? o.z2 : ((first & 0x40000000u) ? o.z1 : o.z0);
+            visit((first & 0x3ffffffcu) + t, oy, oz);
+        }
+        tail = base;
+    }
+};
+
 // Two-phase sweep of the 27-cell stencil around cell (cx, cy, cz).  Each row
 // (3 consecutive cells, one contiguous slot range) is taken in chunks of 32
 // candidates.
@@ -323,14 +393,10 @@ __device__ __forceinline__ uint32_t row_base(uint32_t b0) { return b0 & ~3u; }
 // and one funnel shift that collects its sign bit; one 16-byte load brings four
 // candidates.  The threshold admits every pair the exact test could accept
 // (set_prefilter), about 9% more than are in range.  Phase 2 visits just the
-// set bits, loads the candidate's position, applies the exact FP32 test and
-// calls body(k, q, rx, ry, rz, r2), k the candidate's slot; a candidate that
-// fails loses its bit.  So masks, counts and sums are those of the exact test
-// alone.
-// Both passes are bound by instruction issue: testing the FP32 positions took
-// about 12 instructions and a 16-byte load per candidate, this takes 3 and a
-// quarter of one.  On the 1,003,520-particle dam break, k_lambda 286 M -> 214 M
-// warp instructions, 309-327 -> 281 us; the step 2.35 -> 2.16 ms.
+// set bits of all rows, loads the candidate's position and calls
+// body(k, q, rx, ry, rz, r2), k the candidate's slot, in slot order row by row;
+// the body ignores a candidate that fails the exact test r2 < h^2.  So counts
+// and sums are those of the exact test alone.
 //
 // ANCHORED = false: (px, py, pz) is the absolute FP32 position and r = p - q.
 // ANCHORED = true:  (px, py, pz) is the offset l from the anchor (aix, aiy,
@@ -340,38 +406,50 @@ __device__ __forceinline__ uint32_t row_base(uint32_t b0) { return b0 & ~3u; }
 //
 // Every row of the stencil stores the bits of its first chunk (the particle's
 // own bit cleared) for the delta pass, and a row longer than one chunk sets
-// its bit in the overflow word.  Returns the number of in-range candidates
-// other than the particle itself.
-template <bool ANCHORED, class Body>
-__device__ __forceinline__ uint32_t sweep(const StepConsts& c, const float4* __restrict__ src,
-                                          const uint32_t* __restrict__ qsrc,
-                                          const uint32_t* __restrict__ cstart, int cx, int cy, int cz,
-                                          float px, float py, float pz, float aix, float aiy, float aiz,
-                                          uint32_t qi, int nthr, uint32_t s, const RowMasks& masks,
-                                          Body&& body) {
+// its bit in the overflow word.
+template <bool ANCHORED, uint32_t BS, class Body>
+__device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restrict__ src,
+                                      const uint32_t* __restrict__ qsrc,
+                                      const uint32_t* __restrict__ cstart, int cx, int cy, int cz,
+                                      float px, float py, float pz, float aix, float aiy, float aiz,
+                                      uint32_t qi, int nthr, uint32_t s, const RowMasks& masks,
+                                      PairQueue<BS> queue, Body&& body) {
     const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
     const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
     const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
     const int nx = x1 - x0 + 1;
-    uint32_t hits = 0, over = 0;
+    uint32_t over = 0;
     if (nx <= 0) {  // drifted more than a cell outside a scene's sub-grid: no candidates
         for (int z = z0; z <= z1; ++z)
             for (int y = y0; y <= y1; ++y)
                 masks.rows[uint32_t((z - z0) * 3 + (y - y0)) * masks.stride + s] = 0u;
         masks.overflow[s] = 0u;
-        return 0;
+        return;
+    }
+    auto visit = [&](uint32_t k, float oy, float oz) {
+        const float4 q = __ldg(&src[k]);
+        const float ox = ANCHORED ? __fadd_rn(__fsub_rn(aix, q.w), px) : px;
+        const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
+        body(k, q, rx, ry, rz, dist2(rx, ry, rz));
+    };
+    RowOffsets o{py, py, py, pz, pz, pz};
+    if (ANCHORED) {
+        o.y0 = __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y0)), py);
+        o.y1 = __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y0 + 1)), py);
+        o.y2 = __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y0 + 2)), py);
+        o.z0 = __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z0)), pz);
+        o.z1 = __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z0 + 1)), pz);
+        o.z2 = __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z0 + 2)), pz);
     }
     for (int z = z0; z <= z1; ++z) {
-        const float oz = ANCHORED ? __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z)), pz) : pz;
         for (int y = y0; y <= y1; ++y) {
-            const float oy = ANCHORED ? __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y)), py) : py;
             const uint32_t base = cell_hash(c.g, x0, y, z);
             const uint32_t b0 = cstart[base], b3 = cstart[base + uint32_t(nx)];
             const uint32_t a0 = row_base(b0);
             const uint32_t row = uint32_t((z - z0) * 3 + (y - y0));
             uint32_t first = 0;  // bits of the first chunk (the whole row if b3 - a0 <= 32)
             if (b0 < b3) {
-                uint32_t lo = b0 - a0;  // candidates of the chunk before the row
+                uint32_t drop = 0xffffffffu >> (b0 - a0);  // candidates before the row
                 for (uint32_t c0 = a0; c0 < b3; c0 += 32) {
                     const uint32_t c1 = min(c0 + 32u, b3);
                     uint32_t mask = 0, k = c0;
@@ -384,28 +462,17 @@ __device__ __forceinline__ uint32_t sweep(const StepConsts& c, const float4* __r
                         mask = __funnelshift_l(uint32_t(__dp4a(d2, d2, nthr)), mask, 1);
                         mask = __funnelshift_l(uint32_t(__dp4a(d3, d3, nthr)), mask, 1);
                     }
-                    // first candidate in the top of the k - c0 bits: to bit 0;
-                    // then drop what lies outside the row, and the particle itself
-                    mask = __brev(mask) >> (32u - (k - c0));
-                    mask &= (0xffffffffu << lo) & (0xffffffffu >> (32u - (c1 - c0)));
-                    lo = 0;
-                    if (s - c0 < 32u) mask &= ~(1u << (s - c0));
-                    uint32_t todo = mask;
-                    while (todo) {
-                        const uint32_t bit = todo & (0u - todo);
-                        const uint32_t j = c0 + uint32_t(__ffs(todo) - 1);
-                        todo ^= bit;
-                        const float4 q = __ldg(&src[j]);
-                        const float ox = ANCHORED ? __fadd_rn(__fsub_rn(aix, q.w), px) : px;
-                        const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
-                        const float r2 = dist2(rx, ry, rz);
-                        if (r2 < c.h2)
-                            body(j, q, rx, ry, rz, r2);
-                        else
-                            mask ^= bit;
-                    }
-                    hits += __popc(mask);
+                    // the chunk's first candidate to bit 31; drop what lies outside
+                    // the row, and the particle itself
+                    mask <<= 32u - (k - c0);
+                    mask &= drop & (0xffffffffu << (32u - (c1 - c0)));
+                    drop = 0xffffffffu;
+                    if (s - c0 < 32u) mask &= ~(0x80000000u >> (s - c0));
                     if (c0 == a0) first = mask;
+                    if (mask) {
+                        if (queue.full()) queue.drain(o, visit);  // crowded rows only
+                        queue.push(mask, c0, uint32_t(y - y0), uint32_t(z - z0));
+                    }
                 }
                 if (b3 - a0 > 32u) over |= 1u << row;
             }
@@ -413,7 +480,7 @@ __device__ __forceinline__ uint32_t sweep(const StepConsts& c, const float4* __r
         }
     }
     masks.overflow[s] = over;
-    return hits;
+    queue.drain(o, visit);
 }
 
 // The prefilter's arguments of a particle at offset l from the corner of its
@@ -429,7 +496,7 @@ __device__ __forceinline__ int prefilter(const StepConsts& c, int hx, int hy, in
 // First lambda pass: absolute FP32 predicted positions (reference arithmetic,
 // so the fused neighbour count equals countNeighbors bit for bit); converts
 // the state to anchored offsets for the following passes.
-template <bool LAST>
+template <bool LAST, uint32_t BS>
 __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t s,
                                                   const float4* __restrict__ cur,
                                                   const uint32_t* __restrict__ qpos,
@@ -438,7 +505,8 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t 
                                                   const uint32_t* __restrict__ cstart,
                                                   const uint32_t* __restrict__ sidx,
                                                   float* __restrict__ lambdas,
-                                                  uint32_t* __restrict__ ncount, const RowMasks& rm) {
+                                                  uint32_t* __restrict__ ncount, const RowMasks& rm,
+                                                  uint2* queue) {
     const float4 p = cur[s];
     int cx, cy, cz;
     cell_of(c.g, p.x, p.y, p.z, cx, cy, cz);
@@ -452,11 +520,13 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t 
     const int nthr = prefilter(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, lx, ly, lz, qi);
     LambdaAcc acc;
     acc.self(c);
-    const uint32_t cnt = sweep<false>(c, cur, qpos, cstart, cx, cy, cz, p.x, p.y, p.z, 0.0f, 0.0f, 0.0f, qi,
-                                      nthr, s, rm,
-                                      [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
-                                          acc.add(c, rx, ry, rz, r2);
-                                      });
+    uint32_t cnt = 0;
+    sweep<false, BS>(c, cur, qpos, cstart, cx, cy, cz, p.x, p.y, p.z, 0.0f, 0.0f, 0.0f, qi, nthr, s, rm,
+                     PairQueue<BS>(queue),
+                     [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
+                         cnt += r2 < c.h2 ? 1u : 0u;
+                         acc.add(c, rx, ry, rz, r2);
+                     });
     const float lambda = acc.lambda(c);
     nxt[s] = make_float4(lx, ly, lz, lambda);
     scell[s] = cell_local(c.g, cx, cy, cz);
@@ -467,14 +537,14 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t 
 
 // Later lambda passes on the anchored state: cur is the previous delta pass's
 // output, (l, x anchor of the hash cell) per slot.
-template <bool LAST>
+template <bool LAST, uint32_t BS>
 __device__ __forceinline__ void lambda_item(const StepConsts& c, uint32_t s,
                                             const float4* __restrict__ cur,
                                             const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
                                             const uint32_t* __restrict__ scell,
                                             const uint32_t* __restrict__ cstart,
                                             const uint32_t* __restrict__ sidx,
-                                            float* __restrict__ lambdas, const RowMasks& rm) {
+                                            float* __restrict__ lambdas, const RowMasks& rm, uint2* queue) {
     const float4 l = cur[s];
     int pcx, pcy, pcz, cx, cy, cz;
     decode_cell(c.g, scell[s], pcx, pcy, pcz);
@@ -484,10 +554,11 @@ __device__ __forceinline__ void lambda_item(const StepConsts& c, uint32_t s,
     const int nthr = prefilter(c, pcx + c.g.lx, pcy + c.g.ly, pcz + c.g.lz, l.x, l.y, l.z, qi);
     LambdaAcc acc;
     acc.self(c);
-    sweep<true>(c, cur, qpos, cstart, cx, cy, cz, l.x, l.y, l.z, ax, ay, az, qi, nthr, s, rm,
-                [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
-                    acc.add(c, rx, ry, rz, r2);
-                });
+    sweep<true, BS>(c, cur, qpos, cstart, cx, cy, cz, l.x, l.y, l.z, ax, ay, az, qi, nthr, s, rm,
+                    PairQueue<BS>(queue),
+                    [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
+                        acc.add(c, rx, ry, rz, r2);
+                    });
     const float lambda = acc.lambda(c);
     nxt[s] = make_float4(l.x, l.y, l.z, lambda);
     if (LAST) lambdas[sidx[s]] = lambda;
@@ -545,8 +616,8 @@ __device__ __forceinline__ void finalize_particle(const StepConsts& c, uint32_t 
     if (!(isfinite(X + Y + Z) && isfinite(vx + vy + vz))) atomicOr(err, kDevErrNaN);
 }
 
-// The in-range pairs a lambda pass recorded in its row masks (the particle's
-// own bit cleared), walked with the anchored neighbour vector of sweep<true>:
+// The in-range pairs among those a lambda pass recorded in its row masks (the
+// particle's own bit cleared), walked with the anchored neighbour vector of sweep<true>:
 // body(k, q, rx, ry, rz, r2) for each, in sweep<true>'s order (rows in
 // stencil order, slots ascending).  The candidates of a long row past its
 // first chunk are distance-tested again.  (cx, cy, cz): the stencil cell of the
@@ -578,13 +649,16 @@ __device__ __forceinline__ void masked_pairs(const StepConsts& c, const float4* 
             const uint32_t b2 = nx > 1 ? cstart[base + 2] : b1;
             const uint32_t a0 = row_base(b0);
             while (mask) {
-                const uint32_t k = a0 + uint32_t(__ffs(mask) - 1);
-                mask &= mask - 1;
+                uint32_t t;
+                asm("bfind.shiftamt.u32 %0, %1;" : "=r"(t) : "r"(mask));
+                mask &= 0x7fffffffu >> t;
+                const uint32_t k = a0 + t;
                 const float ox = k < b1 ? ox0 : (k < b2 ? ox1 : ox2);
                 const float4 q = __ldg(&src[k]);
                 const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y);
                 const float rz = __fsub_rn(oz, q.z);
-                body(k, q, rx, ry, rz, dist2(rx, ry, rz));
+                const float r2 = dist2(rx, ry, rz);
+                if (r2 < c.h2) body(k, q, rx, ry, rz, r2);
             }
             if (long_row) {
                 const uint32_t b3 = nx > 2 ? cstart[base + 3] : b2;
@@ -601,14 +675,77 @@ __device__ __forceinline__ void masked_pairs(const StepConsts& c, const float4* 
     }
 }
 
+// The pairs a lambda pass recorded in its row masks, through a PairQueue:
+// body(k, q, rx, ry, rz, r2) for each in masked_pairs' order, the ones out of
+// range included.  xa: the x anchor of every slot's hash cell, so that a
+// candidate's neighbour vector does not need the row's cell bounds.
+template <uint32_t BS, class Body>
+__device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* __restrict__ src,
+                                             const float* __restrict__ xa,
+                                             const uint32_t* __restrict__ cstart, const RowMasks& rm,
+                                             uint32_t s, const float4& l, float ax, float ay, float az,
+                                             int cx, int cy, int cz, PairQueue<BS> queue, Body&& body) {
+    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
+    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
+    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
+    const int nx = x1 - x0 + 1;
+    if (nx <= 0) return;
+    const uint32_t longrows = rm.overflow[s];
+    auto visit = [&](uint32_t k, float oy, float oz) {
+        const float4 q = __ldg(&src[k]);
+        const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
+        const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
+        body(k, q, rx, ry, rz, dist2(rx, ry, rz));
+    };
+    const RowOffsets o{__fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0)), l.y),
+                       __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0 + 1)), l.y),
+                       __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0 + 2)), l.y),
+                       __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0)), l.z),
+                       __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0 + 1)), l.z),
+                       __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0 + 2)), l.z)};
+    for (int z = z0; z <= z1; ++z) {
+        for (int y = y0; y <= y1; ++y) {
+            const uint32_t row = uint32_t((z - z0) * 3 + (y - y0));
+            const uint32_t mask = rm.rows[row * rm.stride + s];
+            const bool long_row = (longrows >> row) & 1u;
+            if (mask == 0u && !long_row) continue;
+            const uint32_t base = cell_hash(c.g, x0, y, z);
+            const uint32_t a0 = row_base(cstart[base]);
+            if (mask) {
+                if (queue.full()) queue.drain(o, visit);
+                queue.push(mask, a0, uint32_t(y - y0), uint32_t(z - z0));
+            }
+            if (long_row) {
+                const float oy = __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y)), l.y);
+                const float oz = __fadd_rn(__fsub_rn(az, anchor_z(c.g, z)), l.z);
+                const uint32_t b3 = cstart[base + uint32_t(nx)];
+                for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
+                    uint32_t more = 0;
+                    for (uint32_t k = c0; k < min(c0 + 32u, b3); ++k) {
+                        const float4 q = __ldg(&src[k]);
+                        const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
+                        const float r2 = dist2(__fsub_rn(ox, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
+                        more |= r2 < c.h2 ? 0x80000000u >> (k - c0) : 0u;
+                    }
+                    if (more) {
+                        if (queue.full()) queue.drain(o, visit);
+                        queue.push(more, c0, uint32_t(y - y0), uint32_t(z - z0));
+                    }
+                }
+            }
+        }
+    }
+    queue.drain(o, visit);
+}
+
 // applyDeltaSorted + sphereCollision on the anchored state; the last
 // iteration also scatters back, finalizes and writes foam.  drec (may be
 // NULL): receives the particle's unclamped correction, for the adjoint.
 // SN: the s_corr exponent when fixed at compile time (4), else 0.
-template <bool LAST, uint32_t SN = 0>
+template <bool LAST, uint32_t SN, uint32_t BS>
 __device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
                                            const float4* __restrict__ src, float4* __restrict__ dst,
-                                           uint32_t* __restrict__ qpos,
+                                           uint32_t* __restrict__ qpos, const float* __restrict__ xa,
                                            const uint32_t* __restrict__ scell,
                                            const uint32_t* __restrict__ cstart,
                                            const uint32_t* __restrict__ sidx,
@@ -617,7 +754,7 @@ __device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
                                            const float4* __restrict__ prev,
                                            const uint32_t* __restrict__ ncount,
                                            float* __restrict__ foam, uint32_t* err,
-                                           const RowMasks& rm, float4* __restrict__ drec) {
+                                           const RowMasks& rm, float4* __restrict__ drec, uint2* queue) {
     const float4 l = src[s];
     int pcx, pcy, pcz;
     decode_cell(c.g, scell[s], pcx, pcy, pcz);
@@ -628,7 +765,7 @@ __device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
     auto body = [&](uint32_t, const float4& q, float rx, float ry, float rz, float r2) {
         delta_add<SN>(c, l.w, q.w, rx, ry, rz, r2, dx, dy, dz);
     };
-    masked_pairs(c, src, cstart, rm, s, l, ax, ay, az, cx, cy, cz, body);
+    queued_pairs<BS>(c, src, xa, cstart, rm, s, l, ax, ay, az, cx, cy, cz, PairQueue<BS>(queue), body);
     dx = __fmul_rn(dx, c.delta_scale);
     dy = __fmul_rn(dy, c.delta_scale);
     dz = __fmul_rn(dz, c.delta_scale);

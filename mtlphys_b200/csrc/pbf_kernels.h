@@ -21,6 +21,7 @@ struct DevState {
     uint32_t* tmp;          // unstable cell-grouped order (before the stable fix-up)
     uint32_t* sidx;         // sortedIndex: slot -> particle, stable within a cell
     uint32_t* qpos;         // quantized position per sorted slot (the lambda passes' prefilter)
+    float* xa;              // x anchor of each slot's hash cell
     uint32_t* scell;        // hash cell per sorted slot (anchor of the solver state)
     uint32_t* row_masks;            // 9 x mask_stride in-range bits per stencil row
     uint32_t* mask_overflow;        // bit r: row r does not fit its 32 bits (delta re-tests the rest)

@@ -18,13 +18,12 @@ namespace {
 
 inline uint32_t cdiv(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
-// Launch shape of the solver kernels, measured on the 1M-particle dam break:
-// blocks of 128 threads (slightly ahead of 256 and 512), and a residency
-// target that caps registers at 65536 / (256 * N) -- the lambda passes run
-// best with N = 4 (64 registers), the middle delta passes with N = 6 (40
-// registers and a small spill: 2% ahead of 48 registers, 3% ahead of 32),
-// the last one, which also finalizes in FP64, with N = 6 (40 registers, a
-// small spill).
+// Launch shape of the solver kernels, measured on the 1,003,520-particle dam
+// break: blocks of 128 threads (1473 us per step; 64: 1606, 256: 1605 us with
+// the delta passes at 48 registers, where 128 takes 1599), and a residency
+// target that caps registers at 65536 / (256 * N): N = 4 (64 registers) for all
+// of them (lambda passes at N = 3: 1698, 5: 1636; delta passes at N = 5, which
+// spills: 1599, 6: 1656 us).
 #ifndef MPB_SOLVER_BLOCK
 #define MPB_SOLVER_BLOCK 128
 #endif
@@ -33,10 +32,10 @@ constexpr uint32_t kSB = MPB_SOLVER_BLOCK;
 #define MPB_LAMBDA_MIN_BLOCKS 4
 #endif
 #ifndef MPB_DELTA_MIN_BLOCKS
-#define MPB_DELTA_MIN_BLOCKS 6
+#define MPB_DELTA_MIN_BLOCKS 4
 #endif
 #ifndef MPB_DELTA_MID_MIN_BLOCKS
-#define MPB_DELTA_MID_MIN_BLOCKS 6
+#define MPB_DELTA_MID_MIN_BLOCKS 4
 #endif
 
 template <bool LAST>
@@ -45,8 +44,10 @@ k_lambda_first(StepConsts c, const float4* __restrict__ cur, const uint32_t* __r
                uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
                const uint32_t* __restrict__ sidx, float* __restrict__ lambdas,
                uint32_t* __restrict__ ncount, RowMasks rm) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < c.n) lambda_first_item<LAST>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm);
+    __shared__ uint2 queue[kQueue * kSB];
+    const uint32_t s = blockIdx.x * kSB + threadIdx.x;
+    if (s < c.n)
+        lambda_first_item<LAST, kSB>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm, queue);
 }
 
 template <bool LAST>
@@ -54,8 +55,9 @@ __global__ void __launch_bounds__(kSB, MPB_LAMBDA_MIN_BLOCKS * 256 / kSB)
 k_lambda(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
          const uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
          const uint32_t* __restrict__ sidx, float* __restrict__ lambdas, RowMasks rm) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < c.n) lambda_item<LAST>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm);
+    __shared__ uint2 queue[kQueue * kSB];
+    const uint32_t s = blockIdx.x * kSB + threadIdx.x;
+    if (s < c.n) lambda_item<LAST, kSB>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm, queue);
 }
 
 // SN = 4: the reference's s_corr exponent, fixed at compile time (the host
@@ -63,24 +65,26 @@ k_lambda(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restric
 template <bool LAST, uint32_t SN>
 __global__ void __launch_bounds__(kSB, (LAST ? MPB_DELTA_MIN_BLOCKS : MPB_DELTA_MID_MIN_BLOCKS) * 256 / kSB)
 k_delta(StepConsts c, const float4* __restrict__ src, float4* __restrict__ dst, uint32_t* __restrict__ qpos,
+        const float* __restrict__ xa,
         const uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
         const uint32_t* __restrict__ sidx, const SphereState* __restrict__ sphere,
         float4* __restrict__ pos, float4* __restrict__ vel, const float4* __restrict__ prev,
         const uint32_t* __restrict__ ncount, float* __restrict__ foam, uint32_t* err, RowMasks rm) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint2 queue[kQueue * kSB];
+    const uint32_t s = blockIdx.x * kSB + threadIdx.x;
     if (s < c.n)
-        delta_item<LAST, SN>(c, s, src, dst, qpos, scell, cstart, sidx, sphere, pos, vel, prev, ncount, foam,
-                             err, rm, nullptr);
+        delta_item<LAST, SN, kSB>(c, s, src, dst, qpos, xa, scell, cstart, sidx, sphere, pos, vel, prev, ncount,
+                                  foam, err, rm, nullptr, queue);
 }
 
 template <bool LAST>
 void launch_delta(const StepConsts& c, const DevState& d, const RowMasks& rm, cudaStream_t s) {
     const dim3 grid(cdiv(c.n, kSB));
     if (c.scorr_n == 4)
-        k_delta<LAST, 4><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.scell, d.cstart, d.sidx, d.sphere,
+        k_delta<LAST, 4><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.xa, d.scell, d.cstart, d.sidx, d.sphere,
                                               d.pos, d.vel, d.prev, d.ncount, d.foam, d.err, rm);
     else
-        k_delta<LAST, 0><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.scell, d.cstart, d.sidx, d.sphere,
+        k_delta<LAST, 0><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.xa, d.scell, d.cstart, d.sidx, d.sphere,
                                               d.pos, d.vel, d.prev, d.ncount, d.foam, d.err, rm);
 }
 
