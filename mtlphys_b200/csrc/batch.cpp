@@ -154,7 +154,7 @@ struct mp_batch {
         for (uint32_t c : counts) most = std::max(most, c);
         const uint32_t chunks = (most + kSumChunk - 1) / kSumChunk;
         const size_t accs = al(cap * 8) + al(cap * 32) + al(32 * size_t(chunks) * std::max<uint32_t>(S, 1u));
-        const size_t total = 8 * v4 + 7 * u + gbytes + inbox + ovf + accs;
+        const size_t total = 8 * v4 + 8 * u + gbytes + inbox + ovf + accs;
         MP_ALLOC(adj_block, total, device);
         MP_CUDA(cudaMemset(adj_block, 0, total));
         char* p = static_cast<char*>(adj_block);
@@ -175,6 +175,7 @@ struct mp_batch {
         adj.lam_extra = reinterpret_cast<float*>(w());
         adj.ccur = reinterpret_cast<uint32_t*>(w());
         adj.cpred = reinterpret_cast<uint32_t*>(w());
+        adj.xa = reinterpret_cast<float*>(w());
         adj.inbox_count = reinterpret_cast<uint32_t*>(w());
         adj.ovf_head = reinterpret_cast<uint32_t*>(w());
         MP_CUDA(cudaMemset(adj.ovf_head, 0xff, 4 * cap));  // kNoPost
@@ -196,6 +197,11 @@ struct mp_batch {
         adj.iterations = iterations;
         adj.stride = uint32_t(cap);
         adj.mask_stride = a.mask_stride;
+        for (const mp_pbf_params& p : params) {
+            GridDev g0;
+            make_grid(p, g0);
+            if (g0.dgx > 2045 || g0.dgy > 2045 || g0.dgz > 1021) adj.wide = 1;
+        }
         return MP_OK;
     }
 
@@ -245,6 +251,7 @@ struct mp_batch {
     int enqueue_adjoint(uint32_t i, const float4* x1, cudaStream_t s) {
         const Slot& sl = slots[i];
         AdjArgs ad = adj;
+        ad.scorr4 = a.scorr4;
         ad.t = AdjStep{sl.rec.scenes, sl.rec.sphere0, sl.x0, x1, sl.sidx, sl.scell, sl.cstart,
                        sl.rec.lam, sl.rec.delta, sl.rec.masks, sl.rec.overflow};
         const cudaError_t e = launch_adjoint_step(ad, s);

@@ -48,7 +48,17 @@ __device__ __forceinline__ uint32_t pack_cell(int x, int y, int z) {
 }
 
 // Whether two packed cells are within one cell of each other on every axis.
-__device__ __forceinline__ bool cells_adjacent(uint32_t a, uint32_t b) {
+// With each field's difference plus one in a field of its own, that is every
+// field 0, 1 or 2: no bit above a field's low two, also after adding one more.
+// The fields of the subtraction cannot borrow their way into that unless two
+// cells are 2046 (x, y) or 1023 (z) apart; `wide` grids, which reach that far,
+// compare axis by axis.
+__device__ __forceinline__ bool cells_adjacent(uint32_t a, uint32_t b, bool wide) {
+    if (!wide) {
+        constexpr uint32_t one = 1u | (1u << 11) | (1u << 22), low2 = 3u * one;
+        const uint32_t d = a - (b - one);
+        return ((d | (d + one)) & ~low2) == 0u;
+    }
     const int dx = int(a & 0x7ffu) - int(b & 0x7ffu);
     const int dy = int((a >> 11) & 0x7ffu) - int((b >> 11) & 0x7ffu);
     const int dz = int(a >> 22) - int(b >> 22);
@@ -58,11 +68,16 @@ __device__ __forceinline__ bool cells_adjacent(uint32_t a, uint32_t b) {
 // Kernel values of a pair at offset r with 1e-12 < |r|^2 = r2 < h^2:
 // spiky gradient g = f r, its Jacobian H v = f v + fp (r . v) r, the poly6
 // weight W and d = h^2 - r2 (grad W = -6 poly6 d^2 r).
+struct PairConsts {
+    float h, h2, poly6, spiky;
+    __device__ __forceinline__ explicit PairConsts(const StepConsts& c)
+        : h(c.h), h2(c.h2), poly6(c.poly6), spiky(c.spiky) {}
+};
 struct PairTerms {
     float d, f, fp, W;
-    __device__ __forceinline__ PairTerms(const StepConsts& c, float r2) {
+    __device__ __forceinline__ PairTerms(const PairConsts& c, float r2) {
         d = c.h2 - r2;
-        const float rinv = rsqrtf(r2);
+        const float rinv = rsqrt_normal(r2);
         const float hd = fmaxf(c.h - r2 * rinv, 0.0f);
         f = -c.spiky * hd * hd * rinv;
         fp = c.spiky * d * rinv * rinv * rinv;
@@ -75,7 +90,11 @@ struct PairTerms {
     }
 };
 
+// x^n; N = 4 is s_corr's exponent fixed at compile time (n - 1 = 3), with the
+// roundings of the loop.
+template <uint32_t N>
 __device__ __forceinline__ float pow_u(float x, uint32_t n) {
+    if (N == 4u) return x * x * x;
     float r = 1.0f;
     for (uint32_t e = 0; e < n; ++e) r *= x;
     return r;
@@ -116,6 +135,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_finalize(AdjArgs a) {
     int px, py, pz;
     decode_cell(c.g, cell, px, py, pz);
     a.cpred[s] = pack_cell(px + c.g.lx, py + c.g.ly, pz + c.g.lz);
+    a.xa[s] = anchor_x(c.g, px);
     const double X[3] = {X4.x, X4.y, X4.z}, P[3] = {P4.x, P4.y, P4.z};
     const double lo_b[3] = {c.bminx, c.bminy, c.bminz}, hi_b[3] = {c.bmaxx, c.bmaxy, c.bmaxz};
     const double kd = double(c.damping) / double(c.dt);
@@ -236,89 +256,90 @@ __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
 // (dbar_j and the j-side terms only for pairs in both lists; the j-side
 // terms of a one-way pair are added to j atomically), and the particle's
 // density sums for the lambda adjoint.
-// The two pair sweeps are compiled for 4 resident blocks per SM (64
-// registers): left alone they take ~90 and run 13-16% slower.
+// Both pair sweeps walk their pairs through a PairQueue (pbf_items.cuh), one
+// loop per slot instead of one per stencil row (10 -> 26 of 32 threads active),
+// and keep the scene's constants in registers.  Bound by issue and load latency.
+// 6 blocks of 128 per SM (80 registers, a small spill): gradient of 10 steps of
+// the 97,336-particle cube, forward included, 9.4 -> 7.6 ms (4 blocks: 8.8, 5:
+// 8.4, 8: 7.8 ms).
 #ifndef MPB_ADJ_SWEEP_MIN_BLOCKS
-#define MPB_ADJ_SWEEP_MIN_BLOCKS 4
+#define MPB_ADJ_SWEEP_MIN_BLOCKS 6
 #endif
 constexpr int kSweepMinBlocks = MPB_ADJ_SWEEP_MIN_BLOCKS;
+constexpr uint32_t kSweepBlock = 128;
 
-__global__ void __launch_bounds__(kBlock, kSweepMinBlocks) k_adj_delta(AdjArgs a, uint32_t it) {
-    const uint32_t m = blockIdx.x * kBlock + threadIdx.x;
-    float kb = 0.0f;
-    if (m < a.n) {
-        const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
-        const size_t off = size_t(it) * a.stride;
-        const float4* src = a.t.lam + off;
-        const float4 l = src[m];
-        const float4 dm = a.dbar[m];
-        const uint32_t pm = a.cpred[m];
-        int pcx, pcy, pcz;
-        decode_cell(c.g, a.t.scell[m], pcx, pcy, pcz);
-        const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
-        int cx, cy, cz;
-        cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
-        const float h2 = c.h2;
-        float dens = c.poly6 * h2 * h2 * h2;  // the particle itself
-        float gx = 0.0f, gy = 0.0f, gz = 0.0f, gsq = 0.0f;
-        float lb = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
-        const uint32_t n = c.scorr_n;
-        const float sgk = n ? 6.0f * c.scorr_k * float(n) * c.inv_wq * c.poly6 : 0.0f;
-        auto body = [&](uint32_t k, const float4& q, float rx, float ry, float rz, float r2) {
-            if (k == m) return;
-            if (!(r2 > 1e-12f)) {
-                dens += c.poly6 * (h2 - r2) * (h2 - r2) * (h2 - r2);
-                return;
-            }
-            const PairTerms t(c, r2);
-            dens += t.W;
-            const float fx = t.f * rx, fy = t.f * ry, fz = t.f * rz;  // g
-            gx += fx;
-            gy += fy;
-            gz += fz;
-            gsq += t.f * t.f * r2;
-            const float ratio = t.W * c.inv_wq;
-            const float rn1 = n ? pow_u(ratio, n - 1) : 0.0f;
-            const float rn = n ? rn1 * ratio : 1.0f;
-            const float coef = l.w + q.w - c.scorr_k * rn;
-            const float sg = sgk * rn1 * t.d * t.d;  // grad s_ij = sg r
-            const float gdm = fx * dm.x + fy * dm.y + fz * dm.z;
-            kb -= rn * gdm;
-            if (cells_adjacent(a.ccur[k], pm)) {
-                const float4 di = a.dbar[k];
-                const float ex = dm.x - di.x, ey = dm.y - di.y, ez = dm.z - di.z;
-                const float gdd = fx * ex + fy * ey + fz * ez;
-                lb += gdd;
-                const float3 hv = t.hess(rx, ry, rz, ex, ey, ez);
-                px += coef * hv.x + sg * gdd * rx;
-                py += coef * hv.y + sg * gdd * ry;
-                pz += coef * hv.z + sg * gdd * rz;
-            } else {
-                lb += gdm;
-                const float3 hv = t.hess(rx, ry, rz, dm.x, dm.y, dm.z);
-                const float vx = coef * hv.x + sg * gdm * rx;
-                const float vy = coef * hv.y + sg * gdm * ry;
-                const float vz = coef * hv.z + sg * gdm * rz;
-                px += vx;
-                py += vy;
-                pz += vz;
-                post(a, k, m,
-                     make_float4(-vx * c.inv_rho0, -vy * c.inv_rho0, -vz * c.inv_rho0, gdm * c.inv_rho0));
-            }
-        };
-        const uint32_t ms = a.mask_stride;
-        const RowMasks rm{const_cast<uint32_t*>(a.t.masks) + size_t(it) * 9 * ms,
-                          const_cast<uint32_t*>(a.t.overflow) + size_t(it) * ms, ms};
-        masked_pairs(c, src, a.t.cstart, rm, m, l, ax, ay, az, cx, cy, cz, body);
-        const float ir = c.inv_rho0;
-        const float4 qb = a.qbar[m];
-        a.qbar[m] = make_float4(qb.x + px * ir, qb.y + py * ir, qb.z + pz * ir, 0.0f);
-        a.lam_part[m] = lb * ir;
-        const float D = ir * ir * (gx * gx + gy * gy + gz * gz + gsq) + c.eps;
-        a.gd[m] = make_float4(gx, gy, gz, D);
-        kb *= ir;
-        a.kacc[m] += double(kb);  // this slot's share of dL/dk
-    }
+template <uint32_t SN>
+__global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjArgs a, uint32_t it) {
+    __shared__ uint2 queue[kQueue * kSweepBlock];
+    const uint32_t m = blockIdx.x * kSweepBlock + threadIdx.x;
+    if (m >= a.n) return;
+    const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
+    const size_t off = size_t(it) * a.stride;
+    const float4* src = a.t.lam + off;
+    const float4 l = src[m];
+    const float4 dm = a.dbar[m];
+    const uint32_t pm = a.cpred[m];
+    int pcx, pcy, pcz;
+    decode_cell(c.g, a.t.scell[m], pcx, pcy, pcz);
+    const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
+    int cx, cy, cz;
+    cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
+    // kept in registers: a post would otherwise make every pair load them again
+    const PairConsts pc(c);
+    const float inv_wq = c.inv_wq, scorr_k = c.scorr_k, ir = c.inv_rho0;
+    const uint32_t n = SN ? SN : c.scorr_n;
+    float dens = pc.poly6 * pc.h2 * pc.h2 * pc.h2;  // the particle itself
+    float gx = 0.0f, gy = 0.0f, gz = 0.0f, gsq = 0.0f;
+    float lb = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f, kb = 0.0f;
+    const float sgk = n ? 6.0f * scorr_k * float(n) * inv_wq * pc.poly6 : 0.0f;
+    auto body = [&](uint32_t k, const float4& q, float rx, float ry, float rz, float r2) {
+        if (!(r2 < pc.h2)) return;
+        if (!(r2 > 1e-12f)) {
+            dens += pc.poly6 * (pc.h2 - r2) * (pc.h2 - r2) * (pc.h2 - r2);
+            return;
+        }
+        const uint32_t cell = __ldg(&a.ccur[k]);
+        const float4 di = __ldg(&a.dbar[k]);
+        const PairTerms t(pc, r2);
+        dens += t.W;
+        const float fx = t.f * rx, fy = t.f * ry, fz = t.f * rz;  // g
+        gx += fx;
+        gy += fy;
+        gz += fz;
+        gsq += t.f * t.f * r2;
+        const float ratio = t.W * inv_wq;
+        const float rn1 = n ? pow_u<SN>(ratio, n - 1) : 0.0f;
+        const float rn = n ? rn1 * ratio : 1.0f;
+        const float coef = l.w + q.w - scorr_k * rn;
+        const float sg = sgk * rn1 * t.d * t.d;  // grad s_ij = sg r
+        kb -= rn * (fx * dm.x + fy * dm.y + fz * dm.z);
+        // a pair in both lists carries the other particle's terms too; a
+        // one-way pair owes it the negative of its own
+        const bool both = cells_adjacent(cell, pm, a.wide);
+        const float ex = dm.x - (both ? di.x : 0.0f), ey = dm.y - (both ? di.y : 0.0f);
+        const float ez = dm.z - (both ? di.z : 0.0f);
+        const float gdd = fx * ex + fy * ey + fz * ez;
+        const float3 hv = t.hess(rx, ry, rz, ex, ey, ez);
+        const float vx = coef * hv.x + sg * gdd * rx;
+        const float vy = coef * hv.y + sg * gdd * ry;
+        const float vz = coef * hv.z + sg * gdd * rz;
+        lb += gdd;
+        px += vx;
+        py += vy;
+        pz += vz;
+        if (!both) post(a, k, m, make_float4(-vx * ir, -vy * ir, -vz * ir, gdd * ir));
+    };
+    const uint32_t ms = a.mask_stride;
+    const RowMasks rm{const_cast<uint32_t*>(a.t.masks) + size_t(it) * 9 * ms,
+                      const_cast<uint32_t*>(a.t.overflow) + size_t(it) * ms, ms};
+    queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, rm, m, l, ax, ay, az, cx, cy, cz,
+                              PairQueue<kSweepBlock>(queue), body);
+    const float4 qb = a.qbar[m];
+    a.qbar[m] = make_float4(qb.x + px * ir, qb.y + py * ir, qb.z + pz * ir, 0.0f);
+    a.lam_part[m] = lb * ir;
+    const float D = ir * ir * (gx * gx + gy * gy + gz * gz + gsq) + c.eps;
+    a.gd[m] = make_float4(gx, gy, gz, D);
+    a.kacc[m] += double(kb * ir);  // this slot's share of dL/dk
 }
 
 // dL/d(density sum, gradient sum, squared-gradient sum) of each particle's
@@ -345,8 +366,9 @@ __global__ void __launch_bounds__(kBlock) k_adj_lbar(AdjArgs a, uint32_t it) {
 //   pbar_i += sum_j (rhobar_i + rhobar_j) grad W_ij
 //             + H_ij (Gbar_i - Gbar_j + 2 (Qbar_i + Qbar_j) g_ij)
 // (j-side terms of one-way pairs added to j atomically).
-__global__ void __launch_bounds__(kBlock, kSweepMinBlocks) k_adj_lambda(AdjArgs a, uint32_t it) {
-    const uint32_t m = blockIdx.x * kBlock + threadIdx.x;
+__global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(AdjArgs a, uint32_t it) {
+    __shared__ uint2 queue[kQueue * kSweepBlock];
+    const uint32_t m = blockIdx.x * kSweepBlock + threadIdx.x;
     if (m >= a.n) return;
     const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
     const size_t off = size_t(it) * a.stride;
@@ -362,35 +384,31 @@ __global__ void __launch_bounds__(kBlock, kSweepMinBlocks) k_adj_lambda(AdjArgs 
     cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
     const float4 qb = a.qbar[m];
     float px = qb.x, py = qb.y, pz = qb.z;
-    const float w6 = -6.0f * c.poly6;
+    const PairConsts pc(c);
+    const float w6 = -6.0f * pc.poly6;
     auto body = [&](uint32_t k, const float4&, float rx, float ry, float rz, float r2) {
-        if (k == m || !(r2 > 1e-12f)) return;
-        const PairTerms t(c, r2);
+        if (!(r2 < pc.h2 && r2 > 1e-12f)) return;
+        const uint32_t cell = __ldg(&a.ccur[k]);
+        const float4 li = __ldg(&a.lbar[k]);
+        const float qi = __ldg(&a.qsc[k]);
+        const PairTerms t(pc, r2);
         const float gw = w6 * t.d * t.d;  // grad W = gw r
-        if (cells_adjacent(a.ccur[k], pm)) {
-            const float4 li = a.lbar[k];
-            const float qs = 2.0f * (qm + a.qsc[k]) * t.f;
-            const float3 hv = t.hess(rx, ry, rz, lm.x - li.x + qs * rx, lm.y - li.y + qs * ry,
-                                     lm.z - li.z + qs * rz);
-            const float w = (lm.w + li.w) * gw;
-            px += w * rx + hv.x;
-            py += w * ry + hv.y;
-            pz += w * rz + hv.z;
-        } else {
-            const float qs = 2.0f * qm * t.f;
-            const float3 hv = t.hess(rx, ry, rz, lm.x + qs * rx, lm.y + qs * ry, lm.z + qs * rz);
-            const float w = lm.w * gw;
-            const float vx = w * rx + hv.x, vy = w * ry + hv.y, vz = w * rz + hv.z;
-            px += vx;
-            py += vy;
-            pz += vz;
-            post(a, k, m, make_float4(-vx, -vy, -vz, 0.0f));
-        }
+        const bool both = cells_adjacent(cell, pm, a.wide);
+        const float qs = 2.0f * (qm + (both ? qi : 0.0f)) * t.f;
+        const float3 hv = t.hess(rx, ry, rz, lm.x - (both ? li.x : 0.0f) + qs * rx,
+                                 lm.y - (both ? li.y : 0.0f) + qs * ry, lm.z - (both ? li.z : 0.0f) + qs * rz);
+        const float w = (lm.w + (both ? li.w : 0.0f)) * gw;
+        const float vx = w * rx + hv.x, vy = w * ry + hv.y, vz = w * rz + hv.z;
+        px += vx;
+        py += vy;
+        pz += vz;
+        if (!both) post(a, k, m, make_float4(-vx, -vy, -vz, 0.0f));
     };
     const uint32_t ms = a.mask_stride;
     const RowMasks rm{const_cast<uint32_t*>(a.t.masks) + size_t(it) * 9 * ms,
                       const_cast<uint32_t*>(a.t.overflow) + size_t(it) * ms, ms};
-    masked_pairs(c, src, a.t.cstart, rm, m, l, ax, ay, az, cx, cy, cz, body);
+    queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, rm, m, l, ax, ay, az, cx, cy, cz,
+                              PairQueue<kSweepBlock>(queue), body);
     a.pbar[m] = make_float4(px, py, pz, 0.0f);
 }
 
@@ -601,14 +619,17 @@ __global__ void __launch_bounds__(128) k_adj_sphere(AdjArgs a) {
 
 cudaError_t launch_adjoint_step(const AdjArgs& a, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
-    const uint32_t grid = cdiv(a.n, kBlock);
+    const uint32_t grid = cdiv(a.n, kBlock), sweep_grid = cdiv(a.n, kSweepBlock);
     k_adj_finalize<<<grid, kBlock, 0, s>>>(a);
     for (uint32_t it = a.iterations; it-- > 0;) {
         k_adj_pre<<<grid, kBlock, 0, s>>>(a, it);
-        k_adj_delta<<<grid, kBlock, 0, s>>>(a, it);
+        if (a.scorr4)
+            k_adj_delta<4><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
+        else
+            k_adj_delta<0><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         k_adj_deliver<true><<<grid, kBlock, 0, s>>>(a);
         k_adj_lbar<<<grid, kBlock, 0, s>>>(a, it);
-        k_adj_lambda<<<grid, kBlock, 0, s>>>(a, it);
+        k_adj_lambda<<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         k_adj_deliver<false><<<grid, kBlock, 0, s>>>(a);
     }
     k_adj_predict<<<grid, kBlock, 0, s>>>(a);

@@ -55,6 +55,9 @@ struct AdjArgs {
     float4 *pbar, *qbar, *dbar, *lbar, *gd, *p_extra;
     float *qsc, *lam_part, *lam_extra;
     uint32_t *ccur, *cpred;
+    float* xa;                    // x anchor of each slot's hash cell
+    uint32_t wide;                // 1: some scene's grid is too wide for the packed cell comparison
+    uint32_t scorr4;              // 1: every scene's s_corr exponent is 4
     // one-way pair posts: per receiver slot a count and kInbox (sender,
     // value) entries (entry e of receiver j at e * stride + j); further posts
     // take pooled entries (sender, value, next) linked from ovf_head[j]

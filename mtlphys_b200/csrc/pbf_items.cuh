@@ -616,69 +616,14 @@ __device__ __forceinline__ void finalize_particle(const StepConsts& c, uint32_t 
     if (!(isfinite(X + Y + Z) && isfinite(vx + vy + vz))) atomicOr(err, kDevErrNaN);
 }
 
-// The in-range pairs among those a lambda pass recorded in its row masks (the
-// particle's own bit cleared), walked with the anchored neighbour vector of sweep<true>:
-// body(k, q, rx, ry, rz, r2) for each, in sweep<true>'s order (rows in
-// stencil order, slots ascending).  The candidates of a long row past its
-// first chunk are distance-tested again.  (cx, cy, cz): the stencil cell of the
-// particle at offset l from anchor (ax, ay, az).
-template <class Body>
-__device__ __forceinline__ void masked_pairs(const StepConsts& c, const float4* __restrict__ src,
-                                             const uint32_t* __restrict__ cstart, const RowMasks& rm,
-                                             uint32_t s, const float4& l, float ax, float ay, float az,
-                                             int cx, int cy, int cz, Body&& body) {
-    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
-    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
-    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
-    const int nx = x1 - x0 + 1;
-    if (nx <= 0) return;
-    const uint32_t longrows = rm.overflow[s];
-    const float ox0 = __fadd_rn(__fsub_rn(ax, anchor_x(c.g, x0)), l.x);
-    const float ox1 = __fadd_rn(__fsub_rn(ax, anchor_x(c.g, x0 + 1)), l.x);
-    const float ox2 = __fadd_rn(__fsub_rn(ax, anchor_x(c.g, x0 + 2)), l.x);
-    for (int z = z0; z <= z1; ++z) {
-        const float oz = __fadd_rn(__fsub_rn(az, anchor_z(c.g, z)), l.z);
-        for (int y = y0; y <= y1; ++y) {
-            const uint32_t row = uint32_t((z - z0) * 3 + (y - y0));
-            uint32_t mask = rm.rows[row * rm.stride + s];
-            const bool long_row = (longrows >> row) & 1u;
-            if (mask == 0u && !long_row) continue;
-            const float oy = __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y)), l.y);
-            const uint32_t base = cell_hash(c.g, x0, y, z);
-            const uint32_t b0 = cstart[base], b1 = cstart[base + 1];
-            const uint32_t b2 = nx > 1 ? cstart[base + 2] : b1;
-            const uint32_t a0 = row_base(b0);
-            while (mask) {
-                uint32_t t;
-                asm("bfind.shiftamt.u32 %0, %1;" : "=r"(t) : "r"(mask));
-                mask &= 0x7fffffffu >> t;
-                const uint32_t k = a0 + t;
-                const float ox = k < b1 ? ox0 : (k < b2 ? ox1 : ox2);
-                const float4 q = __ldg(&src[k]);
-                const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y);
-                const float rz = __fsub_rn(oz, q.z);
-                const float r2 = dist2(rx, ry, rz);
-                if (r2 < c.h2) body(k, q, rx, ry, rz, r2);
-            }
-            if (long_row) {
-                const uint32_t b3 = nx > 2 ? cstart[base + 3] : b2;
-                for (uint32_t k = a0 + 32u; k < b3; ++k) {
-                    const float ox = k < b1 ? ox0 : (k < b2 ? ox1 : ox2);
-                    const float4 q = __ldg(&src[k]);
-                    const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y);
-                    const float rz = __fsub_rn(oz, q.z);
-                    const float r2 = dist2(rx, ry, rz);
-                    if (r2 < c.h2) body(k, q, rx, ry, rz, r2);
-                }
-            }
-        }
-    }
-}
-
-// The pairs a lambda pass recorded in its row masks, through a PairQueue:
-// body(k, q, rx, ry, rz, r2) for each in masked_pairs' order, the ones out of
-// range included.  xa: the x anchor of every slot's hash cell, so that a
-// candidate's neighbour vector does not need the row's cell bounds.
+// The pairs a lambda pass recorded in its row masks (the particle's own bit
+// cleared), walked through a PairQueue with the neighbour vector of sweep<true>:
+// body(k, q, rx, ry, rz, r2) for each, the ones out of range included, in
+// sweep<true>'s order (rows in stencil order, slots ascending).  The candidates
+// of a long row past its first chunk are distance-tested again.  (cx, cy, cz):
+// the stencil cell of the particle at offset l from anchor (ax, ay, az).  xa: the
+// x anchor of every slot's hash cell, so that a candidate's neighbour vector does
+// not need the row's cell bounds.
 template <uint32_t BS, class Body>
 __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* __restrict__ src,
                                              const float* __restrict__ xa,
@@ -725,7 +670,7 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
                         const float4 q = __ldg(&src[k]);
                         const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
                         const float r2 = dist2(__fsub_rn(ox, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
-                        more |= r2 < c.h2 ? 0x80000000u >> (k - c0) : 0u;
+                        more |= r2 < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
                     }
                     if (more) {
                         if (queue.full()) queue.drain(o, visit);
