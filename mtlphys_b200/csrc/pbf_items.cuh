@@ -308,15 +308,20 @@ __device__ __forceinline__ float scorr_pow(float x, uint32_t n) {
 //   (lambda_i + lambda_j - k (W / W(dq))^n) (h - r)^2 / r  r
 // W / W(dq) = d^3 poly6 / W(dq) (c.scorr_pq); the sum of lambdas and s_corr is
 // one fused multiply-add.  No effect unless r2 < h^2.
-template <uint32_t N = 0>
-__device__ __forceinline__ void delta_add(const StepConsts& c, float li, float lj, float rx, float ry,
-                                          float rz, float r2, float& dx, float& dy, float& dz) {
+template <uint32_t N>
+__device__ __forceinline__ float delta_coef(const StepConsts& c, float li, float lj, float r2) {
     const float d = __fsub_rn(c.h2, r2);
     const float ratio = __fmul_rn(__fmul_rn(__fmul_rn(d, d), d), c.scorr_pq);
     const float rinv = rsqrt_normal(r2);
     const float hd = fmaxf(__fsub_rn(c.h, __fmul_rn(r2, rinv)), 0.0f);
-    const float coef = __fmul_rn(__fmaf_rn(-c.scorr_k, scorr_pow<N>(ratio, c.scorr_n), __fadd_rn(li, lj)),
-                                 __fmul_rn(__fmul_rn(hd, hd), rinv));
+    return __fmul_rn(__fmaf_rn(-c.scorr_k, scorr_pow<N>(ratio, c.scorr_n), __fadd_rn(li, lj)),
+                     __fmul_rn(__fmul_rn(hd, hd), rinv));
+}
+
+template <uint32_t N>
+__device__ __forceinline__ void delta_add(const StepConsts& c, float li, float lj, float rx, float ry,
+                                          float rz, float r2, float& dx, float& dy, float& dz) {
+    const float coef = delta_coef<N>(c, li, lj, r2);
     if (r2 < c.h2 && r2 > 1e-12f) {
         dx = __fmaf_rn(coef, rx, dx);
         dy = __fmaf_rn(coef, ry, dy);
@@ -683,34 +688,20 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
     queue.drain(o, visit);
 }
 
-// applyDeltaSorted + sphereCollision on the anchored state; the last
-// iteration also scatters back, finalizes and writes foam.  drec (may be
-// NULL): receives the particle's unclamped correction, for the adjoint.
-// SN: the s_corr exponent when fixed at compile time (4), else 0.
-template <bool LAST, uint32_t SN, uint32_t BS>
-__device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
-                                           const float4* __restrict__ src, float4* __restrict__ dst,
-                                           uint32_t* __restrict__ qpos, const float* __restrict__ xa,
-                                           const uint32_t* __restrict__ scell,
-                                           const uint32_t* __restrict__ cstart,
-                                           const uint32_t* __restrict__ sidx,
-                                           const SphereState* __restrict__ sphere,
-                                           float4* __restrict__ pos, float4* __restrict__ vel,
-                                           const float4* __restrict__ prev,
-                                           const uint32_t* __restrict__ ncount,
-                                           float* __restrict__ foam, uint32_t* err,
-                                           const RowMasks& rm, float4* __restrict__ drec, uint2* queue) {
-    const float4 l = src[s];
-    int pcx, pcy, pcz;
-    decode_cell(c.g, scell[s], pcx, pcy, pcz);
-    const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
-    int cx, cy, cz;
-    cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
-    float dx = 0.0f, dy = 0.0f, dz = 0.0f;
-    auto body = [&](uint32_t, const float4& q, float rx, float ry, float rz, float r2) {
-        delta_add<SN>(c, l.w, q.w, rx, ry, rz, r2, dx, dy, dz);
-    };
-    queued_pairs<BS>(c, src, xa, cstart, rm, s, l, ax, ay, az, cx, cy, cz, PairQueue<BS>(queue), body);
+// The position update of one particle whose pair sums are (dx, dy, dz): box
+// clamp and sphere push in FP64; the last iteration also scatters back, finalizes
+// and writes foam.  drec (may be NULL): receives the unclamped correction, for
+// the adjoint.
+template <bool LAST>
+__device__ __forceinline__ void delta_apply(const StepConsts& c, uint32_t s, const float4& l, float ax, float ay,
+                                            float az, int pcx, int pcy, int pcz, float dx, float dy, float dz,
+                                            float4* __restrict__ dst, uint32_t* __restrict__ qpos,
+                                            const uint32_t* __restrict__ sidx,
+                                            const SphereState* __restrict__ sphere,
+                                            float4* __restrict__ pos, float4* __restrict__ vel,
+                                            const float4* __restrict__ prev,
+                                            const uint32_t* __restrict__ ncount, float* __restrict__ foam,
+                                            uint32_t* err, float4* __restrict__ drec) {
     dx = __fmul_rn(dx, c.delta_scale);
     dy = __fmul_rn(dy, c.delta_scale);
     dz = __fmul_rn(dz, c.delta_scale);
@@ -750,6 +741,38 @@ __device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
         return;
     }
     finalize_particle(c, sidx[s], X, Y, Z, pos, vel, prev, ncount, foam, err);
+}
+
+// applyDeltaSorted + sphereCollision on the anchored state; the last
+// iteration also scatters back, finalizes and writes foam.  drec (may be
+// NULL): receives the particle's unclamped correction, for the adjoint.
+// SN: the s_corr exponent when fixed at compile time (4), else 0.
+template <bool LAST, uint32_t SN, uint32_t BS>
+__device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
+                                           const float4* __restrict__ src, float4* __restrict__ dst,
+                                           uint32_t* __restrict__ qpos, const float* __restrict__ xa,
+                                           const uint32_t* __restrict__ scell,
+                                           const uint32_t* __restrict__ cstart,
+                                           const uint32_t* __restrict__ sidx,
+                                           const SphereState* __restrict__ sphere,
+                                           float4* __restrict__ pos, float4* __restrict__ vel,
+                                           const float4* __restrict__ prev,
+                                           const uint32_t* __restrict__ ncount,
+                                           float* __restrict__ foam, uint32_t* err,
+                                           const RowMasks& rm, float4* __restrict__ drec, uint2* queue) {
+    const float4 l = src[s];
+    int pcx, pcy, pcz;
+    decode_cell(c.g, scell[s], pcx, pcy, pcz);
+    const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
+    int cx, cy, cz;
+    cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
+    float dx = 0.0f, dy = 0.0f, dz = 0.0f;
+    auto body = [&](uint32_t, const float4& q, float rx, float ry, float rz, float r2) {
+        delta_add<SN>(c, l.w, q.w, rx, ry, rz, r2, dx, dy, dz);
+    };
+    queued_pairs<BS>(c, src, xa, cstart, rm, s, l, ax, ay, az, cx, cy, cz, PairQueue<BS>(queue), body);
+    delta_apply<LAST>(c, s, l, ax, ay, az, pcx, pcy, pcz, dx, dy, dz, dst, qpos, sidx, sphere, pos, vel, prev,
+                      ncount, foam, err, drec);
 }
 
 // Zero solver iterations: scatter-back + finalize + foam of the predicted

@@ -101,6 +101,11 @@ cudaError_t launch_count_neighbors(const StepConsts& c, const DevState& d, cudaS
 cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t iterations,
                           cudaStream_t s, KernelTimer* t = nullptr);
 
+// Lanes per particle of the solver passes of n particles (pbf_team.cuh): kTeam,
+// or 0 for one lane each.
+constexpr uint32_t kTeam = 16;
+uint32_t team_lanes(uint32_t n);
+
 // Number of kernel launches one step issues (for the benchmark's count).
 uint32_t step_launch_count(uint32_t iterations);
 

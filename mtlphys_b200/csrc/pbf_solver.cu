@@ -11,7 +11,7 @@
 //   delta          sorted_b (l, lambda) -> sorted_a (l')
 //   lambda         sorted_a (l) -> sorted_b (l, lambda)
 //   last delta     also scatter-back + finalize + foam into original order.
-#include "pbf_items.cuh"
+#include "pbf_team.cuh"
 
 namespace mpb {
 namespace {
@@ -77,15 +77,102 @@ k_delta(StepConsts c, const float4* __restrict__ src, float4* __restrict__ dst, 
                                   foam, err, rm, nullptr, queue);
 }
 
-template <bool LAST>
-void launch_delta(const StepConsts& c, const DevState& d, const RowMasks& rm, cudaStream_t s) {
-    const dim3 grid(cdiv(c.n, kSB));
-    if (c.scorr_n == 4)
-        k_delta<LAST, 4><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.xa, d.scell, d.cstart, d.sidx, d.sphere,
-                                              d.pos, d.vel, d.prev, d.ncount, d.foam, d.err, rm);
+// The same with a team of G lanes per slot (pbf_team.cuh).
+constexpr uint32_t kTB = 64;
+
+template <bool LAST, uint32_t G>
+__global__ void __launch_bounds__(kTB)
+k_lambda_first_team(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restrict__ qpos,
+                    float4* __restrict__ nxt, uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
+                    const uint32_t* __restrict__ sidx, float* __restrict__ lambdas,
+                    uint32_t* __restrict__ ncount, RowMasks rm) {
+    __shared__ TeamBuf bufs[kTB / G];
+    const uint32_t s = (blockIdx.x * kTB + threadIdx.x) / G;
+    if (s < c.n)
+        team_lambda_first<LAST, G>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm, bufs);
+}
+
+template <bool LAST, uint32_t G>
+__global__ void __launch_bounds__(kTB)
+k_lambda_team(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restrict__ qpos,
+              float4* __restrict__ nxt, const uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
+              const uint32_t* __restrict__ sidx, float* __restrict__ lambdas, RowMasks rm) {
+    __shared__ TeamBuf bufs[kTB / G];
+    const uint32_t s = (blockIdx.x * kTB + threadIdx.x) / G;
+    if (s < c.n) team_lambda<LAST, G>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm, bufs);
+}
+
+template <bool LAST, uint32_t SN, uint32_t G>
+__global__ void __launch_bounds__(kTB)
+k_delta_team(StepConsts c, const float4* __restrict__ src, float4* __restrict__ dst, uint32_t* __restrict__ qpos,
+             const float* __restrict__ xa, const uint32_t* __restrict__ scell,
+             const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ sidx,
+             const SphereState* __restrict__ sphere, float4* __restrict__ pos, float4* __restrict__ vel,
+             const float4* __restrict__ prev, const uint32_t* __restrict__ ncount, float* __restrict__ foam,
+             uint32_t* err, RowMasks rm) {
+    __shared__ TeamBuf bufs[kTB / G];
+    const uint32_t s = (blockIdx.x * kTB + threadIdx.x) / G;
+    if (s < c.n)
+        team_delta<LAST, SN, G>(c, s, src, dst, qpos, xa, scell, cstart, sidx, sphere, pos, vel, prev, ncount,
+                                foam, err, rm, nullptr, bufs);
+}
+
+template <uint32_t G, bool LAST>
+void launch_lambda(const StepConsts& c, const DevState& d, bool first, const RowMasks& rm, cudaStream_t s) {
+    const dim3 grid(cdiv(c.n, (G ? kTB / (G ? G : 1) : kSB)));
+    if constexpr (G != 0) {
+        if (first)
+            k_lambda_first_team<LAST, G><<<grid, kTB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart,
+                                                              d.sidx, d.lambdas, d.ncount, rm);
+        else
+            k_lambda_team<LAST, G><<<grid, kTB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart,
+                                                        d.sidx, d.lambdas, rm);
+    } else {
+        if (first)
+            k_lambda_first<LAST><<<grid, kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart,
+                                                      d.sidx, d.lambdas, d.ncount, rm);
+        else
+            k_lambda<LAST><<<grid, kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart, d.sidx,
+                                                d.lambdas, rm);
+    }
+}
+
+template <uint32_t G, bool LAST, uint32_t SN>
+void launch_delta_n(const StepConsts& c, const DevState& d, const RowMasks& rm, cudaStream_t s) {
+    const dim3 grid(cdiv(c.n, (G ? kTB / (G ? G : 1) : kSB)));
+    if constexpr (G != 0)
+        k_delta_team<LAST, SN, G><<<grid, kTB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.xa, d.scell, d.cstart,
+                                                       d.sidx, d.sphere, d.pos, d.vel, d.prev, d.ncount, d.foam,
+                                                       d.err, rm);
     else
-        k_delta<LAST, 0><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.xa, d.scell, d.cstart, d.sidx, d.sphere,
-                                              d.pos, d.vel, d.prev, d.ncount, d.foam, d.err, rm);
+        k_delta<LAST, SN><<<grid, kSB, 0, s>>>(c, d.sorted_b, d.sorted_a, d.qpos, d.xa, d.scell, d.cstart, d.sidx,
+                                               d.sphere, d.pos, d.vel, d.prev, d.ncount, d.foam, d.err, rm);
+}
+
+template <uint32_t G, bool LAST>
+void launch_iteration(const StepConsts& c, const DevState& d, bool first, const RowMasks& rm, cudaStream_t s,
+                      KernelTimer* t) {
+    tbegin(t, s);
+    launch_lambda<G, LAST>(c, d, first, rm, s);
+    tend(t, first ? "lambda_count" : "lambda", s);
+    tbegin(t, s);
+    if (c.scorr_n == 4)
+        launch_delta_n<G, LAST, 4>(c, d, rm, s);
+    else
+        launch_delta_n<G, LAST, 0>(c, d, rm, s);
+    tend(t, LAST ? "delta_finalize" : "delta", s);
+}
+
+template <uint32_t G>
+void launch_iterations(const StepConsts& c, const DevState& d, uint32_t iterations, cudaStream_t s,
+                       KernelTimer* t) {
+    const RowMasks rm{d.row_masks, d.mask_overflow, d.mask_stride};  // 9 x u32 per slot
+    for (uint32_t it = 0; it < iterations; ++it) {
+        if (it + 1 == iterations)
+            launch_iteration<G, true>(c, d, it == 0, rm, s, t);
+        else
+            launch_iteration<G, false>(c, d, it == 0, rm, s, t);
+    }
 }
 
 __global__ void __launch_bounds__(256)
@@ -98,6 +185,14 @@ k_finalize_sorted(StepConsts c, const float4* __restrict__ sorted,
 }
 
 }  // namespace
+
+// 16 lanes per particle up to 16,384 particles: the step of a jittered cube at
+// K = 3 takes 55 us instead of 98 (2,197 particles), 70 / 101 (8,000), 98 / 107
+// (16,000), but 154 / 112 (32,000), where one lane each fills the GPU well
+// enough and does a third of the work.  8 lanes: 65, 78, 113, 164 us.
+uint32_t team_lanes(uint32_t n) {
+    return n <= 16384u ? kTeam : 0u;
+}
 
 cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t iterations,
                           cudaStream_t s, KernelTimer* t) {
@@ -113,30 +208,10 @@ cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t itera
         tend(t, "finalize", s);
         return cudaGetLastError();
     }
-    const RowMasks rm{d.row_masks, d.mask_overflow, d.mask_stride};  // 9 x u32 per slot
-    for (uint32_t it = 0; it < iterations; ++it) {
-        const bool first = it == 0, last = it + 1 == iterations;
-        tbegin(t, s);
-        if (first && last)
-            k_lambda_first<true><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart,
-                                                      d.sidx, d.lambdas, d.ncount, rm);
-        else if (first)
-            k_lambda_first<false><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart,
-                                                       d.sidx, d.lambdas, d.ncount, rm);
-        else if (last)
-            k_lambda<true><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart, d.sidx,
-                                                d.lambdas, rm);
-        else
-            k_lambda<false><<<cdiv(n, kSB), kSB, 0, s>>>(c, d.sorted_a, d.qpos, d.sorted_b, d.scell, d.cstart, d.sidx,
-                                                 d.lambdas, rm);
-        tend(t, first ? "lambda_count" : "lambda", s);
-        tbegin(t, s);
-        if (last)
-            launch_delta<true>(c, d, rm, s);
-        else
-            launch_delta<false>(c, d, rm, s);
-        tend(t, last ? "delta_finalize" : "delta", s);
-    }
+    if (team_lanes(n))
+        launch_iterations<kTeam>(c, d, iterations, s, t);
+    else
+        launch_iterations<0>(c, d, iterations, s, t);
     return cudaGetLastError();
 }
 
