@@ -242,7 +242,7 @@ struct mp_batch {
         args.scell = sl.scell;
         args.cstart = sl.cstart;
         args.rec = sl.rec;
-        const cudaError_t e = launch_batch_step(args, block, blocks(), s);
+        const cudaError_t e = launch_batch_step(args, block, std::min(blocks(), useful_blocks(N)), s);
         if (e != cudaSuccess) return fail(MP_ERR_CUDA, "recorded step launch: %s", cudaGetErrorString(e));
         return MP_OK;
     }
@@ -279,12 +279,25 @@ struct mp_batch {
         if (cap_stream) cudaStreamDestroy(cap_stream);
     }
 
+    // Resident blocks of the current launch shape; the occupancy query is made
+    // once per block size (it costs as much host time as a launch).
+    mutable uint32_t occ_block = 0, occ_blocks = 0, sms = 0;
     uint32_t blocks() const {
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        const int occ = batch_max_blocks_per_sm(block);
-        const int per_sm = blocks_per_sm ? std::min<int>(int(blocks_per_sm), occ) : occ;
-        return uint32_t(std::max(1, per_sm) * std::max(1, sms));
+        if (occ_block != block) {
+            int n = 0;
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+            sms = uint32_t(std::max(1, n));
+            occ_blocks = uint32_t(std::max(1, batch_max_blocks_per_sm(block)));
+            occ_block = block;
+        }
+        return (blocks_per_sm ? std::min(blocks_per_sm, occ_blocks) : occ_blocks) * sms;
+    }
+
+    // Blocks that a launch over n particles can put to work: a grid barrier costs
+    // more the more blocks it waits for (the results do not depend on the grid).
+    uint32_t useful_blocks(uint32_t n) const {
+        const uint64_t lanes = std::max<uint32_t>(1u, team_lanes(n));
+        return uint32_t(std::max<uint64_t>(1u, (n * lanes + block - 1) / block));
     }
 
     // launch arguments with the current bound of the barrier wait
@@ -304,22 +317,19 @@ struct mp_batch {
             args.scene_end = S;
             args.p_begin = 0;
             args.p_end = N;
-            const cudaError_t e = launch_batch_step(args, block, nb, s);
+            const cudaError_t e = launch_batch_step(args, block, std::min(nb, useful_blocks(N)), s);
             if (e != cudaSuccess) return fail(MP_ERR_CUDA, "batch step launch: %s", cudaGetErrorString(e));
             return MP_OK;
         }
-        // The same kernel, one scene per launch, each on a grid no larger
-        // than its particles need (a small scene's grid barriers are cheaper
-        // on fewer blocks; the results do not depend on the grid).
+        // The same kernel, one scene per launch.
         for (uint32_t sc = 0; sc < S; ++sc) {
             if (counts[sc] == 0) continue;
-            const uint32_t need = uint32_t((uint64_t(counts[sc]) + block - 1) / block);
             BatchArgs args = launch_args();
             args.scene_begin = sc;
             args.scene_end = sc + 1;
             args.p_begin = p0[sc];
             args.p_end = p0[sc] + counts[sc];
-            const cudaError_t e = launch_batch_step(args, block, std::min(nb, need), s);
+            const cudaError_t e = launch_batch_step(args, block, std::min(nb, useful_blocks(counts[sc])), s);
             if (e != cudaSuccess) return fail(MP_ERR_CUDA, "batch step launch: %s", cudaGetErrorString(e));
         }
         return MP_OK;
@@ -521,15 +531,15 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         a.cstart = reinterpret_cast<uint32_t*>(static_cast<char*>(b->cell_block) + cbytes);
         a.tile_sums = reinterpret_cast<uint32_t*>(static_cast<char*>(b->cell_block) + 2 * cbytes);
         a.max_cells = b->max_cells;
-        MP_ALLOC(b->small_block, 256, b->device);
-        MP_CUDA(cudaMemset(b->small_block, 0, 256));
+        const size_t small = 256 + sizeof(unsigned) * kBarWords;
+        MP_ALLOC(b->small_block, small, b->device);
+        MP_CUDA(cudaMemset(b->small_block, 0, small));
         uint32_t* sm = static_cast<uint32_t*>(b->small_block);
         a.long_count = sm + 0;
         a.total_cells = sm + 1;
         a.err = sm + 2;
-        a.bar_count = reinterpret_cast<unsigned*>(sm + 32);
-        a.bar_gen = reinterpret_cast<unsigned*>(sm + 33);
         a.abort = sm + 48;
+        a.bar = reinterpret_cast<unsigned*>(sm + 64);
         MP_ALLOC(b->scenes, sizeof(SceneDev) * std::max<uint32_t>(nscenes, 1u), b->device);
         a.scenes = b->scenes;
         a.iterations = iters;
@@ -996,9 +1006,9 @@ int mp_batch_check_errors(mp_batch* b, uint32_t* bits) {
         MP_CUDA(cudaMemcpy(&w, b->a.err, 4, cudaMemcpyDeviceToHost));
         MP_CUDA(cudaMemset(b->a.err, 0, 4));
         if (w & kDevErrSpin) {
-            // a barrier wait gave up: the launch left the barrier counter
+            // a barrier wait gave up: the launch left the barrier's counters
             // mid-count and the abort flag set; re-arm both
-            MP_CUDA(cudaMemset(b->a.bar_count, 0, sizeof(unsigned)));
+            MP_CUDA(cudaMemset(b->a.bar, 0, sizeof(unsigned) * kBarWords));
             MP_CUDA(cudaMemset(b->a.abort, 0, sizeof(uint32_t)));
         }
     }

@@ -28,7 +28,7 @@
 #include <cooperative_groups.h>
 
 #include "pbf_batch.h"
-#include "pbf_items.cuh"
+#include "pbf_team.cuh"
 
 namespace mpb {
 namespace {
@@ -36,47 +36,84 @@ namespace {
 constexpr uint32_t kScanItems = 8;  // per thread and tile in phase 4
 
 // Grid-wide barrier with a generation counter.  Every block calls it the same
-// number of times.  The wait is bounded: a block that waits more than
-// a.spin_limit polls sets the error bit and the abort flag.  Returns false
-// (to every thread of the block) when the launch is aborted, by this block or
-// another one; the block must then return.  A barrier only completes once
-// every block has arrived, i.e. finished the phase before it, so a block that
-// returns true works on complete data; a block that left early never
-// arrives at the next barrier, so nobody passes that one.
-__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, int* s_ok) {
+// number of times.  Blocks arrive at one of several counters, about 32 blocks each
+// (a cache line apart: atomics on one address run one after the other), and each
+// group's last block at the root; the generation that the others poll has a line
+// of its own.  The block that completes the root runs last() before it releases
+// the others, with everything they wrote before the barrier visible: work for
+// one block costs no barrier of its own.
+//
+// Against one counter beside the generation and a barrier on each side of the two
+// one-block phases: 12 scenes of 61,000 particles, 223 -> 184 us per step on 592
+// blocks; one scene of 8,000 (with teams and only the blocks it fills) 221 -> 119.
+//
+// The wait is bounded: a block that waits more than a.spin_limit polls sets the
+// error bit and the abort flag.  Returns false (to every thread of the block)
+// when the launch is aborted, by this block or another one; the block must then
+// return.  A barrier only completes once every block has arrived, i.e. finished
+// the phase before it, so a block that returns true works on complete data; a
+// block that left early never arrives at the next barrier, so nobody passes that
+// one.
+template <class Last>
+__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, int* s_flags, Last&& last) {
     __syncthreads();
+    volatile unsigned* vgen = a.bar + kBarGen;
+    volatile uint32_t* vabort = a.abort;
+    unsigned g = 0;
     if (threadIdx.x == 0) {
-        volatile unsigned* vgen = a.bar_gen;
-        volatile uint32_t* vabort = a.abort;
-        const unsigned g = *vgen;
+        g = *vgen;
         __threadfence();
-        int ok = 1;
-        if (atomicAdd(a.bar_count, 1u) + 1u == gridDim.x + a.bar_extra) {
-            atomicExch(a.bar_count, 0u);
+        // block b belongs to group b mod groups
+        const uint32_t groups = min((gridDim.x + 31u) / 32u, kBarGroups), group = blockIdx.x % groups;
+        const uint32_t members = (gridDim.x - group + groups - 1u) / groups;
+        unsigned* count = a.bar + (1u + group) * kBarLine;
+        int mine = 0;
+        if (atomicAdd(count, 1u) + 1u == members) {
+            atomicExch(count, 0u);
             __threadfence();
-            atomicAdd(a.bar_gen, 1u);
-        } else {
-            uint32_t spins = 0;
-            while (*vgen == g) {
-                if (*vabort) {
-                    ok = 0;
-                    break;
-                }
-                if (++spins > a.spin_limit) {
-                    atomicOr(a.err, kDevErrSpin);
-                    atomicExch(a.abort, 1u);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
+            if (atomicAdd(a.bar + kBarRoot, 1u) + 1u == groups + a.bar_extra) {
+                atomicExch(a.bar + kBarRoot, 0u);
+                __threadfence();
+                mine = 1;
             }
+        }
+        s_flags[0] = mine;
+    }
+    __syncthreads();
+    if (s_flags[0]) {
+        last();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(a.bar + kBarGen, 1u);
+            s_flags[1] = !*vabort;
+        }
+    } else if (threadIdx.x == 0) {
+        int ok = 1;
+        uint32_t spins = 0;
+        while (*vgen == g) {
+            if (*vabort) {
+                ok = 0;
+                break;
+            }
+            if (++spins > a.spin_limit) {
+                atomicOr(a.err, kDevErrSpin);
+                atomicExch(a.abort, 1u);
+                ok = 0;
+                break;
+            }
+            __nanosleep(32);
         }
         if (ok && *vabort) ok = 0;
         __threadfence();
-        *s_ok = ok;
+        s_flags[1] = ok;
     }
     __syncthreads();
-    return *s_ok != 0;
+    return s_flags[1] != 0;
+}
+
+__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, int* s_flags) {
+    return grid_barrier(a, s_flags, [] {});
 }
 
 template <uint32_t BS>
@@ -119,11 +156,16 @@ constexpr int batch_min_blocks() {
 
 // SN: the s_corr exponent fixed at compile time (4, when every scene uses
 // the reference's) or read per scene (0); both give the same bits for 4.
-template <uint32_t BS, uint32_t SN>
+// G: lanes per particle of the solver phases (kTeam) or 0 for one each
+// (team_lanes(); the same bits).
+template <uint32_t BS, uint32_t SN, uint32_t G>
 __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(BatchArgs a) {
     __shared__ uint32_t s_warp[BS / 32 + 1];
-    __shared__ int s_ok;
-    extern __shared__ uint2 queue[];  // kQueue entries per thread
+    __shared__ int s_flags[2];
+    // one lane per particle: kQueue entries per thread; teams: a TeamBuf each
+    extern __shared__ uint2 shared[];
+    uint2* queue = shared;
+    TeamBuf* bufs = reinterpret_cast<TeamBuf*>(shared);
     const uint32_t gtid = blockIdx.x * BS + threadIdx.x;
     // an earlier launch gave up on a barrier and left the barrier counter
     // mid-count: do nothing until the host has re-armed the batch
@@ -145,7 +187,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         if (sc[s].c.sphere) sphere_advance(sc[s].c, &sc[s].sphere);
     }
     if (gtid == 0) *a.long_count = 0;
-    if (!grid_barrier(a, &s_ok)) return;
+    if (!grid_barrier(a, s_flags)) return;
 
     // 1: predict + dense cell of the predicted position -> scene bounding box
     for (uint32_t i = pb + gtid; i < pe_round; i += gsize) {
@@ -176,10 +218,9 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             }
         }
     }
-    if (!grid_barrier(a, &s_ok)) return;
-
-    // 2: sub-grid of every scene and its offset in the cell arrays
-    if (blockIdx.x == 0) {
+    // 2: sub-grid of every scene and its offset in the cell arrays, by the block
+    // that completes the barrier
+    auto lay_out = [&] {
         uint32_t running = 0;
         for (uint32_t s0 = a.scene_begin; s0 < a.scene_end; s0 += BS) {
             const uint32_t s = s0 + threadIdx.x;
@@ -207,8 +248,8 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             running += total;
         }
         if (threadIdx.x == 0) *a.total_cells = running;
-    }
-    if (!grid_barrier(a, &s_ok)) return;
+    };
+    if (!grid_barrier(a, s_flags, lay_out)) return;
 
     // 3: cell id inside the scene's box + warp-aggregated count
     if (a.rec.scenes)
@@ -231,7 +272,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         count_cell(active, cell, a.counts, &rank);
         if (active) a.off[i] = rank;
     }
-    if (!grid_barrier(a, &s_ok)) return;
+    if (!grid_barrier(a, s_flags)) return;
 
     // 4: exclusive scan of counts[0, ncells] into cstart (counts left zero)
     const uint32_t len = cells_ok ? ncells + 1u : 0u;
@@ -247,10 +288,9 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         block_exclusive_scan<BS>(sum, s_warp, total);
         if (threadIdx.x == 0) a.tile_sums[t] = total;
     }
-    if (!grid_barrier(a, &s_ok)) return;
-    if (blockIdx.x == 0) {
-        // slots of this launch start at its first particle (a scene's range
-        // in serial mode)
+    // tile offsets, by the block that completes the barrier; slots of this launch
+    // start at its first particle (a scene's range in serial mode)
+    auto scan_tiles = [&] {
         uint32_t running = pb;
         for (uint32_t t0 = 0; t0 < tiles; t0 += BS) {
             const uint32_t t = t0 + threadIdx.x;
@@ -260,8 +300,8 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             if (t < tiles) a.tile_sums[t] = running + excl;
             running += total;
         }
-    }
-    if (!grid_barrier(a, &s_ok)) return;
+    };
+    if (!grid_barrier(a, s_flags, scan_tiles)) return;
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         // each thread owns kScanItems consecutive items of the tile
         uint32_t v[kScanItems], sum = 0;
@@ -281,27 +321,27 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
                 run += v[k];
             }
     }
-    if (!grid_barrier(a, &s_ok)) return;
+    if (!grid_barrier(a, s_flags)) return;
 
     // 5: scatter; 6: stable re-rank + gather; 7: long segments
     if (cells_ok)
         for (uint32_t i = pb + gtid; i < pe; i += gsize) scatter_item(i, a.hash, a.off, a.cstart, a.tmp);
-    if (!grid_barrier(a, &s_ok)) return;
+    if (!grid_barrier(a, s_flags)) return;
     if (cells_ok)
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             sort_gather_item(sc[a.scene_of[s]].c, s, a.tmp, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
                              a.qpos, a.xa, a.long_list, a.long_count);
-    if (!grid_barrier(a, &s_ok)) return;
-    {
-        const uint32_t nl = cells_ok ? *a.long_count : 0u;
+    if (!grid_barrier(a, s_flags)) return;
+    const uint32_t nl = cells_ok ? *static_cast<volatile uint32_t*>(a.long_count) : 0u;
+    if (nl) {  // the same for every block: long_count is written before the barrier only
         for (uint32_t li = blockIdx.x; li < nl; li += gridDim.x) {
             const uint32_t cell = a.long_list[li];
             const SceneDev& sd = sc[a.scene_of[a.tmp[a.cstart[cell]]]];
             long_segment(sd.c, cell, sd.p0, sd.p0 + sd.c.n, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
                          a.qpos, a.xa, s_warp);
         }
+        if (!grid_barrier(a, s_flags)) return;
     }
-    if (!grid_barrier(a, &s_ok)) return;
 
     // 8+: solver
     const RowMasks rm{a.row_masks, a.mask_overflow, a.mask_stride};
@@ -309,7 +349,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     if (a.iterations == 0) {
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             count_neighbors_item(sc[a.scene_of[s]].c, s, a.sorted_a, a.cstart, a.sidx, a.ncount);
-        if (!grid_barrier(a, &s_ok)) return;
+        if (!grid_barrier(a, s_flags)) return;
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             finalize_sorted_item(sc[a.scene_of[s]].c, s, a.sorted_a, a.sidx, a.pos, a.vel, a.prev,
                                  a.ncount, a.foam, a.err);
@@ -326,69 +366,111 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
                               a.rec.overflow + size_t(it) * a.mask_stride, a.mask_stride}
                    : rm;
         float4* drec = record ? a.rec.delta + size_t(it) * a.rec.stride : nullptr;
-        for (uint32_t s = pb + gtid; s < pe; s += gsize) {
+        constexpr uint32_t lanes = G ? G : 1u;
+        for (uint32_t s = pb + gtid / lanes; s < pe; s += gsize / lanes) {
             const StepConsts& c = sc[a.scene_of[s]].c;
-            if (it == 0) {
+            if constexpr (G != 0) {
+                if (it == 0) {
+                    if (last)
+                        team_lambda_first<true, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                                                   a.lambdas, a.ncount, rmi, bufs);
+                    else
+                        team_lambda_first<false, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                                                    a.lambdas, a.ncount, rmi, bufs);
+                } else if (last) {
+                    team_lambda<true, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                                         rmi, bufs);
+                } else {
+                    team_lambda<false, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                                          rmi, bufs);
+                }
+            } else if (it == 0) {
                 if (last)
                     lambda_first_item<true, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
-                                            a.lambdas, a.ncount, rmi, queue);
+                                                a.lambdas, a.ncount, rmi, queue);
                 else
                     lambda_first_item<false, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
-                                             a.lambdas, a.ncount, rmi, queue);
+                                                 a.lambdas, a.ncount, rmi, queue);
             } else if (last) {
-                lambda_item<true, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi, queue);
+                lambda_item<true, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                                      rmi, queue);
             } else {
-                lambda_item<false, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas, rmi, queue);
+                lambda_item<false, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                                       rmi, queue);
             }
         }
-        if (!grid_barrier(a, &s_ok)) return;
-        for (uint32_t s = pb + gtid; s < pe; s += gsize) {
+        if (!grid_barrier(a, s_flags)) return;
+        for (uint32_t s = pb + gtid / lanes; s < pe; s += gsize / lanes) {
             const SceneDev& sd = sc[a.scene_of[s]];
-            if (last)
-                delta_item<true, SN, BS>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx, &sd.sphere,
-                                 a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec, queue);
-            else
-                delta_item<false, SN, BS>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx, &sd.sphere,
-                                  a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec, queue);
+            if constexpr (G != 0) {
+                if (last)
+                    team_delta<true, SN, G>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                                            &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
+                                            bufs);
+                else
+                    team_delta<false, SN, G>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                                             &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
+                                             bufs);
+            } else if (last) {
+                delta_item<true, SN, BS>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                                         &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
+                                         queue);
+            } else {
+                delta_item<false, SN, BS>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                                          &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
+                                          queue);
+            }
         }
-        if (!last && !grid_barrier(a, &s_ok)) return;
+        if (!last && !grid_barrier(a, s_flags)) return;
     }
 }
 
-// Dynamic shared memory of a launch: the blocks' pair queues (beyond the 48 KB
-// a kernel may use unasked at BS = 512).
+// Dynamic shared memory of a launch: the threads' pair queues or the teams'
+// buffers (beyond the 48 KB a kernel may use unasked at BS = 512).
 template <uint32_t BS>
-constexpr size_t queue_bytes() {
-    return size_t(kQueue) * BS * sizeof(uint2);
+constexpr size_t shared_bytes(bool team) {
+    return team ? sizeof(TeamBuf) * (BS / kTeam) : sizeof(uint2) * kQueue * BS;
 }
 
 template <uint32_t BS>
-cudaError_t allow_shared(const void* fn) {
-    if (queue_bytes<BS>() <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(queue_bytes<BS>()));
+const void* batch_kernel(bool scorr4, bool team) {
+    if (team)
+        return scorr4 ? reinterpret_cast<const void*>(&k_batch_step<BS, 4, kTeam>)
+                      : reinterpret_cast<const void*>(&k_batch_step<BS, 0, kTeam>);
+    return scorr4 ? reinterpret_cast<const void*>(&k_batch_step<BS, 4, 0>)
+                  : reinterpret_cast<const void*>(&k_batch_step<BS, 0, 0>);
+}
+
+cudaError_t allow_shared(const void* fn, size_t bytes) {
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
 }
 
 template <uint32_t BS>
 cudaError_t launch_bs(const BatchArgs& args, uint32_t blocks, cudaStream_t s) {
     void* kargs[] = {const_cast<BatchArgs*>(&args)};
-    const void* fn = args.scorr4 ? reinterpret_cast<const void*>(&k_batch_step<BS, 4>)
-                                 : reinterpret_cast<const void*>(&k_batch_step<BS, 0>);
-    const cudaError_t e = allow_shared<BS>(fn);
+    const bool team = team_lanes(args.p_end - args.p_begin) != 0;
+    const void* fn = batch_kernel<BS>(args.scorr4 != 0, team);
+    const size_t bytes = shared_bytes<BS>(team);
+    const cudaError_t e = allow_shared(fn, bytes);
     if (e != cudaSuccess) return e;
-    return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(BS), kargs, queue_bytes<BS>(), s);
+    return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(BS), kargs, bytes, s);
 }
 
-// Blocks of both instances that fit on one SM at once (the smaller count).
+// Blocks of every instance that fit on one SM at once (the smallest count).
 template <uint32_t BS>
 int occupancy_bs() {
-    int n[2] = {0, 0};
-    const void* fns[2] = {reinterpret_cast<const void*>(&k_batch_step<BS, 0>),
-                          reinterpret_cast<const void*>(&k_batch_step<BS, 4>)};
-    for (int i = 0; i < 2; ++i)
-        if (allow_shared<BS>(fns[i]) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[i], fns[i], BS, queue_bytes<BS>()) != cudaSuccess)
+    int least = 1 << 30;
+    for (int i = 0; i < 4; ++i) {
+        const bool scorr4 = i & 1, team = i & 2;
+        const void* fn = batch_kernel<BS>(scorr4, team);
+        int n = 0;
+        if (allow_shared(fn, shared_bytes<BS>(team)) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, BS, shared_bytes<BS>(team)) != cudaSuccess)
             return 0;
-    return n[0] < n[1] ? n[0] : n[1];
+        least = n < least ? n : least;
+    }
+    return least;
 }
 
 }  // namespace

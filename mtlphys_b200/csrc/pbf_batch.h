@@ -32,6 +32,11 @@ struct BatchRecord {
     uint32_t stride;       // slots per lam / delta array
 };
 
+// Words of the grid barrier's counters, a cache line each: the root, up to kBarGroups arrival counters, the generation.
+constexpr uint32_t kBarLine = 32, kBarGroups = 32;
+constexpr uint32_t kBarRoot = 0, kBarGen = (1 + kBarGroups) * kBarLine;
+constexpr uint32_t kBarWords = (2 + kBarGroups) * kBarLine;
+
 struct BatchArgs {
     SceneDev* scenes;
     uint32_t scene_begin, scene_end;  // scenes of this launch
@@ -47,7 +52,7 @@ struct BatchArgs {
     uint32_t *row_masks, *mask_overflow;
     uint32_t mask_stride;
     uint32_t* total_cells;
-    unsigned *bar_count, *bar_gen;
+    unsigned* bar;                    // grid barrier: kBarWords words (zero, or a generation at kBarGen)
     uint32_t* err;
     // Bounded grid barrier: a block waits at most spin_limit polls.  One
     // that gives up sets kDevErrSpin and *abort, and every block then leaves
