@@ -345,6 +345,8 @@ void set_prefilter(const mp_pbf_params& p, StepConsts& c) {
     c.q_units = 0;
     c.q_inv = 0.0f;
     c.q_thr = 1 << 30;
+    c.q_in = -1;
+    c.q_slack = 0.0f;
     c.q_lim = 0.0f;
     const double cs = p.cell_size, h = p.h;
     const double slack = 4.0;
@@ -361,6 +363,12 @@ void set_prefilter(const mp_pbf_params& p, StepConsts& c) {
     c.q_units = units;
     c.q_inv = float(double(units) / cs);
     c.q_thr = int(std::floor(r * r)) + 2;
+    // the same slack the other way round: a distance of at most r_in steps is
+    // below h.  Between particles inside their cells (give or take q_slack), a
+    // difference that wraps is at least 256 - 2 units - slack >= h / u steps.
+    const double r_in = h / u * (1.0 - 1e-5) - 2.3453 - 1.7321 * fuzz;
+    c.q_in = r_in > 0.0 ? int(std::floor(r_in * r_in)) - 2 : -1;
+    c.q_slack = float(0.4 * u);
     c.q_lim = float(lim);
 }
 
@@ -645,6 +653,7 @@ struct mp_engine {
         char* b = static_cast<char*>(small_block);
         d.long_count = reinterpret_cast<uint32_t*>(b);
         d.err = reinterpret_cast<uint32_t*>(b + 4);
+        d.strays = reinterpret_cast<uint32_t*>(b + 8);
         d.sphere = reinterpret_cast<mpb::SphereState*>(b + 64);
         return MP_OK;
     }

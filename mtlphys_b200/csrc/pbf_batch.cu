@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     if (cells_ok)
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             sort_gather_item(sc[a.scene_of[s]].c, s, a.tmp, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
-                             a.qpos, a.xa, a.long_list, a.long_count);
+                             a.qpos, a.xa, nullptr, a.long_list, a.long_count);
     if (!grid_barrier(a, s_flags)) return;
     const uint32_t nl = cells_ok ? *static_cast<volatile uint32_t*>(a.long_count) : 0u;
     if (nl) {  // the same for every block: long_count is written before the barrier only
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             const uint32_t cell = a.long_list[li];
             const SceneDev& sd = sc[a.scene_of[a.tmp[a.cstart[cell]]]];
             long_segment(sd.c, cell, sd.p0, sd.p0 + sd.c.n, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
-                         a.qpos, a.xa, s_warp);
+                         a.qpos, a.xa, nullptr, s_warp);
         }
         if (!grid_barrier(a, s_flags)) return;
     }
@@ -347,8 +347,10 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     const RowMasks rm{a.row_masks, a.mask_overflow, a.mask_stride};
     if (!cells_ok) return;  // every block takes this branch together
     if (a.iterations == 0) {
-        for (uint32_t s = pb + gtid; s < pe; s += gsize)
-            count_neighbors_item(sc[a.scene_of[s]].c, s, a.sorted_a, a.cstart, a.sidx, a.ncount);
+        if constexpr (G == 0)
+            for (uint32_t s = pb + gtid; s < pe; s += gsize)
+                count_neighbors_item<BS>(sc[a.scene_of[s]].c, s, a.sorted_a, a.qpos, a.cstart, a.sidx, a.ncount,
+                                         1u, PairQueue<BS>(queue));
         if (!grid_barrier(a, s_flags)) return;
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             finalize_sorted_item(sc[a.scene_of[s]].c, s, a.sorted_a, a.sidx, a.pos, a.vel, a.prev,
@@ -449,7 +451,7 @@ cudaError_t allow_shared(const void* fn, size_t bytes) {
 template <uint32_t BS>
 cudaError_t launch_bs(const BatchArgs& args, uint32_t blocks, cudaStream_t s) {
     void* kargs[] = {const_cast<BatchArgs*>(&args)};
-    const bool team = team_lanes(args.p_end - args.p_begin) != 0;
+    const bool team = args.iterations && team_lanes(args.p_end - args.p_begin) != 0;
     const void* fn = batch_kernel<BS>(args.scorr4 != 0, team);
     const size_t bytes = shared_bytes<BS>(team);
     const cudaError_t e = allow_shared(fn, bytes);

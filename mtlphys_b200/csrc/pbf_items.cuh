@@ -122,18 +122,25 @@ __device__ __forceinline__ void scatter_item(uint32_t i, const uint32_t* __restr
 }
 
 // A particle's place in sorted order: its index, predicted position, quantized
-// position and the x anchor of its cell.
+// position and the x anchor of its cell.  strays (may be NULL) is set to 1 when the
+// position lies outside the cell.
 __device__ __forceinline__ void place(const StepConsts& c, uint32_t d, uint32_t j, const float4& p,
                                       uint32_t* __restrict__ sidx, float4* __restrict__ sorted,
-                                      uint32_t* __restrict__ qpos, float* __restrict__ xa) {
+                                      uint32_t* __restrict__ qpos, float* __restrict__ xa,
+                                      uint32_t* strays) {
     int cx, cy, cz;
     cell_of(c.g, p.x, p.y, p.z, cx, cy, cz);
     sidx[d] = j;
     sorted[d] = p;
     const float ax = anchor_x(c.g, cx);
     xa[d] = ax;
-    qpos[d] = quantize<false>(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, __fsub_rn(p.x, ax),
-                              __fsub_rn(p.y, anchor_y(c.g, cy)), __fsub_rn(p.z, anchor_z(c.g, cz)));
+    const float lx = __fsub_rn(p.x, ax), ly = __fsub_rn(p.y, anchor_y(c.g, cy));
+    const float lz = __fsub_rn(p.z, anchor_z(c.g, cz));
+    qpos[d] = quantize<false>(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, lx, ly, lz);
+    // (count_neighbors_item) a position outside its cell, or not finite
+    if (strays && !(fminf(fminf(lx, ly), lz) >= -c.q_slack && fmaxf(fmaxf(lx, ly), lz) <= c.g.cs + c.q_slack &&
+                    lx + ly + lz < 1e30f))  // (fminf and fmaxf drop a NaN)
+        *strays = 1u;
 }
 
 // Stable re-rank inside the cell segment + gatherPositions: the slot's
@@ -147,7 +154,7 @@ __device__ __forceinline__ void sort_gather_item(const StepConsts& sc, uint32_t 
                                                  uint32_t* __restrict__ sidx,
                                                  float4* __restrict__ sorted,
                                                  uint32_t* __restrict__ qpos, float* __restrict__ xa,
-                                                 uint32_t* __restrict__ long_list,
+                                                 uint32_t* strays, uint32_t* __restrict__ long_list,
                                                  uint32_t* __restrict__ long_count) {
     const uint32_t j = tmp[s];
     const uint32_t c = hash[j];
@@ -158,7 +165,7 @@ __device__ __forceinline__ void sort_gather_item(const StepConsts& sc, uint32_t 
     }
     uint32_t rank = 0;
     for (uint32_t k = a; k < b; ++k) rank += (tmp[k] < j) ? 1u : 0u;
-    place(sc, a + rank, j, pos[j], sidx, sorted, qpos, xa);
+    place(sc, a + rank, j, pos[j], sidx, sorted, qpos, xa, strays);
 }
 
 // A long segment, by the whole block: rank(j) = number of particles j' < j of
@@ -169,7 +176,7 @@ __device__ inline void long_segment(const StepConsts& sc, uint32_t c, uint32_t p
                                     const uint32_t* __restrict__ cstart,
                                     const float4* __restrict__ pos, uint32_t* __restrict__ sidx,
                                     float4* __restrict__ sorted, uint32_t* __restrict__ qpos,
-                                    float* __restrict__ xa, uint32_t* s_warp) {
+                                    float* __restrict__ xa, uint32_t* strays, uint32_t* s_warp) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t a = cstart[c], len = cstart[c + 1] - a;
     uint32_t running = 0;
@@ -185,39 +192,11 @@ __device__ inline void long_segment(const StepConsts& sc, uint32_t c, uint32_t p
             blk += s_warp[w];
         }
         if (f)
-            place(sc, a + running + before + __popc(m & lanemask_lt()), j, pos[j], sidx, sorted, qpos, xa);
+            place(sc, a + running + before + __popc(m & lanemask_lt()), j, pos[j], sidx, sorted, qpos, xa,
+                  strays);
         running += blk;
         __syncthreads();
     }
-}
-
-// countNeighbors in sorted order: the 27-cell stencil is 9 contiguous slot
-// ranges (x-fastest hash).
-__device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32_t s,
-                                                     const float4* __restrict__ sorted,
-                                                     const uint32_t* __restrict__ cstart,
-                                                     const uint32_t* __restrict__ sidx,
-                                                     uint32_t* __restrict__ ncount) {
-    const float4 p = sorted[s];
-    int cx, cy, cz;
-    cell_of(c.g, p.x, p.y, p.z, cx, cy, cz);
-    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
-    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
-    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
-    uint32_t cnt = 0;
-    for (int z = z0; z <= z1; ++z)
-        for (int y = y0; y <= y1; ++y) {
-            const uint32_t a = cstart[cell_hash(c.g, x0, y, z)];
-            const uint32_t b = cstart[cell_hash(c.g, x1, y, z) + 1];
-            for (uint32_t k = a; k < b; ++k) {
-                const float4 q = __ldg(&sorted[k]);
-                const float r2 = dist2(q.x - p.x, q.y - p.y, q.z - p.z);
-                cnt += (r2 < c.h2) ? 1u : 0u;
-            }
-        }
-    // the particle itself passed its own distance test unless its position is
-    // not finite
-    ncount[sidx[s]] = cnt - (dist2(p.x - p.x, p.y - p.y, p.z - p.z) < c.h2 ? 1u : 0u);
 }
 
 // ---- solver ------------------------------------------------------------------
@@ -496,6 +475,74 @@ __device__ __forceinline__ int prefilter(const StepConsts& c, int hx, int hy, in
     qi = quantize<true>(c, hx, hy, hz, lx, ly, lz);
     const bool near = fabsf(lx) < c.q_lim && fabsf(ly) < c.q_lim && fabsf(lz) < c.q_lim;
     return near ? -c.q_thr : -kPassAll;
+}
+
+// countNeighbors in sorted order.  Most candidates are decided by their quantized
+// distance: more than q_thr is out of range, at most q_in is in range (when no
+// particle lies outside its cell, so that no byte difference wraps to a small
+// value: `strays` is 0), and only the shell in between, a sixth of the
+// neighbours, is tested exactly.
+template <uint32_t BS>
+__device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32_t s,
+                                                     const float4* __restrict__ sorted,
+                                                     const uint32_t* __restrict__ qsrc,
+                                                     const uint32_t* __restrict__ cstart,
+                                                     const uint32_t* __restrict__ sidx,
+                                                     uint32_t* __restrict__ ncount, uint32_t strays,
+                                                     PairQueue<BS> queue) {
+    const float4 p = sorted[s];
+    int cx, cy, cz;
+    cell_of(c.g, p.x, p.y, p.z, cx, cy, cz);
+    uint32_t qi;
+    const int nthr = prefilter(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, __fsub_rn(p.x, anchor_x(c.g, cx)),
+                               __fsub_rn(p.y, anchor_y(c.g, cy)), __fsub_rn(p.z, anchor_z(c.g, cz)), qi);
+    const int up = strays || nthr != -c.q_thr ? kPassAll : c.q_thr - c.q_in;
+    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
+    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
+    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
+    uint32_t cnt = 0;
+    auto visit = [&](uint32_t k, float, float) {
+        const float4 q = __ldg(&sorted[k]);
+        cnt += dist2(q.x - p.x, q.y - p.y, q.z - p.z) < c.h2 ? 1u : 0u;
+    };
+    const RowOffsets none{};
+    for (int z = z0; z <= z1; ++z)
+        for (int y = y0; y <= y1; ++y) {
+            const uint32_t b0 = cstart[cell_hash(c.g, x0, y, z)];
+            const uint32_t b3 = cstart[cell_hash(c.g, x1, y, z) + 1];
+            const uint32_t a0 = row_base(b0);
+            for (uint32_t c0 = b0 < b3 ? a0 : b3; c0 < b3; c0 += 32) {
+                const uint32_t c1 = min(c0 + 32u, b3);
+                uint32_t maybe = 0, in = 0, k = c0;
+                for (; k < c1; k += 4) {
+                    const uint4 q = __ldg(reinterpret_cast<const uint4*>(qsrc + k));
+                    const int d0 = int(qi - q.x), d1 = int(qi - q.y);
+                    const int d2 = int(qi - q.z), d3 = int(qi - q.w);
+                    const int s0 = __dp4a(d0, d0, nthr), s1 = __dp4a(d1, d1, nthr);
+                    const int s2 = __dp4a(d2, d2, nthr), s3 = __dp4a(d3, d3, nthr);
+                    maybe = __funnelshift_l(uint32_t(s0), maybe, 1);
+                    in = __funnelshift_l(uint32_t(s0 + up), in, 1);
+                    maybe = __funnelshift_l(uint32_t(s1), maybe, 1);
+                    in = __funnelshift_l(uint32_t(s1 + up), in, 1);
+                    maybe = __funnelshift_l(uint32_t(s2), maybe, 1);
+                    in = __funnelshift_l(uint32_t(s2 + up), in, 1);
+                    maybe = __funnelshift_l(uint32_t(s3), maybe, 1);
+                    in = __funnelshift_l(uint32_t(s3 + up), in, 1);
+                }
+                const uint32_t left = 32u - (k - c0);
+                uint32_t row = (0xffffffffu >> (max(b0, c0) - c0)) & (0xffffffffu << (32u - (c1 - c0)));
+                if (s - c0 < 32u) row &= ~(0x80000000u >> (s - c0));
+                in = (in << left) & row;
+                maybe = (maybe << left) & row & ~in;
+                cnt += __popc(in);
+                if (maybe) {
+                    if (queue.full()) queue.drain(none, visit);
+                    queue.push(maybe, c0, 0u, 0u);
+                }
+            }
+        }
+    queue.drain(none, visit);
+    ncount[sidx[s]] = cnt;
 }
 
 // First lambda pass: absolute FP32 predicted positions (reference arithmetic,

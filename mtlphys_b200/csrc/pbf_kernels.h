@@ -33,6 +33,7 @@ struct DevState {
     uint32_t* cstart;       // cells+1 exclusive scan of counts
     uint32_t* long_list;    // cells whose segment exceeds kSegMax
     uint32_t* long_count;   // entries in long_list
+    uint32_t* strays;       // 1: some particle of this hash lies outside its cell
     unsigned long long* scan_status;  // look-back tile descriptors
     unsigned long long* scan_ticket;  // monotonic tile ticket
     uint32_t scan_tiles;

@@ -107,3 +107,35 @@ def test_counts_and_positions_match_the_oracle(cuda, ratio, origin, check_positi
     assert_equal_u32(got["counts"], o["neighbor_counts"], "neighbor counts")
     if check_positions:
         assert_positions(got["pos"], o["pos"], position_tolerance(p, dt, pos, vel))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ratio, strays", [(1.0, 0), (1.0, 30), (0.5, 0), (1.7, 3), (4.0, 0)])
+def test_spatial_hash_counts_match_the_oracle(cuda, ratio, strays):
+    """buildSpatialHash's neighbour counts with every particle inside its cell
+    (decided by the quantized distance but for a shell) and with some outside the
+    grid, whose quantized offsets can wrap; rows of hundreds of candidates."""
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(8)
+    n = 6001
+    pos = np.ones((n, 4), F)
+    pos[:, :3] = rng.uniform(0.0, 1.0, (n, 3))
+    pos[:900, :3] = 0.5 + rng.normal(0, 0.02, (900, 3))
+    pos[900:1000, :3] = rng.choice([0.0, 1.0], (100, 3))  # on the walls
+    if strays:
+        pos[-strays:, :3] = rng.uniform(-0.8, 1.8, (strays, 3))
+        pos[-1, 0] = np.nan
+    p = _abi.default_params()
+    p.set(cell_size=0.1 * ratio, bounds_min=(0.0,) * 3, bounds_max=(1.0,) * 3)
+    e = Engine(0)
+    try:
+        e.set_params(p)
+        e.reset(n, _abi.MP_SCENE_CUBE_DROP)
+        e.set_positions(pos)
+        e.build_spatial_hash()
+        got = e.neighbor_counts()
+        e.error_bits()
+    finally:
+        e.close()
+    assert_equal_u32(got, O.build_spatial_hash(p, pos)[3], "neighbor counts")
