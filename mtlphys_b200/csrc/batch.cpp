@@ -154,7 +154,7 @@ struct mp_batch {
         for (uint32_t c : counts) most = std::max(most, c);
         const uint32_t chunks = (most + kSumChunk - 1) / kSumChunk;
         const size_t accs = al(cap * 8) + al(cap * 32) + al(32 * size_t(chunks) * std::max<uint32_t>(S, 1u));
-        const size_t total = 8 * v4 + 8 * u + gbytes + inbox + ovf + accs;
+        const size_t total = 8 * v4 + 7 * u + gbytes + inbox + ovf + accs;
         MP_ALLOC(adj_block, total, device);
         MP_CUDA(cudaMemset(adj_block, 0, total));
         char* p = static_cast<char*>(adj_block);
@@ -170,10 +170,8 @@ struct mp_batch {
         adj.p_extra = v();
         adj.xbar = v();
         adj.vbar = v();
-        adj.qsc = reinterpret_cast<float*>(w());
+        adj.qc = reinterpret_cast<float2*>(take(2 * u));
         adj.lam_part = reinterpret_cast<float*>(w());
-        adj.lam_extra = reinterpret_cast<float*>(w());
-        adj.ccur = reinterpret_cast<uint32_t*>(w());
         adj.cpred = reinterpret_cast<uint32_t*>(w());
         adj.xa = reinterpret_cast<float*>(w());
         adj.inbox_count = reinterpret_cast<uint32_t*>(w());
@@ -917,7 +915,7 @@ int mp_batch_rollout_backward(mp_batch* b, const float* dpos, const float* dvel,
 
 uint32_t mp_batch_rollout_launch_count(const mp_batch* b, uint32_t steps) {
     if (!b || b->N == 0) return 0;
-    return steps * (1u + adjoint_launch_count(b->iterations)) + (steps ? 1u : 0u);
+    return steps * (1u + adjoint_launch_count(b->iterations)) + (steps ? 2u : 0u);
 }
 
 size_t mp_batch_snapshot_size(const mp_batch* b) {

@@ -27,7 +27,7 @@
 // cell), so each pair term of i's list is delivered to j by j's own sweep
 // when i is in j's list too (a test on the two cells).  Otherwise (a one-way
 // pair, ~0.4% of pairs in a 60-step cube drop) i posts the term to j's inbox
-// and a delivery kernel adds j's posts in ascending order of the sender's
+// and the next kernel over j adds its posts in ascending order of the sender's
 // slot.  The scene gradients (dL/dk, the sphere's center and radius) are
 // accumulated per slot and summed per scene in a fixed order.  Nothing is
 // added with float atomics, so the gradients are the same bytes on every run.
@@ -121,6 +121,47 @@ __device__ __forceinline__ void post(const AdjArgs& a, uint32_t to, uint32_t fro
     }
 }
 
+// The sum of the terms posted to receiver slot j by the last sweep, in ascending
+// order of the sender's slot (a sender posts to a receiver at most once per
+// sweep); empties its inbox.  Posts beyond the inbox are looked up in the
+// overflow list.
+__device__ __forceinline__ float4 collect(const AdjArgs& a, uint32_t j) {
+    float sx = 0.0f, sy = 0.0f, sz = 0.0f, sw = 0.0f;
+    const uint32_t cnt = a.inbox_count[j];
+    if (cnt != 0) {
+        a.inbox_count[j] = 0;
+        const uint32_t nin = min(cnt, kInbox);
+        const uint32_t head = cnt > kInbox ? a.ovf_head[j] : kNoPost;
+        uint32_t last = 0;
+        for (uint32_t done = 0; done < cnt; ++done) {
+            uint32_t best = 0xffffffffu;
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (uint32_t e = 0; e < nin; ++e) {
+                const uint32_t src = a.inbox_src[size_t(e) * a.stride + j];
+                if ((done == 0 || src > last) && src < best) {
+                    best = src;
+                    v = a.inbox_val[size_t(e) * a.stride + j];
+                }
+            }
+            for (uint32_t o = head; o != kNoPost; o = a.ovf_next[o]) {
+                const uint32_t src = a.ovf_src[o];
+                if ((done == 0 || src > last) && src < best) {
+                    best = src;
+                    v = a.ovf_val[o];
+                }
+            }
+            if (best == 0xffffffffu) break;  // posts dropped with the pool exhausted
+            sx += v.x;
+            sy += v.y;
+            sz += v.z;
+            sw += v.w;
+            last = best;
+        }
+        if (head != kNoPost) a.ovf_head[j] = kNoPost;
+    }
+    return make_float4(sx, sy, sz, sw);
+}
+
 // ---- finalize --------------------------------------------------------------
 
 __global__ void __launch_bounds__(kBlock) k_adj_finalize(AdjArgs a) {
@@ -171,7 +212,9 @@ __global__ void __launch_bounds__(kBlock) k_adj_finalize(AdjArgs a) {
 // ---- one solver iteration ---------------------------------------------------
 
 // Through the sphere push, the box clamp and the |delta| clamp of iteration
-// `it`; records the iterate's current cell for the pair sweeps.
+// `it`, from the position adjoint left by the iteration after it (its sweeps'
+// own sums and what they posted); the iterate's current cell goes beside dL/d
+// delta for the pair sweeps.
 __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
     const uint32_t s = blockIdx.x * kBlock + threadIdx.x;
     if (s == 0) *a.ovf_count = 0;  // the delta sweep posts into an empty list
@@ -182,7 +225,9 @@ __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
     const float4 l = __ldg(&a.t.lam[off + s]);
     const float4 dr = __ldg(&a.t.delta[off + s]);
     const uint32_t cell = __ldg(&a.t.scell[s]);
-    const float4 pe = a.p_extra[s];
+    const bool first = it + 1 == a.iterations;  // no sweep has run in this step
+    float4 pe = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (!first) pe = a.p_extra[s];
     const float4 pb4 = a.pbar[s];
     const SceneDev& sd = a.t.scenes[sc];
     const StepConsts& c = sd.c;
@@ -191,7 +236,11 @@ __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
     const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
     int cx, cy, cz;
     cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
-    a.ccur[s] = pack_cell(cx + c.g.lx, cy + c.g.ly, cz + c.g.lz);
+    const uint32_t ccur = pack_cell(cx + c.g.lx, cy + c.g.ly, cz + c.g.lz);
+    if (!first) {
+        const float4 more = collect(a, s);
+        pe = make_float4(pe.x + more.x, pe.y + more.y, pe.z + more.z, 0.0f);
+    }
 
     // the forward update (delta_item): clamp |delta|, A + (l + delta) in FP64
     const float dl = __fsqrt_rn(dist2(dr.x, dr.y, dr.z));
@@ -211,7 +260,6 @@ __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
         qc[k] = fmin(fmax(q[k], lo_b[k]), hi_b[k]);
     }
 
-    a.p_extra[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float pb[3] = {pb4.x + pe.x, pb4.y + pe.y, pb4.z + pe.z};
     if (c.sphere) {
         const double ex = qc[0] - sd.sphere.c[0], ey = qc[1] - sd.sphere.c[1], ez = qc[2] - sd.sphere.c[2];
@@ -245,7 +293,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
         pb[1] = f * (pb[1] - uy * dot);
         pb[2] = f * (pb[2] - uz * dot);
     }
-    a.dbar[s] = make_float4(pb[0], pb[1], pb[2], 0.0f);
+    a.dbar[s] = make_float4(pb[0], pb[1], pb[2], __uint_as_float(ccur));
 }
 
 // Pair sweep of applyDelta's adjoint.  With dbar = dL/d delta:
@@ -298,7 +346,6 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjA
             dens += pc.poly6 * (pc.h2 - r2) * (pc.h2 - r2) * (pc.h2 - r2);
             return;
         }
-        const uint32_t cell = __ldg(&a.ccur[k]);
         const float4 di = __ldg(&a.dbar[k]);
         const PairTerms t(pc, r2);
         dens += t.W;
@@ -315,7 +362,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjA
         kb -= rn * (fx * dm.x + fy * dm.y + fz * dm.z);
         // a pair in both lists carries the other particle's terms too; a
         // one-way pair owes it the negative of its own
-        const bool both = cells_adjacent(cell, pm, a.wide);
+        const bool both = cells_adjacent(__float_as_uint(di.w), pm, a.wide);
         const float ex = dm.x - (both ? di.x : 0.0f), ey = dm.y - (both ? di.y : 0.0f);
         const float ez = dm.z - (both ? di.z : 0.0f);
         const float gdd = fx * ex + fy * ey + fz * ez;
@@ -351,15 +398,17 @@ __global__ void __launch_bounds__(kBlock) k_adj_lbar(AdjArgs a, uint32_t it) {
     if (s == 0) *a.ovf_count = 0;  // the lambda sweep posts into an empty list
     if (s >= a.n) return;
     const StepConsts& c = a.t.scenes[a.scene_of[s]].c;
-    const float lb = a.lam_part[s] + a.lam_extra[s];
-    a.lam_extra[s] = 0.0f;
+    const uint32_t ccur = __float_as_uint(a.dbar[s].w);
+    const float4 posts = collect(a, s);  // of the delta sweep
+    a.p_extra[s] = posts;
+    const float lb = a.lam_part[s] + posts.w;
     const float4 gd = a.gd[s];
     const float lam = a.t.lam[size_t(it) * a.stride + s].w;
     const float ir = c.inv_rho0;
     const float Db = -lb * lam / gd.w;
     const float gG = 2.0f * Db * ir * ir;
     a.lbar[s] = make_float4(gG * gd.x, gG * gd.y, gG * gd.z, -lb * ir / gd.w);
-    a.qsc[s] = Db * ir * ir;
+    a.qc[s] = make_float2(Db * ir * ir, __uint_as_float(ccur));
 }
 
 // Pair sweep of densityLambda's adjoint:
@@ -375,7 +424,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(Adj
     const float4* src = a.t.lam + off;
     const float4 l = src[m];
     const float4 lm = a.lbar[m];
-    const float qm = a.qsc[m];
+    const float qm = a.qc[m].x;
     const uint32_t pm = a.cpred[m];
     int pcx, pcy, pcz;
     decode_cell(c.g, a.t.scell[m], pcx, pcy, pcz);
@@ -388,13 +437,12 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(Adj
     const float w6 = -6.0f * pc.poly6;
     auto body = [&](uint32_t k, const float4&, float rx, float ry, float rz, float r2) {
         if (!(r2 < pc.h2 && r2 > 1e-12f)) return;
-        const uint32_t cell = __ldg(&a.ccur[k]);
         const float4 li = __ldg(&a.lbar[k]);
-        const float qi = __ldg(&a.qsc[k]);
+        const float2 qi = __ldg(&a.qc[k]);
         const PairTerms t(pc, r2);
         const float gw = w6 * t.d * t.d;  // grad W = gw r
-        const bool both = cells_adjacent(cell, pm, a.wide);
-        const float qs = 2.0f * (qm + (both ? qi : 0.0f)) * t.f;
+        const bool both = cells_adjacent(__float_as_uint(qi.y), pm, a.wide);
+        const float qs = 2.0f * (qm + (both ? qi.x : 0.0f)) * t.f;
         const float3 hv = t.hess(rx, ry, rz, lm.x - (both ? li.x : 0.0f) + qs * rx,
                                  lm.y - (both ? li.y : 0.0f) + qs * ry, lm.z - (both ? li.z : 0.0f) + qs * rz);
         const float w = (lm.w + (both ? li.w : 0.0f)) * gw;
@@ -412,52 +460,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(Adj
     a.pbar[m] = make_float4(px, py, pz, 0.0f);
 }
 
-// ---- delivery of one-way pair terms, scene sums ----------------------------------
-
-// Adds every post of receiver slot j in ascending order of the sender's slot
-// (a sender posts to a receiver at most once per sweep): p_extra += the
-// xyz sums, and with LAMBDA lam_extra += the w sum.  Posts beyond the inbox
-// are looked up in the overflow list.
-template <bool LAMBDA>
-__global__ void __launch_bounds__(kBlock) k_adj_deliver(AdjArgs a) {
-    const uint32_t j = blockIdx.x * kBlock + threadIdx.x;
-    if (j >= a.n) return;
-    const uint32_t cnt = a.inbox_count[j];
-    if (cnt == 0) return;
-    a.inbox_count[j] = 0;
-    const uint32_t nin = min(cnt, kInbox);
-    const uint32_t head = cnt > kInbox ? a.ovf_head[j] : kNoPost;
-    float sx = 0.0f, sy = 0.0f, sz = 0.0f, sw = 0.0f;
-    uint32_t last = 0;
-    for (uint32_t done = 0; done < cnt; ++done) {
-        uint32_t best = 0xffffffffu;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (uint32_t e = 0; e < nin; ++e) {
-            const uint32_t src = a.inbox_src[size_t(e) * a.stride + j];
-            if ((done == 0 || src > last) && src < best) {
-                best = src;
-                v = a.inbox_val[size_t(e) * a.stride + j];
-            }
-        }
-        for (uint32_t o = head; o != kNoPost; o = a.ovf_next[o]) {
-            const uint32_t src = a.ovf_src[o];
-            if ((done == 0 || src > last) && src < best) {
-                best = src;
-                v = a.ovf_val[o];
-            }
-        }
-        if (best == 0xffffffffu) break;  // posts dropped with the pool exhausted
-        sx += v.x;
-        sy += v.y;
-        sz += v.z;
-        sw += v.w;
-        last = best;
-    }
-    if (head != kNoPost) a.ovf_head[j] = kNoPost;
-    const float4 pe = a.p_extra[j];
-    a.p_extra[j] = make_float4(pe.x + sx, pe.y + sy, pe.z + sz, 0.0f);
-    if (LAMBDA) a.lam_extra[j] += sw;
-}
+// ---- scene sums ------------------------------------------------------------------
 
 // Fixed-order block sum of one double per thread (blockDim.x == kBlock).
 __device__ __forceinline__ double block_sum(double v, double* sh) {
@@ -512,19 +515,32 @@ __global__ void __launch_bounds__(kBlock) k_adj_sphere_sum(AdjArgs a) {
     if (threadIdx.x == 0) a.spart[size_t(sc) * a.sum_chunks + chunk] = make_double4(cx, cy, cz, r);
 }
 
-// One block per scene: dL/dk = the sum of the per-slot accumulators over the
-// scene's slots (fixed order), which are cleared.
-__global__ void __launch_bounds__(kBlock) k_adj_k_sum(AdjArgs a) {
+// dL/dk of every scene: block (chunk, scene) sums the chunk's per-slot
+// accumulators into spart and clears them; k_adj_k_sum, one warp per scene, adds
+// the chunks.  Both in a fixed order.  (One block per scene walked 80,000 slots
+// in 92 us; both kernels take 6.)
+__global__ void __launch_bounds__(kBlock) k_adj_k_part(AdjArgs a) {
     __shared__ double sh[kBlock];
-    const SceneDev& sd = a.t.scenes[blockIdx.x];
-    const uint32_t p0 = sd.p0, n = sd.c.n;
+    const uint32_t chunk = blockIdx.x, sc = blockIdx.y;
+    const SceneDev& sd = a.t.scenes[sc];
+    const uint32_t first = chunk * kSumChunk, end = min(sd.c.n, first + kSumChunk);
+    double* acc = a.kacc + sd.p0;
     double k = 0.0;
-    for (uint32_t i = threadIdx.x; i < n; i += kBlock) {
-        k += a.kacc[p0 + i];
-        a.kacc[p0 + i] = 0.0;
+    for (uint32_t i = first + threadIdx.x; i < end; i += kBlock) {
+        k += acc[i];
+        acc[i] = 0.0;
     }
     k = block_sum(k, sh);
-    if (threadIdx.x == 0) a.grads[size_t(blockIdx.x) * kGradStride + kGradK] = k;
+    if (threadIdx.x == 0) a.spart[size_t(sc) * a.sum_chunks + chunk].x = k;
+}
+
+__global__ void __launch_bounds__(32) k_adj_k_sum(AdjArgs a) {
+    const uint32_t sc = blockIdx.x;
+    const uint32_t chunks = (a.t.scenes[sc].c.n + kSumChunk - 1) / kSumChunk;
+    double k = 0.0;
+    for (uint32_t i = threadIdx.x; i < chunks; i += 32) k += a.spart[size_t(sc) * a.sum_chunks + i].x;
+    for (int o = 16; o > 0; o >>= 1) k += __shfl_down_sync(kFull, k, o);
+    if (threadIdx.x == 0) a.grads[size_t(sc) * kGradStride + kGradK] = k;
 }
 
 // ---- predict, sphere ----------------------------------------------------------
@@ -535,10 +551,15 @@ __global__ void __launch_bounds__(kBlock) k_adj_predict(AdjArgs a) {
     // loads first (in flight together), stores after
     const uint32_t sc = __ldg(&a.scene_of[s]);
     const uint32_t j = __ldg(&a.t.sidx[s]);
-    const float4 pb = a.pbar[s], pe = a.p_extra[s];
+    const float4 pb = a.pbar[s];
     const float4 xb = a.xbar[j];
     const float dt = a.t.scenes[sc].c.dt;
-    a.p_extra[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 pe = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (a.iterations) {  // what the last iteration's sweeps posted
+        pe = a.p_extra[s];
+        const float4 more = collect(a, s);
+        pe = make_float4(pe.x + more.x, pe.y + more.y, pe.z + more.z, 0.0f);
+    }
     const float bx = pb.x + pe.x, by = pb.y + pe.y, bz = pb.z + pe.z;
     a.xbar[j] = make_float4(xb.x + bx, xb.y + by, xb.z + bz, 0.0f);
     a.vbar[j] = make_float4(bx * dt, by * dt, bz * dt, 0.0f);
@@ -627,10 +648,8 @@ cudaError_t launch_adjoint_step(const AdjArgs& a, cudaStream_t s) {
             k_adj_delta<4><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         else
             k_adj_delta<0><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
-        k_adj_deliver<true><<<grid, kBlock, 0, s>>>(a);
         k_adj_lbar<<<grid, kBlock, 0, s>>>(a, it);
         k_adj_lambda<<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
-        k_adj_deliver<false><<<grid, kBlock, 0, s>>>(a);
     }
     k_adj_predict<<<grid, kBlock, 0, s>>>(a);
     if (a.nscenes && a.sum_chunks) k_adj_sphere_sum<<<dim3(a.sum_chunks, a.nscenes), kBlock, 0, s>>>(a);
@@ -640,10 +659,11 @@ cudaError_t launch_adjoint_step(const AdjArgs& a, cudaStream_t s) {
 
 cudaError_t launch_adjoint_finish(const AdjArgs& a, cudaStream_t s) {
     if (a.n == 0 || a.nscenes == 0) return cudaSuccess;
-    k_adj_k_sum<<<a.nscenes, kBlock, 0, s>>>(a);
+    k_adj_k_part<<<dim3(a.sum_chunks, a.nscenes), kBlock, 0, s>>>(a);
+    k_adj_k_sum<<<a.nscenes, 32, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-uint32_t adjoint_launch_count(uint32_t iterations) { return 4u + 6u * iterations; }
+uint32_t adjoint_launch_count(uint32_t iterations) { return 4u + 4u * iterations; }
 
 }  // namespace mpb

@@ -35,7 +35,7 @@ struct AdjStep {
 // Pair terms that a particle's sweep owes another particle whose own sweep
 // does not see the pair (one-way pairs) are posted to the receiver's inbox:
 // kInbox slots per receiver, then a shared pool of overflow entries linked
-// into a list per receiver.  A delivery kernel then adds each receiver's
+// into a list per receiver.  The next kernel then adds each receiver's
 // posts in ascending order of the sender's slot, so the sums do not depend
 // on the order the posts arrived in (no float atomics: two backward passes
 // give the same bytes).
@@ -52,9 +52,11 @@ struct AdjArgs {
     float4* xbar;                 // in: dL/dx(t+1), out: dL/dx(t) (original order)
     float4* vbar;                 // in: dL/dv(t+1), out: dL/dv(t)
     // per-slot scratch (sorted order)
-    float4 *pbar, *qbar, *dbar, *lbar, *gd, *p_extra;
-    float *qsc, *lam_part, *lam_extra;
-    uint32_t *ccur, *cpred;
+    float4 *pbar, *qbar, *lbar, *gd, *p_extra;
+    float4* dbar;                 // dL/d delta; w: the packed current cell
+    float2* qc;                   // (dL/d squared-gradient sum, packed current cell)
+    float* lam_part;
+    uint32_t* cpred;
     float* xa;                    // x anchor of each slot's hash cell
     uint32_t wide;                // 1: some scene's grid is too wide for the packed cell comparison
     uint32_t scorr4;              // 1: every scene's s_corr exponent is 4
@@ -77,9 +79,8 @@ struct AdjArgs {
 };
 
 // Enqueue the reverse of one step: finalize, every solver iteration in
-// reverse order, predict, and the sphere kinematics.  p_extra, lam_extra,
-// inbox_count and sacc must be zero and ovf_head kNoPost on entry (they are
-// left so); kacc accumulates.
+// reverse order, predict, and the sphere kinematics.  inbox_count and sacc must
+// be zero and ovf_head kNoPost on entry (they are left so); kacc accumulates.
 cudaError_t launch_adjoint_step(const AdjArgs& a, cudaStream_t s);
 // grads[scene][kGradK] = the sum of kacc over the scene's slots (fixed order);
 // kacc is cleared.
