@@ -231,6 +231,29 @@ __device__ __forceinline__ float rsqrt_normal(float x) {
     return r;
 }
 
+// Two FP32 values in one 64-bit register, and the packed operations on them: each
+// half rounds exactly as the single operation does.  They save the lambda pass's
+// pair body three of about 50 instructions (1M-particle dam break: 1463 -> 1440 us
+// per step); packing the neighbour vector's x and y too, or the delta pass's sums,
+// costs as many register moves as it saves.
+struct F2 {
+    unsigned long long v;
+    F2() = default;
+    __device__ __forceinline__ F2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+    __device__ __forceinline__ void get(float& a, float& b) const {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    }
+};
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
 // densityLambdaSorted's sums for one particle (Constraints.metal:99-121): the
 // density starts at the particle's own W(0) whether or not its slot lies in
 // the stencil of its current cell (a particle can drift two cells from its
@@ -246,17 +269,17 @@ struct LambdaAcc {
     // no effect unless r2 < h^2
     __device__ __forceinline__ void add(const StepConsts& c, float rx, float ry, float rz, float r2) {
         const float d = __fsub_rn(c.h2, r2);
-        const float w = __fmul_rn(__fmul_rn(c.poly6, d), d);
         const float rinv = rsqrt_normal(r2);
         const float hd = fmaxf(__fsub_rn(c.h, __fmul_rn(r2, rinv)), 0.0f);
-        const float sc = __fmul_rn(__fmul_rn(__fmul_rn(-c.spiky, hd), hd), rinv);
+        float w, s1;  // poly6 d d and -spiky hd hd
+        const F2 dh(d, hd);
+        mul2(mul2(F2(c.poly6, -c.spiky), dh), dh).get(w, s1);
+        const float sc = __fmul_rn(s1, rinv);
         const float sc2 = __fmul_rn(sc, sc);
         if (r2 < c.h2) dens = __fmaf_rn(w, d, dens);
         if (r2 < c.h2 && r2 > 1e-12f) {
-            gx = __fmaf_rn(sc, rx, gx);
-            gy = __fmaf_rn(sc, ry, gy);
-            gz = __fmaf_rn(sc, rz, gz);
-            gsq = __fmaf_rn(sc2, r2, gsq);
+            fma2(F2(sc, sc), F2(rx, ry), F2(gx, gy)).get(gx, gy);
+            fma2(F2(sc, sc2), F2(rz, r2), F2(gz, gsq)).get(gz, gsq);
         }
     }
     __device__ __forceinline__ float lambda(const StepConsts& c) const {
@@ -345,24 +368,48 @@ struct PairQueue {
         tail += BS * 8u;
         pairs += __popc(mask);
     }
-    // visit(slot, oy, oz) for every bit, in the order queued; empties the queue
-    template <class Visit>
-    __device__ __forceinline__ void drain(const RowOffsets& o, Visit&& visit) {
+    // The next bit's slot and offsets; `at`, `mask`, `first` are the walk's state.
+    __device__ __forceinline__ uint32_t next(const RowOffsets& o, uint32_t& at, uint32_t& mask, uint32_t& first,
+                                             float& oy, float& oz) const {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.eq.u32 p, %0, 0;\n\t"
+            "@p ld.shared.v2.b32 {%0, %1}, [%2];\n\t"
+            "@p add.u32 %2, %2, %3;\n\t}"
+            : "+r"(mask), "+r"(first), "+r"(at)
+            : "n"(BS * 8u));
+        uint32_t t;
+        asm("bfind.shiftamt.u32 %0, %1;" : "=r"(t) : "r"(mask));
+        mask &= 0x7fffffffu >> t;
+        oy = (first & 2u) ? o.y2 : ((first & 1u) ? o.y1 : o.y0);
+        oz = int(first) < 0 ? o.z2 : ((first & 0x40000000u) ? o.z1 : o.z0);
+        return (first & 0x3ffffffcu) + t;
+    }
+    // visit(slot, fetch(slot), oy, oz) for every bit, in the order queued; empties
+    // the queue.  PIPE: each candidate is fetched while the one before it is
+    // visited (1-2% of a step; not for walks in the middle of a sweep, whose
+    // registers it would spill)
+    template <bool PIPE, class Fetch, class Visit>
+    __device__ __forceinline__ void drain(const RowOffsets& o, Fetch&& fetch, Visit&& visit) {
         uint32_t at = base, mask = 0, first = 0;
-        for (; pairs > 0; --pairs) {
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "setp.eq.u32 p, %0, 0;\n\t"
-                "@p ld.shared.v2.b32 {%0, %1}, [%2];\n\t"
-                "@p add.u32 %2, %2, %3;\n\t}"
-                : "+r"(mask), "+r"(first), "+r"(at)
-                : "n"(BS * 8u));
-            uint32_t t;
-            asm("bfind.shiftamt.u32 %0, %1;" : "=r"(t) : "r"(mask));
-            mask &= 0x7fffffffu >> t;
-            const float oy = (first & 2u) ? o.y2 : ((first & 1u) ? o.y1 : o.y0);
-            const float oz = int(first) < 0 ? o.z2 : ((first & 0x40000000u) ? o.z1 : o.z0);
-            visit((first & 0x3ffffffcu) + t, oy, oz);
+        float oy = 0.0f, oz = 0.0f;
+        if (!PIPE) {
+            for (; pairs > 0; --pairs) {
+                const uint32_t k = next(o, at, mask, first, oy, oz);
+                visit(k, fetch(k), oy, oz);
+            }
+        } else if (pairs) {
+            uint32_t k = next(o, at, mask, first, oy, oz);
+            auto q = fetch(k);
+            while (--pairs) {
+                const float y = oy, z = oz;
+                const uint32_t kn = next(o, at, mask, first, oy, oz);
+                const auto qn = fetch(kn);
+                visit(k, q, y, z);
+                k = kn;
+                q = qn;
+            }
+            visit(k, q, oy, oz);
         }
         tail = base;
     }
@@ -410,8 +457,8 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
         masks.overflow[s] = 0u;
         return;
     }
-    auto visit = [&](uint32_t k, float oy, float oz) {
-        const float4 q = __ldg(&src[k]);
+    auto fetch = [&](uint32_t k) { return __ldg(&src[k]); };
+    auto visit = [&](uint32_t k, const float4& q, float oy, float oz) {
         const float ox = ANCHORED ? __fadd_rn(__fsub_rn(aix, q.w), px) : px;
         const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
         body(k, q, rx, ry, rz, dist2(rx, ry, rz));
@@ -454,7 +501,7 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
                     if (s - c0 < 32u) mask &= ~(0x80000000u >> (s - c0));
                     if (c0 == a0) first = mask;
                     if (mask) {
-                        if (queue.full()) queue.drain(o, visit);  // crowded rows only
+                        if (queue.full()) queue.template drain<false>(o, fetch, visit);  // crowded rows only
                         queue.push(mask, c0, uint32_t(y - y0), uint32_t(z - z0));
                     }
                 }
@@ -464,7 +511,7 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
         }
     }
     masks.overflow[s] = over;
-    queue.drain(o, visit);
+    queue.template drain<true>(o, fetch, visit);
 }
 
 // The prefilter's arguments of a particle at offset l from the corner of its
@@ -501,8 +548,8 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
     const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
     const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
     uint32_t cnt = 0;
-    auto visit = [&](uint32_t k, float, float) {
-        const float4 q = __ldg(&sorted[k]);
+    auto fetch = [&](uint32_t k) { return __ldg(&sorted[k]); };
+    auto visit = [&](uint32_t, const float4& q, float, float) {
         cnt += dist2(q.x - p.x, q.y - p.y, q.z - p.z) < c.h2 ? 1u : 0u;
     };
     const RowOffsets none{};
@@ -536,12 +583,12 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
                 maybe = (maybe << left) & row & ~in;
                 cnt += __popc(in);
                 if (maybe) {
-                    if (queue.full()) queue.drain(none, visit);
+                    if (queue.full()) queue.template drain<false>(none, fetch, visit);
                     queue.push(maybe, c0, 0u, 0u);
                 }
             }
         }
-    queue.drain(none, visit);
+    queue.template drain<false>(none, fetch, visit);
     ncount[sidx[s]] = cnt;
 }
 
@@ -688,9 +735,14 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
     const int nx = x1 - x0 + 1;
     if (nx <= 0) return;
     const uint32_t longrows = rm.overflow[s];
-    auto visit = [&](uint32_t k, float oy, float oz) {
-        const float4 q = __ldg(&src[k]);
-        const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
+    struct Candidate {
+        float4 q;
+        float a;
+    };
+    auto fetch = [&](uint32_t k) { return Candidate{__ldg(&src[k]), __ldg(&xa[k])}; };
+    auto visit = [&](uint32_t k, const Candidate& f, float oy, float oz) {
+        const float4& q = f.q;
+        const float ox = __fadd_rn(__fsub_rn(ax, f.a), l.x);
         const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
         body(k, q, rx, ry, rz, dist2(rx, ry, rz));
     };
@@ -709,7 +761,7 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
             const uint32_t base = cell_hash(c.g, x0, y, z);
             const uint32_t a0 = row_base(cstart[base]);
             if (mask) {
-                if (queue.full()) queue.drain(o, visit);
+                if (queue.full()) queue.template drain<false>(o, fetch, visit);
                 queue.push(mask, a0, uint32_t(y - y0), uint32_t(z - z0));
             }
             if (long_row) {
@@ -725,14 +777,14 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
                         more |= r2 < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
                     }
                     if (more) {
-                        if (queue.full()) queue.drain(o, visit);
+                        if (queue.full()) queue.template drain<false>(o, fetch, visit);
                         queue.push(more, c0, uint32_t(y - y0), uint32_t(z - z0));
                     }
                 }
             }
         }
     }
-    queue.drain(o, visit);
+    queue.template drain<true>(o, fetch, visit);
 }
 
 // The position update of one particle whose pair sums are (dx, dy, dz): box

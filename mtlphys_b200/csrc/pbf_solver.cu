@@ -19,27 +19,25 @@ namespace {
 inline uint32_t cdiv(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 // Launch shape of the solver kernels, measured on the 1,003,520-particle dam
-// break: blocks of 128 threads (1473 us per step; 64: 1606, 256: 1605 us with
-// the delta passes at 48 registers, where 128 takes 1599), and a residency
-// target that caps registers at 65536 / (256 * N): N = 4 (64 registers) for all
-// of them (lambda passes at N = 3: 1698, 5: 1636; delta passes at N = 5, which
-// spills: 1599, 6: 1656 us).
+// break: blocks of 128 threads (64 and 256 are within 0.5%), and at least 8 of
+// them per SM, which caps registers at 64: 1440 us per step (lambda passes at 9
+// blocks, 56 registers, +1.5%; delta passes +3.5%; fewer blocks 10% and more).
 #ifndef MPB_SOLVER_BLOCK
 #define MPB_SOLVER_BLOCK 128
 #endif
 constexpr uint32_t kSB = MPB_SOLVER_BLOCK;
 #ifndef MPB_LAMBDA_MIN_BLOCKS
-#define MPB_LAMBDA_MIN_BLOCKS 4
+#define MPB_LAMBDA_MIN_BLOCKS 8
 #endif
 #ifndef MPB_DELTA_MIN_BLOCKS
-#define MPB_DELTA_MIN_BLOCKS 4
+#define MPB_DELTA_MIN_BLOCKS 8
 #endif
 #ifndef MPB_DELTA_MID_MIN_BLOCKS
-#define MPB_DELTA_MID_MIN_BLOCKS 4
+#define MPB_DELTA_MID_MIN_BLOCKS 8
 #endif
 
 template <bool LAST>
-__global__ void __launch_bounds__(kSB, MPB_LAMBDA_MIN_BLOCKS * 256 / kSB)
+__global__ void __launch_bounds__(kSB, MPB_LAMBDA_MIN_BLOCKS)
 k_lambda_first(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
                uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
                const uint32_t* __restrict__ sidx, float* __restrict__ lambdas,
@@ -51,7 +49,7 @@ k_lambda_first(StepConsts c, const float4* __restrict__ cur, const uint32_t* __r
 }
 
 template <bool LAST>
-__global__ void __launch_bounds__(kSB, MPB_LAMBDA_MIN_BLOCKS * 256 / kSB)
+__global__ void __launch_bounds__(kSB, MPB_LAMBDA_MIN_BLOCKS)
 k_lambda(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
          const uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
          const uint32_t* __restrict__ sidx, float* __restrict__ lambdas, RowMasks rm) {
@@ -63,7 +61,7 @@ k_lambda(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restric
 // SN = 4: the reference's s_corr exponent, fixed at compile time (the host
 // launches this instance when scorr_n == 4); SN = 0 reads it from c.
 template <bool LAST, uint32_t SN>
-__global__ void __launch_bounds__(kSB, (LAST ? MPB_DELTA_MIN_BLOCKS : MPB_DELTA_MID_MIN_BLOCKS) * 256 / kSB)
+__global__ void __launch_bounds__(kSB, LAST ? MPB_DELTA_MIN_BLOCKS : MPB_DELTA_MID_MIN_BLOCKS)
 k_delta(StepConsts c, const float4* __restrict__ src, float4* __restrict__ dst, uint32_t* __restrict__ qpos,
         const float* __restrict__ xa,
         const uint32_t* __restrict__ scell, const uint32_t* __restrict__ cstart,
