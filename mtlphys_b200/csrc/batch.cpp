@@ -250,6 +250,8 @@ struct mp_batch {
         const Slot& sl = slots[i];
         AdjArgs ad = adj;
         ad.scorr4 = a.scorr4;
+        ad.common = a.common;
+        ad.pair = a.pair;
         ad.t = AdjStep{sl.rec.scenes, sl.rec.sphere0, sl.x0, x1, sl.sidx, sl.scell, sl.cstart,
                        sl.rec.lam, sl.rec.delta, sl.rec.masks, sl.rec.overflow};
         const cudaError_t e = launch_adjoint_step(ad, s);
@@ -296,6 +298,18 @@ struct mp_batch {
     uint32_t useful_blocks(uint32_t n) const {
         const uint64_t lanes = std::max<uint32_t>(1u, team_lanes(n));
         return uint32_t(std::max<uint64_t>(1u, (n * lanes + block - 1) / block));
+    }
+
+    // What the scenes' constants have in common (kernels fix it, or take it as an argument).
+    void note_consts() {
+        a.scorr4 = 1;
+        a.common = S ? 1 : 0;
+        for (uint32_t s = 0; s < S; ++s) {
+            const PairConsts p = pair_consts(host_scenes[s].c);
+            if (s == 0) a.pair = p;
+            if (std::memcmp(&p, &a.pair, sizeof(p)) != 0) a.common = 0;
+            if (p.scorr_n != 4) a.scorr4 = a.common = 0;
+        }
     }
 
     // launch arguments with the current bound of the barrier wait
@@ -541,9 +555,7 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         MP_ALLOC(b->scenes, sizeof(SceneDev) * std::max<uint32_t>(nscenes, 1u), b->device);
         a.scenes = b->scenes;
         a.iterations = iters;
-        a.scorr4 = 1;
-        for (uint32_t s = 0; s < nscenes; ++s)
-            if (params[s].scorr_n != 4) a.scorr4 = 0;
+        b->note_consts();
         int rc = b->upload_scenes();
         if (rc != MP_OK) return rc;
         if (total) {
@@ -823,10 +835,8 @@ int mp_batch_set_params(mp_batch* b, uint32_t scene, const mp_pbf_params* params
                         b->scene_ids[scene] == MP_SCENE_SPHERE_DROP);
     MP_CUDA(cudaMemcpy(&b->scenes[scene], &cur, sizeof(SceneDev), cudaMemcpyHostToDevice));
     b->params[scene] = *params;
-    b->a.scorr4 = 1;
-    for (const mp_pbf_params& q : b->params)
-        if (q.scorr_n != 4) b->a.scorr4 = 0;
     b->host_scenes[scene].c = cur.c;
+    b->note_consts();
     b->drop_graph();
     return MP_OK;
 }

@@ -68,11 +68,6 @@ __device__ __forceinline__ bool cells_adjacent(uint32_t a, uint32_t b, bool wide
 // Kernel values of a pair at offset r with 1e-12 < |r|^2 = r2 < h^2:
 // spiky gradient g = f r, its Jacobian H v = f v + fp (r . v) r, the poly6
 // weight W and d = h^2 - r2 (grad W = -6 poly6 d^2 r).
-struct PairConsts {
-    float h, h2, poly6, spiky;
-    __device__ __forceinline__ explicit PairConsts(const StepConsts& c)
-        : h(c.h), h2(c.h2), poly6(c.poly6), spiky(c.spiky) {}
-};
 struct PairTerms {
     float d, f, fp, W;
     __device__ __forceinline__ PairTerms(const PairConsts& c, float r2) {
@@ -316,7 +311,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
 constexpr int kSweepMinBlocks = MPB_ADJ_SWEEP_MIN_BLOCKS;
 constexpr uint32_t kSweepBlock = 128;
 
-template <uint32_t SN>
+template <uint32_t SN, bool COMMON>
 __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjArgs a, uint32_t it) {
     __shared__ uint2 queue[kQueue * kSweepBlock];
     const uint32_t m = blockIdx.x * kSweepBlock + threadIdx.x;
@@ -332,10 +327,11 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjA
     const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
     int cx, cy, cz;
     cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
-    // kept in registers: a post would otherwise make every pair load them again
-    const PairConsts pc(c);
-    const float inv_wq = c.inv_wq, scorr_k = c.scorr_k, ir = c.inv_rho0;
-    const uint32_t n = SN ? SN : c.scorr_n;
+    // a kernel argument, or kept in registers: a post would otherwise make every
+    // pair load them again
+    const PairConsts pc = COMMON ? a.pair : pair_consts(c);
+    const float inv_wq = pc.inv_wq, scorr_k = pc.scorr_k, ir = pc.inv_rho0;
+    const uint32_t n = SN ? SN : pc.scorr_n;
     float dens = pc.poly6 * pc.h2 * pc.h2 * pc.h2;  // the particle itself
     float gx = 0.0f, gy = 0.0f, gz = 0.0f, gsq = 0.0f;
     float lb = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f, kb = 0.0f;
@@ -415,6 +411,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_lbar(AdjArgs a, uint32_t it) {
 //   pbar_i += sum_j (rhobar_i + rhobar_j) grad W_ij
 //             + H_ij (Gbar_i - Gbar_j + 2 (Qbar_i + Qbar_j) g_ij)
 // (j-side terms of one-way pairs added to j atomically).
+template <bool COMMON>
 __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(AdjArgs a, uint32_t it) {
     __shared__ uint2 queue[kQueue * kSweepBlock];
     const uint32_t m = blockIdx.x * kSweepBlock + threadIdx.x;
@@ -433,7 +430,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(Adj
     cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
     const float4 qb = a.qbar[m];
     float px = qb.x, py = qb.y, pz = qb.z;
-    const PairConsts pc(c);
+    const PairConsts pc = COMMON ? a.pair : pair_consts(c);
     const float w6 = -6.0f * pc.poly6;
     auto body = [&](uint32_t k, const float4&, float rx, float ry, float rz, float r2) {
         if (!(r2 < pc.h2 && r2 > 1e-12f)) return;
@@ -644,12 +641,17 @@ cudaError_t launch_adjoint_step(const AdjArgs& a, cudaStream_t s) {
     k_adj_finalize<<<grid, kBlock, 0, s>>>(a);
     for (uint32_t it = a.iterations; it-- > 0;) {
         k_adj_pre<<<grid, kBlock, 0, s>>>(a, it);
-        if (a.scorr4)
-            k_adj_delta<4><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
+        if (a.common)
+            k_adj_delta<4, true><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
+        else if (a.scorr4)
+            k_adj_delta<4, false><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         else
-            k_adj_delta<0><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
+            k_adj_delta<0, false><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         k_adj_lbar<<<grid, kBlock, 0, s>>>(a, it);
-        k_adj_lambda<<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
+        if (a.common)
+            k_adj_lambda<true><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
+        else
+            k_adj_lambda<false><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
     }
     k_adj_predict<<<grid, kBlock, 0, s>>>(a);
     if (a.nscenes && a.sum_chunks) k_adj_sphere_sum<<<dim3(a.sum_chunks, a.nscenes), kBlock, 0, s>>>(a);

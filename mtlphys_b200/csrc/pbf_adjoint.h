@@ -59,6 +59,8 @@ struct AdjArgs {
     uint32_t* cpred;
     float* xa;                    // x anchor of each slot's hash cell
     uint32_t wide;                // 1: some scene's grid is too wide for the packed cell comparison
+    uint32_t common;              // 1: every scene has the pair constants `pair`
+    PairConsts pair;
     uint32_t scorr4;              // 1: every scene's s_corr exponent is 4
     // one-way pair posts: per receiver slot a count and kInbox (sender,
     // value) entries (entry e of receiver j at e * stride + j); further posts

@@ -154,11 +154,25 @@ constexpr int batch_min_blocks() {
     return int(65536u / (BS * 64u));
 }
 
+template <bool COMMON>
+__device__ __forceinline__ const auto& pair_constants(const BatchArgs& a, const StepConsts& c) {
+    if constexpr (COMMON)
+        return a.pair;
+    else
+        return c;
+}
+
 // SN: the s_corr exponent fixed at compile time (4, when every scene uses
 // the reference's) or read per scene (0); both give the same bits for 4.
 // G: lanes per particle of the solver phases (kTeam) or 0 for one each
 // (team_lanes(); the same bits).
-template <uint32_t BS, uint32_t SN, uint32_t G>
+// COMMON: every scene has the constants a.pair, which as an argument need no
+// registers; per scene they are loads and a register each, of which the solver
+// phases at 64 have none to spare (spill loads 388 -> 128 bytes with REC fixed
+// too; 256 cubes, 4.2 M particles: 4.44 -> 4.23 ms; 12 small ones 182 -> 168 us).
+// REC: whether the step is recorded, fixed at compile time (0, 1) or read from
+// the arguments (2).
+template <uint32_t BS, uint32_t SN, uint32_t G, bool COMMON, int REC>
 __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(BatchArgs a) {
     __shared__ uint32_t s_warp[BS / 32 + 1];
     __shared__ int s_flags[2];
@@ -359,7 +373,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     }
     // a recorded step keeps every lambda pass's output, row masks and
     // corrections in the record instead of overwriting one buffer
-    const bool record = a.rec.lam != nullptr;
+    const bool record = REC == 2 ? a.rec.lam != nullptr : REC == 1;
     for (uint32_t it = 0; it < a.iterations; ++it) {
         const bool last = it + 1 == a.iterations;
         float4* lam_out = record ? a.rec.lam + size_t(it) * a.rec.stride : a.sorted_b;
@@ -371,6 +385,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         constexpr uint32_t lanes = G ? G : 1u;
         for (uint32_t s = pb + gtid / lanes; s < pe; s += gsize / lanes) {
             const StepConsts& c = sc[a.scene_of[s]].c;
+            const auto& pc = pair_constants<COMMON>(a, c);
             if constexpr (G != 0) {
                 if (it == 0) {
                     if (last)
@@ -388,22 +403,23 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
                 }
             } else if (it == 0) {
                 if (last)
-                    lambda_first_item<true, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                    lambda_first_item<true, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
                                                 a.lambdas, a.ncount, rmi, queue);
                 else
-                    lambda_first_item<false, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                    lambda_first_item<false, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
                                                  a.lambdas, a.ncount, rmi, queue);
             } else if (last) {
-                lambda_item<true, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                lambda_item<true, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
                                       rmi, queue);
             } else {
-                lambda_item<false, BS>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                lambda_item<false, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
                                        rmi, queue);
             }
         }
         if (!grid_barrier(a, s_flags)) return;
         for (uint32_t s = pb + gtid / lanes; s < pe; s += gsize / lanes) {
             const SceneDev& sd = sc[a.scene_of[s]];
+            const auto& pc = pair_constants<COMMON>(a, sd.c);
             if constexpr (G != 0) {
                 if (last)
                     team_delta<true, SN, G>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
@@ -414,11 +430,11 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
                                              &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
                                              bufs);
             } else if (last) {
-                delta_item<true, SN, BS>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                delta_item<true, SN, BS>(sd.c, pc, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
                                          &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
                                          queue);
             } else {
-                delta_item<false, SN, BS>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                delta_item<false, SN, BS>(sd.c, pc, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
                                           &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
                                           queue);
             }
@@ -434,13 +450,17 @@ constexpr size_t shared_bytes(bool team) {
     return team ? sizeof(TeamBuf) * (BS / kTeam) : sizeof(uint2) * kQueue * BS;
 }
 
+// The step kernel for a launch with these properties (common implies scorr4).
 template <uint32_t BS>
-const void* batch_kernel(bool scorr4, bool team) {
+const void* batch_kernel(bool scorr4, bool common, bool team, bool record) {
     if (team)
-        return scorr4 ? reinterpret_cast<const void*>(&k_batch_step<BS, 4, kTeam>)
-                      : reinterpret_cast<const void*>(&k_batch_step<BS, 0, kTeam>);
-    return scorr4 ? reinterpret_cast<const void*>(&k_batch_step<BS, 4, 0>)
-                  : reinterpret_cast<const void*>(&k_batch_step<BS, 0, 0>);
+        return scorr4 ? reinterpret_cast<const void*>(&k_batch_step<BS, 4, kTeam, false, 2>)
+                      : reinterpret_cast<const void*>(&k_batch_step<BS, 0, kTeam, false, 2>);
+    if (common)
+        return record ? reinterpret_cast<const void*>(&k_batch_step<BS, 4, 0, true, 1>)
+                      : reinterpret_cast<const void*>(&k_batch_step<BS, 4, 0, true, 0>);
+    return scorr4 ? reinterpret_cast<const void*>(&k_batch_step<BS, 4, 0, false, 2>)
+                  : reinterpret_cast<const void*>(&k_batch_step<BS, 0, 0, false, 2>);
 }
 
 cudaError_t allow_shared(const void* fn, size_t bytes) {
@@ -452,7 +472,7 @@ template <uint32_t BS>
 cudaError_t launch_bs(const BatchArgs& args, uint32_t blocks, cudaStream_t s) {
     void* kargs[] = {const_cast<BatchArgs*>(&args)};
     const bool team = args.iterations && team_lanes(args.p_end - args.p_begin) != 0;
-    const void* fn = batch_kernel<BS>(args.scorr4 != 0, team);
+    const void* fn = batch_kernel<BS>(args.scorr4 != 0, args.common != 0, team, args.rec.lam != nullptr);
     const size_t bytes = shared_bytes<BS>(team);
     const cudaError_t e = allow_shared(fn, bytes);
     if (e != cudaSuccess) return e;
@@ -463,9 +483,9 @@ cudaError_t launch_bs(const BatchArgs& args, uint32_t blocks, cudaStream_t s) {
 template <uint32_t BS>
 int occupancy_bs() {
     int least = 1 << 30;
-    for (int i = 0; i < 4; ++i) {
-        const bool scorr4 = i & 1, team = i & 2;
-        const void* fn = batch_kernel<BS>(scorr4, team);
+    for (int i = 0; i < 16; ++i) {
+        const bool team = i & 1;
+        const void* fn = batch_kernel<BS>(i & 2, i & 4, team, i & 8);
         int n = 0;
         if (allow_shared(fn, shared_bytes<BS>(team)) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, BS, shared_bytes<BS>(team)) != cudaSuccess)

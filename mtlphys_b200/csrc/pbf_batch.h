@@ -62,6 +62,8 @@ struct BatchArgs {
     // many more blocks than the launch has, so that each wait runs out.
     uint32_t* abort;
     uint32_t spin_limit, bar_extra;
+    uint32_t common;  // 1: every scene has the pair constants `pair`, with an s_corr exponent of 4
+    PairConsts pair;
     uint32_t scorr4;  // 1: every scene's s_corr exponent is 4 (the kernel fixes it at compile time)
     BatchRecord rec;
 };

@@ -62,6 +62,23 @@ struct StepConsts {
     float q_lim;   // particles further than this from their cell's corner skip the prefilter
 };
 
+// The constants of the pair loops.  Where they are a kernel argument (a single
+// scene, or a batch whose scenes share them) they cost no registers.
+struct PairConsts {
+    float h, h2, poly6, spiky;
+    float inv_rho0, inv_wq, scorr_k, scorr_pq;
+    uint32_t scorr_n;
+};
+
+#ifdef __CUDACC__
+__host__ __device__ __forceinline__
+#else
+inline
+#endif
+PairConsts pair_consts(const StepConsts& c) {
+    return PairConsts{c.h, c.h2, c.poly6, c.spiky, c.inv_rho0, c.inv_wq, c.scorr_k, c.scorr_pq, c.scorr_n};
+}
+
 // Device-resident sphere state: center xyz, velocity xyz, radius.
 struct SphereState {
     float c[3];

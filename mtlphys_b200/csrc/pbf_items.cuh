@@ -254,6 +254,9 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
     return r;
 }
+// The pair functions take the constants as C: StepConsts, or PairConsts where a
+// batch's scenes share them.
+
 // densityLambdaSorted's sums for one particle (Constraints.metal:99-121): the
 // density starts at the particle's own W(0) whether or not its slot lies in
 // the stencil of its current cell (a particle can drift two cells from its
@@ -263,11 +266,13 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 struct LambdaAcc {
     float dens = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f, gsq = 0.0f;
     // the particle's own W(0)
-    __device__ __forceinline__ void self(const StepConsts& c) {
+    template <class C>
+    __device__ __forceinline__ void self(const C& c) {
         dens = __fmul_rn(__fmul_rn(__fmul_rn(c.poly6, c.h2), c.h2), c.h2);
     }
     // no effect unless r2 < h^2
-    __device__ __forceinline__ void add(const StepConsts& c, float rx, float ry, float rz, float r2) {
+    template <class C>
+    __device__ __forceinline__ void add(const C& c, float rx, float ry, float rz, float r2) {
         const float d = __fsub_rn(c.h2, r2);
         const float rinv = rsqrt_normal(r2);
         const float hd = fmaxf(__fsub_rn(c.h, __fmul_rn(r2, rinv)), 0.0f);
@@ -310,8 +315,8 @@ __device__ __forceinline__ float scorr_pow(float x, uint32_t n) {
 //   (lambda_i + lambda_j - k (W / W(dq))^n) (h - r)^2 / r  r
 // W / W(dq) = d^3 poly6 / W(dq) (c.scorr_pq); the sum of lambdas and s_corr is
 // one fused multiply-add.  No effect unless r2 < h^2.
-template <uint32_t N>
-__device__ __forceinline__ float delta_coef(const StepConsts& c, float li, float lj, float r2) {
+template <uint32_t N, class C>
+__device__ __forceinline__ float delta_coef(const C& c, float li, float lj, float r2) {
     const float d = __fsub_rn(c.h2, r2);
     const float ratio = __fmul_rn(__fmul_rn(__fmul_rn(d, d), d), c.scorr_pq);
     const float rinv = rsqrt_normal(r2);
@@ -320,8 +325,8 @@ __device__ __forceinline__ float delta_coef(const StepConsts& c, float li, float
                      __fmul_rn(__fmul_rn(hd, hd), rinv));
 }
 
-template <uint32_t N>
-__device__ __forceinline__ void delta_add(const StepConsts& c, float li, float lj, float rx, float ry,
+template <uint32_t N, class C>
+__device__ __forceinline__ void delta_add(const C& c, float li, float lj, float rx, float ry,
                                           float rz, float r2, float& dx, float& dy, float& dz) {
     const float coef = delta_coef<N>(c, li, lj, r2);
     if (r2 < c.h2 && r2 > 1e-12f) {
@@ -595,8 +600,8 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
 // First lambda pass: absolute FP32 predicted positions (reference arithmetic,
 // so the fused neighbour count equals countNeighbors bit for bit); converts
 // the state to anchored offsets for the following passes.
-template <bool LAST, uint32_t BS>
-__device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t s,
+template <bool LAST, uint32_t BS, class C>
+__device__ __forceinline__ void lambda_first_item(const StepConsts& c, const C& pc, uint32_t s,
                                                   const float4* __restrict__ cur,
                                                   const uint32_t* __restrict__ qpos,
                                                   float4* __restrict__ nxt,
@@ -618,13 +623,13 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t 
     uint32_t qi;
     const int nthr = prefilter(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, lx, ly, lz, qi);
     LambdaAcc acc;
-    acc.self(c);
+    acc.self(pc);
     uint32_t cnt = 0;
     sweep<false, BS>(c, cur, qpos, cstart, cx, cy, cz, p.x, p.y, p.z, 0.0f, 0.0f, 0.0f, qi, nthr, s, rm,
                      PairQueue<BS>(queue),
                      [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
-                         cnt += r2 < c.h2 ? 1u : 0u;
-                         acc.add(c, rx, ry, rz, r2);
+                         cnt += r2 < pc.h2 ? 1u : 0u;
+                         acc.add(pc, rx, ry, rz, r2);
                      });
     const float lambda = acc.lambda(c);
     nxt[s] = make_float4(lx, ly, lz, lambda);
@@ -636,8 +641,8 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, uint32_t 
 
 // Later lambda passes on the anchored state: cur is the previous delta pass's
 // output, (l, x anchor of the hash cell) per slot.
-template <bool LAST, uint32_t BS>
-__device__ __forceinline__ void lambda_item(const StepConsts& c, uint32_t s,
+template <bool LAST, uint32_t BS, class C>
+__device__ __forceinline__ void lambda_item(const StepConsts& c, const C& pc, uint32_t s,
                                             const float4* __restrict__ cur,
                                             const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
                                             const uint32_t* __restrict__ scell,
@@ -652,11 +657,11 @@ __device__ __forceinline__ void lambda_item(const StepConsts& c, uint32_t s,
     uint32_t qi;
     const int nthr = prefilter(c, pcx + c.g.lx, pcy + c.g.ly, pcz + c.g.lz, l.x, l.y, l.z, qi);
     LambdaAcc acc;
-    acc.self(c);
+    acc.self(pc);
     sweep<true, BS>(c, cur, qpos, cstart, cx, cy, cz, l.x, l.y, l.z, ax, ay, az, qi, nthr, s, rm,
                     PairQueue<BS>(queue),
                     [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
-                        acc.add(c, rx, ry, rz, r2);
+                        acc.add(pc, rx, ry, rz, r2);
                     });
     const float lambda = acc.lambda(c);
     nxt[s] = make_float4(l.x, l.y, l.z, lambda);
@@ -846,8 +851,8 @@ __device__ __forceinline__ void delta_apply(const StepConsts& c, uint32_t s, con
 // iteration also scatters back, finalizes and writes foam.  drec (may be
 // NULL): receives the particle's unclamped correction, for the adjoint.
 // SN: the s_corr exponent when fixed at compile time (4), else 0.
-template <bool LAST, uint32_t SN, uint32_t BS>
-__device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
+template <bool LAST, uint32_t SN, uint32_t BS, class C>
+__device__ __forceinline__ void delta_item(const StepConsts& c, const C& pc, uint32_t s,
                                            const float4* __restrict__ src, float4* __restrict__ dst,
                                            uint32_t* __restrict__ qpos, const float* __restrict__ xa,
                                            const uint32_t* __restrict__ scell,
@@ -867,7 +872,7 @@ __device__ __forceinline__ void delta_item(const StepConsts& c, uint32_t s,
     cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
     float dx = 0.0f, dy = 0.0f, dz = 0.0f;
     auto body = [&](uint32_t, const float4& q, float rx, float ry, float rz, float r2) {
-        delta_add<SN>(c, l.w, q.w, rx, ry, rz, r2, dx, dy, dz);
+        delta_add<SN>(pc, l.w, q.w, rx, ry, rz, r2, dx, dy, dz);
     };
     queued_pairs<BS>(c, src, xa, cstart, rm, s, l, ax, ay, az, cx, cy, cz, PairQueue<BS>(queue), body);
     delta_apply<LAST>(c, s, l, ax, ay, az, pcx, pcy, pcz, dx, dy, dz, dst, qpos, sidx, sphere, pos, vel, prev,

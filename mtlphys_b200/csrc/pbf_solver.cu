@@ -45,7 +45,7 @@ k_lambda_first(StepConsts c, const float4* __restrict__ cur, const uint32_t* __r
     __shared__ uint2 queue[kQueue * kSB];
     const uint32_t s = blockIdx.x * kSB + threadIdx.x;
     if (s < c.n)
-        lambda_first_item<LAST, kSB>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm, queue);
+        lambda_first_item<LAST, kSB>(c, c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm, queue);
 }
 
 template <bool LAST>
@@ -55,7 +55,7 @@ k_lambda(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restric
          const uint32_t* __restrict__ sidx, float* __restrict__ lambdas, RowMasks rm) {
     __shared__ uint2 queue[kQueue * kSB];
     const uint32_t s = blockIdx.x * kSB + threadIdx.x;
-    if (s < c.n) lambda_item<LAST, kSB>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm, queue);
+    if (s < c.n) lambda_item<LAST, kSB>(c, c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm, queue);
 }
 
 // SN = 4: the reference's s_corr exponent, fixed at compile time (the host
@@ -71,7 +71,7 @@ k_delta(StepConsts c, const float4* __restrict__ src, float4* __restrict__ dst, 
     __shared__ uint2 queue[kQueue * kSB];
     const uint32_t s = blockIdx.x * kSB + threadIdx.x;
     if (s < c.n)
-        delta_item<LAST, SN, kSB>(c, s, src, dst, qpos, xa, scell, cstart, sidx, sphere, pos, vel, prev, ncount,
+        delta_item<LAST, SN, kSB>(c, c, s, src, dst, qpos, xa, scell, cstart, sidx, sphere, pos, vel, prev, ncount,
                                   foam, err, rm, nullptr, queue);
 }
 

@@ -191,3 +191,25 @@ def test_random_cloud_scenes(batch, cuda):
             assert_positions(pos[f:f + n], o["pos"], position_tolerance(p, dt, mid_p, mid_v))
     finally:
         e.close()
+
+
+def test_scenes_with_and_without_common_constants_give_identical_results(batch):
+    """Scenes that share the pair constants run with them as kernel arguments; a
+    scene with another s_corr k, or another exponent, switches the batch to
+    per-scene constants.  The other scenes keep their bits."""
+    w = configs.batch_cubes(num=4, lo=5000, hi=9000)
+    assert sum(w.counts) > 16384  # one lane per particle
+    outs = []
+    for change in (None, {"scorr_k": 0.07}, {"scorr_n": 3}):
+        batch.reset(w.counts, w.params, w.dts, w.scenes, w.descs)
+        if change:
+            batch.set_params(3, batch.params(3).set(**change))
+        for _ in range(3):
+            batch.step()
+        assert batch.check_errors() == 0
+        last = batch.scene_range(3)[0]
+        outs.append((batch.positions(), batch.velocities(), last))
+    for pos, vel, last in outs[1:]:
+        np.testing.assert_array_equal(pos[:last], outs[0][0][:last])
+        np.testing.assert_array_equal(vel[:last], outs[0][1][:last])
+        assert not np.array_equal(pos[last:], outs[0][0][last:])
