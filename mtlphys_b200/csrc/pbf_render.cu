@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) k_splat(RenderConsts c, const float4* __r
 
 // The block's depths with their 4-pixel border and the 81 weights in shared
 // memory: a pixel used to load each tap and evaluate expf 81 times (960 x 540:
-// 16 -> 6 us).
+// 17 -> 8 us).
 __global__ void __launch_bounds__(256) k_smooth(RenderConsts c, const uint32_t* __restrict__ depth,
                                                 float* __restrict__ smoothed) {
     __shared__ uint32_t s_depth[24][25];
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256) k_saturate(uint32_t n, float4* __restrict
 // stepping the major axis through pixel centres.  A thread per edge and pixel;
 // where edges share a pixel, the first one's thread blends all of them in edge
 // order, so the result is deterministic.  (One block running the edges one after
-// another took 22 us at 960 x 540, this takes 4.)
+// another took 22 us at 960 x 540, this takes 5.)
 struct Edge {
     float a0, a1, b0, b1, z0, z1;  // screen coordinate along and across the major axis, NDC z
     int m0, m1;                    // pixels along the major axis (m0 > m1: not visible)
