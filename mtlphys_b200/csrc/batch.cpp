@@ -467,6 +467,7 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         std::copy(tmp.begin(), tmp.end(), pos.begin() + 4 * off);
         std::fill(scene_of.begin() + off, scene_of.begin() + off + counts[s], s);
         std::memset(&hs[s], 0, sizeof(SceneDev));
+        empty_box(hs[s].bb);
         hs[s].c = make_consts(params[s], grids[s], counts[s], dts[s], sid == MP_SCENE_SPHERE_DROP);
         hs[s].p0 = uint32_t(off);
         for (int a = 0; a < 3; ++a) {
@@ -550,8 +551,8 @@ int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const 
         a.long_count = sm + 0;
         a.total_cells = sm + 1;
         a.err = sm + 2;
-        a.abort = sm + 48;
         a.bar = reinterpret_cast<unsigned*>(sm + 64);
+        a.abort = a.bar + kBarGen + 1;
         MP_ALLOC(b->scenes, sizeof(SceneDev) * std::max<uint32_t>(nscenes, 1u), b->device);
         a.scenes = b->scenes;
         a.iterations = iters;
@@ -1015,9 +1016,8 @@ int mp_batch_check_errors(mp_batch* b, uint32_t* bits) {
         MP_CUDA(cudaMemset(b->a.err, 0, 4));
         if (w & kDevErrSpin) {
             // a barrier wait gave up: the launch left the barrier's counters
-            // mid-count and the abort flag set; re-arm both
+            // mid-count and the abort flag (one of its words) set; re-arm both
             MP_CUDA(cudaMemset(b->a.bar, 0, sizeof(unsigned) * kBarWords));
-            MP_CUDA(cudaMemset(b->a.abort, 0, sizeof(uint32_t)));
         }
     }
     if (bits) *bits = w;

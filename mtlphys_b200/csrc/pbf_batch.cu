@@ -15,11 +15,12 @@
 // block that gives up sets MP_DEVERR_SPIN_LIMIT and an abort flag, and every
 // block leaves the launch at its next barrier, so no phase ever runs on the
 // incomplete output of an earlier one):
-//   0  per scene: reset the bounding box, advance the sphere
+//   0  per scene: advance the sphere; in the same phase
 //   1  per particle: predict, dense cell -> scene bounding box (atomics,
 //      reduced per warp first)
 //   2  one block: per-scene sub-grid dims and cell offsets (exclusive scan)
-//   3  per particle: cell id in the scene's box, warp-aggregated count
+//   3  per particle: cell id in the scene's box, warp-aggregated count; per
+//      scene: the bounding box emptied for the next step
 //   4  exclusive scan of the counts (tile sums, scan of the sums, tile scan)
 //   5  scatter, 6 stable re-rank + gather, 7 long segments
 //   8+ K x (lambda, delta); the last delta finalizes.
@@ -54,14 +55,25 @@ constexpr uint32_t kScanItems = 8;  // per thread and tile in phase 4
 // the phase before it, so a block that returns true works on complete data; a
 // block that left early never arrives at the next barrier, so nobody passes that
 // one.
+//
+// Every round trip to L2 on the way counts: a block keeps the generation it is at
+// (read once per launch), and the generation and the abort flag are the two
+// halves of one word.
+struct BarrierState {
+    unsigned gen;  // the generation this block waits to leave
+    int last, ok;
+};
+
+__device__ __forceinline__ uint2 bar_word(const BatchArgs& a) {
+    uint2 w;
+    asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(w.x), "=r"(w.y) : "l"(a.bar + kBarGen));
+    return w;
+}
+
 template <class Last>
-__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, int* s_flags, Last&& last) {
+__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, BarrierState* state, Last&& last) {
     __syncthreads();
-    volatile unsigned* vgen = a.bar + kBarGen;
-    volatile uint32_t* vabort = a.abort;
-    unsigned g = 0;
     if (threadIdx.x == 0) {
-        g = *vgen;
         __threadfence();
         // block b belongs to group b mod groups
         const uint32_t groups = min((gridDim.x + 31u) / 32u, kBarGroups), group = blockIdx.x % groups;
@@ -69,33 +81,31 @@ __device__ __forceinline__ bool grid_barrier(const BatchArgs& a, int* s_flags, L
         unsigned* count = a.bar + (1u + group) * kBarLine;
         int mine = 0;
         if (atomicAdd(count, 1u) + 1u == members) {
-            atomicExch(count, 0u);
+            *static_cast<volatile unsigned*>(count) = 0u;
             __threadfence();
             if (atomicAdd(a.bar + kBarRoot, 1u) + 1u == groups + a.bar_extra) {
-                atomicExch(a.bar + kBarRoot, 0u);
+                *static_cast<volatile unsigned*>(a.bar + kBarRoot) = 0u;
                 __threadfence();
                 mine = 1;
             }
         }
-        s_flags[0] = mine;
+        state->last = mine;
     }
     __syncthreads();
-    if (s_flags[0]) {
+    if (state->last) {
         last();
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
             atomicAdd(a.bar + kBarGen, 1u);
-            s_flags[1] = !*vabort;
+            state->ok = !bar_word(a).y;
+            ++state->gen;
         }
     } else if (threadIdx.x == 0) {
         int ok = 1;
         uint32_t spins = 0;
-        while (*vgen == g) {
-            if (*vabort) {
-                ok = 0;
-                break;
-            }
+        uint2 w = bar_word(a);
+        while (w.x == state->gen && !w.y) {
             if (++spins > a.spin_limit) {
                 atomicOr(a.err, kDevErrSpin);
                 atomicExch(a.abort, 1u);
@@ -103,17 +113,18 @@ __device__ __forceinline__ bool grid_barrier(const BatchArgs& a, int* s_flags, L
                 break;
             }
             __nanosleep(32);
+            w = bar_word(a);
         }
-        if (ok && *vabort) ok = 0;
+        state->ok = ok && !w.y;
+        ++state->gen;
         __threadfence();
-        s_flags[1] = ok;
     }
     __syncthreads();
-    return s_flags[1] != 0;
+    return state->ok != 0;
 }
 
-__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, int* s_flags) {
-    return grid_barrier(a, s_flags, [] {});
+__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, BarrierState* state) {
+    return grid_barrier(a, state, [] {});
 }
 
 template <uint32_t BS>
@@ -175,7 +186,7 @@ __device__ __forceinline__ const auto& pair_constants(const BatchArgs& a, const 
 template <uint32_t BS, uint32_t SN, uint32_t G, bool COMMON, int REC>
 __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(BatchArgs a) {
     __shared__ uint32_t s_warp[BS / 32 + 1];
-    __shared__ int s_flags[2];
+    __shared__ BarrierState s_bar;
     // one lane per particle: kQueue entries per thread; teams: a TeamBuf each
     extern __shared__ uint2 shared[];
     uint2* queue = shared;
@@ -187,21 +198,20 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         if (gtid == 0) atomicOr(a.err, kDevErrSpin);
         return;
     }
+    // (no barrier completes before this block arrives, so none has yet)
+    if (threadIdx.x == 0) s_bar.gen = bar_word(a).x;
     const uint32_t gsize = gridDim.x * BS;
     const uint32_t pb = a.p_begin, pe = a.p_end;
     // loops over particles run in whole warps (warp-level operations inside)
     const uint32_t pe_round = pb + ((pe - pb + 31u) & ~31u);
     SceneDev* sc = a.scenes;
 
-    // 0: reset bounding boxes, advance spheres, clear the long-segment queue
+    // 0: advance the spheres (the solver reads them), clear the long-segment queue
     for (uint32_t s = a.scene_begin + gtid; s < a.scene_end; s += gsize) {
-        sc[s].bb[0] = sc[s].bb[1] = sc[s].bb[2] = 0xffffffffu;
-        sc[s].bb[3] = sc[s].bb[4] = sc[s].bb[5] = 0u;
         if (a.rec.sphere0) a.rec.sphere0[s] = sc[s].sphere;
         if (sc[s].c.sphere) sphere_advance(sc[s].c, &sc[s].sphere);
     }
     if (gtid == 0) *a.long_count = 0;
-    if (!grid_barrier(a, s_flags)) return;
 
     // 1: predict + dense cell of the predicted position -> scene bounding box
     for (uint32_t i = pb + gtid; i < pe_round; i += gsize) {
@@ -263,11 +273,14 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         }
         if (threadIdx.x == 0) *a.total_cells = running;
     };
-    if (!grid_barrier(a, s_flags, lay_out)) return;
+    if (!grid_barrier(a, &s_bar, lay_out)) return;
 
-    // 3: cell id inside the scene's box + warp-aggregated count
-    if (a.rec.scenes)
-        for (uint32_t s = a.scene_begin + gtid; s < a.scene_end; s += gsize) a.rec.scenes[s] = sc[s];
+    // 3: cell id inside the scene's box + warp-aggregated count; the boxes are
+    // empty again for the next step
+    for (uint32_t s = a.scene_begin + gtid; s < a.scene_end; s += gsize) {
+        if (a.rec.scenes) a.rec.scenes[s] = sc[s];
+        empty_box(sc[s].bb);
+    }
     const uint32_t ncells = *a.total_cells;
     if (ncells > a.max_cells && gtid == 0) atomicOr(a.err, kDevErrIndex);
     const bool cells_ok = ncells <= a.max_cells;
@@ -286,7 +299,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         count_cell(active, cell, a.counts, &rank);
         if (active) a.off[i] = rank;
     }
-    if (!grid_barrier(a, s_flags)) return;
+    if (!grid_barrier(a, &s_bar)) return;
 
     // 4: exclusive scan of counts[0, ncells] into cstart (counts left zero)
     const uint32_t len = cells_ok ? ncells + 1u : 0u;
@@ -315,7 +328,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             running += total;
         }
     };
-    if (!grid_barrier(a, s_flags, scan_tiles)) return;
+    if (!grid_barrier(a, &s_bar, scan_tiles)) return;
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         // each thread owns kScanItems consecutive items of the tile
         uint32_t v[kScanItems], sum = 0;
@@ -335,17 +348,17 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
                 run += v[k];
             }
     }
-    if (!grid_barrier(a, s_flags)) return;
+    if (!grid_barrier(a, &s_bar)) return;
 
     // 5: scatter; 6: stable re-rank + gather; 7: long segments
     if (cells_ok)
         for (uint32_t i = pb + gtid; i < pe; i += gsize) scatter_item(i, a.hash, a.off, a.cstart, a.tmp);
-    if (!grid_barrier(a, s_flags)) return;
+    if (!grid_barrier(a, &s_bar)) return;
     if (cells_ok)
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             sort_gather_item(sc[a.scene_of[s]].c, s, a.tmp, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
                              a.qpos, a.xa, nullptr, a.long_list, a.long_count);
-    if (!grid_barrier(a, s_flags)) return;
+    if (!grid_barrier(a, &s_bar)) return;
     const uint32_t nl = cells_ok ? *static_cast<volatile uint32_t*>(a.long_count) : 0u;
     if (nl) {  // the same for every block: long_count is written before the barrier only
         for (uint32_t li = blockIdx.x; li < nl; li += gridDim.x) {
@@ -354,7 +367,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             long_segment(sd.c, cell, sd.p0, sd.p0 + sd.c.n, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
                          a.qpos, a.xa, nullptr, s_warp);
         }
-        if (!grid_barrier(a, s_flags)) return;
+        if (!grid_barrier(a, &s_bar)) return;
     }
 
     // 8+: solver
@@ -365,7 +378,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             for (uint32_t s = pb + gtid; s < pe; s += gsize)
                 count_neighbors_item<BS>(sc[a.scene_of[s]].c, s, a.sorted_a, a.qpos, a.cstart, a.sidx, a.ncount,
                                          1u, PairQueue<BS>(queue));
-        if (!grid_barrier(a, s_flags)) return;
+        if (!grid_barrier(a, &s_bar)) return;
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             finalize_sorted_item(sc[a.scene_of[s]].c, s, a.sorted_a, a.sidx, a.pos, a.vel, a.prev,
                                  a.ncount, a.foam, a.err);
@@ -416,7 +429,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
                                        rmi, queue);
             }
         }
-        if (!grid_barrier(a, s_flags)) return;
+        if (!grid_barrier(a, &s_bar)) return;
         for (uint32_t s = pb + gtid / lanes; s < pe; s += gsize / lanes) {
             const SceneDev& sd = sc[a.scene_of[s]];
             const auto& pc = pair_constants<COMMON>(a, sd.c);
@@ -439,7 +452,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
                                           queue);
             }
         }
-        if (!last && !grid_barrier(a, s_flags)) return;
+        if (!last && !grid_barrier(a, &s_bar)) return;
     }
 }
 

@@ -14,10 +14,21 @@ namespace mpb {
 struct SceneDev {
     StepConsts c;
     uint32_t p0;         // first particle (and first sorted slot) of the scene
-    uint32_t bb[6];      // min x, y, z / max x, y, z dense cell of this step
+    uint32_t bb[6];      // min x, y, z / max x, y, z dense cell of this step (empty between steps)
     uint32_t pad;
     SphereState sphere;  // used when c.sphere != 0
 };
+
+// An empty bounding box: what a step expects in SceneDev::bb, and leaves there.
+#ifdef __CUDACC__
+__host__ __device__ __forceinline__
+#else
+inline
+#endif
+void empty_box(uint32_t bb[6]) {
+    bb[0] = bb[1] = bb[2] = 0xffffffffu;
+    bb[3] = bb[4] = bb[5] = 0u;
+}
 
 // Recording of one step for the adjoint (lam == nullptr: not recording).
 // The step's prev, sidx, scell and cstart arrays are kept as well: for a
@@ -32,7 +43,8 @@ struct BatchRecord {
     uint32_t stride;       // slots per lam / delta array
 };
 
-// Words of the grid barrier's counters, a cache line each: the root, up to kBarGroups arrival counters, the generation.
+// Words of the grid barrier's counters, a cache line each: the root, up to kBarGroups arrival counters, the generation (and beside it
+// the abort flag).
 constexpr uint32_t kBarLine = 32, kBarGroups = 32;
 constexpr uint32_t kBarRoot = 0, kBarGen = (1 + kBarGroups) * kBarLine;
 constexpr uint32_t kBarWords = (2 + kBarGroups) * kBarLine;
