@@ -32,7 +32,7 @@
 // accumulated per slot and summed per scene in a fixed order.  Nothing is
 // added with float atomics, so the gradients are the same bytes on every run.
 #include "pbf_adjoint.h"
-#include "pbf_items.cuh"
+#include "pbf_team.cuh"
 
 namespace mpb {
 namespace {
@@ -65,35 +65,43 @@ __device__ __forceinline__ bool cells_adjacent(uint32_t a, uint32_t b, bool wide
     return abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1;
 }
 
-// Kernel values of a pair at offset r with 1e-12 < |r|^2 = r2 < h^2:
-// spiky gradient g = f r, its Jacobian H v = f v + fp (r . v) r, the poly6
-// weight W and d = h^2 - r2 (grad W = -6 poly6 d^2 r).
-struct PairTerms {
-    float d, f, fp, W;
-    __device__ __forceinline__ PairTerms(const PairConsts& c, float r2) {
-        d = c.h2 - r2;
-        const float rinv = rsqrt_normal(r2);
-        const float hd = fmaxf(c.h - r2 * rinv, 0.0f);
-        f = -c.spiky * hd * hd * rinv;
-        fp = c.spiky * d * rinv * rinv * rinv;
-        W = c.poly6 * d * d * d;
-    }
-    __device__ __forceinline__ float3 hess(float rx, float ry, float rz, float vx, float vy,
-                                           float vz) const {
-        const float a = fp * (rx * vx + ry * vy + rz * vz);
-        return make_float3(f * vx + a * rx, f * vy + a * ry, f * vz + a * rz);
-    }
-};
-
 // x^n; N = 4 is s_corr's exponent fixed at compile time (n - 1 = 3), with the
 // roundings of the loop.
 template <uint32_t N>
 __device__ __forceinline__ float pow_u(float x, uint32_t n) {
-    if (N == 4u) return x * x * x;
+    if (N == 4u) return __fmul_rn(__fmul_rn(x, x), x);
     float r = 1.0f;
-    for (uint32_t e = 0; e < n; ++e) r *= x;
+    for (uint32_t e = 0; e < n; ++e) r = __fmul_rn(r, x);
     return r;
 }
+
+// The pair terms below are written with explicit roundings, so that the sweeps
+// with one lane and with a team of lanes per slot give the same bits.
+
+__device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz) {
+    return __fmaf_rn(az, bz, __fmaf_rn(ay, by, __fmul_rn(ax, bx)));
+}
+
+// Kernel values of a pair at offset r with 1e-12 < |r|^2 = r2 < h^2:
+// spiky gradient g = f r, its Jacobian H v = f v + fp (r . v) r, d = h^2 - r2
+// (poly6 weight W = w d, grad W = -6 poly6 d^2 r).
+struct PairTerms {
+    float d, f, fp, w;
+    __device__ __forceinline__ PairTerms(const PairConsts& c, float r2) {
+        d = __fsub_rn(c.h2, r2);
+        const float rinv = rsqrt_normal(r2);
+        const float hd = fmaxf(__fmaf_rn(-r2, rinv, c.h), 0.0f);
+        f = __fmul_rn(__fmul_rn(__fmul_rn(-c.spiky, hd), hd), rinv);
+        fp = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(c.spiky, d), rinv), rinv), rinv);
+        w = __fmul_rn(__fmul_rn(c.poly6, d), d);
+    }
+    __device__ __forceinline__ float3 hess(float rx, float ry, float rz, float vx, float vy,
+                                           float vz) const {
+        const float a = __fmul_rn(fp, dot3(rx, ry, rz, vx, vy, vz));
+        return make_float3(__fmaf_rn(a, rx, __fmul_rn(f, vx)), __fmaf_rn(a, ry, __fmul_rn(f, vy)),
+                           __fmaf_rn(a, rz, __fmul_rn(f, vz)));
+    }
+};
 
 // Posts the term v that sender slot `from` owes receiver slot `to` (a
 // one-way pair): into one of the receiver's kInbox entries, or a pooled
@@ -302,14 +310,96 @@ __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
 // Both pair sweeps walk their pairs through a PairQueue (pbf_items.cuh), one
 // loop per slot instead of one per stencil row (10 -> 26 of 32 threads active),
 // and keep the scene's constants in registers.  Bound by issue and load latency.
-// 6 blocks of 128 per SM (80 registers, a small spill): gradient of 10 steps of
-// the 97,336-particle cube, forward included, 9.4 -> 7.6 ms (4 blocks: 8.8, 5:
-// 8.4, 8: 7.8 ms).
+// 7 blocks of 128 per SM (72 registers, a small spill): gradients of eight lakes
+// (386,000 particles) 8.0 ms, of the 97,336-particle cube 6.6 ms (5 blocks: 8.3 and
+// 7.3, 6: 8.05 and 6.55, 8: 8.0 and 6.65 ms).
 #ifndef MPB_ADJ_SWEEP_MIN_BLOCKS
-#define MPB_ADJ_SWEEP_MIN_BLOCKS 6
+#define MPB_ADJ_SWEEP_MIN_BLOCKS 7
 #endif
 constexpr int kSweepMinBlocks = MPB_ADJ_SWEEP_MIN_BLOCKS;
 constexpr uint32_t kSweepBlock = 128;
+
+// What a slot's delta sweep reads of its own.
+struct DeltaSlot {
+    float4 l, dm;
+    uint32_t pm;
+    float ax, ay, az;
+    int cx, cy, cz;
+    __device__ __forceinline__ DeltaSlot(const AdjArgs& a, const StepConsts& c, const float4* src, uint32_t m) {
+        l = src[m];
+        dm = a.dbar[m];
+        pm = a.cpred[m];
+        int pcx, pcy, pcz;
+        decode_cell(c.g, a.t.scell[m], pcx, pcy, pcz);
+        ax = anchor_x(c.g, pcx);
+        ay = anchor_y(c.g, pcy);
+        az = anchor_z(c.g, pcz);
+        cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
+    }
+};
+
+// A pair's terms in the delta sweep of slot m (1e-12 < r2 < h^2): the gradient
+// sums' (f r, f^2 r2), dL/dk's (-rn gdm), dL/d lambda's (gdd) and dL/d position's
+// (v).
+struct DeltaTerms {
+    float f, f2, rn, gdm, gdd, vx, vy, vz;
+};
+
+template <uint32_t SN>
+__device__ __forceinline__ DeltaTerms delta_terms(const AdjArgs& a, const PairConsts& pc, uint32_t n, float sgk,
+                                                  float li, const float4& dm, uint32_t pm, uint32_t m, uint32_t k,
+                                                  const float4& q, float rx, float ry, float rz, float r2) {
+    DeltaTerms r;
+    const float4 di = __ldg(&a.dbar[k]);
+    const PairTerms t(pc, r2);
+    r.f = t.f;
+    r.f2 = __fmul_rn(t.f, t.f);
+    const float fx = __fmul_rn(t.f, rx), fy = __fmul_rn(t.f, ry), fz = __fmul_rn(t.f, rz);  // g
+    const float ratio = __fmul_rn(__fmul_rn(t.w, t.d), pc.inv_wq);
+    const float rn1 = n ? pow_u<SN>(ratio, n - 1) : 0.0f;
+    r.rn = n ? __fmul_rn(rn1, ratio) : 1.0f;
+    const float coef = __fmaf_rn(-pc.scorr_k, r.rn, __fadd_rn(li, q.w));
+    const float sg = __fmul_rn(__fmul_rn(__fmul_rn(sgk, rn1), t.d), t.d);  // grad s_ij = sg r
+    r.gdm = dot3(fx, fy, fz, dm.x, dm.y, dm.z);
+    // a pair in both lists carries the other particle's terms too; a
+    // one-way pair owes it the negative of its own
+    const bool both = cells_adjacent(__float_as_uint(di.w), pm, a.wide);
+    const float ex = __fsub_rn(dm.x, both ? di.x : 0.0f), ey = __fsub_rn(dm.y, both ? di.y : 0.0f);
+    const float ez = __fsub_rn(dm.z, both ? di.z : 0.0f);
+    r.gdd = dot3(fx, fy, fz, ex, ey, ez);
+    const float3 hv = t.hess(rx, ry, rz, ex, ey, ez);
+    const float sgd = __fmul_rn(sg, r.gdd);
+    r.vx = __fmaf_rn(coef, hv.x, __fmul_rn(sgd, rx));
+    r.vy = __fmaf_rn(coef, hv.y, __fmul_rn(sgd, ry));
+    r.vz = __fmaf_rn(coef, hv.z, __fmul_rn(sgd, rz));
+    if (!both) {
+        const float ir = pc.inv_rho0;
+        post(a, k, m, make_float4(-r.vx * ir, -r.vy * ir, -r.vz * ir, r.gdd * ir));
+    }
+    return r;
+}
+
+// The sums of a slot's delta sweep, written out.
+__device__ __forceinline__ void delta_out(const AdjArgs& a, const StepConsts& c, uint32_t m, float gx, float gy,
+                                          float gz, float gsq, float kb, float lb, float px, float py, float pz) {
+    const float ir = c.inv_rho0;
+    const float4 qb = a.qbar[m];
+    a.qbar[m] = make_float4(__fmaf_rn(px, ir, qb.x), __fmaf_rn(py, ir, qb.y), __fmaf_rn(pz, ir, qb.z), 0.0f);
+    a.lam_part[m] = __fmul_rn(lb, ir);
+    const float g2 = __fadd_rn(dot3(gx, gy, gz, gx, gy, gz), gsq);
+    a.gd[m] = make_float4(gx, gy, gz, __fmaf_rn(__fmul_rn(ir, ir), g2, c.eps));
+    a.kacc[m] += double(__fmul_rn(kb, ir));  // this slot's share of dL/dk
+}
+
+__device__ __forceinline__ float scorr_grad(const PairConsts& pc, uint32_t n) {
+    return n ? 6.0f * pc.scorr_k * float(n) * pc.inv_wq * pc.poly6 : 0.0f;
+}
+
+__device__ __forceinline__ RowMasks recorded_masks(const AdjArgs& a, uint32_t it) {
+    const uint32_t ms = a.mask_stride;
+    return RowMasks{const_cast<uint32_t*>(a.t.masks) + size_t(it) * 9 * ms,
+                    const_cast<uint32_t*>(a.t.overflow) + size_t(it) * ms, ms};
+}
 
 template <uint32_t SN, bool COMMON>
 __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjArgs a, uint32_t it) {
@@ -317,72 +407,81 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjA
     const uint32_t m = blockIdx.x * kSweepBlock + threadIdx.x;
     if (m >= a.n) return;
     const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
-    const size_t off = size_t(it) * a.stride;
-    const float4* src = a.t.lam + off;
-    const float4 l = src[m];
-    const float4 dm = a.dbar[m];
-    const uint32_t pm = a.cpred[m];
-    int pcx, pcy, pcz;
-    decode_cell(c.g, a.t.scell[m], pcx, pcy, pcz);
-    const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
-    int cx, cy, cz;
-    cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
+    const float4* src = a.t.lam + size_t(it) * a.stride;
+    const DeltaSlot o(a, c, src, m);
     // a kernel argument, or kept in registers: a post would otherwise make every
     // pair load them again
     const PairConsts pc = COMMON ? a.pair : pair_consts(c);
-    const float inv_wq = pc.inv_wq, scorr_k = pc.scorr_k, ir = pc.inv_rho0;
     const uint32_t n = SN ? SN : pc.scorr_n;
-    float dens = pc.poly6 * pc.h2 * pc.h2 * pc.h2;  // the particle itself
+    const float sgk = scorr_grad(pc, n);
     float gx = 0.0f, gy = 0.0f, gz = 0.0f, gsq = 0.0f;
-    float lb = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f, kb = 0.0f;
-    const float sgk = n ? 6.0f * scorr_k * float(n) * inv_wq * pc.poly6 : 0.0f;
+    float kb = 0.0f, lb = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
     auto body = [&](uint32_t k, const float4& q, float rx, float ry, float rz, float r2) {
-        if (!(r2 < pc.h2)) return;
-        if (!(r2 > 1e-12f)) {
-            dens += pc.poly6 * (pc.h2 - r2) * (pc.h2 - r2) * (pc.h2 - r2);
-            return;
-        }
-        const float4 di = __ldg(&a.dbar[k]);
-        const PairTerms t(pc, r2);
-        dens += t.W;
-        const float fx = t.f * rx, fy = t.f * ry, fz = t.f * rz;  // g
-        gx += fx;
-        gy += fy;
-        gz += fz;
-        gsq += t.f * t.f * r2;
-        const float ratio = t.W * inv_wq;
-        const float rn1 = n ? pow_u<SN>(ratio, n - 1) : 0.0f;
-        const float rn = n ? rn1 * ratio : 1.0f;
-        const float coef = l.w + q.w - scorr_k * rn;
-        const float sg = sgk * rn1 * t.d * t.d;  // grad s_ij = sg r
-        kb -= rn * (fx * dm.x + fy * dm.y + fz * dm.z);
-        // a pair in both lists carries the other particle's terms too; a
-        // one-way pair owes it the negative of its own
-        const bool both = cells_adjacent(__float_as_uint(di.w), pm, a.wide);
-        const float ex = dm.x - (both ? di.x : 0.0f), ey = dm.y - (both ? di.y : 0.0f);
-        const float ez = dm.z - (both ? di.z : 0.0f);
-        const float gdd = fx * ex + fy * ey + fz * ez;
-        const float3 hv = t.hess(rx, ry, rz, ex, ey, ez);
-        const float vx = coef * hv.x + sg * gdd * rx;
-        const float vy = coef * hv.y + sg * gdd * ry;
-        const float vz = coef * hv.z + sg * gdd * rz;
-        lb += gdd;
-        px += vx;
-        py += vy;
-        pz += vz;
-        if (!both) post(a, k, m, make_float4(-vx * ir, -vy * ir, -vz * ir, gdd * ir));
+        if (!(r2 < pc.h2 && r2 > 1e-12f)) return;
+        const DeltaTerms t = delta_terms<SN>(a, pc, n, sgk, o.l.w, o.dm, o.pm, m, k, q, rx, ry, rz, r2);
+        gx = __fmaf_rn(t.f, rx, gx);
+        gy = __fmaf_rn(t.f, ry, gy);
+        gz = __fmaf_rn(t.f, rz, gz);
+        gsq = __fmaf_rn(t.f2, r2, gsq);
+        kb = __fmaf_rn(-t.rn, t.gdm, kb);
+        lb = __fadd_rn(lb, t.gdd);
+        px = __fadd_rn(px, t.vx);
+        py = __fadd_rn(py, t.vy);
+        pz = __fadd_rn(pz, t.vz);
     };
-    const uint32_t ms = a.mask_stride;
-    const RowMasks rm{const_cast<uint32_t*>(a.t.masks) + size_t(it) * 9 * ms,
-                      const_cast<uint32_t*>(a.t.overflow) + size_t(it) * ms, ms};
-    queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, rm, m, l, ax, ay, az, cx, cy, cz,
-                              PairQueue<kSweepBlock>(queue), body);
-    const float4 qb = a.qbar[m];
-    a.qbar[m] = make_float4(qb.x + px * ir, qb.y + py * ir, qb.z + pz * ir, 0.0f);
-    a.lam_part[m] = lb * ir;
-    const float D = ir * ir * (gx * gx + gy * gy + gz * gz + gsq) + c.eps;
-    a.gd[m] = make_float4(gx, gy, gz, D);
-    a.kacc[m] += double(kb * ir);  // this slot's share of dL/dk
+    queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, recorded_masks(a, it), m, o.l, o.ax, o.ay, o.az, o.cx,
+                              o.cy, o.cz, PairQueue<kSweepBlock>(queue), body);
+    delta_out(a, c, m, gx, gy, gz, gsq, kb, lb, px, py, pz);
+}
+
+// The same with a team of kTeam lanes per slot (pbf_team.cuh): 8,000 slots, 25 -> 9
+// us a sweep; ten steps forward and backward 4.16 -> 3.21 ms.
+constexpr uint32_t kTeamBlock = 64;
+
+template <uint32_t SN>
+__global__ void __launch_bounds__(kTeamBlock) k_adj_delta_team(AdjArgs a, uint32_t it) {
+    __shared__ TeamBufOf<9> bufs[kTeamBlock / kTeam];
+    const uint32_t m = (blockIdx.x * kTeamBlock + threadIdx.x) / kTeam;
+    if (m >= a.n) return;
+    const Team<kTeam, TeamBufOf<9>> team(bufs);
+    const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
+    const float4* src = a.t.lam + size_t(it) * a.stride;
+    const DeltaSlot o(a, c, src, m);
+    const PairConsts pc = pair_consts(c);
+    const uint32_t n = SN ? SN : pc.scorr_n;
+    const float sgk = scorr_grad(pc, n);
+    const RowMasks rm = recorded_masks(a, it);
+    const TeamWalk walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, max(o.cy - 1, 0), max(o.cz - 1, 0)};
+    auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* out) {
+        const float4 q = __ldg(&src[k]);
+        float rx, ry, rz;
+        walk.offset(k, q, y, z, rx, ry, rz);
+        const float r2 = dist2(rx, ry, rz);
+        DeltaTerms t{};
+        const bool apart = r2 < pc.h2 && r2 > 1e-12f;
+        if (apart) t = delta_terms<SN>(a, pc, n, sgk, o.l.w, o.dm, o.pm, m, k, q, rx, ry, rz, r2);
+        auto put = [&](uint32_t i, float x, float y) {
+            out[i * kTermStride] = apart ? make_float2(x, y) : make_float2(0.0f, 0.0f);
+        };
+        put(0, t.f, rx);
+        put(1, t.f, ry);
+        put(2, t.f, rz);
+        put(3, t.f2, r2);
+        put(4, -t.rn, t.gdm);
+        put(5, t.gdd, 1.0f);
+        put(6, t.vx, 1.0f);
+        put(7, t.vy, 1.0f);
+        put(8, t.vz, 1.0f);
+    };
+    float sum = 0.0f;
+    team_pairs<kTeam, 9>(
+        team, c, a.t.cstart, o.cx, o.cy, o.cz, sum,
+        [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) { return walk.bits(row, c0, b0, b3); },
+        [](uint32_t) {}, terms);
+    float r[9];
+#pragma unroll
+    for (uint32_t i = 0; i < 9; ++i) r[i] = team.from(sum, i);
+    if (team.lane == 0) delta_out(a, c, m, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8]);
 }
 
 // dL/d(density sum, gradient sum, squared-gradient sum) of each particle's
@@ -411,50 +510,81 @@ __global__ void __launch_bounds__(kBlock) k_adj_lbar(AdjArgs a, uint32_t it) {
 //   pbar_i += sum_j (rhobar_i + rhobar_j) grad W_ij
 //             + H_ij (Gbar_i - Gbar_j + 2 (Qbar_i + Qbar_j) g_ij)
 // (j-side terms of one-way pairs added to j atomically).
+// A pair's position term in the lambda sweep of slot m (1e-12 < r2 < h^2).
+__device__ __forceinline__ float3 lambda_term(const AdjArgs& a, const PairConsts& pc, const float4& lm, float qm,
+                                              uint32_t pm, uint32_t m, uint32_t k, float rx, float ry, float rz,
+                                              float r2) {
+    const float4 li = __ldg(&a.lbar[k]);
+    const float2 qi = __ldg(&a.qc[k]);
+    const PairTerms t(pc, r2);
+    const float gw = __fmul_rn(__fmul_rn(__fmul_rn(-6.0f, pc.poly6), t.d), t.d);  // grad W = gw r
+    const bool both = cells_adjacent(__float_as_uint(qi.y), pm, a.wide);
+    const float qs = __fmul_rn(__fmul_rn(2.0f, __fadd_rn(qm, both ? qi.x : 0.0f)), t.f);
+    const float3 hv = t.hess(rx, ry, rz, __fmaf_rn(qs, rx, __fsub_rn(lm.x, both ? li.x : 0.0f)),
+                             __fmaf_rn(qs, ry, __fsub_rn(lm.y, both ? li.y : 0.0f)),
+                             __fmaf_rn(qs, rz, __fsub_rn(lm.z, both ? li.z : 0.0f)));
+    const float w = __fmul_rn(__fadd_rn(lm.w, both ? li.w : 0.0f), gw);
+    const float3 v = make_float3(__fmaf_rn(w, rx, hv.x), __fmaf_rn(w, ry, hv.y), __fmaf_rn(w, rz, hv.z));
+    if (!both) post(a, k, m, make_float4(-v.x, -v.y, -v.z, 0.0f));
+    return v;
+}
+
 template <bool COMMON>
 __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(AdjArgs a, uint32_t it) {
     __shared__ uint2 queue[kQueue * kSweepBlock];
     const uint32_t m = blockIdx.x * kSweepBlock + threadIdx.x;
     if (m >= a.n) return;
     const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
-    const size_t off = size_t(it) * a.stride;
-    const float4* src = a.t.lam + off;
-    const float4 l = src[m];
+    const float4* src = a.t.lam + size_t(it) * a.stride;
+    const DeltaSlot o(a, c, src, m);
     const float4 lm = a.lbar[m];
     const float qm = a.qc[m].x;
-    const uint32_t pm = a.cpred[m];
-    int pcx, pcy, pcz;
-    decode_cell(c.g, a.t.scell[m], pcx, pcy, pcz);
-    const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
-    int cx, cy, cz;
-    cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
     const float4 qb = a.qbar[m];
     float px = qb.x, py = qb.y, pz = qb.z;
     const PairConsts pc = COMMON ? a.pair : pair_consts(c);
-    const float w6 = -6.0f * pc.poly6;
     auto body = [&](uint32_t k, const float4&, float rx, float ry, float rz, float r2) {
         if (!(r2 < pc.h2 && r2 > 1e-12f)) return;
-        const float4 li = __ldg(&a.lbar[k]);
-        const float2 qi = __ldg(&a.qc[k]);
-        const PairTerms t(pc, r2);
-        const float gw = w6 * t.d * t.d;  // grad W = gw r
-        const bool both = cells_adjacent(__float_as_uint(qi.y), pm, a.wide);
-        const float qs = 2.0f * (qm + (both ? qi.x : 0.0f)) * t.f;
-        const float3 hv = t.hess(rx, ry, rz, lm.x - (both ? li.x : 0.0f) + qs * rx,
-                                 lm.y - (both ? li.y : 0.0f) + qs * ry, lm.z - (both ? li.z : 0.0f) + qs * rz);
-        const float w = (lm.w + (both ? li.w : 0.0f)) * gw;
-        const float vx = w * rx + hv.x, vy = w * ry + hv.y, vz = w * rz + hv.z;
-        px += vx;
-        py += vy;
-        pz += vz;
-        if (!both) post(a, k, m, make_float4(-vx, -vy, -vz, 0.0f));
+        const float3 v = lambda_term(a, pc, lm, qm, o.pm, m, k, rx, ry, rz, r2);
+        px = __fadd_rn(px, v.x);
+        py = __fadd_rn(py, v.y);
+        pz = __fadd_rn(pz, v.z);
     };
-    const uint32_t ms = a.mask_stride;
-    const RowMasks rm{const_cast<uint32_t*>(a.t.masks) + size_t(it) * 9 * ms,
-                      const_cast<uint32_t*>(a.t.overflow) + size_t(it) * ms, ms};
-    queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, rm, m, l, ax, ay, az, cx, cy, cz,
-                              PairQueue<kSweepBlock>(queue), body);
+    queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, recorded_masks(a, it), m, o.l, o.ax, o.ay, o.az, o.cx,
+                              o.cy, o.cz, PairQueue<kSweepBlock>(queue), body);
     a.pbar[m] = make_float4(px, py, pz, 0.0f);
+}
+
+__global__ void __launch_bounds__(kTeamBlock) k_adj_lambda_team(AdjArgs a, uint32_t it) {
+    __shared__ TeamBufOf<3> bufs[kTeamBlock / kTeam];
+    const uint32_t m = (blockIdx.x * kTeamBlock + threadIdx.x) / kTeam;
+    if (m >= a.n) return;
+    const Team<kTeam, TeamBufOf<3>> team(bufs);
+    const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
+    const float4* src = a.t.lam + size_t(it) * a.stride;
+    const DeltaSlot o(a, c, src, m);
+    const float4 lm = a.lbar[m];
+    const float qm = a.qc[m].x;
+    const float4 qb = a.qbar[m];
+    const PairConsts pc = pair_consts(c);
+    const RowMasks rm = recorded_masks(a, it);
+    const TeamWalk walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, max(o.cy - 1, 0), max(o.cz - 1, 0)};
+    auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* out) {
+        float rx, ry, rz;
+        walk.offset(k, __ldg(&src[k]), y, z, rx, ry, rz);
+        const float r2 = dist2(rx, ry, rz);
+        float3 v = make_float3(0.0f, 0.0f, 0.0f);
+        if (r2 < pc.h2 && r2 > 1e-12f) v = lambda_term(a, pc, lm, qm, o.pm, m, k, rx, ry, rz, r2);
+        out[0] = make_float2(v.x, 1.0f);
+        out[kTermStride] = make_float2(v.y, 1.0f);
+        out[2 * kTermStride] = make_float2(v.z, 1.0f);
+    };
+    float sum = team.lane == 0 ? qb.x : team.lane == 1 ? qb.y : qb.z;
+    team_pairs<kTeam, 3>(
+        team, c, a.t.cstart, o.cx, o.cy, o.cz, sum,
+        [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) { return walk.bits(row, c0, b0, b3); },
+        [](uint32_t) {}, terms);
+    const float px = team.from(sum, 0), py = team.from(sum, 1), pz = team.from(sum, 2);
+    if (team.lane == 0) a.pbar[m] = make_float4(px, py, pz, 0.0f);
 }
 
 // ---- scene sums ------------------------------------------------------------------
@@ -638,17 +768,25 @@ __global__ void __launch_bounds__(128) k_adj_sphere(AdjArgs a) {
 cudaError_t launch_adjoint_step(const AdjArgs& a, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
     const uint32_t grid = cdiv(a.n, kBlock), sweep_grid = cdiv(a.n, kSweepBlock);
+    const bool team = team_lanes(a.n) != 0;
+    const uint32_t team_grid = cdiv(a.n, kTeamBlock / kTeam);
     k_adj_finalize<<<grid, kBlock, 0, s>>>(a);
     for (uint32_t it = a.iterations; it-- > 0;) {
         k_adj_pre<<<grid, kBlock, 0, s>>>(a, it);
-        if (a.common)
+        if (team && a.scorr4)
+            k_adj_delta_team<4><<<team_grid, kTeamBlock, 0, s>>>(a, it);
+        else if (team)
+            k_adj_delta_team<0><<<team_grid, kTeamBlock, 0, s>>>(a, it);
+        else if (a.common)
             k_adj_delta<4, true><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         else if (a.scorr4)
             k_adj_delta<4, false><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         else
             k_adj_delta<0, false><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         k_adj_lbar<<<grid, kBlock, 0, s>>>(a, it);
-        if (a.common)
+        if (team)
+            k_adj_lambda_team<<<team_grid, kTeamBlock, 0, s>>>(a, it);
+        else if (a.common)
             k_adj_lambda<true><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);
         else
             k_adj_lambda<false><<<sweep_grid, kSweepBlock, 0, s>>>(a, it);

@@ -25,18 +25,20 @@ constexpr uint32_t kTeamChunks = 10;  // row chunks (of 32 candidates) expanded 
 constexpr uint32_t kTeamPairs = 32;   // pairs whose terms are computed at a time
 constexpr uint32_t kTeamMaxSlots = 1u << 28;  // list entries hold 28-bit slots
 
-// Shared memory of one team.
-struct TeamBuf {
+// Shared memory of one team that adds up SUMS sums.
+template <uint32_t SUMS>
+struct TeamBufOf {
     uint32_t b0[9], b3[9], chunks[9];      // rows: slot range, number of chunks
     uint32_t list[kTeamChunks * 32];       // slot | y << 28 | z << 30
-    float2 term[5][kTeamPairs + 1];        // per sum: the factors of each pair's term
+    float2 term[SUMS][kTeamPairs + 1];     // per sum: the factors of each pair's term
 };
+using TeamBuf = TeamBufOf<5>;
 
-template <uint32_t G>
+template <uint32_t G, class Buf = TeamBuf>
 struct Team {
     uint32_t lane, mask;  // lane in the team; the team's lanes in the warp
-    TeamBuf* buf;
-    __device__ __forceinline__ explicit Team(TeamBuf* bufs)
+    Buf* buf;
+    __device__ __forceinline__ explicit Team(Buf* bufs)
         : lane(threadIdx.x % G),
           mask((G == 32 ? 0xffffffffu : (1u << G) - 1u) << ((threadIdx.x & 31u) & ~(G - 1u))),
           buf(bufs + threadIdx.x / G) {}
@@ -54,12 +56,12 @@ struct Team {
 // terms(k, y, z, t) writes the NT term factors of candidate slot k (t[i * stride],
 // i < NT), and lane i adds x * y of factor pair i over all candidates to `sum`.
 // empty(row) is called for rows without candidates.
-template <uint32_t G, uint32_t NT, class Bits, class Empty, class Terms>
-__device__ __forceinline__ void team_pairs(const Team<G>& team, const StepConsts& c,
+template <uint32_t G, uint32_t NT, class Buf, class Bits, class Empty, class Terms>
+__device__ __forceinline__ void team_pairs(const Team<G, Buf>& team, const StepConsts& c,
                                            const uint32_t* __restrict__ cstart, int cx, int cy, int cz,
                                            float& sum, Bits&& bits, Empty&& empty, Terms&& terms) {
     static_assert(NT <= G, "one lane per sum");
-    TeamBuf& buf = *team.buf;
+    Buf& buf = *team.buf;
     const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
     const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
     const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
@@ -260,6 +262,38 @@ __device__ __forceinline__ void team_lambda(const StepConsts& c, uint32_t s, con
     if (LAST) lambdas[sidx[s]] = lambda;
 }
 
+// Neighbour vectors and chunk masks of a pass that walks recorded row masks, for a
+// particle at offset l from anchor (ax, ay, az) (see queued_pairs()).
+struct TeamWalk {
+    const StepConsts& c;
+    const float4* __restrict__ src;
+    const float* __restrict__ xa;
+    const RowMasks& rm;
+    uint32_t s;
+    float4 l;
+    float ax, ay, az;
+    int y0, z0;
+    __device__ __forceinline__ void offset(uint32_t k, const float4& q, uint32_t y, uint32_t z, float& rx,
+                                           float& ry, float& rz) const {
+        const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
+        const float oy = __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0 + int(y))), l.y);
+        const float oz = __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0 + int(z))), l.z);
+        rx = __fsub_rn(ox, q.x);
+        ry = __fsub_rn(oy, q.y);
+        rz = __fsub_rn(oz, q.z);
+    }
+    __device__ __forceinline__ uint32_t bits(uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) const {
+        if (c0 == row_base(b0)) return rm.rows[row * rm.stride + s];
+        uint32_t more = 0;
+        for (uint32_t k = c0; k < min(c0 + 32u, b3); ++k) {
+            float rx, ry, rz;
+            offset(k, __ldg(&src[k]), row % 3u, row / 3u, rx, ry, rz);
+            more |= dist2(rx, ry, rz) < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
+        }
+        return more;
+    }
+};
+
 template <bool LAST, uint32_t SN, uint32_t G>
 __device__ __forceinline__ void team_delta(const StepConsts& c, uint32_t s, const float4* __restrict__ src,
                                            float4* __restrict__ dst, uint32_t* __restrict__ qpos,
@@ -278,29 +312,12 @@ __device__ __forceinline__ void team_delta(const StepConsts& c, uint32_t s, cons
     const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
     int cx, cy, cz;
     cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
-    const int y0 = max(cy - 1, 0), z0 = max(cz - 1, 0);
-    auto offset = [&](uint32_t k, const float4& q, uint32_t y, uint32_t z, float& rx, float& ry, float& rz) {
-        const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
-        const float oy = __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0 + int(y))), l.y);
-        const float oz = __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0 + int(z))), l.z);
-        rx = __fsub_rn(ox, q.x);
-        ry = __fsub_rn(oy, q.y);
-        rz = __fsub_rn(oz, q.z);
-    };
-    auto bits = [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) {
-        if (c0 == row_base(b0)) return rm.rows[row * rm.stride + s];
-        uint32_t more = 0;
-        for (uint32_t k = c0; k < min(c0 + 32u, b3); ++k) {
-            float rx, ry, rz;
-            offset(k, __ldg(&src[k]), row % 3u, row / 3u, rx, ry, rz);
-            more |= dist2(rx, ry, rz) < c.h2 ? 0x80000000u >> (k - c0) : 0u;
-        }
-        return more;
-    };
+    const TeamWalk walk{c, src, xa, rm, s, l, ax, ay, az, max(cy - 1, 0), max(cz - 1, 0)};
+    auto bits = [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) { return walk.bits(row, c0, b0, b3); };
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* t) {
         const float4 q = __ldg(&src[k]);
         float rx, ry, rz;
-        offset(k, q, y, z, rx, ry, rz);
+        walk.offset(k, q, y, z, rx, ry, rz);
         const float r2 = dist2(rx, ry, rz);
         const float coef = delta_coef<SN>(c, l.w, q.w, r2);
         const bool apart = r2 < c.h2 && r2 > 1e-12f;
