@@ -57,7 +57,6 @@ def kernel_bytes(n: int, c: int) -> dict:
         "scan": 24 * c,
         "scatter": 8 * n + 12 * c,
         "sort_gather": 36 * n,
-        "long_segments": 0,
         "lambda_count": 68 * n + 8 * c,
         "lambda": 28 * n + 4 * c,
         "delta": 36 * n + 4 * c,

@@ -562,7 +562,7 @@ struct mp_engine {
         particle_block = nullptr;
         list_block = nullptr;
         d.pos = d.vel = d.prev = d.sorted_a = d.sorted_b = nullptr;
-        d.hash = d.off = d.tmp = d.sidx = d.qpos = d.scell = d.ncount = d.long_list = nullptr;
+        d.hash = d.off = d.tmp = d.sidx = d.qpos = d.scell = d.ncount = nullptr;
         d.lambdas = d.foam = d.xa = nullptr;
         d.row_masks = nullptr;
         d.mask_overflow = nullptr;
@@ -592,8 +592,7 @@ struct mp_engine {
         if (cap == n_alloc) return MP_OK;
         free_particles();
         const size_t v4 = size_t(cap) * 16, u = size_t(cap) * 4;
-        const size_t longs = (size_t(cap) / mpb::kSegMax + 2) * 4;
-        const size_t total = 5 * v4 + 10 * u + longs + 18 * 256;
+        const size_t total = 5 * v4 + 10 * u + 18 * 256;
         MP_ALLOC(particle_block, total, device);
         char* b = static_cast<char*>(particle_block);
         auto take = [&](size_t bytes) {
@@ -616,7 +615,6 @@ struct mp_engine {
         d.lambdas = reinterpret_cast<float*>(take(u));
         d.foam = reinterpret_cast<float*>(take(u));
         d.xa = reinterpret_cast<float*>(take(u));
-        d.long_list = reinterpret_cast<uint32_t*>(take(longs));
         MP_CUDA(cudaMemset(particle_block, 0, total));
         // 9 row masks (4 bytes each) + an overflow flag per particle
         MP_ALLOC(list_block, 10 * u, device);
@@ -651,7 +649,6 @@ struct mp_engine {
         MP_ALLOC(small_block, 256, device);
         MP_CUDA(cudaMemset(small_block, 0, 256));
         char* b = static_cast<char*>(small_block);
-        d.long_count = reinterpret_cast<uint32_t*>(b);
         d.err = reinterpret_cast<uint32_t*>(b + 4);
         d.strays = reinterpret_cast<uint32_t*>(b + 8);
         d.sphere = reinterpret_cast<mpb::SphereState*>(b + 64);

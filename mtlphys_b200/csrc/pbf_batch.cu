@@ -357,7 +357,8 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     if (cells_ok)
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
             sort_gather_item(sc[a.scene_of[s]].c, s, a.tmp, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,
-                             a.qpos, a.xa, nullptr, a.long_list, a.long_count);
+                             a.qpos, a.xa, nullptr,
+                             [&](uint32_t cell) { a.long_list[atomicAdd(a.long_count, 1u)] = cell; });
     if (!grid_barrier(a, &s_bar)) return;
     const uint32_t nl = cells_ok ? *static_cast<volatile uint32_t*>(a.long_count) : 0u;
     if (nl) {  // the same for every block: long_count is written before the barrier only

@@ -26,10 +26,8 @@ namespace {
 __global__ void __launch_bounds__(256)
 k_predict_hash(StepConsts c, float4* __restrict__ pos, const float4* __restrict__ vel,
                float4* __restrict__ prev, uint32_t* __restrict__ hash, uint32_t* __restrict__ off,
-               uint32_t* __restrict__ counts, uint32_t* __restrict__ long_count,
-               uint32_t* __restrict__ strays, SphereState* __restrict__ sphere, int predict, uint32_t* __restrict__ err) {
+               uint32_t* __restrict__ counts, uint32_t* __restrict__ strays, SphereState* __restrict__ sphere, int predict, uint32_t* __restrict__ err) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *long_count = 0;
         *strays = 0;
         if (predict && c.sphere) sphere_advance(c, sphere);
     }
@@ -235,27 +233,24 @@ k_scatter(uint32_t n, const uint32_t* __restrict__ hash, const uint32_t* __restr
     if (i < n) scatter_item(i, hash, off, cstart, tmp);
 }
 
-__global__ void __launch_bounds__(256)
+// A block's 256 slots hold the first slot of at most one segment of more than
+// kSegMax particles; the block ranks that one (a launch of its own for them took 2
+// us, mostly to find none).
+__global__ void __launch_bounds__(kSegMax)
 k_sort_gather(StepConsts c, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ hash,
               const uint32_t* __restrict__ cstart, const float4* __restrict__ pos,
               uint32_t* __restrict__ sidx, float4* __restrict__ sorted, uint32_t* __restrict__ qpos,
-              float* __restrict__ xa, uint32_t* strays, uint32_t* __restrict__ long_list,
-              uint32_t* __restrict__ long_count) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < c.n) sort_gather_item(c, s, tmp, hash, cstart, pos, sidx, sorted, qpos, xa, strays, long_list, long_count);
-}
-
-// One block per queued long segment.
-__global__ void __launch_bounds__(256)
-k_long_segments(StepConsts c, const uint32_t* __restrict__ hash, const uint32_t* __restrict__ cstart,
-                const float4* __restrict__ pos, uint32_t* __restrict__ sidx,
-                float4* __restrict__ sorted, uint32_t* __restrict__ qpos, float* __restrict__ xa,
-                uint32_t* strays, const uint32_t* __restrict__ long_list,
-                const uint32_t* __restrict__ long_count) {
-    __shared__ uint32_t s_warp[8];
-    const uint32_t total = *long_count;
-    for (uint32_t li = blockIdx.x; li < total; li += gridDim.x)
-        long_segment(c, long_list[li], 0u, c.n, hash, cstart, pos, sidx, sorted, qpos, xa, strays, s_warp);
+              float* __restrict__ xa, uint32_t* strays) {
+    constexpr uint32_t kNone = 0xffffffffu;
+    __shared__ uint32_t s_warp[kSegMax / 32], s_long;
+    if (threadIdx.x == 0) s_long = kNone;
+    __syncthreads();
+    const uint32_t s = blockIdx.x * kSegMax + threadIdx.x;
+    if (s < c.n)
+        sort_gather_item(c, s, tmp, hash, cstart, pos, sidx, sorted, qpos, xa, strays,
+                         [&](uint32_t cell) { s_long = cell; });
+    __syncthreads();
+    if (s_long != kNone) long_segment(c, s_long, 0u, c.n, hash, cstart, pos, sidx, sorted, qpos, xa, strays, s_warp);
 }
 
 // Bound by instruction issue, like the lambda passes whose prefilter it shares:
@@ -296,7 +291,7 @@ cudaError_t launch_hash_pass(const StepConsts& c, const DevState& d, bool predic
     const uint32_t n = c.n;
     tbegin(t, s);
     k_predict_hash<<<n ? cdiv(n, 256) : 1, 256, 0, s>>>(c, d.pos, d.vel, d.prev, d.hash, d.off,
-                                                        d.counts, d.long_count, d.strays, d.sphere,
+                                                        d.counts, d.strays, d.sphere,
                                                         predict ? 1 : 0, d.err);
     tend(t, predict ? "predict_hash" : "hash", s);
     cudaError_t e = cudaGetLastError();
@@ -308,13 +303,9 @@ cudaError_t launch_hash_pass(const StepConsts& c, const DevState& d, bool predic
     k_scatter<<<cdiv(n, 256), 256, 0, s>>>(n, d.hash, d.off, d.cstart, d.tmp);
     tend(t, "scatter", s);
     tbegin(t, s);
-    k_sort_gather<<<cdiv(n, 256), 256, 0, s>>>(c, d.tmp, d.hash, d.cstart, d.pos, d.sidx,
-                                                d.sorted_a, d.qpos, d.xa, d.strays, d.long_list, d.long_count);
+    k_sort_gather<<<cdiv(n, kSegMax), kSegMax, 0, s>>>(c, d.tmp, d.hash, d.cstart, d.pos, d.sidx, d.sorted_a,
+                                                       d.qpos, d.xa, d.strays);
     tend(t, "sort_gather", s);
-    tbegin(t, s);
-    k_long_segments<<<148, 256, 0, s>>>(c, d.hash, d.cstart, d.pos, d.sidx, d.sorted_a,
-                                        d.qpos, d.xa, d.strays, d.long_list, d.long_count);
-    tend(t, "long_segments", s);
     return cudaGetLastError();
 }
 

@@ -145,7 +145,9 @@ __device__ __forceinline__ void place(const StepConsts& c, uint32_t d, uint32_t 
 
 // Stable re-rank inside the cell segment + gatherPositions: the slot's
 // particle j moves to cellStart + (number of particles of its cell with a
-// smaller index).  Segments longer than kSegMax are queued instead.
+// smaller index).  A cell of more than kSegMax particles is left to
+// long_segment: on_long(cell) is called once, by its first slot.
+template <class OnLong>
 __device__ __forceinline__ void sort_gather_item(const StepConsts& sc, uint32_t s,
                                                  const uint32_t* __restrict__ tmp,
                                                  const uint32_t* __restrict__ hash,
@@ -154,13 +156,12 @@ __device__ __forceinline__ void sort_gather_item(const StepConsts& sc, uint32_t 
                                                  uint32_t* __restrict__ sidx,
                                                  float4* __restrict__ sorted,
                                                  uint32_t* __restrict__ qpos, float* __restrict__ xa,
-                                                 uint32_t* strays, uint32_t* __restrict__ long_list,
-                                                 uint32_t* __restrict__ long_count) {
+                                                 uint32_t* strays, OnLong&& on_long) {
     const uint32_t j = tmp[s];
     const uint32_t c = hash[j];
     const uint32_t a = cstart[c], b = cstart[c + 1];
     if (b - a > kSegMax) {
-        if (s == a) long_list[atomicAdd(long_count, 1u)] = c;
+        if (s == a) on_long(c);
         return;
     }
     uint32_t rank = 0;

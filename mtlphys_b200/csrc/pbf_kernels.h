@@ -31,8 +31,6 @@ struct DevState {
     float* foam;            // foam intensity per particle
     uint32_t* counts;       // cells+1 per-cell counts (all zero between passes)
     uint32_t* cstart;       // cells+1 exclusive scan of counts
-    uint32_t* long_list;    // cells whose segment exceeds kSegMax
-    uint32_t* long_count;   // entries in long_list
     uint32_t* strays;       // 1: some particle of this hash lies outside its cell
     unsigned long long* scan_status;  // look-back tile descriptors
     unsigned long long* scan_ticket;  // monotonic tile ticket
@@ -44,7 +42,7 @@ struct DevState {
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanItemsPerThread = 16;
 constexpr uint32_t kScanTile = kScanThreads * kScanItemsPerThread;  // 4096
-constexpr uint32_t kSegMax = 256;  // longest cell segment ranked in place
+constexpr uint32_t kSegMax = 256;  // longest cell segment ranked slot by slot
 
 inline uint32_t scan_tiles_for(uint64_t n) { return uint32_t((n + kScanTile - 1) / kScanTile); }
 

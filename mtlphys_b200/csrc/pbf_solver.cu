@@ -214,9 +214,9 @@ cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t itera
 }
 
 uint32_t step_launch_count(uint32_t iterations) {
-    // predict+hash, scan, scatter, sort+gather, long segments, then 2 per
-    // iteration (or count + finalize for zero iterations).
-    return 5u + (iterations ? 2u * iterations : 2u);
+    // predict+hash, scan, scatter, sort+gather, then 2 per iteration (or count +
+    // finalize for zero iterations).
+    return 4u + (iterations ? 2u * iterations : 2u);
 }
 
 }  // namespace mpb
