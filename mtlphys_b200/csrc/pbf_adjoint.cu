@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_adj_delta_team(AdjArgs a, uint32
     const uint32_t n = SN ? SN : pc.scorr_n;
     const float sgk = scorr_grad(pc, n);
     const RowMasks rm = recorded_masks(a, it);
-    const TeamWalk walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, max(o.cy - 1, 0), max(o.cz - 1, 0)};
+    const TeamWalk walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, o.cy - 1, o.cz - 1};
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* out) {
         const float4 q = __ldg(&src[k]);
         float rx, ry, rz;
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_adj_lambda_team(AdjArgs a, uint3
     const float4 qb = a.qbar[m];
     const PairConsts pc = pair_consts(c);
     const RowMasks rm = recorded_masks(a, it);
-    const TeamWalk walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, max(o.cy - 1, 0), max(o.cz - 1, 0)};
+    const TeamWalk walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, o.cy - 1, o.cz - 1};
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* out) {
         float rx, ry, rz;
         walk.offset(k, __ldg(&src[k]), y, z, rx, ry, rz);

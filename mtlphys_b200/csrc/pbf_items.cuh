@@ -344,12 +344,22 @@ __device__ __forceinline__ uint32_t row_base(uint32_t b0) { return b0 & ~3u; }
 // Offsets of a particle to the three stencil rows along y and along z.
 struct RowOffsets {
     float y0, y1, y2, z0, z1, z2;
+    // (A_i - A_row) + l_i for the rows around cell (cy, cz)
+    __device__ __forceinline__ static RowOffsets anchored(const GridDev& g, int cy, int cz, float ay, float az,
+                                                          float ly, float lz) {
+        return RowOffsets{__fadd_rn(__fsub_rn(ay, anchor_y(g, cy - 1)), ly),
+                          __fadd_rn(__fsub_rn(ay, anchor_y(g, cy)), ly),
+                          __fadd_rn(__fsub_rn(ay, anchor_y(g, cy + 1)), ly),
+                          __fadd_rn(__fsub_rn(az, anchor_z(g, cz - 1)), lz),
+                          __fadd_rn(__fsub_rn(az, anchor_z(g, cz)), lz),
+                          __fadd_rn(__fsub_rn(az, anchor_z(g, cz + 1)), lz)};
+    }
 };
 
 // Per-thread queue of row chunks with candidates to visit, in shared memory:
 // entry e of thread t at (e * BS + t), 8 bytes: the chunk's bits (first
-// candidate in bit 31), and its first slot (a multiple of 4, below 2^30) with the
-// row's y index in bits 0-1 and z index in bits 30-31.  The lanes of a warp have
+// candidate in bit 31), and 4 times its first slot (a multiple of 4, below 2^30) with
+// the row's y index in bits 0-1 and its z index in bits 2-3.  The lanes of a warp have
 // very different numbers of candidates per row but similar totals: walking all
 // rows' bits in one loop, each lane moving to its next chunk by itself with a
 // predicated load, takes 38 iterations where row by row takes 87 (lattice or
@@ -357,8 +367,17 @@ struct RowOffsets {
 // 1,003,520-particle dam break: 214 M -> 150 M warp instructions, 17 -> 25 of 32
 // threads active, 281 -> 184 us; k_delta 161 M -> 95 M, 14 -> 27, 150-171 -> 130 us.
 // 16-byte entries that hold the two offsets instead of the row's indices leave
-// too little of the SM's memory for L1 (k_delta 258 us, 13% hits).
-constexpr uint32_t kQueue = 10;  // 9 rows and a second chunk of one of them
+// too little of the SM's memory for L1 (k_delta 258 us, 13% hits).  With the rows
+// in a loop of nine fixed ones, their bounds a row ahead (lambda) or all loads up
+// front (delta): 167 and 107 us.
+//
+// 9 rows and 6 more chunks of long ones.  A lane whose queue is full walks it in the
+// middle of the sweep while its warp waits: with 10 entries a few such warps
+// decided the time of a scene that fits the GPU at once (97,336 particles: 31 us
+// per lambda pass on the slowest SM, 20 on average).  15 is the most that leaves L1
+// as large as 10 do (eight blocks of 128 use 131 KB).
+constexpr uint32_t kQueue = 15;
+static_assert(kQueue >= 10, "room for every row's first chunk and an empty one");
 
 template <uint32_t BS>
 struct PairQueue {
@@ -368,10 +387,14 @@ struct PairQueue {
 
     __device__ __forceinline__ explicit PairQueue(uint2* shared)
         : base(uint32_t(__cvta_generic_to_shared(shared + threadIdx.x))), tail(base) {}
-    __device__ __forceinline__ bool full() const { return tail == base + kQueue * BS * 8u; }
-    __device__ __forceinline__ void push(uint32_t mask, uint32_t first, uint32_t y, uint32_t z) {
-        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(tail), "r"(mask), "r"(first | y | (z << 30)));
-        tail += BS * 8u;
+    // whether fewer than `entries` more fit
+    __device__ __forceinline__ bool short_of(uint32_t entries) const {
+        return tail + entries * (BS * 8u) > base + kQueue * BS * 8u;
+    }
+    // code: y | z << 2.  An empty mask takes no entry.
+    __device__ __forceinline__ void push(uint32_t mask, uint32_t first, uint32_t code) {
+        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(tail), "r"(mask), "r"(first * 4u | code));
+        tail += mask ? BS * 8u : 0u;
         pairs += __popc(mask);
     }
     // The next bit's slot and offsets; `at`, `mask`, `first` are the walk's state.
@@ -388,8 +411,8 @@ struct PairQueue {
         asm("bfind.shiftamt.u32 %0, %1;" : "=r"(t) : "r"(mask));
         mask &= 0x7fffffffu >> t;
         oy = (first & 2u) ? o.y2 : ((first & 1u) ? o.y1 : o.y0);
-        oz = int(first) < 0 ? o.z2 : ((first & 0x40000000u) ? o.z1 : o.z0);
-        return (first & 0x3ffffffcu) + t;
+        oz = (first & 8u) ? o.z2 : ((first & 4u) ? o.z1 : o.z0);
+        return (first >> 4) * 4u + t;
     }
     // visit(slot, fetch(slot), oy, oz) for every bit, in the order queued; empties
     // the queue.  PIPE: each candidate is fetched while the one before it is
@@ -421,6 +444,51 @@ struct PairQueue {
     }
 };
 
+// The 9 rows of the stencil around cell (cx, cy, cz), z outer, y inner: row
+// (cy - 1 + y, cz - 1 + z) is number 3 z + y and starts at cell `base`, advanced by
+// next_y after each row and by next_z after each plane.  Rows outside the grid are
+// not valid (all of them for a particle that drifted more than a cell past a
+// scene's sub-grid in x).
+struct StencilRows {
+    uint32_t base, nx, next_y, next_z;
+    int gy, gz;
+    __device__ __forceinline__ StencilRows(const GridDev& g, int cx, int cy, int cz) {
+        const int x0 = max(cx - 1, 0), n = min(cx + 1, g.gx - 1) - x0 + 1;
+        nx = uint32_t(n);
+        gy = n > 0 ? g.gy : 0;
+        gz = g.gz;
+        next_y = uint32_t(g.gx);
+        next_z = uint32_t(g.gx) * uint32_t(g.gy - 3);
+        base = cell_hash(g, x0, cy - 1, cz - 1);
+    }
+    __device__ __forceinline__ bool valid(int y, int z) const {
+        return uint32_t(y) < uint32_t(gy) && uint32_t(z) < uint32_t(gz);
+    }
+};
+
+// Phase 1 of a sweep: the prefilter's bits of slots [c0, c1), c0 a multiple of 4, at
+// most 32 of them (first one in bit 31), without slot s.  Reads up to 7 slots past
+// c1.
+__device__ __forceinline__ uint32_t row_bits(const uint32_t* __restrict__ qsrc, uint32_t qi, int nthr, uint32_t c0,
+                                             uint32_t c1, uint32_t s) {
+    uint32_t mask = 0, k = c0;
+    auto test = [&](uint32_t w) {
+        const int d = int(qi - w);
+        mask = __funnelshift_l(uint32_t(__dp4a(d, d, nthr)), mask, 1);
+    };
+    for (; k < c1; k += 4) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(qsrc + k));
+        test(q.x);
+        test(q.y);
+        test(q.z);
+        test(q.w);
+    }
+    mask <<= 32u - (k - c0);
+    mask &= 0xffffffffu << (32u - (c1 - c0));
+    if (s - c0 < 32u) mask &= ~(0x80000000u >> (s - c0));
+    return mask;
+}
+
 // Two-phase sweep of the 27-cell stencil around cell (cx, cy, cz).  Each row
 // (3 consecutive cells, one contiguous slot range) is taken in chunks of 32
 // candidates.
@@ -451,18 +519,6 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
                                       float px, float py, float pz, float aix, float aiy, float aiz,
                                       uint32_t qi, int nthr, uint32_t s, const RowMasks& masks,
                                       PairQueue<BS> queue, Body&& body) {
-    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
-    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
-    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
-    const int nx = x1 - x0 + 1;
-    uint32_t over = 0;
-    if (nx <= 0) {  // drifted more than a cell outside a scene's sub-grid: no candidates
-        for (int z = z0; z <= z1; ++z)
-            for (int y = y0; y <= y1; ++y)
-                masks.rows[uint32_t((z - z0) * 3 + (y - y0)) * masks.stride + s] = 0u;
-        masks.overflow[s] = 0u;
-        return;
-    }
     auto fetch = [&](uint32_t k) { return __ldg(&src[k]); };
     auto visit = [&](uint32_t k, const float4& q, float oy, float oz) {
         const float ox = ANCHORED ? __fadd_rn(__fsub_rn(aix, q.w), px) : px;
@@ -470,50 +526,44 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
         body(k, q, rx, ry, rz, dist2(rx, ry, rz));
     };
     RowOffsets o{py, py, py, pz, pz, pz};
-    if (ANCHORED) {
-        o.y0 = __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y0)), py);
-        o.y1 = __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y0 + 1)), py);
-        o.y2 = __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y0 + 2)), py);
-        o.z0 = __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z0)), pz);
-        o.z1 = __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z0 + 1)), pz);
-        o.z2 = __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z0 + 2)), pz);
+    if (ANCHORED) o = RowOffsets::anchored(c.g, cy, cz, aiy, aiz, py, pz);
+    const StencilRows rows(c.g, cx, cy, cz);
+    uint32_t over = 0, base = rows.base, b0 = 0, b3 = 0;
+    uint32_t* out = masks.rows + s;
+    if (rows.valid(cy - 1, cz - 1)) {
+        b0 = cstart[base];
+        b3 = cstart[base + rows.nx];
     }
-    for (int z = z0; z <= z1; ++z) {
-        for (int y = y0; y <= y1; ++y) {
-            const uint32_t base = cell_hash(c.g, x0, y, z);
-            const uint32_t b0 = cstart[base], b3 = cstart[base + uint32_t(nx)];
-            const uint32_t a0 = row_base(b0);
-            const uint32_t row = uint32_t((z - z0) * 3 + (y - y0));
-            uint32_t first = 0;  // bits of the first chunk (the whole row if b3 - a0 <= 32)
-            if (b0 < b3) {
-                uint32_t drop = 0xffffffffu >> (b0 - a0);  // candidates before the row
-                for (uint32_t c0 = a0; c0 < b3; c0 += 32) {
-                    const uint32_t c1 = min(c0 + 32u, b3);
-                    uint32_t mask = 0, k = c0;
-                    for (; k < c1; k += 4) {
-                        const uint4 q = __ldg(reinterpret_cast<const uint4*>(qsrc + k));
-                        const int d0 = int(qi - q.x), d1 = int(qi - q.y);
-                        const int d2 = int(qi - q.z), d3 = int(qi - q.w);
-                        mask = __funnelshift_l(uint32_t(__dp4a(d0, d0, nthr)), mask, 1);
-                        mask = __funnelshift_l(uint32_t(__dp4a(d1, d1, nthr)), mask, 1);
-                        mask = __funnelshift_l(uint32_t(__dp4a(d2, d2, nthr)), mask, 1);
-                        mask = __funnelshift_l(uint32_t(__dp4a(d3, d3, nthr)), mask, 1);
-                    }
-                    // the chunk's first candidate to bit 31; drop what lies outside
-                    // the row, and the particle itself
-                    mask <<= 32u - (k - c0);
-                    mask &= drop & (0xffffffffu << (32u - (c1 - c0)));
-                    drop = 0xffffffffu;
-                    if (s - c0 < 32u) mask &= ~(0x80000000u >> (s - c0));
-                    if (c0 == a0) first = mask;
-                    if (mask) {
-                        if (queue.full()) queue.template drain<false>(o, fetch, visit);  // crowded rows only
-                        queue.push(mask, c0, uint32_t(y - y0), uint32_t(z - z0));
-                    }
-                }
-                if (b3 - a0 > 32u) over |= 1u << row;
+#pragma unroll 1  // (unrolled, the rows' code no longer fits the instruction cache)
+    for (int z = 0; z < 3; ++z) {
+#pragma unroll 1
+        for (int y = 0; y < 3; ++y, out += masks.stride) {
+            // the next row's bounds are on their way while this one is tested
+            const int y1 = y < 2 ? y + 1 : 0, z1 = y < 2 ? z : z + 1;
+            base += rows.next_y + (y < 2 ? 0u : rows.next_z);
+            uint32_t n0 = 0, n3 = 0;
+            if (z1 < 3 && rows.valid(cy - 1 + y1, cz - 1 + z1)) {
+                n0 = cstart[base];
+                n3 = cstart[base + rows.nx];
             }
-            masks.rows[row * masks.stride + s] = first;
+            uint32_t mask = 0;
+            const uint32_t a0 = row_base(b0);
+            if (b0 < b3) mask = row_bits(qsrc, qi, nthr, a0, min(a0 + 32u, b3), s) & (0xffffffffu >> (b0 - a0));
+            // the bits of the row's first chunk (the whole row if b3 - a0 <= 32)
+            *out = mask;
+            const uint32_t code = uint32_t(y) | (uint32_t(z) << 2);
+            queue.push(mask, a0, code);
+            if (b3 > a0 + 32u) {  // (never an empty row)
+                const uint32_t row = uint32_t(3 * z + y);
+                over |= 1u << row;
+                for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
+                    // room for this chunk and the first ones of the rows to come
+                    if (queue.short_of(9u - row)) queue.template drain<false>(o, fetch, visit);
+                    queue.push(row_bits(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s), c0, code);
+                }
+            }
+            b0 = n0;
+            b3 = n3;
         }
     }
     masks.overflow[s] = over;
@@ -588,10 +638,8 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
                 in = (in << left) & row;
                 maybe = (maybe << left) & row & ~in;
                 cnt += __popc(in);
-                if (maybe) {
-                    if (queue.full()) queue.template drain<false>(none, fetch, visit);
-                    queue.push(maybe, c0, 0u, 0u);
-                }
+                if (queue.short_of(1u)) queue.template drain<false>(none, fetch, visit);
+                queue.push(maybe, c0, 0u);
             }
         }
     queue.template drain<false>(none, fetch, visit);
@@ -735,11 +783,6 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
                                              const uint32_t* __restrict__ cstart, const RowMasks& rm,
                                              uint32_t s, const float4& l, float ax, float ay, float az,
                                              int cx, int cy, int cz, PairQueue<BS> queue, Body&& body) {
-    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
-    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
-    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
-    const int nx = x1 - x0 + 1;
-    if (nx <= 0) return;
     const uint32_t longrows = rm.overflow[s];
     struct Candidate {
         float4 q;
@@ -752,39 +795,48 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
         const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
         body(k, q, rx, ry, rz, dist2(rx, ry, rz));
     };
-    const RowOffsets o{__fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0)), l.y),
-                       __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0 + 1)), l.y),
-                       __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0 + 2)), l.y),
-                       __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0)), l.z),
-                       __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0 + 1)), l.z),
-                       __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0 + 2)), l.z)};
-    for (int z = z0; z <= z1; ++z) {
-        for (int y = y0; y <= y1; ++y) {
-            const uint32_t row = uint32_t((z - z0) * 3 + (y - y0));
-            const uint32_t mask = rm.rows[row * rm.stride + s];
-            const bool long_row = (longrows >> row) & 1u;
-            if (mask == 0u && !long_row) continue;
-            const uint32_t base = cell_hash(c.g, x0, y, z);
-            const uint32_t a0 = row_base(cstart[base]);
-            if (mask) {
-                if (queue.full()) queue.template drain<false>(o, fetch, visit);
-                queue.push(mask, a0, uint32_t(y - y0), uint32_t(z - z0));
-            }
-            if (long_row) {
-                const float oy = __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y)), l.y);
-                const float oz = __fadd_rn(__fsub_rn(az, anchor_z(c.g, z)), l.z);
-                const uint32_t b3 = cstart[base + uint32_t(nx)];
-                for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
-                    uint32_t more = 0;
-                    for (uint32_t k = c0; k < min(c0 + 32u, b3); ++k) {
-                        const float4 q = __ldg(&src[k]);
-                        const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
-                        const float r2 = dist2(__fsub_rn(ox, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
-                        more |= r2 < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
-                    }
-                    if (more) {
-                        if (queue.full()) queue.template drain<false>(o, fetch, visit);
-                        queue.push(more, c0, uint32_t(y - y0), uint32_t(z - z0));
+    const RowOffsets o = RowOffsets::anchored(c.g, cy, cz, ay, az, l.y, l.z);
+    const StencilRows rows(c.g, cx, cy, cz);
+    uint32_t base = rows.base;
+    const uint32_t* in = rm.rows + s;
+    if (longrows == 0u) {
+        // all masks and row starts on their way at once
+        uint32_t mask[9], b0[9];
+#pragma unroll
+        for (uint32_t r = 0; r < 9; ++r) {
+            mask[r] = in[r * rm.stride];
+            b0[r] = rows.valid(cy - 1 + int(r % 3u), cz - 1 + int(r / 3u))
+                        ? cstart[base + r * rows.next_y + (r / 3u) * rows.next_z]
+                        : 0u;
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < 9; ++r) queue.push(mask[r], row_base(b0[r]), (r % 3u) | ((r / 3u) << 2));
+    } else {
+#pragma unroll 1
+        for (int z = 0; z < 3; ++z, base += rows.next_z) {
+#pragma unroll 1
+            for (int y = 0; y < 3; ++y, base += rows.next_y, in += rm.stride) {
+                const uint32_t mask = *in;
+                const uint32_t row = uint32_t(3 * z + y);
+                const bool long_row = (longrows >> row) & 1u;
+                if (mask == 0u && !long_row) continue;
+                const uint32_t a0 = row_base(cstart[base]);
+                const uint32_t code = uint32_t(y) | (uint32_t(z) << 2);
+                queue.push(mask, a0, code);
+                if (long_row) {
+                    const float oy = y == 0 ? o.y0 : (y == 1 ? o.y1 : o.y2);
+                    const float oz = z == 0 ? o.z0 : (z == 1 ? o.z1 : o.z2);
+                    const uint32_t b3 = cstart[base + rows.nx];
+                    for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
+                        uint32_t more = 0;
+                        for (uint32_t k = c0; k < min(c0 + 32u, b3); ++k) {
+                            const float4 q = __ldg(&src[k]);
+                            const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
+                            const float r2 = dist2(__fsub_rn(ox, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
+                            more |= r2 < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
+                        }
+                        if (queue.short_of(9u - row)) queue.template drain<false>(o, fetch, visit);
+                        queue.push(more, c0, code);
                     }
                 }
             }

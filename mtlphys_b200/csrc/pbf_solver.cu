@@ -20,8 +20,9 @@ inline uint32_t cdiv(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 // Launch shape of the solver kernels, measured on the 1,003,520-particle dam
 // break: blocks of 128 threads (64 and 256 are within 0.5%), and at least 8 of
-// them per SM, which caps registers at 64: 1440 us per step (lambda passes at 9
-// blocks, 56 registers, +1.5%; delta passes +3.5%; fewer blocks 10% and more).
+// them per SM, which caps registers at 64: 1285 us per step (with 9 blocks, 56
+// registers, the lambda passes cost a step 1.5% more and the delta passes 3.5%;
+// fewer blocks 10% and more).
 #ifndef MPB_SOLVER_BLOCK
 #define MPB_SOLVER_BLOCK 128
 #endif

@@ -62,20 +62,17 @@ __device__ __forceinline__ void team_pairs(const Team<G, Buf>& team, const StepC
                                            float& sum, Bits&& bits, Empty&& empty, Terms&& terms) {
     static_assert(NT <= G, "one lane per sum");
     Buf& buf = *team.buf;
-    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, c.g.gx - 1);
-    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
-    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
-    const int nx = x1 - x0 + 1;
+    const StencilRows rows(c.g, cx, cy, cz);
     team.sync();  // the buffer may still be read for the team's previous slot
     for (uint32_t row = team.lane; row < 9; row += G) {
-        const int y = y0 + int(row % 3u), z = z0 + int(row / 3u);
+        const uint32_t y = row % 3u, z = row / 3u;
         uint32_t b0 = 0, b3 = 0;
-        if (nx > 0 && y <= y1 && z <= z1) {
-            const uint32_t base = cell_hash(c.g, x0, y, z);
+        if (rows.valid(cy - 1 + int(y), cz - 1 + int(z))) {
+            const uint32_t base = rows.base + row * rows.next_y + z * rows.next_z;
             b0 = cstart[base];
-            b3 = cstart[base + uint32_t(nx)];
-            if (b0 >= b3) empty(row);
+            b3 = cstart[base + rows.nx];
         }
+        if (b0 >= b3) empty(row);
         buf.b0[row] = b0;
         buf.b3[row] = b3;
         buf.chunks[row] = b0 < b3 ? (b3 - row_base(b0) + 31u) / 32u : 0u;
@@ -159,23 +156,11 @@ __device__ __forceinline__ uint32_t team_sweep(const Team<G>& team, const StepCo
                                                float px, float py, float pz, float aix, float aiy, float aiz,
                                                uint32_t qi, int nthr, uint32_t s, const RowMasks& masks,
                                                LambdaAcc& acc) {
-    const int y0 = max(cy - 1, 0), z0 = max(cz - 1, 0);
+    const int y0 = cy - 1, z0 = cz - 1;
     uint32_t hits = 0, over = 0;
     auto bits = [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) {
-        const uint32_t c1 = min(c0 + 32u, b3);
-        uint32_t mask = 0, k = c0;
-        for (; k < c1; k += 4) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4*>(qsrc + k));
-            const int d0 = int(qi - q.x), d1 = int(qi - q.y);
-            const int d2 = int(qi - q.z), d3 = int(qi - q.w);
-            mask = __funnelshift_l(uint32_t(__dp4a(d0, d0, nthr)), mask, 1);
-            mask = __funnelshift_l(uint32_t(__dp4a(d1, d1, nthr)), mask, 1);
-            mask = __funnelshift_l(uint32_t(__dp4a(d2, d2, nthr)), mask, 1);
-            mask = __funnelshift_l(uint32_t(__dp4a(d3, d3, nthr)), mask, 1);
-        }
-        mask <<= 32u - (k - c0);
-        mask &= (0xffffffffu >> (max(b0, c0) - c0)) & (0xffffffffu << (32u - (c1 - c0)));
-        if (s - c0 < 32u) mask &= ~(0x80000000u >> (s - c0));
+        uint32_t mask = row_bits(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s);
+        mask &= 0xffffffffu >> (max(b0, c0) - c0);
         if (c0 == row_base(b0)) {
             masks.rows[row * masks.stride + s] = mask;
             if (b3 - c0 > 32u) over |= 1u << row;
@@ -312,7 +297,7 @@ __device__ __forceinline__ void team_delta(const StepConsts& c, uint32_t s, cons
     const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
     int cx, cy, cz;
     cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
-    const TeamWalk walk{c, src, xa, rm, s, l, ax, ay, az, max(cy - 1, 0), max(cz - 1, 0)};
+    const TeamWalk walk{c, src, xa, rm, s, l, ax, ay, az, cy - 1, cz - 1};
     auto bits = [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) { return walk.bits(row, c0, b0, b3); };
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* t) {
         const float4 q = __ldg(&src[k]);
