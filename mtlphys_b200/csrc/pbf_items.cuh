@@ -804,7 +804,7 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
         uint32_t mask[9], b0[9];
 #pragma unroll
         for (uint32_t r = 0; r < 9; ++r) {
-            mask[r] = in[r * rm.stride];
+            mask[r] = in[size_t(r) * rm.stride];  // (9 rows of 2^30 slots pass 2^32)
             b0[r] = rows.valid(cy - 1 + int(r % 3u), cz - 1 + int(r / 3u))
                         ? cstart[base + r * rows.next_y + (r / 3u) * rows.next_z]
                         : 0u;

@@ -162,12 +162,12 @@ __device__ __forceinline__ uint32_t team_sweep(const Team<G>& team, const StepCo
         uint32_t mask = row_bits(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s);
         mask &= 0xffffffffu >> (max(b0, c0) - c0);
         if (c0 == row_base(b0)) {
-            masks.rows[row * masks.stride + s] = mask;
+            masks.rows[size_t(row) * masks.stride + s] = mask;
             if (b3 - c0 > 32u) over |= 1u << row;
         }
         return mask;
     };
-    auto empty = [&](uint32_t row) { masks.rows[row * masks.stride + s] = 0u; };
+    auto empty = [&](uint32_t row) { masks.rows[size_t(row) * masks.stride + s] = 0u; };
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* t) {
         const float4 q = __ldg(&src[k]);
         float ox = px, oy = py, oz = pz;
@@ -268,7 +268,7 @@ struct TeamWalk {
         rz = __fsub_rn(oz, q.z);
     }
     __device__ __forceinline__ uint32_t bits(uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) const {
-        if (c0 == row_base(b0)) return rm.rows[row * rm.stride + s];
+        if (c0 == row_base(b0)) return rm.rows[size_t(row) * rm.stride + s];
         uint32_t more = 0;
         for (uint32_t k = c0; k < min(c0 + 32u, b3); ++k) {
             float rx, ry, rz;
