@@ -186,9 +186,10 @@ k_finalize_sorted(StepConsts c, const float4* __restrict__ sorted,
 }  // namespace
 
 // 16 lanes per particle up to 16,384 particles: the step of a jittered cube at
-// K = 3 takes 55 us instead of 98 (2,197 particles), 70 / 101 (8,000), 98 / 107
-// (16,000), but 154 / 112 (32,000), where one lane each fills the GPU well
-// enough and does a third of the work.  8 lanes: 65, 78, 113, 164 us.
+// K = 3 takes 53 us instead of 90 (2,197 particles), 69 / 97 (8,000), 76 / 94
+// (10,648: the most that one wave of blocks holds), 97 / 97 (16,000), but 112 / 101
+// (19,683) and 156 / 104 (32,768), where one lane each fills the GPU well enough and
+// does a third of the work.  8 lanes: 65 (2,197), 78 (8,000), 113 us (16,000).
 uint32_t team_lanes(uint32_t n) {
     return n <= 16384u ? kTeam : 0u;
 }
