@@ -36,31 +36,34 @@ namespace {
 
 constexpr uint32_t kScanItems = 8;  // per thread and tile in phase 4
 
-// Grid-wide barrier with a generation counter.  Every block calls it the same
-// number of times.  Blocks arrive at one of several counters, about 32 blocks each
-// (a cache line apart: atomics on one address run one after the other), and each
-// group's last block at the root; the generation that the others poll has a line
-// of its own.  The block that completes the root runs last() before it releases
-// the others, with everything they wrote before the barrier visible: work for
-// one block costs no barrier of its own.
+// Grid-wide barrier.  Every block calls it the same number of times.  All blocks
+// count their arrivals on the word that they then poll: the first block adds bit 31
+// less the number of the others, those add 1, so the last one to arrive flips bit 31
+// and leaves the other bits zero, and nothing has to be reset or passed on.  With
+// `last`, the arrivals are counted elsewhere, and the block that completes them runs
+// last() before it flips the polled word, with everything the others wrote before
+// the barrier visible: work for one block costs no barrier of its own.
 //
-// Against one counter beside the generation and a barrier on each side of the two
-// one-block phases: 12 scenes of 61,000 particles, 223 -> 184 us per step on 592
-// blocks; one scene of 8,000 (with teams and only the blocks it fills) 221 -> 119.
+// Latency of the chain of fences, atomics and polls is all there is to it, so it has
+// as few links as can be: a fence, one atomic and the poll that sees it (2 us between
+// the last arrival and the others' return).  One scene of 8,000 particles 109 -> 92 us
+// per step (11 barriers), 12 of 61,000 in all 156 -> 137, 64 scenes of 4,000 to 20,000
+// on all 1,184 blocks 636 -> 615, against arrivals at counters of 32 blocks each,
+// their sums at a root and a generation word behind it (three atomics and four fences
+// in a row); that form with the blocks polling the root: 101, 147, 624.  The length of
+// the pause between polls makes no difference (0 to 200 ns).
 //
 // The wait is bounded: a block that waits more than a.spin_limit polls sets the
-// error bit and the abort flag.  Returns false (to every thread of the block)
-// when the launch is aborted, by this block or another one; the block must then
-// return.  A barrier only completes once every block has arrived, i.e. finished
-// the phase before it, so a block that returns true works on complete data; a
-// block that left early never arrives at the next barrier, so nobody passes that
-// one.
-//
-// Every round trip to L2 on the way counts: a block keeps the generation it is at
-// (read once per launch), and the generation and the abort flag are the two
-// halves of one word.
+// error bit and the abort flag, the other half of the polled word.  Returns false (to
+// every thread of the block) when the launch is aborted, by this block or another one;
+// the block must then return.  A barrier only completes once every block has arrived,
+// i.e. finished the phase before it, so a block that returns true works on complete
+// data; a block that left early never arrives at the next barrier, so nobody passes
+// that one.
+constexpr unsigned kBarPhase = 0x80000000u;
+
 struct BarrierState {
-    unsigned gen;  // the generation this block waits to leave
+    unsigned phase;  // bit 31 of the phase word until the next barrier completes
     int last, ok;
 };
 
@@ -70,26 +73,51 @@ __device__ __forceinline__ uint2 bar_word(const BatchArgs& a) {
     return w;
 }
 
+// Thread 0: this block is at the barrier that `word` counts.  Returns whether that
+// completes it.
+__device__ __forceinline__ bool arrive(const BatchArgs& a, uint32_t word) {
+    __threadfence();
+    const unsigned inc = blockIdx.x == 0u ? kBarPhase - (gridDim.x - 1u + a.bar_extra) : 1u;
+    const unsigned old = atomicAdd(a.bar + word, inc);
+    return ((old + inc) ^ old) & kBarPhase;
+}
+
+// Thread 0: waits for the barrier's phase to end.
+__device__ __forceinline__ void wait_phase(const BatchArgs& a, BarrierState* state) {
+    int ok = 1;
+    uint32_t spins = 0;
+    uint2 w = bar_word(a);
+    while (((w.x ^ state->phase) & kBarPhase) == 0u && !w.y) {
+        if (++spins > a.spin_limit) {
+            atomicOr(a.err, kDevErrSpin);
+            atomicExch(a.abort, 1u);
+            ok = 0;
+            break;
+        }
+        __nanosleep(32);
+        w = bar_word(a);
+    }
+    state->ok = ok && !w.y;
+    state->phase ^= kBarPhase;
+    __threadfence();
+}
+
+__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, BarrierState* state) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        arrive(a, kBarGen);
+        wait_phase(a, state);
+    }
+    __syncthreads();
+    return state->ok != 0;
+}
+
 template <class Last>
 __device__ __forceinline__ bool grid_barrier(const BatchArgs& a, BarrierState* state, Last&& last) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        // block b belongs to group b mod groups
-        const uint32_t groups = min((gridDim.x + 31u) / 32u, kBarGroups), group = blockIdx.x % groups;
-        const uint32_t members = (gridDim.x - group + groups - 1u) / groups;
-        unsigned* count = a.bar + (1u + group) * kBarLine;
-        int mine = 0;
-        if (atomicAdd(count, 1u) + 1u == members) {
-            *static_cast<volatile unsigned*>(count) = 0u;
-            __threadfence();
-            if (atomicAdd(a.bar + kBarRoot, 1u) + 1u == groups + a.bar_extra) {
-                *static_cast<volatile unsigned*>(a.bar + kBarRoot) = 0u;
-                __threadfence();
-                mine = 1;
-            }
-        }
-        state->last = mine;
+        state->last = arrive(a, kBarRoot);
+        if (state->last) __threadfence();
     }
     __syncthreads();
     if (state->last) {
@@ -97,34 +125,12 @@ __device__ __forceinline__ bool grid_barrier(const BatchArgs& a, BarrierState* s
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
-            atomicAdd(a.bar + kBarGen, 1u);
-            state->ok = !bar_word(a).y;
-            ++state->gen;
+            atomicAdd(a.bar + kBarGen, kBarPhase);
         }
-    } else if (threadIdx.x == 0) {
-        int ok = 1;
-        uint32_t spins = 0;
-        uint2 w = bar_word(a);
-        while (w.x == state->gen && !w.y) {
-            if (++spins > a.spin_limit) {
-                atomicOr(a.err, kDevErrSpin);
-                atomicExch(a.abort, 1u);
-                ok = 0;
-                break;
-            }
-            __nanosleep(32);
-            w = bar_word(a);
-        }
-        state->ok = ok && !w.y;
-        ++state->gen;
-        __threadfence();
     }
+    if (threadIdx.x == 0) wait_phase(a, state);
     __syncthreads();
     return state->ok != 0;
-}
-
-__device__ __forceinline__ bool grid_barrier(const BatchArgs& a, BarrierState* state) {
-    return grid_barrier(a, state, [] {});
 }
 
 template <uint32_t BS>
@@ -199,7 +205,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         return;
     }
     // (no barrier completes before this block arrives, so none has yet)
-    if (threadIdx.x == 0) s_bar.gen = bar_word(a).x;
+    if (threadIdx.x == 0) s_bar.phase = bar_word(a).x;
     const uint32_t gsize = gridDim.x * BS;
     const uint32_t pb = a.p_begin, pe = a.p_end;
     // loops over particles run in whole warps (warp-level operations inside)

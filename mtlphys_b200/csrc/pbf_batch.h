@@ -43,11 +43,10 @@ struct BatchRecord {
     uint32_t stride;       // slots per lam / delta array
 };
 
-// Words of the grid barrier's counters, a cache line each: the root, up to kBarGroups arrival counters, the generation (and beside it
-// the abort flag).
-constexpr uint32_t kBarLine = 32, kBarGroups = 32;
-constexpr uint32_t kBarRoot = 0, kBarGen = (1 + kBarGroups) * kBarLine;
-constexpr uint32_t kBarWords = (2 + kBarGroups) * kBarLine;
+// The grid barrier's words, a cache line each: arrivals at barriers whose last block
+// has work to do, and the word that the blocks poll (its neighbour is the abort flag).
+constexpr uint32_t kBarLine = 32, kBarRoot = 0, kBarGen = kBarLine;
+constexpr uint32_t kBarWords = 2 * kBarLine;
 
 struct BatchArgs {
     SceneDev* scenes;
@@ -64,7 +63,7 @@ struct BatchArgs {
     uint32_t *row_masks, *mask_overflow;
     uint32_t mask_stride;
     uint32_t* total_cells;
-    unsigned* bar;                    // grid barrier: kBarWords words (zero, or a generation at kBarGen)
+    unsigned* bar;                    // grid barrier: kBarWords words (a phase in bit 31, the rest zero)
     uint32_t* err;
     // Bounded grid barrier: a block waits at most spin_limit polls.  One
     // that gives up sets kDevErrSpin and *abort, and every block then leaves
