@@ -213,3 +213,28 @@ def test_scenes_with_and_without_common_constants_give_identical_results(batch):
         np.testing.assert_array_equal(pos[:last], outs[0][0][:last])
         np.testing.assert_array_equal(vel[:last], outs[0][1][:last])
         assert not np.array_equal(pos[last:], outs[0][0][last:])
+
+
+@pytest.mark.parametrize("num, lo, hi", [(5, 1, 9000), (1, 100, 128), (8, 500, 30000)])
+def test_launches_of_different_grid_sizes_share_the_barrier(batch, num, lo, hi):
+    """Every launch leaves the barrier's counter at zero arrivals in either phase:
+    launches of one block, of a few and of hundreds (a scene by itself, all scenes
+    together, other block sizes) follow one another on it and give the same bits."""
+    w = configs.batch_cubes(num=num, lo=lo, hi=hi, steps=6)
+    ref = None
+    for mixed in (False, True):
+        batch.reset(w.counts, w.params, w.dts, w.scenes, w.descs)
+        for i in range(6):
+            if mixed:
+                batch.set_serial(i % 2 == 1)
+                batch.set_launch((128, 256, 512)[i % 3], 0)
+            batch.step()
+        assert batch.check_errors() == 0
+        out = batch.positions(), batch.velocities()
+        batch.set_serial(False)
+        batch.set_launch(256, 0)
+        if ref is None:
+            ref = out
+        else:
+            np.testing.assert_array_equal(out[0], ref[0])
+            np.testing.assert_array_equal(out[1], ref[1])
