@@ -343,12 +343,16 @@ int mp_batch_get_params(const mp_batch* b, uint32_t scene, mp_pbf_params* params
  * mp_engine_check_errors).  When a grid barrier gave up (MP_ERR_SPIN_LIMIT),
  * the launch left every block at its next barrier, so the state of that step
  * is invalid, and every step after it did nothing; this call re-arms the
- * batch, which steps again from its (invalid) state: restore or reset it. */
+ * batch, which steps again from its (invalid) state: restore or reset it, or
+ * upload positions and velocities and set the spheres. */
 int mp_batch_check_errors(mp_batch* b, uint32_t* bits);
 /* Test hook: every grid barrier of the following steps waits for `extra`
  * more blocks than the launch has (0 = normal), so every wait runs out after
  * the mp_set_spin_limit bound.  For failure-path tests only. */
 int mp_batch_debug_barrier_extra(mp_batch* b, uint32_t extra);
+/* Test hook: lets the first `barriers` barriers of every launch pass as usual
+ * (0 = none) before mp_batch_debug_barrier_extra's wait runs out. */
+int mp_batch_debug_barrier_pass(mp_batch* b, uint32_t barriers);
 
 /* ---- differentiable rollouts (no reference counterpart: the reference
  *      engine is not differentiable) ------------------------------------------

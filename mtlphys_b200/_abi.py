@@ -238,6 +238,7 @@ PROTOTYPES = {
     "mp_set_spin_limit": (_INT, [_U32]),
     "mp_set_device_allocator": (_INT, [_VP, _VP, _VP]),
     "mp_batch_debug_barrier_extra": (_INT, [_VP, _U32]),
+    "mp_batch_debug_barrier_pass": (_INT, [_VP, _U32]),
 }
 
 # mp_device_alloc_fn / mp_device_free_fn

@@ -63,7 +63,7 @@ struct mp_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     uint32_t graph_spin_epoch = 0;  // spin limits the captured graph was made with
-    uint32_t bar_extra = 0;         // test hook: mp_batch_debug_barrier_extra
+    uint32_t bar_extra = 0, bar_pass = 0;  // test hooks: mp_batch_debug_barrier_extra, _pass
 
     // ---- differentiable rollouts ----
     // One recorded step: the record arrays of the step kernel plus its own
@@ -317,6 +317,7 @@ struct mp_batch {
         BatchArgs args = a;
         args.spin_limit = barrier_spin_limit();
         args.bar_extra = bar_extra;
+        args.bar_pass = bar_pass;
         return args;
     }
 
@@ -1016,8 +1017,15 @@ int mp_batch_check_errors(mp_batch* b, uint32_t* bits) {
         MP_CUDA(cudaMemset(b->a.err, 0, 4));
         if (w & kDevErrSpin) {
             // a barrier wait gave up: the launch left the barrier's counters
-            // mid-count and the abort flag (one of its words) set; re-arm both
+            // mid-count, the abort flag (one of its words) set, and perhaps what
+            // a step expects clean of the one before it: the cell counts (else
+            // ranks and slots run past the particles) and the bounding boxes
             MP_CUDA(cudaMemset(b->a.bar, 0, sizeof(unsigned) * kBarWords));
+            MP_CUDA(cudaMemset(b->a.counts, 0, (size_t(b->max_cells) + 1) * 4));
+            std::vector<SceneDev> cur(b->S);
+            MP_CUDA(cudaMemcpy(cur.data(), b->scenes, sizeof(SceneDev) * b->S, cudaMemcpyDeviceToHost));
+            for (SceneDev& sd : cur) empty_box(sd.bb);
+            MP_CUDA(cudaMemcpy(b->scenes, cur.data(), sizeof(SceneDev) * b->S, cudaMemcpyHostToDevice));
         }
     }
     if (bits) *bits = w;
@@ -1030,6 +1038,13 @@ int mp_batch_debug_barrier_extra(mp_batch* b, uint32_t extra) {
     if (!b) return fail(MP_ERR_INVALID_ARGUMENT, "NULL batch");
     if (extra > 1024) return fail(MP_ERR_INVALID_ARGUMENT, "extra = %u > 1024", extra);
     b->bar_extra = extra;
+    b->drop_graph();
+    return MP_OK;
+}
+
+int mp_batch_debug_barrier_pass(mp_batch* b, uint32_t barriers) {
+    if (!b) return fail(MP_ERR_INVALID_ARGUMENT, "NULL batch");
+    b->bar_pass = barriers;
     b->drop_graph();
     return MP_OK;
 }

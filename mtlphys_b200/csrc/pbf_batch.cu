@@ -64,6 +64,7 @@ constexpr unsigned kBarPhase = 0x80000000u;
 
 struct BarrierState {
     unsigned phase;  // bit 31 of the phase word until the next barrier completes
+    unsigned passed;  // barriers so far (counted by the first block, for bar_pass only)
     int last, ok;
 };
 
@@ -75,9 +76,13 @@ __device__ __forceinline__ uint2 bar_word(const BatchArgs& a) {
 
 // Thread 0: this block is at the barrier that `word` counts.  Returns whether that
 // completes it.
-__device__ __forceinline__ bool arrive(const BatchArgs& a, uint32_t word) {
+__device__ __forceinline__ bool arrive(const BatchArgs& a, uint32_t word, BarrierState* state) {
     __threadfence();
-    const unsigned inc = blockIdx.x == 0u ? kBarPhase - (gridDim.x - 1u + a.bar_extra) : 1u;
+    unsigned inc = 1u;
+    if (blockIdx.x == 0u) {
+        inc = kBarPhase - (gridDim.x - 1u);
+        if (a.bar_extra && state->passed++ >= a.bar_pass) inc -= a.bar_extra;
+    }
     const unsigned old = atomicAdd(a.bar + word, inc);
     return ((old + inc) ^ old) & kBarPhase;
 }
@@ -105,7 +110,7 @@ __device__ __forceinline__ void wait_phase(const BatchArgs& a, BarrierState* sta
 __device__ __forceinline__ bool grid_barrier(const BatchArgs& a, BarrierState* state) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        arrive(a, kBarGen);
+        arrive(a, kBarGen, state);
         wait_phase(a, state);
     }
     __syncthreads();
@@ -116,7 +121,7 @@ template <class Last>
 __device__ __forceinline__ bool grid_barrier(const BatchArgs& a, BarrierState* state, Last&& last) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        state->last = arrive(a, kBarRoot);
+        state->last = arrive(a, kBarRoot, state);
         if (state->last) __threadfence();
     }
     __syncthreads();
@@ -205,7 +210,10 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         return;
     }
     // (no barrier completes before this block arrives, so none has yet)
-    if (threadIdx.x == 0) s_bar.phase = bar_word(a).x;
+    if (threadIdx.x == 0) {
+        s_bar.phase = bar_word(a).x;
+        s_bar.passed = 0;
+    }
     const uint32_t gsize = gridDim.x * BS;
     const uint32_t pb = a.p_begin, pe = a.p_end;
     // loops over particles run in whole warps (warp-level operations inside)

@@ -69,10 +69,11 @@ struct BatchArgs {
     // that gives up sets kDevErrSpin and *abort, and every block then leaves
     // the launch at its next barrier; a launch that starts with *abort set
     // does nothing (the host clears it in mp_batch_check_errors).
-    // bar_extra (a test hook, normally 0) makes every barrier wait for that
-    // many more blocks than the launch has, so that each wait runs out.
+    // bar_extra (a test hook, normally 0) makes every barrier after the first
+    // bar_pass ones of a launch wait for that many more blocks than the launch
+    // has, so that the wait runs out.
     uint32_t* abort;
-    uint32_t spin_limit, bar_extra;
+    uint32_t spin_limit, bar_extra, bar_pass;
     uint32_t common;  // 1: every scene has the pair constants `pair`, with an s_corr exponent of 4
     PairConsts pair;
     uint32_t scorr4;  // 1: every scene's s_corr exponent is 4 (the kernel fixes it at compile time)
