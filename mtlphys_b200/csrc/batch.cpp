@@ -240,7 +240,7 @@ struct mp_batch {
         args.scell = sl.scell;
         args.cstart = sl.cstart;
         args.rec = sl.rec;
-        const cudaError_t e = launch_batch_step(args, block, std::min(blocks(), useful_blocks(N)), s);
+        const cudaError_t e = launch_batch_step(args, block, std::min(blocks(), useful_blocks(N, N)), s);
         if (e != cudaSuccess) return fail(MP_ERR_CUDA, "recorded step launch: %s", cudaGetErrorString(e));
         return MP_OK;
     }
@@ -293,10 +293,11 @@ struct mp_batch {
         return (blocks_per_sm ? std::min(blocks_per_sm, occ_blocks) : occ_blocks) * sms;
     }
 
-    // Blocks that a launch over n particles can put to work: a grid barrier costs
-    // more the more blocks it waits for (the results do not depend on the grid).
-    uint32_t useful_blocks(uint32_t n) const {
-        const uint64_t lanes = std::max<uint32_t>(1u, team_lanes(n));
+    // Blocks that a launch over the n particles up to slot `end` can put to work: a
+    // grid barrier costs more the more blocks it waits for (the results do not depend
+    // on the grid).
+    uint32_t useful_blocks(uint32_t n, uint32_t end) const {
+        const uint64_t lanes = std::max<uint32_t>(1u, team_lanes(n, end));
         return uint32_t(std::max<uint64_t>(1u, (n * lanes + block - 1) / block));
     }
 
@@ -330,7 +331,7 @@ struct mp_batch {
             args.scene_end = S;
             args.p_begin = 0;
             args.p_end = N;
-            const cudaError_t e = launch_batch_step(args, block, std::min(nb, useful_blocks(N)), s);
+            const cudaError_t e = launch_batch_step(args, block, std::min(nb, useful_blocks(N, N)), s);
             if (e != cudaSuccess) return fail(MP_ERR_CUDA, "batch step launch: %s", cudaGetErrorString(e));
             return MP_OK;
         }
@@ -342,7 +343,7 @@ struct mp_batch {
             args.scene_end = sc + 1;
             args.p_begin = p0[sc];
             args.p_end = p0[sc] + counts[sc];
-            const cudaError_t e = launch_batch_step(args, block, std::min(nb, useful_blocks(counts[sc])), s);
+            const cudaError_t e = launch_batch_step(args, block, std::min(nb, useful_blocks(counts[sc], args.p_end)), s);
             if (e != cudaSuccess) return fail(MP_ERR_CUDA, "batch step launch: %s", cudaGetErrorString(e));
         }
         return MP_OK;

@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(128) k_adj_sphere(AdjArgs a) {
 cudaError_t launch_adjoint_step(const AdjArgs& a, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
     const uint32_t grid = cdiv(a.n, kBlock), sweep_grid = cdiv(a.n, kSweepBlock);
-    const bool team = team_lanes(a.n) != 0;
+    const bool team = team_lanes(a.n, a.n) != 0;
     const uint32_t team_grid = cdiv(a.n, kTeamBlock / kTeam);
     k_adj_finalize<<<grid, kBlock, 0, s>>>(a);
     for (uint32_t it = a.iterations; it-- > 0;) {

@@ -499,7 +499,7 @@ cudaError_t allow_shared(const void* fn, size_t bytes) {
 template <uint32_t BS>
 cudaError_t launch_bs(const BatchArgs& args, uint32_t blocks, cudaStream_t s) {
     void* kargs[] = {const_cast<BatchArgs*>(&args)};
-    const bool team = args.iterations && team_lanes(args.p_end - args.p_begin) != 0;
+    const bool team = args.iterations && team_lanes(args.p_end - args.p_begin, args.p_end) != 0;
     const void* fn = batch_kernel<BS>(args.scorr4 != 0, args.common != 0, team, args.rec.lam != nullptr);
     const size_t bytes = shared_bytes<BS>(team);
     const cudaError_t e = allow_shared(fn, bytes);

@@ -101,9 +101,20 @@ cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t itera
                           cudaStream_t s, KernelTimer* t = nullptr);
 
 // Lanes per particle of the solver passes of n particles (pbf_team.cuh): kTeam,
-// or 0 for one lane each.
+// or 0 for one lane each.  end: the slot after the launch's last one; a team's
+// list of candidates holds 28-bit slots, so a small scene that lies beyond them in
+// a batch of 268 million particles or more takes one lane each.
+//
+// 16 lanes per particle up to 16,384 particles: the step of a jittered cube at
+// K = 3 takes 53 us instead of 90 (2,197 particles), 69 / 97 (8,000), 76 / 94
+// (10,648: the most that one wave of blocks holds), 97 / 97 (16,000), but 112 / 101
+// (19,683) and 156 / 104 (32,768), where one lane each fills the GPU well enough and
+// does a third of the work.  8 lanes: 65 (2,197), 78 (8,000), 113 us (16,000).
 constexpr uint32_t kTeam = 16;
-uint32_t team_lanes(uint32_t n);
+constexpr uint32_t kTeamMaxSlots = 1u << 28;
+inline uint32_t team_lanes(uint32_t n, uint32_t end) {
+    return n <= 16384u && end <= kTeamMaxSlots ? kTeam : 0u;
+}
 
 // Number of kernel launches one step issues (for the benchmark's count).
 uint32_t step_launch_count(uint32_t iterations);

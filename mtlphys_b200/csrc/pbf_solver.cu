@@ -185,15 +185,6 @@ k_finalize_sorted(StepConsts c, const float4* __restrict__ sorted,
 
 }  // namespace
 
-// 16 lanes per particle up to 16,384 particles: the step of a jittered cube at
-// K = 3 takes 53 us instead of 90 (2,197 particles), 69 / 97 (8,000), 76 / 94
-// (10,648: the most that one wave of blocks holds), 97 / 97 (16,000), but 112 / 101
-// (19,683) and 156 / 104 (32,768), where one lane each fills the GPU well enough and
-// does a third of the work.  8 lanes: 65 (2,197), 78 (8,000), 113 us (16,000).
-uint32_t team_lanes(uint32_t n) {
-    return n <= 16384u ? kTeam : 0u;
-}
-
 cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t iterations,
                           cudaStream_t s, KernelTimer* t) {
     const uint32_t n = c.n;
@@ -208,7 +199,7 @@ cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t itera
         tend(t, "finalize", s);
         return cudaGetLastError();
     }
-    if (team_lanes(n))
+    if (team_lanes(n, n))
         launch_iterations<kTeam>(c, d, iterations, s, t);
     else
         launch_iterations<0>(c, d, iterations, s, t);

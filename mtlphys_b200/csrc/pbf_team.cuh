@@ -23,13 +23,12 @@ namespace mpb {
 
 constexpr uint32_t kTeamChunks = 10;  // row chunks (of 32 candidates) expanded at a time
 constexpr uint32_t kTeamPairs = 32;   // pairs whose terms are computed at a time
-constexpr uint32_t kTeamMaxSlots = 1u << 28;  // list entries hold 28-bit slots
 
 // Shared memory of one team that adds up SUMS sums.
 template <uint32_t SUMS>
 struct TeamBufOf {
     uint32_t b0[9], b3[9], chunks[9];      // rows: slot range, number of chunks
-    uint32_t list[kTeamChunks * 32];       // slot | y << 28 | z << 30
+    uint32_t list[kTeamChunks * 32];       // slot (below kTeamMaxSlots) | y << 28 | z << 30
     float2 term[SUMS][kTeamPairs + 1];     // per sum: the factors of each pair's term
 };
 using TeamBuf = TeamBufOf<5>;
