@@ -100,6 +100,9 @@ struct mp_batch {
                            al(sizeof(SphereState) * std::max<uint32_t>(S, 1u)) + al(v4) + 2 * al(u) +
                            al((size_t(max_cells) + 1) * 4) + K * (2 * al(v4) + al(9 * u) + al(u));
         MP_ALLOC(tape_block, per * nslots, device);
+        // a recorded step that gave up at a barrier leaves the rest of its record as it
+        // was; the adjoint kernels follow its indices
+        MP_CUDA(cudaMemset(tape_block, 0, per * nslots));
         char* p = static_cast<char*>(tape_block);
         auto take = [&](size_t bytes) {
             char* r = p;
@@ -188,6 +191,7 @@ struct mp_batch {
         adj.spart = reinterpret_cast<double4*>(take(32 * size_t(chunks) * std::max<uint32_t>(S, 1u)));
         adj.sum_chunks = chunks;
         adj.err = a.err;
+        adj.abort = a.abort;
         adj.grads = reinterpret_cast<double*>(p);
         adj.scene_of = a.scene_of;
         adj.n = N;

@@ -395,6 +395,11 @@ __device__ __forceinline__ float scorr_grad(const PairConsts& pc, uint32_t n) {
     return n ? 6.0f * pc.scorr_k * float(n) * pc.inv_wq * pc.poly6 : 0.0f;
 }
 
+// Whether a recorded step gave up at a barrier.  Its record may mix two steps', so
+// the pair sweeps leave their sums alone (the kernels that follow one index per slot
+// stay inside their arrays).  Loaded beside the slot's own values, where it is free.
+__device__ __forceinline__ bool stopped(const AdjArgs& a) { return __ldg(a.abort) != 0u; }
+
 __device__ __forceinline__ RowMasks recorded_masks(const AdjArgs& a, uint32_t it) {
     const uint32_t ms = a.mask_stride;
     return RowMasks{const_cast<uint32_t*>(a.t.masks) + size_t(it) * 9 * ms,
@@ -406,6 +411,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjA
     __shared__ uint2 queue[kQueue * kSweepBlock];
     const uint32_t m = blockIdx.x * kSweepBlock + threadIdx.x;
     if (m >= a.n) return;
+    const bool stop = stopped(a);
     const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
     const float4* src = a.t.lam + size_t(it) * a.stride;
     const DeltaSlot o(a, c, src, m);
@@ -429,6 +435,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjA
         py = __fadd_rn(py, t.vy);
         pz = __fadd_rn(pz, t.vz);
     };
+    if (stop) return;
     queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, recorded_masks(a, it), m, o.l, o.ax, o.ay, o.az, o.cx,
                               o.cy, o.cz, PairQueue<kSweepBlock>(queue), body);
     delta_out(a, c, m, gx, gy, gz, gsq, kb, lb, px, py, pz);
@@ -444,6 +451,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_adj_delta_team(AdjArgs a, uint32
     const uint32_t m = (blockIdx.x * kTeamBlock + threadIdx.x) / kTeam;
     if (m >= a.n) return;
     const Team<kTeam, TeamBufOf<9>> team(bufs);
+    const bool stop = stopped(a);
     const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
     const float4* src = a.t.lam + size_t(it) * a.stride;
     const DeltaSlot o(a, c, src, m);
@@ -474,6 +482,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_adj_delta_team(AdjArgs a, uint32
         put(8, t.vz, 1.0f);
     };
     float sum = 0.0f;
+    if (stop) return;
     team_pairs<kTeam, 9>(
         team, c, a.t.cstart, o.cx, o.cy, o.cz, sum,
         [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) { return walk.bits(row, c0, b0, b3); },
@@ -534,6 +543,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(Adj
     __shared__ uint2 queue[kQueue * kSweepBlock];
     const uint32_t m = blockIdx.x * kSweepBlock + threadIdx.x;
     if (m >= a.n) return;
+    const bool stop = stopped(a);
     const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
     const float4* src = a.t.lam + size_t(it) * a.stride;
     const DeltaSlot o(a, c, src, m);
@@ -549,6 +559,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(Adj
         py = __fadd_rn(py, v.y);
         pz = __fadd_rn(pz, v.z);
     };
+    if (stop) return;
     queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, recorded_masks(a, it), m, o.l, o.ax, o.ay, o.az, o.cx,
                               o.cy, o.cz, PairQueue<kSweepBlock>(queue), body);
     a.pbar[m] = make_float4(px, py, pz, 0.0f);
@@ -559,6 +570,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_adj_lambda_team(AdjArgs a, uint3
     const uint32_t m = (blockIdx.x * kTeamBlock + threadIdx.x) / kTeam;
     if (m >= a.n) return;
     const Team<kTeam, TeamBufOf<3>> team(bufs);
+    const bool stop = stopped(a);
     const StepConsts& c = a.t.scenes[a.scene_of[m]].c;
     const float4* src = a.t.lam + size_t(it) * a.stride;
     const DeltaSlot o(a, c, src, m);
@@ -579,6 +591,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_adj_lambda_team(AdjArgs a, uint3
         out[2 * kTermStride] = make_float2(v.z, 1.0f);
     };
     float sum = team.lane == 0 ? qb.x : team.lane == 1 ? qb.y : qb.z;
+    if (stop) return;
     team_pairs<kTeam, 3>(
         team, c, a.t.cstart, o.cx, o.cy, o.cz, sum,
         [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) { return walk.bits(row, c0, b0, b3); },

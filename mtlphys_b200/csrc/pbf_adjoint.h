@@ -77,6 +77,7 @@ struct AdjArgs {
     double4 *sacc, *spart;
     uint32_t sum_chunks;
     uint32_t* err;                // device error word (kDevErrIndex: a post was dropped)
+    const uint32_t* abort;        // set: a recorded step was stopped, its record is not whole
     double* grads;                // nscenes x kGradStride
 };
 

@@ -56,3 +56,42 @@ def test_a_stopped_step_leaves_nothing_behind(cuda, passed):
         lib.mp_set_spin_limit(0)
         b.close()
         ref.close()
+
+
+@pytest.mark.parametrize("passed", [0, 3, 6, 9])
+def test_a_backward_pass_whose_recorded_step_stops_can_be_repeated(cuda, passed):
+    """The adjoint kernels that follow a stopped step stay inside their arrays (the
+    record is a new one, then one that holds other steps), and the same rollout gives
+    its gradients once the error has been read."""
+    import torch
+
+    lib = _abi.load()
+    b = small_batch()
+    try:
+        n = b.particle_count()
+        g = torch.from_numpy(np.random.default_rng(4).normal(size=(n, 4)).astype(np.float32)).cuda()
+
+        def stop():
+            lib.mp_set_spin_limit(SHORT)
+            assert lib.mp_batch_debug_barrier_extra(b._h, 1) == _abi.MP_OK
+            assert lib.mp_batch_debug_barrier_pass(b._h, passed) == _abi.MP_OK
+            b.rollout_backward(g, g)
+            assert lib.mp_batch_check_errors(b._h, None) == _abi.MP_ERR_SPIN_LIMIT
+            lib.mp_set_spin_limit(0)
+            assert lib.mp_batch_debug_barrier_extra(b._h, 0) == _abi.MP_OK
+
+        b.rollout_forward(4, 2)
+        end = b.positions()
+        stop()
+        first = [t.cpu().numpy() for t in b.rollout_backward(g, g)]
+        assert b.check_errors() == 0
+        stop()
+        again = [t.cpu().numpy() for t in b.rollout_backward(g, g)]
+        assert b.check_errors() == 0
+        for x, y in zip(first, again):
+            assert np.isfinite(x).all()
+            np.testing.assert_array_equal(x, y)
+        np.testing.assert_array_equal(end, b.positions())
+    finally:
+        lib.mp_set_spin_limit(0)
+        b.close()
