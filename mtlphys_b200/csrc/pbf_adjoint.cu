@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_delta(AdjA
         pz = __fadd_rn(pz, t.vz);
     };
     if (stop) return;
-    queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, recorded_masks(a, it), m, o.l, o.ax, o.ay, o.az, o.cx,
+    queued_pairs<true, kSweepBlock>(c, src, a.xa, a.t.cstart, recorded_masks(a, it), m, o.l, o.ax, o.ay, o.az, o.cx,
                               o.cy, o.cz, PairQueue<kSweepBlock>(queue), body);
     delta_out(a, c, m, gx, gy, gz, gsq, kb, lb, px, py, pz);
 }
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_adj_delta_team(AdjArgs a, uint32
     const uint32_t n = SN ? SN : pc.scorr_n;
     const float sgk = scorr_grad(pc, n);
     const RowMasks rm = recorded_masks(a, it);
-    const TeamWalk walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, o.cy - 1, o.cz - 1};
+    const TeamWalk<true> walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, o.cy - 1, o.cz - 1};
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* out) {
         const float4 q = __ldg(&src[k]);
         float rx, ry, rz;
@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(Adj
         pz = __fadd_rn(pz, v.z);
     };
     if (stop) return;
-    queued_pairs<kSweepBlock>(c, src, a.xa, a.t.cstart, recorded_masks(a, it), m, o.l, o.ax, o.ay, o.az, o.cx,
+    queued_pairs<true, kSweepBlock>(c, src, a.xa, a.t.cstart, recorded_masks(a, it), m, o.l, o.ax, o.ay, o.az, o.cx,
                               o.cy, o.cz, PairQueue<kSweepBlock>(queue), body);
     a.pbar[m] = make_float4(px, py, pz, 0.0f);
 }
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_adj_lambda_team(AdjArgs a, uint3
     const float4 qb = a.qbar[m];
     const PairConsts pc = pair_consts(c);
     const RowMasks rm = recorded_masks(a, it);
-    const TeamWalk walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, o.cy - 1, o.cz - 1};
+    const TeamWalk<true> walk{c, src, a.xa, rm, m, o.l, o.ax, o.ay, o.az, o.cy - 1, o.cz - 1};
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* out) {
         float rx, ry, rz;
         walk.offset(k, __ldg(&src[k]), y, z, rx, ry, rz);

@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     if (a.iterations == 0) {
         if constexpr (G == 0)
             for (uint32_t s = pb + gtid; s < pe; s += gsize)
-                count_neighbors_item<BS>(sc[a.scene_of[s]].c, s, a.sorted_a, a.qpos, a.cstart, a.sidx, a.ncount,
+                count_neighbors_item<false, BS>(sc[a.scene_of[s]].c, s, a.sorted_a, a.qpos, a.cstart, a.sidx, a.ncount,
                                          1u, PairQueue<BS>(queue));
         if (!grid_barrier(a, &s_bar)) return;
         for (uint32_t s = pb + gtid; s < pe; s += gsize)
@@ -417,30 +417,30 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             if constexpr (G != 0) {
                 if (it == 0) {
                     if (last)
-                        team_lambda_first<true, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                        team_lambda_first<true, false, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
                                                    a.lambdas, a.ncount, rmi, bufs);
                     else
-                        team_lambda_first<false, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                        team_lambda_first<false, false, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
                                                     a.lambdas, a.ncount, rmi, bufs);
                 } else if (last) {
-                    team_lambda<true, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                    team_lambda<true, false, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
                                          rmi, bufs);
                 } else {
-                    team_lambda<false, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                    team_lambda<false, false, G>(c, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
                                           rmi, bufs);
                 }
             } else if (it == 0) {
                 if (last)
-                    lambda_first_item<true, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                    lambda_first_item<true, false, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
                                                 a.lambdas, a.ncount, rmi, queue);
                 else
-                    lambda_first_item<false, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
+                    lambda_first_item<false, false, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx,
                                                  a.lambdas, a.ncount, rmi, queue);
             } else if (last) {
-                lambda_item<true, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                lambda_item<true, false, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
                                       rmi, queue);
             } else {
-                lambda_item<false, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
+                lambda_item<false, false, BS>(c, pc, s, a.sorted_a, a.qpos, lam_out, a.scell, a.cstart, a.sidx, a.lambdas,
                                        rmi, queue);
             }
         }
@@ -450,19 +450,19 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
             const auto& pc = pair_constants<COMMON>(a, sd.c);
             if constexpr (G != 0) {
                 if (last)
-                    team_delta<true, SN, G>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                    team_delta<true, SN, false, G>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
                                             &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
                                             bufs);
                 else
-                    team_delta<false, SN, G>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                    team_delta<false, SN, false, G>(sd.c, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
                                              &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
                                              bufs);
             } else if (last) {
-                delta_item<true, SN, BS>(sd.c, pc, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                delta_item<true, SN, false, BS>(sd.c, pc, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
                                          &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
                                          queue);
             } else {
-                delta_item<false, SN, BS>(sd.c, pc, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
+                delta_item<false, SN, false, BS>(sd.c, pc, s, lam_out, a.sorted_a, a.qpos, a.xa, a.scell, a.cstart, a.sidx,
                                           &sd.sphere, a.pos, a.vel, a.prev, a.ncount, a.foam, a.err, rmi, drec,
                                           queue);
             }

@@ -264,7 +264,7 @@ k_count_neighbors(StepConsts c, const float4* __restrict__ sorted, const uint32_
     __shared__ uint2 queue[kQueue * kCB];
     const uint32_t s = blockIdx.x * kCB + threadIdx.x;
     if (s < c.n)
-        count_neighbors_item<kCB>(c, s, sorted, qpos, cstart, sidx, ncount, *strays, PairQueue<kCB>(queue));
+        count_neighbors_item<true, kCB>(c, s, sorted, qpos, cstart, sidx, ncount, *strays, PairQueue<kCB>(queue));
 }
 
 inline uint32_t cdiv(uint32_t a, uint32_t b) { return (a + b - 1) / b; }

@@ -337,6 +337,35 @@ __device__ __forceinline__ void delta_add(const C& c, float li, float lj, float 
     }
 }
 
+// A load of an array that other kernels write.  RO: nothing in this launch writes it,
+// so it may go through the read-only path.  The persistent batch kernel writes these
+// arrays in one phase and reads them in another, which only an ordinary load may do
+// (its grid barrier orders those).  Written as instructions: as plain C++ loads the
+// compiler moves and splits them, spills more (144 -> 232 bytes of spill loads) and a
+// step of 256 cubes takes 4.28 ms instead of 4.00.
+__device__ __forceinline__ float load_ordinary(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 load_ordinary(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 load_ordinary(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+template <bool RO, class T>
+__device__ __forceinline__ T load(const T* p) {
+    if constexpr (RO)
+        return __ldg(p);
+    else
+        return load_ordinary(p);
+}
+
 // First slot of a row mask: the row's first slot, rounded down to a 16-byte
 // boundary of the quantized positions.
 __device__ __forceinline__ uint32_t row_base(uint32_t b0) { return b0 & ~3u; }
@@ -469,6 +498,7 @@ struct StencilRows {
 // Phase 1 of a sweep: the prefilter's bits of slots [c0, c1), c0 a multiple of 4, at
 // most 32 of them (first one in bit 31), without slot s.  Reads up to 7 slots past
 // c1.
+template <bool RO>
 __device__ __forceinline__ uint32_t row_bits(const uint32_t* __restrict__ qsrc, uint32_t qi, int nthr, uint32_t c0,
                                              uint32_t c1, uint32_t s) {
     uint32_t mask = 0, k = c0;
@@ -477,7 +507,7 @@ __device__ __forceinline__ uint32_t row_bits(const uint32_t* __restrict__ qsrc, 
         mask = __funnelshift_l(uint32_t(__dp4a(d, d, nthr)), mask, 1);
     };
     for (; k < c1; k += 4) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(qsrc + k));
+        const uint4 q = load<RO>(reinterpret_cast<const uint4*>(qsrc + k));
         test(q.x);
         test(q.y);
         test(q.z);
@@ -512,14 +542,14 @@ __device__ __forceinline__ uint32_t row_bits(const uint32_t* __restrict__ qsrc, 
 // Every row of the stencil stores the bits of its first chunk (the particle's
 // own bit cleared) for the delta pass, and a row longer than one chunk sets
 // its bit in the overflow word.
-template <bool ANCHORED, uint32_t BS, class Body>
+template <bool ANCHORED, bool RO, uint32_t BS, class Body>
 __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restrict__ src,
                                       const uint32_t* __restrict__ qsrc,
                                       const uint32_t* __restrict__ cstart, int cx, int cy, int cz,
                                       float px, float py, float pz, float aix, float aiy, float aiz,
                                       uint32_t qi, int nthr, uint32_t s, const RowMasks& masks,
                                       PairQueue<BS> queue, Body&& body) {
-    auto fetch = [&](uint32_t k) { return __ldg(&src[k]); };
+    auto fetch = [&](uint32_t k) { return load<RO>(&src[k]); };
     auto visit = [&](uint32_t k, const float4& q, float oy, float oz) {
         const float ox = ANCHORED ? __fadd_rn(__fsub_rn(aix, q.w), px) : px;
         const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
@@ -548,7 +578,7 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
             }
             uint32_t mask = 0;
             const uint32_t a0 = row_base(b0);
-            if (b0 < b3) mask = row_bits(qsrc, qi, nthr, a0, min(a0 + 32u, b3), s) & (0xffffffffu >> (b0 - a0));
+            if (b0 < b3) mask = row_bits<RO>(qsrc, qi, nthr, a0, min(a0 + 32u, b3), s) & (0xffffffffu >> (b0 - a0));
             // the bits of the row's first chunk (the whole row if b3 - a0 <= 32)
             *out = mask;
             const uint32_t code = uint32_t(y) | (uint32_t(z) << 2);
@@ -559,7 +589,7 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
                 for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
                     // room for this chunk and the first ones of the rows to come
                     if (queue.short_of(9u - row)) queue.template drain<false>(o, fetch, visit);
-                    queue.push(row_bits(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s), c0, code);
+                    queue.push(row_bits<RO>(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s), c0, code);
                 }
             }
             b0 = n0;
@@ -585,7 +615,7 @@ __device__ __forceinline__ int prefilter(const StepConsts& c, int hx, int hy, in
 // particle lies outside its cell, so that no byte difference wraps to a small
 // value: `strays` is 0), and only the shell in between, a sixth of the
 // neighbours, is tested exactly.
-template <uint32_t BS>
+template <bool RO, uint32_t BS>
 __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32_t s,
                                                      const float4* __restrict__ sorted,
                                                      const uint32_t* __restrict__ qsrc,
@@ -604,7 +634,7 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
     const int y0 = max(cy - 1, 0), y1 = min(cy + 1, c.g.gy - 1);
     const int z0 = max(cz - 1, 0), z1 = min(cz + 1, c.g.gz - 1);
     uint32_t cnt = 0;
-    auto fetch = [&](uint32_t k) { return __ldg(&sorted[k]); };
+    auto fetch = [&](uint32_t k) { return load<RO>(&sorted[k]); };
     auto visit = [&](uint32_t, const float4& q, float, float) {
         cnt += dist2(q.x - p.x, q.y - p.y, q.z - p.z) < c.h2 ? 1u : 0u;
     };
@@ -618,7 +648,7 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
                 const uint32_t c1 = min(c0 + 32u, b3);
                 uint32_t maybe = 0, in = 0, k = c0;
                 for (; k < c1; k += 4) {
-                    const uint4 q = __ldg(reinterpret_cast<const uint4*>(qsrc + k));
+                    const uint4 q = load<RO>(reinterpret_cast<const uint4*>(qsrc + k));
                     const int d0 = int(qi - q.x), d1 = int(qi - q.y);
                     const int d2 = int(qi - q.z), d3 = int(qi - q.w);
                     const int s0 = __dp4a(d0, d0, nthr), s1 = __dp4a(d1, d1, nthr);
@@ -649,7 +679,7 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
 // First lambda pass: absolute FP32 predicted positions (reference arithmetic,
 // so the fused neighbour count equals countNeighbors bit for bit); converts
 // the state to anchored offsets for the following passes.
-template <bool LAST, uint32_t BS, class C>
+template <bool LAST, bool RO, uint32_t BS, class C>
 __device__ __forceinline__ void lambda_first_item(const StepConsts& c, const C& pc, uint32_t s,
                                                   const float4* __restrict__ cur,
                                                   const uint32_t* __restrict__ qpos,
@@ -674,7 +704,7 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, const C& 
     LambdaAcc acc;
     acc.self(pc);
     uint32_t cnt = 0;
-    sweep<false, BS>(c, cur, qpos, cstart, cx, cy, cz, p.x, p.y, p.z, 0.0f, 0.0f, 0.0f, qi, nthr, s, rm,
+    sweep<false, RO, BS>(c, cur, qpos, cstart, cx, cy, cz, p.x, p.y, p.z, 0.0f, 0.0f, 0.0f, qi, nthr, s, rm,
                      PairQueue<BS>(queue),
                      [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
                          cnt += r2 < pc.h2 ? 1u : 0u;
@@ -690,7 +720,7 @@ __device__ __forceinline__ void lambda_first_item(const StepConsts& c, const C& 
 
 // Later lambda passes on the anchored state: cur is the previous delta pass's
 // output, (l, x anchor of the hash cell) per slot.
-template <bool LAST, uint32_t BS, class C>
+template <bool LAST, bool RO, uint32_t BS, class C>
 __device__ __forceinline__ void lambda_item(const StepConsts& c, const C& pc, uint32_t s,
                                             const float4* __restrict__ cur,
                                             const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
@@ -707,7 +737,7 @@ __device__ __forceinline__ void lambda_item(const StepConsts& c, const C& pc, ui
     const int nthr = prefilter(c, pcx + c.g.lx, pcy + c.g.ly, pcz + c.g.lz, l.x, l.y, l.z, qi);
     LambdaAcc acc;
     acc.self(pc);
-    sweep<true, BS>(c, cur, qpos, cstart, cx, cy, cz, l.x, l.y, l.z, ax, ay, az, qi, nthr, s, rm,
+    sweep<true, RO, BS>(c, cur, qpos, cstart, cx, cy, cz, l.x, l.y, l.z, ax, ay, az, qi, nthr, s, rm,
                     PairQueue<BS>(queue),
                     [&](uint32_t, const float4&, float rx, float ry, float rz, float r2) {
                         acc.add(pc, rx, ry, rz, r2);
@@ -777,7 +807,7 @@ __device__ __forceinline__ void finalize_particle(const StepConsts& c, uint32_t 
 // the stencil cell of the particle at offset l from anchor (ax, ay, az).  xa: the
 // x anchor of every slot's hash cell, so that a candidate's neighbour vector does
 // not need the row's cell bounds.
-template <uint32_t BS, class Body>
+template <bool RO, uint32_t BS, class Body>
 __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* __restrict__ src,
                                              const float* __restrict__ xa,
                                              const uint32_t* __restrict__ cstart, const RowMasks& rm,
@@ -788,7 +818,7 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
         float4 q;
         float a;
     };
-    auto fetch = [&](uint32_t k) { return Candidate{__ldg(&src[k]), __ldg(&xa[k])}; };
+    auto fetch = [&](uint32_t k) { return Candidate{load<RO>(&src[k]), load<RO>(&xa[k])}; };
     auto visit = [&](uint32_t k, const Candidate& f, float oy, float oz) {
         const float4& q = f.q;
         const float ox = __fadd_rn(__fsub_rn(ax, f.a), l.x);
@@ -830,8 +860,8 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
                     for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
                         uint32_t more = 0;
                         for (uint32_t k = c0; k < min(c0 + 32u, b3); ++k) {
-                            const float4 q = __ldg(&src[k]);
-                            const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
+                            const float4 q = load<RO>(&src[k]);
+                            const float ox = __fadd_rn(__fsub_rn(ax, load<RO>(&xa[k])), l.x);
                             const float r2 = dist2(__fsub_rn(ox, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
                             more |= r2 < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
                         }
@@ -904,7 +934,7 @@ __device__ __forceinline__ void delta_apply(const StepConsts& c, uint32_t s, con
 // iteration also scatters back, finalizes and writes foam.  drec (may be
 // NULL): receives the particle's unclamped correction, for the adjoint.
 // SN: the s_corr exponent when fixed at compile time (4), else 0.
-template <bool LAST, uint32_t SN, uint32_t BS, class C>
+template <bool LAST, uint32_t SN, bool RO, uint32_t BS, class C>
 __device__ __forceinline__ void delta_item(const StepConsts& c, const C& pc, uint32_t s,
                                            const float4* __restrict__ src, float4* __restrict__ dst,
                                            uint32_t* __restrict__ qpos, const float* __restrict__ xa,
@@ -927,7 +957,7 @@ __device__ __forceinline__ void delta_item(const StepConsts& c, const C& pc, uin
     auto body = [&](uint32_t, const float4& q, float rx, float ry, float rz, float r2) {
         delta_add<SN>(pc, l.w, q.w, rx, ry, rz, r2, dx, dy, dz);
     };
-    queued_pairs<BS>(c, src, xa, cstart, rm, s, l, ax, ay, az, cx, cy, cz, PairQueue<BS>(queue), body);
+    queued_pairs<RO, BS>(c, src, xa, cstart, rm, s, l, ax, ay, az, cx, cy, cz, PairQueue<BS>(queue), body);
     delta_apply<LAST>(c, s, l, ax, ay, az, pcx, pcy, pcz, dx, dy, dz, dst, qpos, sidx, sphere, pos, vel, prev,
                       ncount, foam, err, drec);
 }

@@ -46,7 +46,7 @@ k_lambda_first(StepConsts c, const float4* __restrict__ cur, const uint32_t* __r
     __shared__ uint2 queue[kQueue * kSB];
     const uint32_t s = blockIdx.x * kSB + threadIdx.x;
     if (s < c.n)
-        lambda_first_item<LAST, kSB>(c, c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm, queue);
+        lambda_first_item<LAST, true, kSB>(c, c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm, queue);
 }
 
 template <bool LAST>
@@ -56,7 +56,7 @@ k_lambda(StepConsts c, const float4* __restrict__ cur, const uint32_t* __restric
          const uint32_t* __restrict__ sidx, float* __restrict__ lambdas, RowMasks rm) {
     __shared__ uint2 queue[kQueue * kSB];
     const uint32_t s = blockIdx.x * kSB + threadIdx.x;
-    if (s < c.n) lambda_item<LAST, kSB>(c, c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm, queue);
+    if (s < c.n) lambda_item<LAST, true, kSB>(c, c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm, queue);
 }
 
 // SN = 4: the reference's s_corr exponent, fixed at compile time (the host
@@ -72,7 +72,7 @@ k_delta(StepConsts c, const float4* __restrict__ src, float4* __restrict__ dst, 
     __shared__ uint2 queue[kQueue * kSB];
     const uint32_t s = blockIdx.x * kSB + threadIdx.x;
     if (s < c.n)
-        delta_item<LAST, SN, kSB>(c, c, s, src, dst, qpos, xa, scell, cstart, sidx, sphere, pos, vel, prev, ncount,
+        delta_item<LAST, SN, true, kSB>(c, c, s, src, dst, qpos, xa, scell, cstart, sidx, sphere, pos, vel, prev, ncount,
                                   foam, err, rm, nullptr, queue);
 }
 
@@ -88,7 +88,7 @@ k_lambda_first_team(StepConsts c, const float4* __restrict__ cur, const uint32_t
     __shared__ TeamBuf bufs[kTB / G];
     const uint32_t s = (blockIdx.x * kTB + threadIdx.x) / G;
     if (s < c.n)
-        team_lambda_first<LAST, G>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm, bufs);
+        team_lambda_first<LAST, true, G>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, ncount, rm, bufs);
 }
 
 template <bool LAST, uint32_t G>
@@ -98,7 +98,7 @@ k_lambda_team(StepConsts c, const float4* __restrict__ cur, const uint32_t* __re
               const uint32_t* __restrict__ sidx, float* __restrict__ lambdas, RowMasks rm) {
     __shared__ TeamBuf bufs[kTB / G];
     const uint32_t s = (blockIdx.x * kTB + threadIdx.x) / G;
-    if (s < c.n) team_lambda<LAST, G>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm, bufs);
+    if (s < c.n) team_lambda<LAST, true, G>(c, s, cur, qpos, nxt, scell, cstart, sidx, lambdas, rm, bufs);
 }
 
 template <bool LAST, uint32_t SN, uint32_t G>
@@ -112,7 +112,7 @@ k_delta_team(StepConsts c, const float4* __restrict__ src, float4* __restrict__ 
     __shared__ TeamBuf bufs[kTB / G];
     const uint32_t s = (blockIdx.x * kTB + threadIdx.x) / G;
     if (s < c.n)
-        team_delta<LAST, SN, G>(c, s, src, dst, qpos, xa, scell, cstart, sidx, sphere, pos, vel, prev, ncount,
+        team_delta<LAST, SN, true, G>(c, s, src, dst, qpos, xa, scell, cstart, sidx, sphere, pos, vel, prev, ncount,
                                 foam, err, rm, nullptr, bufs);
 }
 

@@ -147,7 +147,7 @@ __device__ __forceinline__ void lambda_terms(const StepConsts& c, float rx, floa
 
 // The sums of a lambda pass for slot s (see sweep()).  Returns the number of
 // in-range candidates other than the particle; acc is complete on every lane.
-template <uint32_t G, bool ANCHORED>
+template <uint32_t G, bool ANCHORED, bool RO>
 __device__ __forceinline__ uint32_t team_sweep(const Team<G>& team, const StepConsts& c,
                                                const float4* __restrict__ src,
                                                const uint32_t* __restrict__ qsrc,
@@ -158,7 +158,7 @@ __device__ __forceinline__ uint32_t team_sweep(const Team<G>& team, const StepCo
     const int y0 = cy - 1, z0 = cz - 1;
     uint32_t hits = 0, over = 0;
     auto bits = [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) {
-        uint32_t mask = row_bits(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s);
+        uint32_t mask = row_bits<RO>(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s);
         mask &= 0xffffffffu >> (max(b0, c0) - c0);
         if (c0 == row_base(b0)) {
             masks.rows[size_t(row) * masks.stride + s] = mask;
@@ -168,7 +168,7 @@ __device__ __forceinline__ uint32_t team_sweep(const Team<G>& team, const StepCo
     };
     auto empty = [&](uint32_t row) { masks.rows[size_t(row) * masks.stride + s] = 0u; };
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* t) {
-        const float4 q = __ldg(&src[k]);
+        const float4 q = load<RO>(&src[k]);
         float ox = px, oy = py, oz = pz;
         if (ANCHORED) {
             ox = __fadd_rn(__fsub_rn(aix, q.w), px);
@@ -193,7 +193,7 @@ __device__ __forceinline__ uint32_t team_sweep(const Team<G>& team, const StepCo
     return __reduce_add_sync(team.mask, hits);
 }
 
-template <bool LAST, uint32_t G>
+template <bool LAST, bool RO, uint32_t G>
 __device__ __forceinline__ void team_lambda_first(const StepConsts& c, uint32_t s,
                                                   const float4* __restrict__ cur,
                                                   const uint32_t* __restrict__ qpos,
@@ -212,7 +212,7 @@ __device__ __forceinline__ void team_lambda_first(const StepConsts& c, uint32_t 
     uint32_t qi;
     const int nthr = prefilter(c, cx + c.g.lx, cy + c.g.ly, cz + c.g.lz, lx, ly, lz, qi);
     LambdaAcc acc;
-    const uint32_t cnt = team_sweep<G, false>(team, c, cur, qpos, cstart, cx, cy, cz, p.x, p.y, p.z, 0.0f, 0.0f,
+    const uint32_t cnt = team_sweep<G, false, RO>(team, c, cur, qpos, cstart, cx, cy, cz, p.x, p.y, p.z, 0.0f, 0.0f,
                                               0.0f, qi, nthr, s, rm, acc);
     if (team.lane != 0) return;
     const float lambda = acc.lambda(c);
@@ -223,7 +223,7 @@ __device__ __forceinline__ void team_lambda_first(const StepConsts& c, uint32_t 
     if (LAST) lambdas[j] = lambda;
 }
 
-template <bool LAST, uint32_t G>
+template <bool LAST, bool RO, uint32_t G>
 __device__ __forceinline__ void team_lambda(const StepConsts& c, uint32_t s, const float4* __restrict__ cur,
                                             const uint32_t* __restrict__ qpos, float4* __restrict__ nxt,
                                             const uint32_t* __restrict__ scell,
@@ -239,7 +239,7 @@ __device__ __forceinline__ void team_lambda(const StepConsts& c, uint32_t s, con
     uint32_t qi;
     const int nthr = prefilter(c, pcx + c.g.lx, pcy + c.g.ly, pcz + c.g.lz, l.x, l.y, l.z, qi);
     LambdaAcc acc;
-    team_sweep<G, true>(team, c, cur, qpos, cstart, cx, cy, cz, l.x, l.y, l.z, ax, ay, az, qi, nthr, s, rm, acc);
+    team_sweep<G, true, RO>(team, c, cur, qpos, cstart, cx, cy, cz, l.x, l.y, l.z, ax, ay, az, qi, nthr, s, rm, acc);
     if (team.lane != 0) return;
     const float lambda = acc.lambda(c);
     nxt[s] = make_float4(l.x, l.y, l.z, lambda);
@@ -248,6 +248,7 @@ __device__ __forceinline__ void team_lambda(const StepConsts& c, uint32_t s, con
 
 // Neighbour vectors and chunk masks of a pass that walks recorded row masks, for a
 // particle at offset l from anchor (ax, ay, az) (see queued_pairs()).
+template <bool RO>
 struct TeamWalk {
     const StepConsts& c;
     const float4* __restrict__ src;
@@ -259,7 +260,7 @@ struct TeamWalk {
     int y0, z0;
     __device__ __forceinline__ void offset(uint32_t k, const float4& q, uint32_t y, uint32_t z, float& rx,
                                            float& ry, float& rz) const {
-        const float ox = __fadd_rn(__fsub_rn(ax, __ldg(&xa[k])), l.x);
+        const float ox = __fadd_rn(__fsub_rn(ax, load<RO>(&xa[k])), l.x);
         const float oy = __fadd_rn(__fsub_rn(ay, anchor_y(c.g, y0 + int(y))), l.y);
         const float oz = __fadd_rn(__fsub_rn(az, anchor_z(c.g, z0 + int(z))), l.z);
         rx = __fsub_rn(ox, q.x);
@@ -271,14 +272,14 @@ struct TeamWalk {
         uint32_t more = 0;
         for (uint32_t k = c0; k < min(c0 + 32u, b3); ++k) {
             float rx, ry, rz;
-            offset(k, __ldg(&src[k]), row % 3u, row / 3u, rx, ry, rz);
+            offset(k, load<RO>(&src[k]), row % 3u, row / 3u, rx, ry, rz);
             more |= dist2(rx, ry, rz) < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
         }
         return more;
     }
 };
 
-template <bool LAST, uint32_t SN, uint32_t G>
+template <bool LAST, uint32_t SN, bool RO, uint32_t G>
 __device__ __forceinline__ void team_delta(const StepConsts& c, uint32_t s, const float4* __restrict__ src,
                                            float4* __restrict__ dst, uint32_t* __restrict__ qpos,
                                            const float* __restrict__ xa, const uint32_t* __restrict__ scell,
@@ -296,10 +297,10 @@ __device__ __forceinline__ void team_delta(const StepConsts& c, uint32_t s, cons
     const float ax = anchor_x(c.g, pcx), ay = anchor_y(c.g, pcy), az = anchor_z(c.g, pcz);
     int cx, cy, cz;
     cell_of(c.g, __fadd_rn(ax, l.x), __fadd_rn(ay, l.y), __fadd_rn(az, l.z), cx, cy, cz);
-    const TeamWalk walk{c, src, xa, rm, s, l, ax, ay, az, cy - 1, cz - 1};
+    const TeamWalk<RO> walk{c, src, xa, rm, s, l, ax, ay, az, cy - 1, cz - 1};
     auto bits = [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) { return walk.bits(row, c0, b0, b3); };
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* t) {
-        const float4 q = __ldg(&src[k]);
+        const float4 q = load<RO>(&src[k]);
         float rx, ry, rz;
         walk.offset(k, q, y, z, rx, ry, rz);
         const float r2 = dist2(rx, ry, rz);
