@@ -320,6 +320,8 @@ int mp_batch_set_mode(mp_batch* b, int serial);
 int mp_batch_set_graph_mode(mp_batch* b, int enable);
 /* Launch shape (block = 128/256/512, blocks_per_sm 0 = as many as fit). */
 int mp_batch_set_launch(mp_batch* b, uint32_t block, uint32_t blocks_per_sm);
+/* Threads per block and blocks of a step's launch (serial mode: of its largest
+ * scene's): no more than are resident at once, nor than the particles fill. */
 int mp_batch_get_launch(const mp_batch* b, uint32_t* block, uint32_t* blocks);
 /* Time `steps` steps for every launch shape from the same saved state
  * (restored afterwards), keep the fastest, and remember it for batches of

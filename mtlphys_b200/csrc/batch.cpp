@@ -305,6 +305,15 @@ struct mp_batch {
         return uint32_t(std::max<uint64_t>(1u, (n * lanes + block - 1) / block));
     }
 
+    // Blocks of a step's launch (serial mode: of its largest scene's).
+    uint32_t step_blocks() const {
+        uint32_t useful = 1;
+        if (!serial) useful = useful_blocks(N, N);
+        else
+            for (uint32_t s = 0; s < S; ++s) useful = std::max(useful, useful_blocks(counts[s], p0[s] + counts[s]));
+        return std::min(blocks(), useful);
+    }
+
     // What the scenes' constants have in common (kernels fix it, or take it as an argument).
     void note_consts() {
         a.scorr4 = 1;
@@ -658,7 +667,7 @@ int mp_batch_set_launch(mp_batch* b, uint32_t block, uint32_t blocks_per_sm) {
 int mp_batch_get_launch(const mp_batch* b, uint32_t* block, uint32_t* blocks) {
     if (!b || !block || !blocks) return fail(MP_ERR_INVALID_ARGUMENT, "NULL argument");
     *block = b->block;
-    *blocks = b->blocks();
+    *blocks = b->step_blocks();
     return MP_OK;
 }
 
@@ -694,7 +703,7 @@ int mp_batch_autotune(mp_batch* b, uint32_t steps, mp_batch_tuning* best) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     float best_ms = 1e30f;
-    uint32_t best_block = saved_block, best_bps = saved_bps;
+    uint32_t best_block = saved_block, best_bps = saved_bps, timed_bps = saved_bps;
     for (uint32_t block : {128u, 256u, 512u}) {
         const int occ = batch_max_blocks_per_sm(block);
         for (int bps = 1; rc == MP_OK && bps <= occ; ++bps) {
@@ -710,11 +719,16 @@ int mp_batch_autotune(mp_batch* b, uint32_t steps, mp_batch_tuning* best) {
             float ms = 0.0f;
             cudaEventElapsedTime(&ms, e0, e1);
             ms /= float(steps);
+            // a grid that the particles do not fill: more blocks per SM would launch
+            // the same one, and the count is no limit for other batches of this bucket
+            const bool all = b->step_blocks() < b->blocks();
             if (rc == MP_OK && ms < best_ms) {
                 best_ms = ms;
                 best_block = block;
-                best_bps = uint32_t(bps);
+                timed_bps = uint32_t(bps);
+                best_bps = all ? 0u : uint32_t(bps);
             }
+            if (all) break;
         }
     }
     cudaEventDestroy(e0);
@@ -735,7 +749,7 @@ int mp_batch_autotune(mp_batch* b, uint32_t steps, mp_batch_tuning* best) {
     }
     if (best) {
         best->block = best_block;
-        best->blocks_per_sm = best_bps;
+        best->blocks_per_sm = timed_bps;
         best->ms_per_step = best_ms;
     }
     MP_CUDA(cudaDeviceSynchronize());
