@@ -34,7 +34,7 @@
 namespace mpb {
 namespace {
 
-constexpr uint32_t kScanItems = 8;  // per thread and tile in phase 4
+constexpr uint32_t kScanItems = kBatchScanItems;
 
 // Grid-wide barrier.  Every block calls it the same number of times.  All blocks
 // count their arrivals on the word that they then poll: the first block adds bit 31
@@ -64,6 +64,7 @@ constexpr unsigned kBarPhase = 0x80000000u;
 
 struct BarrierState {
     unsigned phase;  // bit 31 of the phase word until the next barrier completes
+    unsigned blocks;  // that take part
     unsigned passed;  // barriers so far (counted by the first block, for bar_pass only)
     int last, ok;
 };
@@ -80,7 +81,7 @@ __device__ __forceinline__ bool arrive(const BatchArgs& a, uint32_t word, Barrie
     __threadfence();
     unsigned inc = 1u;
     if (blockIdx.x == 0u) {
-        inc = kBarPhase - (gridDim.x - 1u);
+        inc = kBarPhase - (state->blocks - 1u);
         if (a.bar_extra && state->passed++ >= a.bar_pass) inc -= a.bar_extra;
     }
     const unsigned old = atomicAdd(a.bar + word, inc);
@@ -213,8 +214,9 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     if (threadIdx.x == 0) {
         s_bar.phase = bar_word(a).x;
         s_bar.passed = 0;
+        s_bar.blocks = gridDim.x;
     }
-    const uint32_t gsize = gridDim.x * BS;
+    uint32_t nblocks = gridDim.x, gsize = nblocks * BS;
     const uint32_t pb = a.p_begin, pe = a.p_end;
     // loops over particles run in whole warps (warp-level operations inside)
     const uint32_t pe_round = pb + ((pe - pb + 31u) & ~31u);
@@ -288,6 +290,14 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         if (threadIdx.x == 0) *a.total_cells = running;
     };
     if (!grid_barrier(a, &s_bar, lay_out)) return;
+    if (a.particle_blocks < nblocks) {
+        // blocks launched for the scan of cells that there could have been leave
+        const uint32_t round = BS * kScanItems * kBatchScanRounds;
+        nblocks = min(nblocks, max(a.particle_blocks, *a.total_cells / round + 1u));
+        if (blockIdx.x >= nblocks) return;
+        gsize = nblocks * BS;
+        if (threadIdx.x == 0) s_bar.blocks = nblocks;
+    }
 
     // 3: cell id inside the scene's box + warp-aggregated count; the boxes are
     // empty again for the next step
@@ -319,7 +329,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     const uint32_t len = cells_ok ? ncells + 1u : 0u;
     const uint32_t tile = BS * kScanItems;
     const uint32_t tiles = (len + tile - 1) / tile;
-    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < tiles; t += nblocks) {
         uint32_t sum = 0;
         for (uint32_t k = 0; k < kScanItems; ++k) {
             const uint32_t idx = t * tile + k * BS + threadIdx.x;
@@ -343,7 +353,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
         }
     };
     if (!grid_barrier(a, &s_bar, scan_tiles)) return;
-    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < tiles; t += nblocks) {
         // each thread owns kScanItems consecutive items of the tile
         uint32_t v[kScanItems], sum = 0;
         const uint32_t first = t * tile + threadIdx.x * kScanItems;
@@ -376,7 +386,7 @@ __global__ void __launch_bounds__(BS, batch_min_blocks<BS>()) k_batch_step(Batch
     if (!grid_barrier(a, &s_bar)) return;
     const uint32_t nl = cells_ok ? *static_cast<volatile uint32_t*>(a.long_count) : 0u;
     if (nl) {  // the same for every block: long_count is written before the barrier only
-        for (uint32_t li = blockIdx.x; li < nl; li += gridDim.x) {
+        for (uint32_t li = blockIdx.x; li < nl; li += nblocks) {
             const uint32_t cell = a.long_list[li];
             const SceneDev& sd = sc[a.scene_of[a.tmp[a.cstart[cell]]]];
             long_segment(sd.c, cell, sd.p0, sd.p0 + sd.c.n, a.hash, a.cstart, a.pos, a.sidx, a.sorted_a,

@@ -48,11 +48,15 @@ struct BatchRecord {
 constexpr uint32_t kBarLine = 32, kBarRoot = 0, kBarGen = kBarLine;
 constexpr uint32_t kBarWords = 2 * kBarLine;
 
+constexpr uint32_t kBatchScanItems = 8;   // cells per thread and tile of the step's scan
+constexpr uint32_t kBatchScanRounds = 4;  // tiles that a block scans before more blocks are worth their barriers
+
 struct BatchArgs {
     SceneDev* scenes;
     uint32_t scene_begin, scene_end;  // scenes of this launch
     const uint32_t* scene_of;         // scene of every particle / slot
     uint32_t p_begin, p_end;          // particles (= slots) of this launch
+    uint32_t particle_blocks;         // blocks that these fill; more are there for the scan, if the boxes are large
     uint32_t iterations;
     float4 *pos, *vel, *prev, *sorted_a, *sorted_b;
     uint32_t *hash, *off, *tmp, *sidx, *scell, *ncount, *qpos;
