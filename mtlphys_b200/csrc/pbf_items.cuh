@@ -385,6 +385,11 @@ struct RowOffsets {
     }
 };
 
+// Whether p holds on any lane that is here too.  Lanes that walk full queues do so
+// together: each on its own, while the others of its warp wait, 50,000 particles in a
+// cloud with clumps of thousands took 31.4 ms per step; together, 12.7.
+__device__ __forceinline__ bool warp_any(bool p) { return __any_sync(__activemask(), p); }
+
 // Per-thread queue of row chunks with candidates to visit, in shared memory:
 // entry e of thread t at (e * BS + t), 8 bytes: the chunk's bits (first
 // candidate in bit 31), and 4 times its first slot (a multiple of 4, below 2^30) with
@@ -583,12 +588,12 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
             *out = mask;
             const uint32_t code = uint32_t(y) | (uint32_t(z) << 2);
             queue.push(mask, a0, code);
-            if (b3 > a0 + 32u) {  // (never an empty row)
+            if (__builtin_expect(b3 > a0 + 32u, 0)) {  // (never an empty row)
                 const uint32_t row = uint32_t(3 * z + y);
                 over |= 1u << row;
                 for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
                     // room for this chunk and the first ones of the rows to come
-                    if (queue.short_of(9u - row)) queue.template drain<false>(o, fetch, visit);
+                    if (warp_any(queue.short_of(9u - row))) queue.template drain<false>(o, fetch, visit);
                     queue.push(row_bits<RO>(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s), c0, code);
                 }
             }
@@ -668,7 +673,7 @@ __device__ __forceinline__ void count_neighbors_item(const StepConsts& c, uint32
                 in = (in << left) & row;
                 maybe = (maybe << left) & row & ~in;
                 cnt += __popc(in);
-                if (queue.short_of(1u)) queue.template drain<false>(none, fetch, visit);
+                if (warp_any(queue.short_of(1u))) queue.template drain<false>(none, fetch, visit);
                 queue.push(maybe, c0, 0u);
             }
         }
@@ -865,7 +870,7 @@ __device__ __forceinline__ void queued_pairs(const StepConsts& c, const float4* 
                             const float r2 = dist2(__fsub_rn(ox, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
                             more |= r2 < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
                         }
-                        if (queue.short_of(9u - row)) queue.template drain<false>(o, fetch, visit);
+                        if (warp_any(queue.short_of(9u - row))) queue.template drain<false>(o, fetch, visit);
                         queue.push(more, c0, code);
                     }
                 }
