@@ -565,6 +565,23 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
     const StencilRows rows(c.g, cx, cy, cz);
     uint32_t over = 0, base = rows.base, b0 = 0, b3 = 0;
     uint32_t* out = masks.rows + s;
+    // bits of slots [c0, c1), c0 a multiple of 4, at most 32 of them, in row (y, z)
+    auto bits = [&](uint32_t c0, uint32_t c1, int y, int z) {
+        if (nthr != -kPassAll) return row_bits<RO>(qsrc, qi, nthr, c0, c1, s);
+        // nothing the prefilter could tell apart: the exact test decides, or the
+        // queue would carry every candidate (100,000 particles 300 m outside the box
+        // 5.6 ms per step, this way 1.8)
+        const float oy = y == 0 ? o.y0 : (y == 1 ? o.y1 : o.y2), oz = z == 0 ? o.z0 : (z == 1 ? o.z1 : o.z2);
+        uint32_t mask = 0;
+#pragma unroll 1
+        for (uint32_t k = c0; k < c1; ++k) {
+            const float4 q = fetch(k);
+            const float ox = ANCHORED ? __fadd_rn(__fsub_rn(aix, q.w), px) : px;
+            const float r2 = dist2(__fsub_rn(ox, q.x), __fsub_rn(oy, q.y), __fsub_rn(oz, q.z));
+            mask |= r2 < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
+        }
+        return mask;
+    };
     if (rows.valid(cy - 1, cz - 1)) {
         b0 = cstart[base];
         b3 = cstart[base + rows.nx];
@@ -583,7 +600,7 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
             }
             uint32_t mask = 0;
             const uint32_t a0 = row_base(b0);
-            if (b0 < b3) mask = row_bits<RO>(qsrc, qi, nthr, a0, min(a0 + 32u, b3), s) & (0xffffffffu >> (b0 - a0));
+            if (b0 < b3) mask = bits(a0, min(a0 + 32u, b3), y, z) & (0xffffffffu >> (b0 - a0));
             // the bits of the row's first chunk (the whole row if b3 - a0 <= 32)
             *out = mask;
             const uint32_t code = uint32_t(y) | (uint32_t(z) << 2);
@@ -594,7 +611,7 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
                 for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
                     // room for this chunk and the first ones of the rows to come
                     if (warp_any(queue.short_of(9u - row))) queue.template drain<false>(o, fetch, visit);
-                    queue.push(row_bits<RO>(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s), c0, code);
+                    queue.push(bits(c0, min(c0 + 32u, b3), y, z), c0, code);
                 }
             }
             b0 = n0;

@@ -157,8 +157,31 @@ __device__ __forceinline__ uint32_t team_sweep(const Team<G>& team, const StepCo
                                                LambdaAcc& acc) {
     const int y0 = cy - 1, z0 = cz - 1;
     uint32_t hits = 0, over = 0;
+    auto offset = [&](const float4& q, uint32_t y, uint32_t z, float& rx, float& ry, float& rz) {
+        float ox = px, oy = py, oz = pz;
+        if (ANCHORED) {
+            ox = __fadd_rn(__fsub_rn(aix, q.w), px);
+            oy = __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y0 + int(y))), py);
+            oz = __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z0 + int(z))), pz);
+        }
+        rx = __fsub_rn(ox, q.x);
+        ry = __fsub_rn(oy, q.y);
+        rz = __fsub_rn(oz, q.z);
+        return dist2(rx, ry, rz);
+    };
     auto bits = [&](uint32_t row, uint32_t c0, uint32_t b0, uint32_t b3) {
-        uint32_t mask = row_bits<RO>(qsrc, qi, nthr, c0, min(c0 + 32u, b3), s);
+        const uint32_t c1 = min(c0 + 32u, b3);
+        uint32_t mask = 0;
+        if (nthr != -kPassAll) {
+            mask = row_bits<RO>(qsrc, qi, nthr, c0, c1, s);
+        } else {  // as sweep() does
+#pragma unroll 1
+            for (uint32_t k = c0; k < c1; ++k) {
+                float rx, ry, rz;
+                const float r2 = offset(load<RO>(&src[k]), row % 3u, row / 3u, rx, ry, rz);
+                mask |= r2 < c.h2 && k != s ? 0x80000000u >> (k - c0) : 0u;
+            }
+        }
         mask &= 0xffffffffu >> (max(b0, c0) - c0);
         if (c0 == row_base(b0)) {
             masks.rows[size_t(row) * masks.stride + s] = mask;
@@ -168,15 +191,8 @@ __device__ __forceinline__ uint32_t team_sweep(const Team<G>& team, const StepCo
     };
     auto empty = [&](uint32_t row) { masks.rows[size_t(row) * masks.stride + s] = 0u; };
     auto terms = [&](uint32_t k, uint32_t y, uint32_t z, float2* t) {
-        const float4 q = load<RO>(&src[k]);
-        float ox = px, oy = py, oz = pz;
-        if (ANCHORED) {
-            ox = __fadd_rn(__fsub_rn(aix, q.w), px);
-            oy = __fadd_rn(__fsub_rn(aiy, anchor_y(c.g, y0 + int(y))), py);
-            oz = __fadd_rn(__fsub_rn(aiz, anchor_z(c.g, z0 + int(z))), pz);
-        }
-        const float rx = __fsub_rn(ox, q.x), ry = __fsub_rn(oy, q.y), rz = __fsub_rn(oz, q.z);
-        const float r2 = dist2(rx, ry, rz);
+        float rx, ry, rz;
+        const float r2 = offset(load<RO>(&src[k]), y, z, rx, ry, rz);
         hits += r2 < c.h2 ? 1u : 0u;
         lambda_terms(c, rx, ry, rz, r2, t);
     };

@@ -64,3 +64,45 @@ def test_a_warp_walks_full_queues_together(cuda):
     crowded = best_ms(cloud_params(), *random_scene(3, 50000))
     teams = best_ms(cloud_params(), *random_scene(3, 16000))
     assert crowded < 22.0 * teams, (crowded, teams)
+
+
+def test_far_particles_test_candidates_exactly_at_once(cuda):
+    """100,000 particles 300 m outside the box, where the prefilter cannot place them
+    and the border cells hold 184 candidates a row: 12 times an ordinary state; 37 when
+    all of them went through the queue."""
+    p = configs.base_params(3)
+    far, near = best_ms(p, *cube(100000, 300.0)), best_ms(p, *cube(100000))
+    assert far < 22.0 * near, (far, near)
+
+
+def test_far_particles_get_the_same_bits_from_teams_and_one_lane(cuda):
+    counts = [33, 4001, 16384]
+    p = configs.base_params(3)
+    p.set(bounds_max=(3.0, 3.0, 3.0))
+    states = [cube(n, off) for n, off in zip(counts, (300.0, 41.0, -2000.0))]
+    states[1][0][::7, 0] -= 41.0  # far and near ones in one warp
+    which = (_abi.MP_BUF_POSITIONS, _abi.MP_BUF_VELOCITIES, _abi.MP_BUF_LAMBDAS, _abi.MP_BUF_NEIGHBOR_COUNTS)
+    b = Batch(0)
+    try:
+        b.reset(counts, p, [DT] * len(counts))
+        b.write(_abi.MP_BUF_POSITIONS, np.concatenate([x for x, _ in states]))
+        b.write(_abi.MP_BUF_VELOCITIES, np.concatenate([v for _, v in states]))
+        b.step()
+        assert b.check_errors() == 0
+        together = [b.read(w) for w in which]
+        ranges = [b.scene_range(s) for s in range(len(counts))]
+    finally:
+        b.close()
+    for (first, n), (pos, vel) in zip(ranges, states):
+        e = Engine(0)
+        try:
+            e.set_params(p)
+            e.reset(n, _abi.MP_SCENE_CUBE_DROP)
+            e.set_positions(pos)
+            e.set_velocities(vel)
+            e.step(DT)
+            assert e.check_errors() == 0
+            for w, every in zip(which, together):
+                np.testing.assert_array_equal(e.read(w), every[first:first + n], err_msg=f"{n} particles, buffer {w}")
+        finally:
+            e.close()
