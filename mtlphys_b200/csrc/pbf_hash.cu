@@ -258,7 +258,7 @@ k_sort_gather(StepConsts c, const uint32_t* __restrict__ tmp, const uint32_t* __
 constexpr uint32_t kCB = 128;
 
 __global__ void __launch_bounds__(kCB)
-k_count_neighbors(StepConsts c, const float4* __restrict__ sorted, const uint32_t* __restrict__ qpos,
+k_count_neighbors(const __grid_constant__ StepConsts c, const float4* __restrict__ sorted, const uint32_t* __restrict__ qpos,
                   const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ sidx,
                   uint32_t* __restrict__ ncount, const uint32_t* __restrict__ strays) {
     __shared__ uint2 queue[kQueue * kCB];

@@ -106,3 +106,41 @@ def test_far_particles_get_the_same_bits_from_teams_and_one_lane(cuda):
                 np.testing.assert_array_equal(e.read(w), every[first:first + n], err_msg=f"{n} particles, buffer {w}")
         finally:
             e.close()
+
+
+def test_counts_of_crowded_cells_with_strays_go_straight_through(cuda):
+    """buildSpatialHash of a crowded cloud with a tenth of its particles outside the
+    box, where no inner threshold holds, against the same inside: 1.6 times as long;
+    5 times when every candidate went through the queue."""
+    pos, vel = random_scene(3, 50000)
+    inside = pos.copy()
+    inside[:, :3] = np.clip(inside[:, :3], [-2.9, -2.9, -2.9], [2.9, 5.9, 2.9])
+    strays = best_ms(cloud_params(), pos, vel, hash_only=True)
+    none = best_ms(cloud_params(), inside, vel, hash_only=True)
+    assert strays < 3.0 * none, (strays, none)
+
+
+@pytest.mark.parametrize("n, clump, offset", [(6001, 4000, 0.0), (6001, 300, 0.0), (5000, 0, 300.0), (70, 40, 0.0)])
+def test_counts_without_the_inner_threshold_match_the_oracle(cuda, n, clump, offset):
+    """Rows of few, dozens and hundreds of candidates, most of them in range or none."""
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(6)
+    pos = np.ones((n, 4), np.float32)
+    pos[:, :3] = rng.uniform(0.0, 1.0, (n, 3))
+    pos[:clump, :3] = 0.5 + rng.normal(0, 0.02, (clump, 3))
+    pos[:, 0] += np.float32(offset)
+    pos[-20:, :3] = rng.uniform(-0.8, 1.8, (20, 3))
+    p = _abi.default_params()
+    p.set(cell_size=0.1, bounds_min=(0.0,) * 3, bounds_max=(1.0,) * 3)
+    e = Engine(0)
+    try:
+        e.set_params(p)
+        e.reset(n, _abi.MP_SCENE_CUBE_DROP)
+        e.set_positions(pos)
+        e.build_spatial_hash()
+        got = e.neighbor_counts()
+        assert e.check_errors() == 0
+    finally:
+        e.close()
+    assert_equal_u32(got, O.build_spatial_hash(p, pos)[3], "neighbor counts")
