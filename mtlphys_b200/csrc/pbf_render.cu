@@ -289,11 +289,15 @@ __device__ __forceinline__ Edge box_edge(const RenderConsts& c, int e) {
     return g;
 }
 
-// The pixel across the major axis and the NDC z at pixel m along it.
+// The pixel across the major axis and the NDC z at pixel m along it.  Explicit
+// roundings: two threads that meet at a pixel must agree on which edges pass it, or
+// both blend it (or neither).
 __device__ __forceinline__ int edge_at(const Edge& g, int m, float& z) {
-    const float t = (g.a1 != g.a0) ? ((float(m) + 0.5f) - g.a0) / (g.a1 - g.a0) : 0.0f;
-    z = g.z0 + t * (g.z1 - g.z0);
-    return int(floorf(g.b0 + t * (g.b1 - g.b0)));
+    const float t = (g.a1 != g.a0)
+                        ? __fdiv_rn(__fsub_rn(__fadd_rn(float(m), 0.5f), g.a0), __fsub_rn(g.a1, g.a0))
+                        : 0.0f;
+    z = __fmaf_rn(t, __fsub_rn(g.z1, g.z0), g.z0);
+    return int(floorf(__fmaf_rn(t, __fsub_rn(g.b1, g.b0), g.b0)));
 }
 
 __global__ void __launch_bounds__(128) k_wire_box(RenderConsts c, const float* __restrict__ ndc,
