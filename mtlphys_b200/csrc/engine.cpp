@@ -333,7 +333,7 @@ size_t elem_bytes(uint32_t which) {
 //     the byte below shift a byte's difference by less than 1 step on x and 1.5
 //     on y and z, together sqrt(1 + 1.5^2 + 1.5^2) < 2.3453 steps, plus
 //     `fuzz` per axis for FP32 rounding of coordinates and offsets.  q_thr is
-//     the square of h / u plus that (plus 1: byte 3 can hold a borrow).
+//     above the square of h / u plus that (plus 1: byte 3 can hold a borrow).
 //   - Bytes hold differences up to 127 steps: units <= (127 - slack) / (h / cs).
 //     Candidates up to 2 cells away must not wrap to within range:
 //     256 - 2 units >= h / u + slack.  (A wrapped candidate only costs an exact

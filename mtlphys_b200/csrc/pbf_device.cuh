@@ -56,8 +56,8 @@ struct StepConsts {
     // byte-quantized distance prefilter of the lambda passes (set_prefilter):
     int q_units;   // quantization steps per cell
     float q_inv;   // q_units / cellSize
-    int q_thr;     // largest quantized squared distance an in-range pair can have
-    int q_in;      // quantized squared distances up to this are in range (nothing wrapped)
+    int q_thr;     // quantized squared distances from this on are out of range
+    int q_in;      // quantized squared distances below this are in range (nothing wrapped)
     float q_slack; // how far outside its cell a particle may be for q_in to hold
     float q_lim;   // particles further than this from their cell's corner skip the prefilter
 };
