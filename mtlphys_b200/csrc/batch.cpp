@@ -202,7 +202,7 @@ struct mp_batch {
         for (const mp_pbf_params& p : params) {
             GridDev g0;
             make_grid(p, g0);
-            if (g0.dgx > 2045 || g0.dgy > 2045 || g0.dgz > 1021) adj.wide = 1;
+            if (wide_grid(g0.dgx, g0.dgy, g0.dgz)) adj.wide = 1;
         }
         return MP_OK;
     }

@@ -41,30 +41,6 @@ constexpr uint32_t kBlock = 256;
 
 inline uint32_t cdiv(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
-// Dense cell coordinates packed 11 / 11 / 10 bits (x, y, z); the host checks
-// that the dense grid fits.
-__device__ __forceinline__ uint32_t pack_cell(int x, int y, int z) {
-    return uint32_t(x) | (uint32_t(y) << 11) | (uint32_t(z) << 22);
-}
-
-// Whether two packed cells are within one cell of each other on every axis.
-// With each field's difference plus one in a field of its own, that is every
-// field 0, 1 or 2: no bit above a field's low two, also after adding one more.
-// The fields of the subtraction cannot borrow their way into that unless two
-// cells are 2046 (x, y) or 1023 (z) apart; `wide` grids, which reach that far,
-// compare axis by axis.
-__device__ __forceinline__ bool cells_adjacent(uint32_t a, uint32_t b, bool wide) {
-    if (!wide) {
-        constexpr uint32_t one = 1u | (1u << 11) | (1u << 22), low2 = 3u * one;
-        const uint32_t d = a - (b - one);
-        return ((d | (d + one)) & ~low2) == 0u;
-    }
-    const int dx = int(a & 0x7ffu) - int(b & 0x7ffu);
-    const int dy = int((a >> 11) & 0x7ffu) - int((b >> 11) & 0x7ffu);
-    const int dz = int(a >> 22) - int(b >> 22);
-    return abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1;
-}
-
 // x^n; N = 4 is s_corr's exponent fixed at compile time (n - 1 = 3), with the
 // roundings of the loop.
 template <uint32_t N>

@@ -32,6 +32,39 @@ struct AdjStep {
     const uint32_t* overflow;     // iterations x mask_stride: bit r set for a long row r
 };
 
+#ifdef __CUDACC__
+#define MPB_BOTH __host__ __device__ __forceinline__
+#else
+#define MPB_BOTH inline
+#endif
+
+// Dense cell coordinates packed 11 / 11 / 10 bits (x, y, z); the host checks
+// that the dense grid fits.
+MPB_BOTH uint32_t pack_cell(int x, int y, int z) {
+    return uint32_t(x) | (uint32_t(y) << 11) | (uint32_t(z) << 22);
+}
+
+// Whether two packed cells are within one cell of each other on every axis.
+// With each field's difference plus one in a field of its own, that is every
+// field 0, 1 or 2: no bit above a field's low two, also after adding one more.
+// The fields of the subtraction cannot borrow their way into that unless two
+// cells are 2046 (x, y) or 1023 (z) apart; `wide` grids, which reach that far,
+// compare axis by axis.
+MPB_BOTH bool cells_adjacent(uint32_t a, uint32_t b, bool wide) {
+    if (!wide) {
+        constexpr uint32_t one = 1u | (1u << 11) | (1u << 22), low2 = 3u * one;
+        const uint32_t d = a - (b - one);
+        return ((d | (d + one)) & ~low2) == 0u;
+    }
+    const int dx = int(a & 0x7ffu) - int(b & 0x7ffu);
+    const int dy = int((a >> 11) & 0x7ffu) - int((b >> 11) & 0x7ffu);
+    const int dz = int(a >> 22) - int(b >> 22);
+    return dx * dx <= 1 && dy * dy <= 1 && dz * dz <= 1;
+}
+
+// Whether a grid of these dense dims is wide in that sense.
+inline bool wide_grid(int dx, int dy, int dz) { return dx > 2045 || dy > 2045 || dz > 1021; }
+
 // Pair terms that a particle's sweep owes another particle whose own sweep
 // does not see the pair (one-way pairs) are posted to the receiver's inbox:
 // kInbox slots per receiver, then a shared pool of overflow entries linked
