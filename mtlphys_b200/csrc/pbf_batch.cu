@@ -521,9 +521,10 @@ cudaError_t launch_bs(const BatchArgs& args, uint32_t blocks, cudaStream_t s) {
 template <uint32_t BS>
 int occupancy_bs() {
     int least = 1 << 30;
-    for (int i = 0; i < 16; ++i) {
-        const bool team = i & 1;
-        const void* fn = batch_kernel<BS>(i & 2, i & 4, team, i & 8);
+    for (int i = 0; i < 6; ++i) {
+        // two instances each: teams, shared constants, neither
+        const bool team = i < 2, common = i / 2 == 1, odd = i & 1;
+        const void* fn = batch_kernel<BS>(common || odd, common, team, common && odd);
         int n = 0;
         if (allow_shared(fn, shared_bytes<BS>(team)) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, BS, shared_bytes<BS>(team)) != cudaSuccess)
