@@ -308,7 +308,8 @@ int mp_batch_create(int device, mp_batch** out);
 int mp_batch_destroy(mp_batch* b);
 /* nscenes scenes: counts[s] particles, scene_ids[s] (MP_SCENE_*, NULL = cube
  * drop), params[s], descs[s] (NULL = reference placement), dts[s] > 0.  All
- * scenes use the same solver_iterations. */
+ * scenes use the same solver_iterations, and have 2^30 particles together at
+ * most. */
 int mp_batch_reset(mp_batch* b, uint32_t nscenes, const uint32_t* counts, const uint32_t* scene_ids,
                    const mp_pbf_params* params, const mp_scene_desc* descs, const float* dts);
 int mp_batch_set_dts(mp_batch* b, const float* dts);

@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_pre(AdjArgs a, uint32_t it) {
 //                        + grad s_ij g_ij . (dbar_i - dbar_j)) / rho0
 //   kbar       += sum_j -(W_ij / W(dq))^n g_ij . dbar_i / rho0
 // (dbar_j and the j-side terms only for pairs in both lists; the j-side
-// terms of a one-way pair are added to j atomically), and the particle's
-// density sums for the lambda adjoint.
+// terms of a one-way pair are posted to j, and the next kernel over j adds
+// them), and the particle's density sums for the lambda adjoint.
 // Both pair sweeps walk their pairs through a PairQueue (pbf_items.cuh), one
 // loop per slot instead of one per stencil row (10 -> 26 of 32 threads active),
 // and keep the scene's constants in registers.  Bound by issue and load latency.
@@ -491,10 +491,6 @@ __global__ void __launch_bounds__(kBlock) k_adj_lbar(AdjArgs a, uint32_t it) {
     a.qc[s] = make_float2(Db * ir * ir, __uint_as_float(ccur));
 }
 
-// Pair sweep of densityLambda's adjoint:
-//   pbar_i += sum_j (rhobar_i + rhobar_j) grad W_ij
-//             + H_ij (Gbar_i - Gbar_j + 2 (Qbar_i + Qbar_j) g_ij)
-// (j-side terms of one-way pairs added to j atomically).
 // A pair's position term in the lambda sweep of slot m (1e-12 < r2 < h^2).
 __device__ __forceinline__ float3 lambda_term(const AdjArgs& a, const PairConsts& pc, const float4& lm, float qm,
                                               uint32_t pm, uint32_t m, uint32_t k, float rx, float ry, float rz,
@@ -514,6 +510,10 @@ __device__ __forceinline__ float3 lambda_term(const AdjArgs& a, const PairConsts
     return v;
 }
 
+// Pair sweep of densityLambda's adjoint:
+//   pbar_i += sum_j (rhobar_i + rhobar_j) grad W_ij
+//             + H_ij (Gbar_i - Gbar_j + 2 (Qbar_i + Qbar_j) g_ij)
+// (j-side terms of one-way pairs are posted to j, as in the delta sweep).
 template <bool COMMON>
 __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) k_adj_lambda(AdjArgs a, uint32_t it) {
     __shared__ uint2 queue[kQueue * kSweepBlock];
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_sphere_sum(AdjArgs a) {
 // dL/dk of every scene: block (chunk, scene) sums the chunk's per-slot
 // accumulators into spart and clears them; k_adj_k_sum, one warp per scene, adds
 // the chunks.  Both in a fixed order.  (One block per scene walked 80,000 slots
-// in 92 us; both kernels take 6.)
+// in 92 us; the two kernels take 8.)
 __global__ void __launch_bounds__(kBlock) k_adj_k_part(AdjArgs a) {
     __shared__ double sh[kBlock];
     const uint32_t chunk = blockIdx.x, sc = blockIdx.y;

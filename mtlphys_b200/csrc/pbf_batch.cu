@@ -18,7 +18,8 @@
 //   0  per scene: advance the sphere; in the same phase
 //   1  per particle: predict, dense cell -> scene bounding box (atomics,
 //      reduced per warp first)
-//   2  one block: per-scene sub-grid dims and cell offsets (exclusive scan)
+//   2  one block: per-scene sub-grid dims and cell offsets (exclusive scan); blocks
+//      that only a larger box would have needed leave
 //   3  per particle: cell id in the scene's box, warp-aggregated count; per
 //      scene: the bounding box emptied for the next step
 //   4  exclusive scan of the counts (tile sums, scan of the sums, tile scan)
@@ -26,8 +27,6 @@
 //   8+ K x (lambda, delta); the last delta finalizes.
 // The per-particle work is the single-scene engine's (pbf_items.cuh).  The
 // serial mode launches this same kernel once per scene.
-#include <cooperative_groups.h>
-
 #include "pbf_batch.h"
 #include "pbf_team.cuh"
 
@@ -39,7 +38,8 @@ constexpr uint32_t kScanItems = kBatchScanItems;
 // Grid-wide barrier.  Every block calls it the same number of times.  All blocks
 // count their arrivals on the word that they then poll: the first block adds bit 31
 // less the number of the others, those add 1, so the last one to arrive flips bit 31
-// and leaves the other bits zero, and nothing has to be reset or passed on.  With
+// and leaves the other bits zero, and nothing has to be reset or passed on (the
+// arithmetic of the grid barrier in the CUDA toolkit's cooperative groups).  With
 // `last`, the arrivals are counted elsewhere, and the block that completes them runs
 // last() before it flips the polled word, with everything the others wrote before
 // the barrier visible: work for one block costs no barrier of its own.
@@ -191,8 +191,9 @@ __device__ __forceinline__ const auto& pair_constants(const BatchArgs& a, const 
 // (team_lanes(); the same bits).
 // COMMON: every scene has the constants a.pair, which as an argument need no
 // registers; per scene they are loads and a register each, of which the solver
-// phases at 64 have none to spare (spill loads 388 -> 128 bytes with REC fixed
-// too; 256 cubes, 4.2 M particles: 4.44 -> 4.23 ms; 12 small ones 182 -> 168 us).
+// phases at 64 have none to spare (spill loads 368 -> 140 bytes with REC fixed
+// too, 164 recording; 256 cubes, 4.2 M particles: 4.44 -> 4.23 ms; 12 small ones
+// 182 -> 168 us).
 // REC: whether the step is recorded, fixed at compile time (0, 1) or read from
 // the arguments (2).
 template <uint32_t BS, uint32_t SN, uint32_t G, bool COMMON, int REC>

@@ -501,8 +501,8 @@ struct StencilRows {
 };
 
 // Phase 1 of a sweep: the prefilter's bits of slots [c0, c1), c0 a multiple of 4, at
-// most 32 of them (first one in bit 31), without slot s.  Reads up to 7 slots past
-// c1.
+// most 32 of them (first one in bit 31), without slot s.  Reads up to 3 slots past
+// c1 (whole groups of four).
 template <bool RO>
 __device__ __forceinline__ uint32_t row_bits(const uint32_t* __restrict__ qsrc, uint32_t qi, int nthr, uint32_t c0,
                                              uint32_t c1, uint32_t s) {

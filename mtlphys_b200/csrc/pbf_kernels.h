@@ -110,6 +110,11 @@ cudaError_t launch_solver(const StepConsts& c, const DevState& d, uint32_t itera
 // (10,648: the most that one wave of blocks holds), 97 / 97 (16,000), but 112 / 101
 // (19,683) and 156 / 104 (32,768), where one lane each fills the GPU well enough and
 // does a third of the work.  8 lanes: 65 (2,197), 78 (8,000), 113 us (16,000).
+// The same line serves a batch's launches (81 / 117 us at 2,197 particles, 102 / 127 at
+// 8,000, 134 / 135 at 12,000, 132 / 124 at 16,000, 160 / 124 at 20,000) and the adjoint
+// (four steps forward and backward 1.16 / 1.82 ms at 2,197, 1.35 / 1.83 at 8,000, 1.79 /
+// 1.90 at 16,000, 2.12 / 1.90 at 20,000).  Clumps of hundreds per cell favour teams far
+// beyond it: 1.2 / 5.4 ms for a batch of 16,000.
 constexpr uint32_t kTeam = 16;
 constexpr uint32_t kTeamMaxSlots = 1u << 28;
 inline uint32_t team_lanes(uint32_t n, uint32_t end) {

@@ -15,7 +15,8 @@
 //                surface normal's screen derivatives are differences within
 //                the pixel's 2x2 quad, as a fragment quad computes them.
 //   k_wire_box   wireBox* (:296-335): 12 edges, LessEqual against the fluid
-//                depth, alpha blend 0.85; one block, edges in order.
+//                depth, alpha blend 0.85; a thread per edge and pixel, shared
+//                pixels blended in edge order by one thread.
 //   k_sphere     sphereDraw* (:394-458): opaque, Less, writes depth.
 //   k_foam       foam* (:337-389): additive sprites, LessEqual, no depth write.
 //   k_saturate   the [0, 1] clamp of the unorm colour target after the sprites.
