@@ -90,7 +90,7 @@ struct mp_batch {
     size_t cap_slots() const { return round_up(std::max<uint32_t>(N, 1u), 256u); }
     static size_t al(size_t bytes) { return (bytes + 255) & ~size_t(255); }
 
-    int ensure_tape(uint32_t nslots) {
+    int ensure_tape(uint32_t nslots, cudaStream_t s) {
         if (slots.size() >= nslots) return MP_OK;
         dev_free(tape_block);
         tape_block = nullptr;
@@ -102,7 +102,7 @@ struct mp_batch {
         MP_ALLOC(tape_block, per * nslots, device);
         // a recorded step that gave up at a barrier leaves the rest of its record as it
         // was; the adjoint kernels follow its indices
-        MP_CUDA(cudaMemset(tape_block, 0, per * nslots));
+        MP_CUDA(cudaMemsetAsync(tape_block, 0, per * nslots, s));
         char* p = static_cast<char*>(tape_block);
         auto take = [&](size_t bytes) {
             char* r = p;
@@ -146,7 +146,7 @@ struct mp_batch {
         return MP_OK;
     }
 
-    int ensure_adjoint() {
+    int ensure_adjoint(cudaStream_t s) {
         if (adj_block) return MP_OK;
         const size_t cap = cap_slots(), v4 = al(cap * 16), u = al(cap * 4);
         const size_t gbytes = al(sizeof(double) * kGradStride * std::max<uint32_t>(S, 1u));
@@ -159,7 +159,7 @@ struct mp_batch {
         const size_t accs = al(cap * 8) + al(cap * 32) + al(32 * size_t(chunks) * std::max<uint32_t>(S, 1u));
         const size_t total = 8 * v4 + 7 * u + gbytes + inbox + ovf + accs;
         MP_ALLOC(adj_block, total, device);
-        MP_CUDA(cudaMemset(adj_block, 0, total));
+        MP_CUDA(cudaMemsetAsync(adj_block, 0, total, s));  // on the pass's stream: in order with its kernels
         char* p = static_cast<char*>(adj_block);
         auto v = [&]() { float4* r = reinterpret_cast<float4*>(p); p += v4; return r; };
         auto w = [&]() { char* r = p; p += u; return r; };
@@ -179,7 +179,7 @@ struct mp_batch {
         adj.xa = reinterpret_cast<float*>(w());
         adj.inbox_count = reinterpret_cast<uint32_t*>(w());
         adj.ovf_head = reinterpret_cast<uint32_t*>(w());
-        MP_CUDA(cudaMemset(adj.ovf_head, 0xff, 4 * cap));  // kNoPost
+        MP_CUDA(cudaMemsetAsync(adj.ovf_head, 0xff, 4 * cap, s));  // kNoPost
         adj.inbox_src = reinterpret_cast<uint32_t*>(take(kInbox * u));
         adj.inbox_val = reinterpret_cast<float4*>(take(kInbox * v4));
         adj.ovf_count = reinterpret_cast<uint32_t*>(take(256));
@@ -920,8 +920,8 @@ int mp_batch_rollout_backward(mp_batch* b, const float* dpos, const float* dvel,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint32_t steps = b->roll_steps, every = b->roll_every;
     const uint32_t nck = (steps + every - 1) / every;
-    int rc = b->ensure_tape(std::min(steps, every));
-    if (rc == MP_OK) rc = b->ensure_adjoint();
+    int rc = b->ensure_tape(std::min(steps, every), st);
+    if (rc == MP_OK) rc = b->ensure_adjoint(st);
     if (rc != MP_OK) return rc;
     const size_t v4 = size_t(b->N) * 16;
     AdjArgs& ad = b->adj;
@@ -1050,7 +1050,7 @@ int mp_batch_check_errors(mp_batch* b, uint32_t* bits) {
     uint32_t w = 0;
     if (b->a.err) {
         MP_CUDA(cudaMemcpy(&w, b->a.err, 4, cudaMemcpyDeviceToHost));
-        MP_CUDA(cudaMemset(b->a.err, 0, 4));
+        if (w) MP_CUDA(cudaMemset(b->a.err, 0, 4));
         if (w & kDevErrSpin) {
             // a barrier wait gave up: the launch left the barrier's counters
             // mid-count, the abort flag (one of its words) set, and perhaps what
@@ -1063,6 +1063,7 @@ int mp_batch_check_errors(mp_batch* b, uint32_t* bits) {
             for (SceneDev& sd : cur) empty_box(sd.bb);
             MP_CUDA(cudaMemcpy(b->scenes, cur.data(), sizeof(SceneDev) * b->S, cudaMemcpyHostToDevice));
         }
+        if (w) MP_CUDA(cudaDeviceSynchronize());  // before a step on any stream
     }
     if (bits) *bits = w;
     if (w & kDevErrSpin) return fail(MP_ERR_SPIN_LIMIT, "a bounded device wait gave up (bits 0x%x)", w);

@@ -1189,7 +1189,10 @@ int mp_engine_check_errors(mp_engine* e, uint32_t* bits) {
     MP_CUDA(cudaDeviceSynchronize());
     uint32_t w = 0;
     MP_CUDA(cudaMemcpy(&w, e->d.err, 4, cudaMemcpyDeviceToHost));
-    MP_CUDA(cudaMemset(e->d.err, 0, 4));
+    if (w) {
+        MP_CUDA(cudaMemset(e->d.err, 0, 4));
+        MP_CUDA(cudaDeviceSynchronize());  // before a step on any stream
+    }
     if (bits) *bits = w;
     if (w & mpb::kDevErrSpin) return fail(MP_ERR_SPIN_LIMIT, "a bounded device wait gave up (bits 0x%x)", w);
     if (w) return fail(MP_ERR_DEVICE, "device error word 0x%x", w);
