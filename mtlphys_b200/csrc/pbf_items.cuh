@@ -387,7 +387,7 @@ struct RowOffsets {
 
 // Whether p holds on any lane that is here too.  Lanes that walk full queues do so
 // together: each on its own, while the others of its warp wait, 50,000 particles in a
-// cloud with clumps of thousands took 31.4 ms per step; together, 12.7.
+// cloud with clumps of thousands took 31.4 ms per step; together, 13.5.
 __device__ __forceinline__ bool warp_any(bool p) { return __any_sync(__activemask(), p); }
 
 // Per-thread queue of row chunks with candidates to visit, in shared memory:
@@ -570,7 +570,7 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
         if (nthr != -kPassAll) return row_bits<RO>(qsrc, qi, nthr, c0, c1, s);
         // nothing the prefilter could tell apart: the exact test decides, or the
         // queue would carry every candidate (100,000 particles 300 m outside the box
-        // 5.6 ms per step, this way 1.8)
+        // 5.6 ms per step, this way 2.1)
         const float oy = y == 0 ? o.y0 : (y == 1 ? o.y1 : o.y2), oz = z == 0 ? o.z0 : (z == 1 ? o.z1 : o.z2);
         uint32_t mask = 0;
 #pragma unroll 1
@@ -609,8 +609,14 @@ __device__ __forceinline__ void sweep(const StepConsts& c, const float4* __restr
                 const uint32_t row = uint32_t(3 * z + y);
                 over |= 1u << row;
                 for (uint32_t c0 = a0 + 32u; c0 < b3; c0 += 32) {
-                    // room for this chunk and the first ones of the rows to come
-                    if (warp_any(queue.short_of(9u - row))) queue.template drain<false>(o, fetch, visit);
+                    // Room for this chunk and the first ones of the rows to come.  A vote
+                    // here costs the single-scene kernels 1-2% of ordinary states (the
+                    // batch kernel nothing), so there the lanes, which mostly walk one
+                    // row, meet at every eighth chunk of it, where those with room for
+                    // less than four more walk their queues.
+                    const bool meet = RO && ((c0 - a0) & 224u) == 32u;
+                    const bool full = queue.short_of(meet ? 13u - row : 9u - row);
+                    if (RO ? full : warp_any(full)) queue.template drain<false>(o, fetch, visit);
                     queue.push(bits(c0, min(c0 + 32u, b3), y, z), c0, code);
                 }
             }
