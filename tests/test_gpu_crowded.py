@@ -68,7 +68,7 @@ def test_a_warp_walks_full_queues_together(cuda):
 
 def test_far_particles_test_candidates_exactly_at_once(cuda):
     """100,000 particles 300 m outside the box, where the prefilter cannot place them
-    and the border cells hold 184 candidates a row: 12 times an ordinary state; 37 when
+    and the border cells hold 184 candidates a row: 14 times an ordinary state; 37 when
     all of them went through the queue."""
     p = configs.base_params(3)
     far, near = best_ms(p, *cube(100000, 300.0)), best_ms(p, *cube(100000))
